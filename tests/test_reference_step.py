@@ -1,0 +1,95 @@
+"""The fused training step of the reference architecture (csrc/reference_step.cu, small_optimizer_kernel)
+against the same engine running operator by operator on CUDA cores."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import relative
+from turbogpt_b200 import bridge
+from turbogpt_b200.bridge import Config, ConfigEx, Native
+
+pytestmark = pytest.mark.gpu
+
+# Tile edges: one padded sequence; sequences that straddle a warp's 16 rows; a last tile with fewer sequences;
+# a sequence longer than a warp and one that fills a tile; the shipped experiment; more tiles than SMs (two
+# rounds: gradients accumulate across tiles); the deepest model that fits.
+SHAPES = [(1, 2, 3), (2, 5, 7), (4, 4, 16), (3, 16, 9), (2, 33, 5), (2, 128, 3), (4, 4, 2880), (8, 8, 2001), (16, 7, 41)]
+NAMES = ["x", "normed1", "qkv", "attended", "middle", "normed2", "activated"]
+
+
+def engine_pair(depth, context, batch, scheduled):
+    rng = np.random.default_rng(depth * 1000 + context)
+    data = rng.integers(32, 127, 4096 + context, dtype=np.uint8)
+    engines = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.reference(Config(depth=depth, context=context, batch=batch), flags=flags)
+        engine = Native(ex)
+        engine.set_weights(bridge.initialize_weights(ex))
+        if scheduled:
+            engine.set_onecycle(100)
+        engine.set_data(data)
+        engines.append(engine)
+    return engines, bridge.parameter_layout(ex)
+
+
+@pytest.mark.parametrize("depth,context,batch", SHAPES)
+def test_step_matches_the_operator_path(depth, context, batch):
+    (fused, plain), layout = engine_pair(depth, context, batch, True)
+    with fused, plain:
+        before = fused.weights()
+        for engine in (fused, plain):
+            engine.train(1)
+        # Losses: the operator path rounds logits to BF16 (half an ulp is 2^-9 of the value; |logit| < 1 at these
+        # weights) in the target's logit and in the log-sum.
+        np.testing.assert_allclose(fused.training_losses(1), plain.training_losses(1), rtol=0, atol=2 * 2 ** -9)
+        for name in NAMES:
+            for layer in (0, depth - 1):
+                assert relative(fused.activation(layer, name), plain.activation(layer, name)) <= 5e-3, (layer, name)
+        assert relative(fused.activation(-1, "final_normed"), plain.activation(-1, "final_normed")) <= 5e-3
+        # After one step the momentum is a fixed multiple of the gradient: the reference's per-tensor bound.
+        (m, v, step), (pm, pv, _) = fused.optimizer_state(), plain.optimizer_state()
+        assert step == 1
+        for offset, rows, cols in layout:
+            part = slice(offset, offset + rows * max(cols, 1))
+            assert relative(m[part], pm[part]) <= 0.02, (offset, rows, cols)
+            if np.any(pv[part]):
+                assert relative(v[part], pv[part]) <= 0.04, (offset, rows, cols)
+        # The update itself: the operator path's optimizer on the gradient this step used (the first step's sign-like
+        # AdamW update and Muon's null directions amplify the gradients' own differences, so those are kept out), with the
+        # reference's bounds for AdamW and Muon (tests/verify.py).
+        plain.set_weights(before)
+        rates = bridge.StepRates()
+        bridge.load_library().tg_onecycle_point(C.byref(bridge.OneCycle(100)), 0, C.byref(rates))
+        plain.optimizer_test(m / np.float32(1 - rates.momentum))
+        expected, got = plain.weights(), fused.weights()
+        for offset, rows, cols in layout:
+            part = slice(offset, offset + rows * max(cols, 1))
+            if cols and rows != 256:
+                assert relative(got[part] - before[part], expected[part] - before[part]) <= 0.04, (offset, rows, cols)
+            else:
+                np.testing.assert_allclose(got[part], expected[part], atol=2e-6, rtol=2e-5)
+
+
+@pytest.mark.parametrize("depth,context,batch", [(4, 4, 16), (2, 5, 7), (8, 8, 2001)])
+def test_graph_direct_and_streamed_steps_are_the_same(depth, context, batch):
+    """Replayed graphs, direct launches and steps fed from host bytes leave bit-identical weights."""
+    rng = np.random.default_rng(1)
+    data = rng.integers(32, 127, 4096, dtype=np.uint8)
+    results = []
+    for flags, streamed in ((0, False), (bridge.FLAG_NO_GRAPH, False), (0, True)):
+        ex = ConfigEx.reference(Config(depth=depth, context=context, batch=batch), flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(bridge.initialize_weights(ex))
+            engine.set_data(data)
+            if streamed:
+                losses = np.stack([engine.train_batch(*engine.sample(step)) for step in range(30)])
+            else:
+                engine.train(19)
+                first = engine.training_losses(19)
+                engine.train(11)
+                losses = np.concatenate([first, engine.training_losses(11)])
+            results.append((losses, engine.weights(), engine.optimizer_state()[0]))
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            np.testing.assert_array_equal(a, b)

@@ -79,3 +79,13 @@ __device__ __forceinline__ float gelu_derivative(float x) {
 __device__ __forceinline__ float join_weight(bf16 high, uint16_t low) {
     return __uint_as_float((unsigned(__bfloat16_as_ushort(high)) << 16) | low);
 }
+
+// A warp's 16 x 8 product on the register-operand tensor cores, BF16 in, FP32 sums: lane (g = lane / 4, t = lane % 4) holds
+// d0, d1 = row g, columns 2t, 2t+1 and d2, d3 = row g + 8; a = {row g, k 2t..}, {row g + 8}, {row g, k 8 + 2t..}, {row g + 8};
+// b = {k 2t, 2t+1}, {k 8 + 2t..} of column g.
+__device__ __forceinline__ void mma_bf16(float &d0, float &d1, float &d2, float &d3, const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(d0), "+f"(d1), "+f"(d2), "+f"(d3)
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}

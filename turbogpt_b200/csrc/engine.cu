@@ -5,6 +5,7 @@
 // (sampling seed, schedule point, loss-history row) read from device-resident counters.
 #include "engine.h"
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <dlfcn.h>
 
@@ -54,6 +55,7 @@ void Nccl::check(int result, const char *what) const {
                                  (GetErrorString ? GetErrorString(result) : "NCCL error"));
 }
 
+constexpr int ReferenceGraphSteps = 8; // steps of the reference architecture (three kernels each) per captured graph
 constexpr int ExchangeSms = 4; // CTAs of the gradient all-reduce = SMs the backward GEMMs leave free for it
 
 // ------------------------------------------------------------------------------- setup -------
@@ -195,6 +197,8 @@ void Engine::initialize() {
         allocate(muon_b, square, false);
         allocate(muon_sumsq, size_t(depth) * MuonBlocks);
     }
+    if (tensor_cores && c.world == 1 && reference_step_supported(c))
+        prepare_reference_step();
     if (c.world > 1 && !(c.flags & TG_FLAG_NO_COMMUNICATOR)) {
         const Nccl &nccl = Nccl::get();
         Nccl::UniqueId id;
@@ -224,6 +228,28 @@ void Engine::initialize() {
             allocate(gradient_bf16, P, false);
     }
     CHECK_CUDA(cudaStreamSynchronize(stream));
+}
+
+void Engine::prepare_reference_step() {
+    const TgConfigEx &c = config;
+    reference_step = true;
+    reference_plan = reference_step_plan(c, sms);
+    allocate(reference_partial, size_t(reference_plan.blocks) * reference_plan.partial_stride, false);
+    allocate(reference_norm, reference_plan.gradient_blocks);
+    allocate(small_ticket, 1);
+    std::vector<float2> rope(c.base.context);
+    for (int p = 0; p < c.base.context; ++p)
+        rope[p] = make_float2(float(std::cos(double(p))), float(std::sin(double(p))));
+    std::vector<SmallMatrix> matrices;
+    for (const TensorInfo &t : layout.tensors)
+        if (t.kind == 2)
+            matrices.push_back({int(t.offset), t.rows, t.cols});
+    small_matrix_count = int(matrices.size());
+    allocate(reference_rope, rope.size(), false);
+    allocate(small_matrices, matrices.size(), false);
+    CHECK_CUDA(cudaMemcpyAsync(reference_rope, rope.data(), rope.size() * sizeof(float2), cudaMemcpyHostToDevice, stream));
+    CHECK_CUDA(cudaMemcpyAsync(small_matrices, matrices.data(), matrices.size() * sizeof(SmallMatrix), cudaMemcpyHostToDevice, stream));
+    CHECK_CUDA(cudaStreamSynchronize(stream)); // the host arrays are about to go out of scope
 }
 
 void Engine::release() {
@@ -650,7 +676,35 @@ void Engine::optimize() {
 }
 
 // ------------------------------------------------------------------------------- modes -------
-void Engine::one_step(RunMode mode) {
+// One optimizer step of the reference architecture.  `save`: leave the activations where read_activation finds them.
+void Engine::reference_train_step(bool sample, bool save) {
+    const TgConfig &b = config.base;
+    ReferenceActivations saved{};
+    if (save) {
+        for (int l = 0; l < b.depth; ++l) {
+            const LayerActivations &a = layers[l];
+            saved.layer[l] = {a.x, a.normed1, a.qkv, a.attended, a.middle, a.normed2, a.activated};
+        }
+        saved.final_x = final_x, saved.final_normed = final_normed;
+    }
+    ReferenceStepArgs step{sample ? data : nullptr, data_size, b.seed, x, y, counters, weight_high, weight_low, reference_rope,
+                           reference_partial, token_losses, loss_history, gradient, reference_norm, b.batch, b.context, b.depth,
+                           save ? &saved : nullptr};
+    run(FMisc, [&] { launch_reference_step(step, reference_plan, stream); });
+    ++launches; // step kernel + reduce kernel
+    SmallOptimizerArgs update{{gradient, momentum, variance, weight_high, weight_low, nullptr, adam_mode, reference_norm,
+                               reference_plan.gradient_blocks, schedule, counters, b.learning_rate, b.beta1, b.beta2, b.weight_decay,
+                               b.epsilon, b.clip, layout.count},
+                              b.muon_lr, b.momentum, b.ns_steps, small_matrices, small_matrix_count, counters, small_ticket};
+    run(FOptimizer, [&] { launch_small_optimizer(update, stream); });
+}
+
+// `last`: no other step follows in this call, so the activations it leaves can be read.
+void Engine::one_step(RunMode mode, bool last) {
+    if (mode == RunMode::Train && reference_step) {
+        reference_train_step(true, last);
+        return;
+    }
     if (mode == RunMode::Train) {
         SampleArgs s{data, data_size, config.base.seed, counters, -1, config.base.batch, config.base.context,
                      config.world, config.rank, x, y};
@@ -694,10 +748,14 @@ void Engine::train(int steps) {
     // A step reads everything that changes from device memory, so its kernel sequence is captured
     // once (after one eager step has sized every workspace) and replayed as a CUDA graph.
     const bool use_graph = !profile && !comm && !(config.flags & TG_FLAG_NO_GRAPH);
-    for (int i = 0; i < steps; ++i) {
-        if (!use_graph || !graph_warm) {
-            one_step(RunMode::Train);
+    // The last step of a call leaves its activations for read_activation: the reference architecture's step kernel, whose
+    // activations otherwise stay on chip, is launched in another form for it, outside the graph.
+    const int outside = reference_step ? 1 : 0, graph_steps = reference_step ? ReferenceGraphSteps : 1;
+    for (int i = 0; i < steps;) {
+        if (!use_graph || !graph_warm || steps - i - outside < graph_steps) {
+            one_step(RunMode::Train, i + 1 == steps);
             graph_warm = true;
+            ++i;
             continue;
         }
         if (step_graph && graph_generation != gemm_workspace.generation)
@@ -708,7 +766,8 @@ void Engine::train(int steps) {
             cudaGraph_t graph = nullptr;
             CHECK_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
             try {
-                one_step(RunMode::Train);
+                for (int k = 0; k < graph_steps; ++k)
+                    one_step(RunMode::Train, false);
             } catch (...) {
                 cudaStreamEndCapture(stream, &graph);
                 if (graph)
@@ -724,6 +783,7 @@ void Engine::train(int steps) {
         }
         CHECK_CUDA(cudaGraphLaunch(step_graph, stream));
         launches += graph_launches;
+        i += graph_steps;
     }
     last_train_steps = steps;
     losses_reduced = false;
@@ -931,12 +991,16 @@ void Engine::train_batch(const uint8_t *bx, const uint8_t *by, float *per_positi
     CHECK_CUDA(cudaMemcpyAsync(x, bx, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemcpyAsync(y, by, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemsetAsync(&counters->iteration, 0, sizeof(int), stream));
-    forward(true, false);
-    run(FMisc, [&] {
-        launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context, stream);
-    });
-    backward();
-    optimize();
+    if (reference_step) {
+        reference_train_step(false, true);
+    } else {
+        forward(true, false);
+        run(FMisc, [&] {
+            launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context, stream);
+        });
+        backward();
+        optimize();
+    }
     step += 1;
     last_train_steps = 1;
     losses_reduced = false;

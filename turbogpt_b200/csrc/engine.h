@@ -83,6 +83,14 @@ struct Engine {
     // Muon scratch
     bf16 *muon_x[2] = {nullptr, nullptr}, *muon_a = nullptr, *muon_b = nullptr;
     float *muon_sumsq = nullptr;
+    // the reference architecture's step in three kernels (reference_step.cu, small_optimizer_kernel); unset: operator by operator
+    bool reference_step = false;
+    ReferenceStepPlan reference_plan;
+    float *reference_partial = nullptr, *reference_norm = nullptr;
+    float2 *reference_rope = nullptr;
+    SmallMatrix *small_matrices = nullptr;
+    int small_matrix_count = 0;
+    unsigned *small_ticket = nullptr;
     // host mirrors
     uint64_t step = 0;
     int last_train_steps = 0;
@@ -146,6 +154,8 @@ struct Engine {
     void finish_exchange();
     void optimize();
     void muon_family(int64_t first_offset, int rows, int cols);
-    void one_step(RunMode mode);
+    void prepare_reference_step();
+    void reference_train_step(bool sample, bool save);
+    void one_step(RunMode mode, bool last = true);
     void check_device_error();
 };

@@ -203,6 +203,39 @@ void launch_weight_gradient_static(const void *dy, const void *x, float *dw, int
                                    cudaStream_t s);
 size_t gemm_tc_static_scratch_bytes();
 
+// ---- whole step of the reference architecture (reference_step.cu) ----
+constexpr int ReferenceMaxDepth = 16; // deeper models leave no room for a tile of tokens beside their weights
+struct ReferenceActivations { // where a step leaves its activations, [tokens][features] BF16
+    struct {
+        void *x, *normed1, *qkv, *attended, *middle, *normed2, *activated;
+    } layer[ReferenceMaxDepth];
+    void *final_x, *final_normed;
+};
+struct ReferenceStepPlan { // how a batch is cut into tiles, and the scratch that takes
+    int sequences = 0, rows = 0, tiles = 0; // per tile: whole sequences, their tokens in groups of 16
+    int blocks = 0, gradient_blocks = 0;    // of the step and reduce kernels
+    int64_t partial_stride = 0;             // floats per block of gradient sums
+};
+struct ReferenceStepArgs {
+    const uint8_t *data; // corpus to sample the batch from (as launch_sample does for world 1); nullptr: x and y hold it
+    int64_t data_size;
+    uint64_t seed;
+    const uint8_t *x, *y;
+    const StepCounters *counters;
+    const bf16 *weight_high;
+    const uint16_t *weight_low;
+    const float2 *rope;  // [context] cos, sin of the position in radians
+    float *partial;      // [blocks][partial_stride] scratch
+    float *token_losses, *history, *gradient;
+    float *norm_partial; // [gradient_blocks] sums of squares of the gradient, for clipping
+    int batch, context, depth;
+    const ReferenceActivations *save; // nullptr: activations stay inside the kernel
+};
+bool reference_step_supported(const TgConfigEx &c);
+ReferenceStepPlan reference_step_plan(const TgConfigEx &c, int sms);
+// Sampling, forward, loss, backward, gradient reduction and loss history: two kernels.
+void launch_reference_step(const ReferenceStepArgs &a, const ReferenceStepPlan &plan, cudaStream_t s);
+
 // ---- optimizer (reference cuda/optim.cuh) ----
 void launch_sum_squares(const float *gradient, int64_t count, float *partial, int blocks, cudaStream_t s);
 struct AdamArgs {
@@ -252,6 +285,22 @@ struct MuonApplyArgs {
 };
 void launch_muon_apply(const MuonApplyArgs &a, cudaStream_t s);
 void launch_advance(StepCounters *counters, cudaStream_t s);
+// AdamW, Muon and the advance of the step counters in one kernel, for models whose hidden matrices are at most 16 x 48
+// (or 48 x 16): one warp orthogonalises one matrix in registers.
+struct SmallMatrix {
+    int offset, rows, cols;
+};
+struct SmallOptimizerArgs {
+    AdamArgs adam;
+    float muon_lr, momentum_rate;
+    int ns_steps;
+    const SmallMatrix *matrices; // device
+    int matrix_count;
+    StepCounters *counters;      // advanced by the last block
+    unsigned *ticket;            // zero between launches
+};
+bool small_optimizer_supported(int rows, int cols);
+void launch_small_optimizer(const SmallOptimizerArgs &a, cudaStream_t s);
 
 // ---- self-test: a wait on a barrier nothing arms, with a short limit (selftest.cu) ----
 int launch_starved_wait(StepCounters *counters, double limit_ms, int code, cudaStream_t s);

@@ -4,6 +4,7 @@
 // stages sit either side of Newton-Schulz GEMMs issued by the host.
 #include "device_utils.cuh"
 #include "kernels.cuh"
+#include "sm100.cuh"
 
 // Fixed-order partial sums of squares: block b covers a contiguous slice.
 __global__ void __launch_bounds__(256) sum_squares_kernel(const float *gradient, int64_t count, float *partial) {
@@ -51,34 +52,46 @@ __device__ __forceinline__ float clip_factor(const float *norm_partial, int norm
     return fminf(1.f, clip / (sqrtf(norm) + 1e-6f));
 }
 
-__global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a) {
-    __shared__ float scratch[32];
-    const float clip = clip_factor(a.norm_partial, a.norm_blocks, a.clip, scratch);
-    const unsigned long long step = a.counters->step;
-    float multiplier = 1, beta1 = a.beta1;
-    if (a.schedule) { // every update reads its own schedule point (reference cuda/optim.cuh:82-89)
-        TgStepRates rates = a.schedule[step];
-        multiplier = rates.multiplier;
-        beta1 = rates.momentum;
+// What every AdamW thread needs of the step: its own schedule point (reference cuda/optim.cuh:82-89), and bias
+// correction with the current, possibly cycled, beta1 as torch.optim.AdamW does.
+struct AdamRates {
+    float clip = 1.f, lr, beta1, step_size, inv_sqrt_bc2;
+    __device__ __forceinline__ explicit AdamRates(const AdamArgs &a) {
+        const unsigned long long step = a.counters->step;
+        float multiplier = 1;
+        beta1 = a.beta1;
+        if (a.schedule) {
+            TgStepRates rates = a.schedule[step];
+            multiplier = rates.multiplier;
+            beta1 = rates.momentum;
+        }
+        lr = a.learning_rate * multiplier;
+        step_size = lr / (1 - powf(beta1, float(step + 1)));
+        inv_sqrt_bc2 = 1.f / sqrtf(1 - powf(a.beta2, float(step + 1)));
     }
-    const float lr = a.learning_rate * multiplier;
-    // Bias correction with the current, possibly cycled, beta1 as torch.optim.AdamW does.
-    const float bc1 = 1 - powf(beta1, float(step + 1)), bc2 = 1 - powf(a.beta2, float(step + 1));
-    const float step_size = lr / bc1, inv_sqrt_bc2 = 1.f / sqrtf(bc2);
-    const int64_t groups = a.count / 8;
-    for (int64_t group = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; group < groups;
-         group += int64_t(gridDim.x) * blockDim.x) {
-        const int mode = a.mode[group];
-        if (mode == 0)
-            continue;
+};
+// Eight consecutive parameters and their state, fetched before the rates are known.
+struct AdamGroup {
+    int mode = 0;
+    float g[8], m[8], v[8];
+    uint4 high, low;
+    __device__ __forceinline__ AdamGroup() {}
+    __device__ __forceinline__ AdamGroup(const AdamArgs &a, int64_t group) : mode(a.mode[group]) {
+        if (mode == 0) // Muon's
+            return;
         const int64_t i = group * 8;
-        const float decay = 1 - lr * (mode == 2 ? a.weight_decay : 0.f);
-        float g[8], m[8], v[8], w[8];
         load8(a.gradient + i, g);
         load8(a.momentum + i, m);
         load8(a.variance + i, v);
-        uint4 high = *reinterpret_cast<const uint4 *>(a.weight_high + i);
-        uint4 low = *reinterpret_cast<const uint4 *>(a.weight_low + i);
+        high = *reinterpret_cast<const uint4 *>(a.weight_high + i);
+        low = *reinterpret_cast<const uint4 *>(a.weight_low + i);
+    }
+    __device__ __forceinline__ void update(const AdamArgs &a, const AdamRates &rates, int64_t group) {
+        if (mode == 0)
+            return;
+        const int64_t i = group * 8;
+        const float decay = 1 - rates.lr * (mode == 2 ? a.weight_decay : 0.f);
+        float w[8];
         const unsigned hw[4] = {high.x, high.y, high.z, high.w}, lw[4] = {low.x, low.y, low.z, low.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -87,10 +100,10 @@ __global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a) {
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            float gj = g[j] * clip;
-            m[j] = m[j] + (1 - beta1) * (gj - m[j]);
+            float gj = g[j] * rates.clip;
+            m[j] = m[j] + (1 - rates.beta1) * (gj - m[j]);
             v[j] = a.beta2 * v[j] + (1 - a.beta2) * gj * gj;
-            w[j] = w[j] * decay - step_size * m[j] / (sqrtf(v[j]) * inv_sqrt_bc2 + a.epsilon);
+            w[j] = w[j] * decay - rates.step_size * m[j] / (sqrtf(v[j]) * rates.inv_sqrt_bc2 + a.epsilon);
         }
         store8(a.momentum + i, m);
         store8(a.variance + i, v);
@@ -106,6 +119,15 @@ __global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a) {
         if (a.weight_fp32)
             store8(a.weight_fp32 + i, w);
     }
+};
+__global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a) {
+    __shared__ float scratch[32];
+    AdamRates rates(a);
+    rates.clip = clip_factor(a.norm_partial, a.norm_blocks, a.clip, scratch);
+    const int64_t groups = a.count / 8;
+    for (int64_t group = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; group < groups;
+         group += int64_t(gridDim.x) * blockDim.x)
+        AdamGroup(a, group).update(a, rates, group);
 }
 void launch_adamw(const AdamArgs &a, int sms, cudaStream_t s) {
     int64_t groups = a.count / 8;
@@ -428,4 +450,172 @@ __global__ void advance_kernel(StepCounters *counters) {
 }
 void launch_advance(StepCounters *counters, cudaStream_t s) {
     advance_kernel<<<1, 1, 0, s>>>(counters);
+}
+
+// ------------------------------------------------------------------------------------------
+// Whole update of a model of 16-wide matrices.  As separate kernels it was 5 x (prepare, normalise, Newton-Schulz in
+// shared memory, apply), AdamW and the counter: 22 launches and 0.2 ms, all latency (now ~9 us).  One warp takes one matrix: X
+// (16 x n, n = 16 or 48, the wide orientation) lives in registers as m16n8k16 operand fragments, and an iteration is
+// n/8 + 2 + n/8 products per 16-deep step with the roundings of muon_newton_schulz_small_kernel:
+//   A = X X^T     X's fragments are both operands
+//   B = 2.0315 A A - 4.775 A,  X' = B X + 3.4445 X     the right operands are 8 x 8 blocks transposed in registers
+// ------------------------------------------------------------------------------------------
+constexpr int SmallWarps = 4; // matrices per block
+__device__ __forceinline__ uint32_t transposed_block(uint32_t block) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(block));
+    return r;
+}
+__device__ __forceinline__ float low_half(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float high_half(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+
+template <int Steps> struct SmallMuon { // Steps: columns of X / 16
+    SmallMatrix matrix;
+    int g, t;
+    float mu, multiplier;
+    float grad[Steps][4][2], momentum[Steps][4][2];
+    bf16 high[Steps][4][2];
+    uint16_t low[Steps][4][2];
+
+    // register i of step k, half j: row g + 8 (i % 2), column 16 k + 8 (i / 2) + 2 t + j of X
+    __device__ __forceinline__ int index(int k, int i, int j) const {
+        const int row = g + 8 * (i % 2), column = 16 * k + 8 * (i / 2) + 2 * t + j;
+        return matrix.offset + (matrix.rows > matrix.cols ? column * matrix.cols + row : row * matrix.cols + column);
+    }
+    template <class F> __device__ __forceinline__ void each(F &&f) const {
+#pragma unroll
+        for (int k = 0; k < Steps; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    f(k, i, j);
+    }
+    // Every load is issued before the clip norm is awaited and before the first store (they may alias as far as the
+    // compiler knows: interleaved, each of the 24 elements paid a round trip to L2).
+    __device__ __forceinline__ SmallMuon(const SmallOptimizerArgs &a, const SmallMatrix &matrix, int lane)
+        : matrix(matrix), g(lane / 4), t(lane % 4), mu(a.momentum_rate), multiplier(1.f) {
+        each([&](int k, int i, int j) {
+            const int at = index(k, i, j);
+            grad[k][i][j] = a.adam.gradient[at], momentum[k][i][j] = a.adam.momentum[at];
+            high[k][i][j] = a.adam.weight_high[at], low[k][i][j] = a.adam.weight_low[at];
+        });
+        if (a.adam.schedule) {
+            const TgStepRates rates = a.adam.schedule[a.adam.counters->step];
+            mu = rates.momentum, multiplier = rates.multiplier;
+        }
+    }
+    __device__ __forceinline__ void update(const SmallOptimizerArgs &a, float clip) {
+        uint32_t x[Steps][4];
+        float squares = 0;
+#pragma unroll
+        for (int k = 0; k < Steps; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float u[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float d = grad[k][i][j] * clip, m = momentum[k][i][j] + (1 - mu) * (d - momentum[k][i][j]);
+                    a.adam.momentum[index(k, i, j)] = m;
+                    u[j] = rounded<bf16>(d + mu * (m - d));
+                    squares += u[j] * u[j];
+                }
+                x[k][i] = pack_bf16(u[0], u[1]);
+            }
+        const float inverse = 1.f / fmaxf(rounded<bf16>(sqrtf(warp_sum(squares))), rounded<bf16>(1e-7f));
+#pragma unroll
+        for (int k = 0; k < Steps; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                x[k][i] = pack_bf16(low_half(x[k][i]) * inverse, high_half(x[k][i]) * inverse);
+        for (int step = 0; step < a.ns_steps; ++step) {
+            float acc[8] = {};
+#pragma unroll
+            for (int k = 0; k < Steps; ++k) {
+                mma_bf16(acc[0], acc[1], acc[2], acc[3], x[k], x[k][0], x[k][2]);
+                mma_bf16(acc[4], acc[5], acc[6], acc[7], x[k], x[k][1], x[k][3]);
+            }
+            uint32_t square[4], b[4]; // A, then B, as left operands
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                square[i] = pack_bf16(acc[2 * i], acc[2 * i + 1]), acc[2 * i] = acc[2 * i + 1] = 0.f;
+            mma_bf16(acc[0], acc[1], acc[2], acc[3], square, transposed_block(square[0]), transposed_block(square[1]));
+            mma_bf16(acc[4], acc[5], acc[6], acc[7], square, transposed_block(square[2]), transposed_block(square[3]));
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                b[i] = pack_bf16(2.0315f * acc[2 * i] - 4.775f * low_half(square[i]), 2.0315f * acc[2 * i + 1] - 4.775f * high_half(square[i]));
+#pragma unroll
+            for (int k = 0; k < Steps; ++k)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { // eight columns
+                    float y[4] = {};
+                    mma_bf16(y[0], y[1], y[2], y[3], b, transposed_block(x[k][2 * h]), transposed_block(x[k][2 * h + 1]));
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+                        x[k][2 * h + r] =
+                            pack_bf16(y[2 * r] + 3.4445f * low_half(x[k][2 * h + r]), y[2 * r + 1] + 3.4445f * high_half(x[k][2 * h + r]));
+                }
+        }
+        const float lr = a.muon_lr * multiplier, keep = 1 - lr * a.adam.weight_decay;
+        const float adjusted = lr * sqrtf(fmaxf(1.f, float(matrix.rows) / matrix.cols));
+        each([&](int k, int i, int j) {
+            const int at = index(k, i, j);
+            float w = join_weight(high[k][i][j], low[k][i][j]) * keep;
+            w -= adjusted * (j ? high_half(x[k][i]) : low_half(x[k][i]));
+            const unsigned bits = __float_as_uint(w);
+            a.adam.weight_high[at] = __ushort_as_bfloat16((unsigned short)(bits >> 16));
+            a.adam.weight_low[at] = uint16_t(bits);
+        });
+    }
+};
+// clip_factor for one warp on its own: a few hundred partial sums, the same order in every warp.
+__device__ __forceinline__ float clip_of_warp(const AdamArgs &a) {
+    if (!(a.clip > 0))
+        return 1.f;
+    float local = 0;
+#pragma unroll 4
+    for (int b = threadIdx.x % 32; b < a.norm_blocks; b += 32)
+        local += a.norm_partial[b];
+    return fminf(1.f, a.clip / (sqrtf(warp_sum(local)) + 1e-6f));
+}
+__global__ void __launch_bounds__(SmallWarps * 32) small_optimizer_kernel(const __grid_constant__ SmallOptimizerArgs a, int matrix_blocks) {
+    sm100::grid_launch_dependents();
+    const int index = blockIdx.x * SmallWarps + threadIdx.x / 32;
+    SmallMatrix matrix{0, 16, 16};
+    if (index < a.matrix_count)
+        matrix = a.matrices[index];
+    sm100::grid_dependency_wait();
+    if (int(blockIdx.x) >= matrix_blocks) {
+        const int64_t group = int64_t(blockIdx.x - matrix_blocks) * blockDim.x + threadIdx.x;
+        AdamGroup parameters;
+        if (group < a.adam.count / 8)
+            parameters = AdamGroup(a.adam, group);
+        AdamRates rates(a.adam);
+        rates.clip = clip_of_warp(a.adam);
+        parameters.update(a.adam, rates, group);
+    } else {
+        if (max(matrix.rows, matrix.cols) == 48) {
+            SmallMuon<3> muon(a, matrix, threadIdx.x % 32);
+            muon.update(a, clip_of_warp(a.adam));
+        } else if (index < a.matrix_count) {
+            SmallMuon<1> muon(a, matrix, threadIdx.x % 32);
+            muon.update(a, clip_of_warp(a.adam));
+        }
+    }
+    __syncthreads(); // every thread has read the step before the block's arrival is counted
+    if (threadIdx.x == 0 && atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1) {
+        a.counters->step += 1;
+        a.counters->iteration += 1;
+    }
+}
+bool small_optimizer_supported(int rows, int cols) { return (rows == 16 && (cols == 16 || cols == 48)) || (rows == 48 && cols == 16); }
+void launch_small_optimizer(const SmallOptimizerArgs &a, cudaStream_t s) {
+    const int matrix_blocks = (a.matrix_count + SmallWarps - 1) / SmallWarps, per_block = SmallWarps * 32;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(matrix_blocks + unsigned((a.adam.count / 8 + per_block - 1) / per_block));
+    config.blockDim = dim3(per_block), config.stream = s, config.attrs = &attribute, config.numAttrs = 1;
+    CHECK_CUDA(cudaLaunchKernelEx(&config, small_optimizer_kernel, a, matrix_blocks));
 }
