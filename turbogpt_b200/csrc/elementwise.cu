@@ -595,7 +595,6 @@ int norm_backward_blocks(int rows, int sms) {
 }
 void launch_norm_backward(Dtype t, const NormBackwardArgs &a, cudaStream_t s) {
     size_t shared = size_t(2) * a.width * sizeof(float);
-    const int reduce_blocks = blocks_for(2 * a.width, 8);
     if (a.width % 256 == 0 && a.width <= 1024) {
         DISPATCH(t, {
             switch (a.width / 256) {
@@ -605,7 +604,6 @@ void launch_norm_backward(Dtype t, const NormBackwardArgs &a, cudaStream_t s) {
             default: launch_norm_backward_rows<T, 4>(a, s); break;
             }
         });
-        norm_backward_reduce_kernel<<<reduce_blocks, 256, 0, s>>>(a.partial, a.dscale, a.dbias, a.width, a.blocks);
         return;
     }
     // as many warps per block (up to 8) as 200 KB of per-warp sums allow
@@ -619,7 +617,9 @@ void launch_norm_backward(Dtype t, const NormBackwardArgs &a, cudaStream_t s) {
                                             int(shared)));
         norm_backward_kernel<T><<<a.blocks, warps * 32, shared, s>>>(a);
     });
-    norm_backward_reduce_kernel<<<reduce_blocks, 256, 0, s>>>(a.partial, a.dscale, a.dbias, a.width, a.blocks);
+}
+void launch_norm_backward_reduce(const NormBackwardArgs &a, cudaStream_t s) {
+    norm_backward_reduce_kernel<<<blocks_for(2 * a.width, 8), 256, 0, s>>>(a.partial, a.dscale, a.dbias, a.width, a.blocks);
 }
 
 // ------------------------------------------------------------------------------------------

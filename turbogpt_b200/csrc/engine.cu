@@ -103,6 +103,11 @@ void Engine::initialize() {
     tokens = c.base.batch * c.base.context;
     gemm_sms = sms;
     CHECK_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    lanes[0].stream = stream;
+    // Profiling times kernels one at a time, and gradient buckets leave in the order the layers finish: both keep one lane.
+    concurrent = !profile && c.world == 1 && tensor_cores;
+    for (int l = 1; l < LaneCount && concurrent; ++l)
+        CHECK_CUDA(cudaStreamCreateWithFlags(&lanes[l].stream, cudaStreamNonBlocking));
 
     const int64_t P = layout.count;
     const int W = c.width, Hd = c.hidden, T = c.base.context, depth = c.base.depth;
@@ -153,18 +158,22 @@ void Engine::initialize() {
     bytes(final_normed, M * W);
     allocate(final_stats, M * 2, false);
     bytes(logits, M * Vocabulary);
-    bytes(dhidden[0], M * W);
-    bytes(dhidden[1], M * W);
+    for (void *&p : dhidden)
+        bytes(p, M * W);
     bytes(dbranch, M * W);
-    bytes(dwide, M * wide);
+    for (int i = 0; i < LayerRing; ++i) {
+        bytes(dwide[i], M * wide);
+        bytes(dqkv[i], M * 3 * W);
+    }
     bytes(dactivated, M * Hd);
-    bytes(dqkv, M * 3 * W);
     allocate(attention_scratch,
              std::max<size_t>(size_t(M) * c.heads, flash_attention_backward_scratch_bytes(c.base.batch, T, c.heads) / sizeof(float)),
              false);
-    allocate(simt_scratch, SimtScratchBytes / sizeof(float), false);
+    for (int l = 0; l < (concurrent ? 2 : 1); ++l) // the lanes of the forward and backward pass
+        allocate(simt_scratch[l], SimtScratchBytes / sizeof(float), false);
     norm_blocks = norm_backward_blocks(tokens, sms);
-    allocate(norm_partial, size_t(norm_blocks) * 2 * W, false);
+    for (float *&p : norm_partial)
+        allocate(p, size_t(norm_blocks) * 2 * W, false);
     if (W <= 1024 && tokens >= 4096)
         allocate(embedding_partial, size_t(EmbeddingSlices) * Vocabulary * W, false);
     sumsq_blocks = sms * 8;
@@ -187,15 +196,22 @@ void Engine::initialize() {
     }
     CHECK_CUDA(cudaMemcpyAsync(adam_mode, mode.data(), mode.size(), cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaStreamSynchronize(stream)); // `mode` is about to go out of scope
-    if (any_muon) {
-        size_t largest = std::max(size_t(3) * W * W, size_t(Hd) * W) * depth;
-        size_t square = size_t(std::min(3 * W, W)) * std::min(3 * W, W);
-        square = std::max(square, size_t(std::min(Hd, W)) * std::min(Hd, W)) * depth;
-        allocate(muon_x[0], largest, false);
-        allocate(muon_x[1], largest, false);
-        allocate(muon_a, square, false);
-        allocate(muon_b, square, false);
-        allocate(muon_sumsq, size_t(depth) * MuonBlocks);
+    if (any_muon) { // q, k and v orthogonalised as one matrix (reference cuda/optim.cuh:109-117)
+        const LayerOffsets &p = layout.layers[0];
+        muon.push_back({p.qkv, 3 * W, W});
+        muon.push_back({p.attention, W, W});
+        muon.push_back({p.gate, Hd, W});
+        muon.push_back({p.down, W, Hd});
+        if (c.mlp == TG_MLP_SWIGLU)
+            muon.push_back({p.up, Hd, W});
+        for (MuonFamily &f : muon) {
+            const size_t square = size_t(std::min(f.rows, f.cols)) * std::min(f.rows, f.cols) * depth;
+            for (bf16 *&x : f.x)
+                allocate(x, size_t(f.rows) * f.cols * depth, false);
+            allocate(f.a, square, false);
+            allocate(f.b, square, false);
+            allocate(f.sumsq, size_t(depth) * MuonBlocks);
+        }
     }
     if (tensor_cores && c.world == 1 && reference_step_supported(c))
         prepare_reference_step();
@@ -260,7 +276,12 @@ void Engine::release() {
         cudaStreamSynchronize(exchange_stream);
     if (comm)
         Nccl::get().CommDestroy(comm);
-    drop_graph();
+    drop_graphs();
+    for (Lane &l : lanes)
+        if (l.stream)
+            cudaStreamSynchronize(l.stream);
+    for (cudaEvent_t ev : fork_events)
+        cudaEventDestroy(ev);
     for (auto &t : timed) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
@@ -273,7 +294,11 @@ void Engine::release() {
         cudaEventDestroy(exchange_done);
     for (void *p : allocations)
         cudaFree(p);
-    release_gemm_workspace(gemm_workspace);
+    for (Lane &l : lanes) {
+        release_gemm_workspace(l.workspace);
+        if (l.stream && l.stream != stream)
+            cudaStreamDestroy(l.stream);
+    }
     if (exchange_stream)
         cudaStreamDestroy(exchange_stream);
     if (stream)
@@ -284,7 +309,7 @@ void Engine::release() {
 template <class F> void Engine::run(Family f, F &&launch) {
     ++launches;
     if (!profile) {
-        launch();
+        launch(lanes[lane].stream);
         return;
     }
     auto take = [&] {
@@ -299,7 +324,7 @@ template <class F> void Engine::run(Family f, F &&launch) {
     };
     Timed t{int(f), take(), take()};
     CHECK_CUDA(cudaEventRecord(t.start, stream));
-    launch();
+    launch(stream);
     CHECK_CUDA(cudaEventRecord(t.stop, stream));
     timed.push_back(t);
     if (timed.size() >= 8192)
@@ -321,13 +346,26 @@ void Engine::flush_profile() {
 }
 void Engine::gemm(Family f, GemmArgs g) {
     g.in = act;
-    run(f, [&] {
+    run(f, [&](cudaStream_t s) {
         if (tensor_cores && gemm_tc_supported(g))
-            launches += launch_gemm_tc(g, gemm_sms, counters, stream, &gemm_workspace) - 1;
+            launches += launch_gemm_tc(g, gemm_sms, counters, s, &lanes[lane].workspace) - 1;
         else
-            launch_gemm_simt(g, stream, gemm_simt_scratch_bytes(g) <= SimtScratchBytes ? simt_scratch : nullptr);
+            launch_gemm_simt(g, s, gemm_simt_scratch_bytes(g) <= SimtScratchBytes ? simt_scratch[lane] : nullptr);
     });
 }
+cudaEvent_t Engine::mark(int on) {
+    if (fork_events.size() < 64) { // more than are ever awaited late: see backward()
+        cudaEvent_t event;
+        CHECK_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+        fork_events.push_back(event);
+        next_fork_event = fork_events.size() - 1;
+    } else {
+        next_fork_event = (next_fork_event + 1) % fork_events.size();
+    }
+    CHECK_CUDA(cudaEventRecord(fork_events[next_fork_event], lanes[on].stream));
+    return fork_events[next_fork_event];
+}
+void Engine::await(int on, cudaEvent_t event) { CHECK_CUDA(cudaStreamWaitEvent(lanes[on].stream, event, 0)); }
 void Engine::check_device_error() {
     StepCounters host{};
     CHECK_CUDA(cudaMemcpyAsync(&host, counters, sizeof(host), cudaMemcpyDeviceToHost, stream));
@@ -358,7 +396,7 @@ void Engine::get_weights(float *w) {
     CHECK_CUDA(cudaStreamSynchronize(stream));
 }
 void Engine::set_data(const uint8_t *bytes, int64_t size) {
-    drop_graph();
+    drop_graphs();
     set_device();
     if (size <= 8)
         throw std::runtime_error("Dataset needs at least 9 bytes");
@@ -372,7 +410,7 @@ void Engine::set_data(const uint8_t *bytes, int64_t size) {
     CHECK_CUDA(cudaStreamSynchronize(stream));
 }
 void Engine::set_onecycle(const TgOneCycle &s) {
-    drop_graph();
+    drop_graphs();
     set_device();
     if (schedule || step)
         throw std::runtime_error("Set OneCycle once, before training");
@@ -397,9 +435,9 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
     auto norm = [&](const void *in, int64_t scale, int64_t bias, void *out, float *stats) {
         NormArgs a{c.norm, in, weight_high + scale, layer_norm ? weight_high + bias : nullptr, weight_low + scale,
                    layer_norm ? weight_low + bias : nullptr, out, M, W, stats};
-        run(FNorm, [&] { launch_norm(act, a, stream); });
+        run(FNorm, [&](cudaStream_t s) { launch_norm(act, a, s); });
     };
-    run(FEmbedding, [&] { launch_embedding(act, weight(layout.embedding), x, layers[0].x, M, W, stream); });
+    run(FEmbedding, [&](cudaStream_t s) { launch_embedding(act, weight(layout.embedding), x, layers[0].x, M, W, s); });
     for (int l = 0; l < depth; ++l) {
         LayerActivations &a = layers[l];
         const LayerOffsets &p = layout.layers[l];
@@ -410,17 +448,17 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
         qkv.m = M, qkv.n = 3 * W, qkv.k = W, qkv.out = act;
         gemm(FGemmForward, qkv);
         if (c.rope == TG_ROPE_PARTIAL)
-            run(FMisc, [&] { launch_rope(act, a.qkv, M, T, W, H, false, stream); });
+            run(FMisc, [&](cudaStream_t s) { launch_rope(act, a.qkv, M, T, W, H, false, s); });
         if (c.attention == TG_ATTENTION_ARGMAX) {
             ArgmaxAttentionArgs at{a.qkv, a.attended, a.selected, a.gates, a.derivatives, B, T, W, H};
-            run(FAttentionForward, [&] { launch_argmax_attention(act, at, stream); });
+            run(FAttentionForward, [&](cudaStream_t s) { launch_argmax_attention(act, at, s); });
         } else {
             SoftmaxAttentionArgs at{a.qkv, a.attended, a.lse, B, T, W, H};
-            run(FAttentionForward, [&] {
+            run(FAttentionForward, [&](cudaStream_t s) {
                 if (tensor_cores && act == Dtype::BF16 && flash_attention_supported(W, H))
-                    launch_flash_attention_forward(a.qkv, a.attended, a.lse, B, T, H, counters, stream);
+                    launch_flash_attention_forward(a.qkv, a.attended, a.lse, B, T, H, counters, s);
                 else
-                    launch_softmax_attention(act, at, stream);
+                    launch_softmax_attention(act, at, s);
             });
         }
         GemmArgs proj;
@@ -435,7 +473,7 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
         if (c.mlp == TG_MLP_SWIGLU) { // gate and up are adjacent: one projection computes both
             up.n = 2 * Hd, up.ldc = 2 * Hd;
             gemm(FGemmForward, up);
-            run(FActivation, [&] { launch_swiglu(act, a.wide, a.activated, M, Hd, stream); });
+            run(FActivation, [&](cudaStream_t s) { launch_swiglu(act, a.wide, a.activated, M, Hd, s); });
         } else {
             up.n = Hd, up.ldc = Hd, up.epilogue = Epilogue::GeluDual, up.c2 = a.activated;
             gemm(FGemmForward, up);
@@ -463,7 +501,7 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
     gemm(FGemmForward, head);
     CrossEntropyArgs ce{logits, y, token_losses, want_gradient ? logits : nullptr,
                         dump_logits ? logits_fp32 : nullptr, divisor, M};
-    run(FCrossEntropy, [&] { launch_cross_entropy(act, ce, stream); });
+    run(FCrossEntropy, [&](cudaStream_t s) { launch_cross_entropy(act, ce, s); });
 }
 
 // ------------------------------------------------------------------------------- backward ----
@@ -499,8 +537,17 @@ void Engine::backward() {
     const int depth = c.base.depth;
     const bool layer_norm = c.norm == TG_NORM_LAYER;
     const int wide = c.mlp == TG_MLP_SWIGLU ? 2 * Hd : Hd;
+    // Nothing in backward waits for a weight gradient or for the sums of a norm's scale and bias gradients: they run on
+    // a lane of their own beside the chain of input gradients.
+    const int side = concurrent ? 1 : 0;
+    auto aside = [&] { // launches go to the side lane, after everything the main lane holds
+        if (side)
+            fork(0, side);
+        return OnLane(*this, side);
+    };
     // dW[out, in] = dy^T x: both operands are read "MN-major" (tokens are the contraction).
     auto weight_grad = [&](const void *dy, int out, const void *xin, int in, int64_t offset) {
+        const OnLane on = aside();
         GemmArgs g;
         g.a = dy, g.a_row = 1, g.a_col = out, g.b = xin, g.b_row = 1, g.b_col = in;
         g.c = gradient + offset, g.ldc = in, g.m = out, g.n = in, g.k = M, g.out = Dtype::FP32;
@@ -513,14 +560,18 @@ void Engine::backward() {
         g.c = dx, g.ldc = in, g.m = M, g.n = in, g.k = out, g.out = act;
         return g;
     };
+    int norms = 0;
     auto norm_back = [&](const void *xin, const void *dy, int64_t scale, int64_t bias, const void *residual,
                          void *dx, const float *stats) {
-        NormBackwardArgs a{c.norm, xin, dy, weight_high + scale, weight_low + scale, residual, dx, norm_partial,
+        NormBackwardArgs a{c.norm, xin, dy, weight_high + scale, weight_low + scale, residual, dx, norm_partial[norms++ % HiddenRing],
                            gradient + scale, layer_norm ? gradient + bias : nullptr, M, W, norm_blocks, stats};
-        run(FNormBackward, [&] { launch_norm_backward(act, a, stream); });
-        ++launches; // rows kernel + reduce kernel
+        run(FNormBackward, [&](cudaStream_t s) { launch_norm_backward(act, a, s); });
+        const OnLane on = aside();
+        run(FNormBackward, [&](cudaStream_t s) { launch_norm_backward_reduce(a, s); });
     };
-    void *dh = dhidden[0], *dh_other = dhidden[1];
+    int hidden = 0; // ring position of the running residual-stream gradient
+    auto dh = [&] { return dhidden[hidden % HiddenRing]; };
+    auto dh_next = [&] { return dhidden[(hidden + 1) % HiddenRing]; };
     // From the first bucket to the end of backward a collective may be running beside the GEMMs.
     struct Reserve {
         Engine &e;
@@ -533,71 +584,81 @@ void Engine::backward() {
 
     weight_grad(logits, Vocabulary, final_normed, W, layout.head);
     gemm(FGemmInputGrad, input_grad(logits, Vocabulary, layout.head, W, dbranch));
-    norm_back(final_x, dbranch, layout.final_norm, layout.final_norm_bias, nullptr, dh, final_stats);
+    norm_back(final_x, dbranch, layout.final_norm, layout.final_norm_bias, nullptr, dh(), final_stats);
     if (!c.tied) // final norm + head form the first bucket; a tied head waits for the embedding scatter
         exchange_bucket(layout.final_norm, layout.count, depth);
     else
         exchange_bucket(layout.final_norm, layout.final_norm + (layer_norm ? 2 : 1) * W, depth);
 
+    std::vector<cudaEvent_t> layer_done(depth); // the side lane's end of each layer
+    const cudaEvent_t head_done = side ? mark(side) : nullptr;
     for (int l = depth - 1; l >= 0; --l) {
+        if (side && l + 2 < depth)
+            await(0, layer_done[l + 2]); // its buffers are about to be written again
+        void *dwide = this->dwide[l % LayerRing], *dqkv = this->dqkv[l % LayerRing];
         LayerActivations &a = layers[l];
         const LayerOffsets &p = layout.layers[l];
-        weight_grad(dh, W, a.activated, Hd, p.down);
-        GemmArgs dact = input_grad(dh, W, p.down, Hd, c.mlp == TG_MLP_SWIGLU ? dactivated : dwide);
+        weight_grad(dh(), W, a.activated, Hd, p.down);
+        GemmArgs dact = input_grad(dh(), W, p.down, Hd, c.mlp == TG_MLP_SWIGLU ? dactivated : dwide);
         if (c.mlp == TG_MLP_SWIGLU) {
             gemm(FGemmInputGrad, dact);
-            run(FActivation, [&] { launch_swiglu_backward(act, a.wide, dactivated, dwide, M, Hd, stream); });
+            run(FActivation, [&](cudaStream_t s) { launch_swiglu_backward(act, a.wide, dactivated, dwide, M, Hd, s); });
         } else {
             dact.epilogue = Epilogue::GeluGrad, dact.r = a.wide, dact.ldr = Hd;
             gemm(FGemmInputGrad, dact);
         }
         weight_grad(dwide, wide, a.normed2, W, p.gate);
         gemm(FGemmInputGrad, input_grad(dwide, wide, p.gate, W, dbranch));
-        norm_back(a.middle, dbranch, p.mlp_norm, p.mlp_norm_bias, dh, dh_other, a.stats2);
-        std::swap(dh, dh_other);
+        norm_back(a.middle, dbranch, p.mlp_norm, p.mlp_norm_bias, dh(), dh_next(), a.stats2);
+        ++hidden;
 
-        weight_grad(dh, W, a.attended, W, p.attention);
-        gemm(FGemmInputGrad, input_grad(dh, W, p.attention, W, dbranch));
+        weight_grad(dh(), W, a.attended, W, p.attention);
+        gemm(FGemmInputGrad, input_grad(dh(), W, p.attention, W, dbranch));
         if (c.attention == TG_ATTENTION_ARGMAX) {
             ArgmaxAttentionBackwardArgs at{a.qkv, dbranch, a.selected, a.gates, a.derivatives, attention_scratch,
                                            dqkv, B, T, W, H};
-            run(FAttentionBackward, [&] { launch_argmax_attention_backward(act, at, stream); });
+            run(FAttentionBackward, [&](cudaStream_t s) { launch_argmax_attention_backward(act, at, s); });
         } else {
             SoftmaxAttentionBackwardArgs at{a.qkv, a.attended, dbranch, a.lse, attention_scratch, dqkv, B, T, W, H};
-            run(FAttentionBackward, [&] {
+            run(FAttentionBackward, [&](cudaStream_t s) {
                 if (tensor_cores && act == Dtype::BF16 && flash_attention_supported(W, H)) {
                     launch_flash_attention_backward(a.qkv, a.attended, dbranch, a.lse, attention_scratch, dqkv, B, T, H,
-                                                    counters, stream);
+                                                    counters, s);
                     ++launches; // dq kernel + dk/dv kernel
                 } else {
-                    launch_softmax_attention_backward(act, at, stream);
+                    launch_softmax_attention_backward(act, at, s);
                 }
             });
         }
         if (c.rope == TG_ROPE_PARTIAL)
-            run(FMisc, [&] { launch_rope(act, dqkv, M, T, W, H, true, stream); });
+            run(FMisc, [&](cudaStream_t s) { launch_rope(act, dqkv, M, T, W, H, true, s); });
         weight_grad(dqkv, 3 * W, a.normed1, W, p.qkv);
         gemm(FGemmInputGrad, input_grad(dqkv, 3 * W, p.qkv, W, dbranch));
-        norm_back(a.x, dbranch, p.attention_norm, p.attention_norm_bias, dh, dh_other, a.stats1);
-        std::swap(dh, dh_other);
+        norm_back(a.x, dbranch, p.attention_norm, p.attention_norm_bias, dh(), dh_next(), a.stats1);
+        ++hidden;
+        if (side)
+            layer_done[l] = mark(side);
         int64_t layer_end = l + 1 < depth ? layout.layers[l + 1].attention_norm : layout.final_norm;
         exchange_bucket(p.attention_norm, layer_end, l);
     }
-    run(FEmbeddingBackward, [&] {
-        launch_embedding_backward(act, dh, x, gradient + layout.embedding, M, W, c.tied != 0, embedding_partial,
-                                  stream);
+    if (side)
+        await(0, head_done); // a tied head's gradient is added to
+    run(FEmbeddingBackward, [&](cudaStream_t s) {
+        launch_embedding_backward(act, dh(), x, gradient + layout.embedding, M, W, c.tied != 0, embedding_partial,
+                                  s);
     });
     if (embedding_partial)
         ++launches; // slices kernel + sum kernel
     exchange_bucket(layout.embedding, layout.embedding + int64_t(Vocabulary) * W, depth + 1);
     finish_exchange();
+    fork(side, 0); // join
 }
 
 // ------------------------------------------------------------------------------- optimizer ---
-void Engine::muon_family(int64_t first_offset, int rows, int cols) {
+void Engine::muon_family(const MuonFamily &family) {
     const TgConfigEx &c = config;
-    const int depth = c.base.depth;
-    const int64_t stride = depth > 1 ? layout.layers[1].qkv - layout.layers[0].qkv : 0;
+    const int depth = c.base.depth, rows = family.rows, cols = family.cols;
+    const int64_t first_offset = family.first, stride = depth > 1 ? layout.layers[1].qkv - layout.layers[0].qkv : 0;
     const int r = std::min(rows, cols), n = std::max(rows, cols); // orthogonalise the wide orientation
     const int64_t per = int64_t(rows) * cols;
     // Under data parallelism the gradients are identical on every rank after the exchange, so the
@@ -607,15 +668,15 @@ void Engine::muon_family(int64_t first_offset, int rows, int cols) {
     // stay bit-identical and any rank can write a checkpoint.
     const bool sharded = comm && depth % c.world == 0 && depth >= c.world;
     const int mine = sharded ? depth / c.world : depth, first = sharded ? c.rank * mine : 0;
-    MuonPrepareArgs prep{gradient + first_offset, momentum + first_offset, muon_x[0], muon_sumsq, sumsq_partial,
+    MuonPrepareArgs prep{gradient + first_offset, momentum + first_offset, family.x[0], family.sumsq, sumsq_partial,
                          sumsq_blocks, schedule, counters, c.base.momentum, c.base.clip, rows, cols, depth, stride};
-    run(FMuon, [&] { launch_muon_prepare(prep, stream); });
-    run(FMuon, [&] { launch_muon_normalize(muon_x[0], muon_sumsq, per, depth, stream); });
-    bf16 *cur = muon_x[0] + first * per, *nxt = muon_x[1] + first * per;
-    bf16 *a_buffer = muon_a + int64_t(first) * r * r, *b_buffer = muon_b + int64_t(first) * r * r;
+    run(FMuon, [&](cudaStream_t s) { launch_muon_prepare(prep, s); });
+    run(FMuon, [&](cudaStream_t s) { launch_muon_normalize(family.x[0], family.sumsq, per, depth, s); });
+    bf16 *cur = family.x[0] + first * per, *nxt = family.x[1] + first * per;
+    bf16 *a_buffer = family.a + int64_t(first) * r * r, *b_buffer = family.b + int64_t(first) * r * r;
     const bool small = muon_newton_schulz_small_supported(r, n); // the reference architecture: one launch, in place
     if (small)
-        run(FMuon, [&] { launch_muon_newton_schulz_small(cur, r, n, c.base.ns_steps, mine, stream); });
+        run(FMuon, [&](cudaStream_t s) { launch_muon_newton_schulz_small(cur, r, n, c.base.ns_steps, mine, s); });
     for (int it = 0; !small && it < c.base.ns_steps; ++it) {
         GemmArgs a; // A = X X^T
         a.a = cur, a.a_row = n, a.b = cur, a.b_row = n, a.c = a_buffer, a.ldc = r, a.m = r, a.n = r, a.k = n;
@@ -632,12 +693,12 @@ void Engine::muon_family(int64_t first_offset, int rows, int cols) {
         x2.epilogue = Epilogue::Axpby, x2.alpha = 1.f, x2.beta = 3.4445f, x2.r = cur, x2.ldr = n;
         x2.out = Dtype::BF16;
         for (GemmArgs *g : {&a, &b, &x2}) {
-            run(FMuon, [&] {
+            run(FMuon, [&](cudaStream_t s) {
                 g->in = Dtype::BF16;
                 if (tensor_cores && gemm_tc_supported(*g))
-                    launches += launch_gemm_tc(*g, sms, counters, stream, &gemm_workspace) - 1;
+                    launches += launch_gemm_tc(*g, sms, counters, s, &lanes[lane].workspace) - 1;
                 else
-                    launch_gemm_simt(*g, stream);
+                    launch_gemm_simt(*g, s);
             });
         }
         std::swap(cur, nxt);
@@ -645,34 +706,35 @@ void Engine::muon_family(int64_t first_offset, int rows, int cols) {
     bf16 *all = cur - first * per; // the buffer holding every layer's result
     if (sharded) {
         const Nccl &nccl = Nccl::get();
-        run(FExchange, [&] {
-            nccl.check(nccl.AllGather(cur, all, size_t(mine) * per, Nccl::Bfloat16, comm, stream), "ncclAllGather");
+        run(FExchange, [&](cudaStream_t s) {
+            nccl.check(nccl.AllGather(cur, all, size_t(mine) * per, Nccl::Bfloat16, comm, s), "ncclAllGather");
         });
     }
     MuonApplyArgs apply{all, weight_high + first_offset, weight_low + first_offset,
                         weight_fp32 ? weight_fp32 + first_offset : nullptr, schedule, counters, c.base.muon_lr,
                         c.base.weight_decay, rows, cols, depth, stride};
-    run(FMuon, [&] { launch_muon_apply(apply, stream); });
+    run(FMuon, [&](cudaStream_t s) { launch_muon_apply(apply, s); });
 }
 
 void Engine::optimize() {
     const TgConfigEx &c = config;
-    run(FOptimizer, [&] { launch_sum_squares(gradient, layout.count, sumsq_partial, sumsq_blocks, stream); });
+    run(FOptimizer, [&](cudaStream_t s) { launch_sum_squares(gradient, layout.count, sumsq_partial, sumsq_blocks, s); });
     AdamArgs a{gradient, momentum, variance, weight_high, weight_low, weight_fp32, adam_mode, sumsq_partial,
                sumsq_blocks, schedule, counters, c.base.learning_rate, c.base.beta1, c.base.beta2,
                c.base.weight_decay, c.base.epsilon, c.base.clip, layout.count};
-    run(FOptimizer, [&] { launch_adamw(a, sms, stream); });
-    if (c.hidden_optimizer == TG_HIDDEN_MUON) {
-        const LayerOffsets &p = layout.layers[0];
-        const int W = c.width, Hd = c.hidden;
-        muon_family(p.qkv, 3 * W, W); // q, k and v orthogonalised as one matrix (reference cuda/optim.cuh:109-117)
-        muon_family(p.attention, W, W);
-        muon_family(p.gate, Hd, W);
-        if (c.mlp == TG_MLP_SWIGLU)
-            muon_family(p.up, Hd, W);
-        muon_family(p.down, W, Hd);
+    const cudaEvent_t norm_ready = concurrent && !muon.empty() ? mark(0) : nullptr;
+    run(FOptimizer, [&](cudaStream_t s) { launch_adamw(a, sms, s); });
+    // The families are independent chains of small products: each on a lane of its own.
+    const int chains = concurrent ? std::min(int(muon.size()), LaneCount - 1) : 0;
+    for (int l = 1; l <= chains; ++l)
+        await(l, norm_ready);
+    for (size_t f = 0; f < muon.size(); ++f) {
+        OnLane on(*this, chains ? 1 + int(f) % chains : 0);
+        muon_family(muon[f]);
     }
-    run(FMisc, [&] { launch_advance(counters, stream); });
+    for (int l = 1; l <= chains; ++l)
+        fork(l, 0); // join
+    run(FMisc, [&](cudaStream_t s) { launch_advance(counters, s); });
 }
 
 // ------------------------------------------------------------------------------- modes -------
@@ -690,13 +752,13 @@ void Engine::reference_train_step(bool sample, bool save) {
     ReferenceStepArgs step{sample ? data : nullptr, data_size, b.seed, x, y, counters, weight_high, weight_low, reference_rope,
                            reference_partial, token_losses, loss_history, gradient, reference_norm, b.batch, b.context, b.depth,
                            save ? &saved : nullptr};
-    run(FMisc, [&] { launch_reference_step(step, reference_plan, stream); });
+    run(FMisc, [&](cudaStream_t s) { launch_reference_step(step, reference_plan, s); });
     ++launches; // step kernel + reduce kernel
     SmallOptimizerArgs update{{gradient, momentum, variance, weight_high, weight_low, nullptr, adam_mode, reference_norm,
                                reference_plan.gradient_blocks, schedule, counters, b.learning_rate, b.beta1, b.beta2, b.weight_decay,
                                b.epsilon, b.clip, layout.count},
                               b.muon_lr, b.momentum, b.ns_steps, small_matrices, small_matrix_count, counters, small_ticket};
-    run(FOptimizer, [&] { launch_small_optimizer(update, stream); });
+    run(FOptimizer, [&](cudaStream_t s) { launch_small_optimizer(update, s); });
 }
 
 // `last`: no other step follows in this call, so the activations it leaves can be read.
@@ -706,18 +768,18 @@ void Engine::one_step(RunMode mode, bool last) {
         return;
     }
     if (mode == RunMode::Train) {
-        SampleArgs s{data, data_size, config.base.seed, counters, -1, config.base.batch, config.base.context,
+        SampleArgs sampling{data, data_size, config.base.seed, counters, -1, config.base.batch, config.base.context,
                      config.world, config.rank, x, y};
-        run(FSample, [&] { launch_sample(s, stream); });
+        run(FSample, [&](cudaStream_t s) { launch_sample(sampling, s); });
     }
     if (mode != RunMode::OptimizerOnly) {
         forward(mode != RunMode::Evaluate, mode != RunMode::Train && logits_fp32 != nullptr);
         if (mode == RunMode::Evaluate)
             return;
         if (mode == RunMode::Train)
-            run(FMisc, [&] {
+            run(FMisc, [&](cudaStream_t s) {
                 launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context,
-                                    stream);
+                                    s);
             });
         backward();
         if (mode == RunMode::Gradients)
@@ -726,11 +788,52 @@ void Engine::one_step(RunMode mode, bool last) {
     optimize();
 }
 
-// The captured step holds raw pointers: it is dropped whenever one of them may change.
-void Engine::drop_graph() {
-    if (step_graph)
-        cudaGraphExecDestroy(step_graph);
-    step_graph = nullptr;
+void Engine::drop_graphs() {
+    for (StepGraph &g : graphs) {
+        if (g.exec)
+            cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
+}
+
+// Runs a kernel sequence that reads everything that changes between calls from device memory: directly the first time (which
+// sizes every workspace), then captured once and replayed.
+template <class F> void Engine::replay(GraphKind kind, F &&body) {
+    StepGraph &g = graphs[kind];
+    if (!use_graphs() || !g.warm) {
+        body();
+        g.warm = true;
+        return;
+    }
+    uint64_t generation = 0;
+    for (const Lane &l : lanes)
+        generation += l.workspace.generation;
+    if (g.exec && g.generation != generation) { // a split-K workspace moved since the capture
+        cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
+    if (!g.exec) {
+        g.generation = generation;
+        const int64_t before = launches;
+        cudaGraph_t graph = nullptr;
+        CHECK_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        try {
+            body();
+        } catch (...) {
+            cudaStreamEndCapture(stream, &graph);
+            if (graph)
+                cudaGraphDestroy(graph);
+            throw;
+        }
+        CHECK_CUDA(cudaStreamEndCapture(stream, &graph));
+        const cudaError_t status = cudaGraphInstantiate(&g.exec, graph, 0);
+        cudaGraphDestroy(graph);
+        CHECK_CUDA(status);
+        g.launches = launches - before;
+        launches = before;
+    }
+    CHECK_CUDA(cudaGraphLaunch(g.exec, stream));
+    launches += g.launches;
 }
 
 void Engine::train(int steps) {
@@ -745,44 +848,19 @@ void Engine::train(int steps) {
     if (schedule && step + uint64_t(steps) > uint64_t(schedule_steps))
         throw std::runtime_error("Training would exceed the OneCycle schedule");
     CHECK_CUDA(cudaMemsetAsync(&counters->iteration, 0, sizeof(int), stream));
-    // A step reads everything that changes from device memory, so its kernel sequence is captured
-    // once (after one eager step has sized every workspace) and replayed as a CUDA graph.
-    const bool use_graph = !profile && !comm && !(config.flags & TG_FLAG_NO_GRAPH);
     // The last step of a call leaves its activations for read_activation: the reference architecture's step kernel, whose
     // activations otherwise stay on chip, is launched in another form for it, outside the graph.
     const int outside = reference_step ? 1 : 0, graph_steps = reference_step ? ReferenceGraphSteps : 1;
     for (int i = 0; i < steps;) {
-        if (!use_graph || !graph_warm || steps - i - outside < graph_steps) {
+        if (steps - i - outside < graph_steps) {
             one_step(RunMode::Train, i + 1 == steps);
-            graph_warm = true;
             ++i;
             continue;
         }
-        if (step_graph && graph_generation != gemm_workspace.generation)
-            drop_graph(); // the split-K workspace moved since the capture
-        if (!step_graph) {
-            graph_generation = gemm_workspace.generation;
-            const int64_t before = launches;
-            cudaGraph_t graph = nullptr;
-            CHECK_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            try {
-                for (int k = 0; k < graph_steps; ++k)
-                    one_step(RunMode::Train, false);
-            } catch (...) {
-                cudaStreamEndCapture(stream, &graph);
-                if (graph)
-                    cudaGraphDestroy(graph);
-                throw;
-            }
-            CHECK_CUDA(cudaStreamEndCapture(stream, &graph));
-            cudaError_t status = cudaGraphInstantiate(&step_graph, graph, 0);
-            cudaGraphDestroy(graph);
-            CHECK_CUDA(status);
-            graph_launches = launches - before;
-            launches = before;
-        }
-        CHECK_CUDA(cudaGraphLaunch(step_graph, stream));
-        launches += graph_launches;
+        replay(GraphTrain, [&] {
+            for (int k = 0; k < graph_steps; ++k)
+                one_step(RunMode::Train, false);
+        });
         i += graph_steps;
     }
     last_train_steps = steps;
@@ -834,7 +912,8 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
         allocate(logits_fp32, size_t(tokens) * Vocabulary, false);
     CHECK_CUDA(cudaMemcpyAsync(x, bx, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemcpyAsync(y, by, tokens, cudaMemcpyHostToDevice, stream));
-    one_step(gradient_out ? RunMode::Gradients : RunMode::Evaluate);
+    replay(gradient_out ? GraphGradients : GraphEvaluate,
+           [&] { one_step(gradient_out ? RunMode::Gradients : RunMode::Evaluate); });
     if (logits_out)
         CHECK_CUDA(cudaMemcpyAsync(logits_out, logits_fp32, size_t(tokens) * Vocabulary * 4, cudaMemcpyDeviceToHost,
                                    stream));
@@ -868,7 +947,7 @@ void Engine::predict(const uint8_t *context, float *logits256) {
     CHECK_CUDA(cudaMemsetAsync(y, 0, T, stream));
     forward_batch = 1;
     try {
-        one_step(RunMode::Evaluate);
+        replay(GraphPredict, [&] { one_step(RunMode::Evaluate); });
     } catch (...) {
         forward_batch = 0;
         throw;
@@ -898,9 +977,9 @@ void Engine::sample(uint64_t at_step, uint8_t *bx, uint8_t *by) {
     set_device();
     if (!data)
         throw std::runtime_error("Load data first");
-    SampleArgs s{data, data_size, config.base.seed, counters, (long long)at_step, config.base.batch,
+    SampleArgs sampling{data, data_size, config.base.seed, counters, (long long)at_step, config.base.batch,
                  config.base.context, config.world, config.rank, x, y};
-    run(FSample, [&] { launch_sample(s, stream); });
+    run(FSample, [&](cudaStream_t s) { launch_sample(sampling, s); });
     CHECK_CUDA(cudaMemcpyAsync(bx, x, tokens, cudaMemcpyDeviceToHost, stream));
     CHECK_CUDA(cudaMemcpyAsync(by, y, tokens, cudaMemcpyDeviceToHost, stream));
     CHECK_CUDA(cudaStreamSynchronize(stream));
@@ -991,16 +1070,18 @@ void Engine::train_batch(const uint8_t *bx, const uint8_t *by, float *per_positi
     CHECK_CUDA(cudaMemcpyAsync(x, bx, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemcpyAsync(y, by, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemsetAsync(&counters->iteration, 0, sizeof(int), stream));
-    if (reference_step) {
-        reference_train_step(false, true);
-    } else {
+    replay(GraphTrainBatch, [&] {
+        if (reference_step) {
+            reference_train_step(false, true);
+            return;
+        }
         forward(true, false);
-        run(FMisc, [&] {
-            launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context, stream);
+        run(FMisc, [&](cudaStream_t s) {
+            launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context, s);
         });
         backward();
         optimize();
-    }
+    });
     step += 1;
     last_train_steps = 1;
     losses_reduced = false;

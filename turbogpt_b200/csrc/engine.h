@@ -46,6 +46,23 @@ struct LayerActivations { // saved by forward for backward (reference cuda/types
     float *stats1, *stats2; // per row: mean and 1/sigma of the two norms, saved by forward for backward
 };
 
+// Kernels that do not depend on one another run side by side on the engine's lanes: lane 0 is the engine's stream, the
+// others carry work forked from it (weight gradients beside the input-gradient chain, the families of Muon matrices) and
+// are joined before the step ends.  Each lane has its own split-K scratch.
+constexpr int LaneCount = 5;
+struct Lane {
+    cudaStream_t stream = nullptr;
+    GemmWorkspace workspace;
+};
+// A captured kernel sequence; pointers it holds are fixed, so it is dropped when one of them may change.
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    bool warm = false; // the sequence has run once directly, which sizes every workspace
+    int64_t launches = 0;
+    uint64_t generation = 0;
+};
+enum GraphKind { GraphTrain, GraphTrainBatch, GraphEvaluate, GraphGradients, GraphPredict, GraphKinds };
+
 enum class RunMode { Evaluate, Gradients, Train, OptimizerOnly }; // reference cuda/trainer.cuh:6
 
 struct Engine {
@@ -71,18 +88,24 @@ struct Engine {
     std::vector<LayerActivations> layers;
     void *final_x = nullptr, *final_normed = nullptr, *logits = nullptr;
     float *final_stats = nullptr;
-    void *dhidden[2] = {nullptr, nullptr}, *dbranch = nullptr, *dwide = nullptr, *dactivated = nullptr,
-         *dqkv = nullptr;
+    // Gradients that the weight-gradient lane reads: it may be up to two layers behind, so the buffers rotate.
+    static constexpr int HiddenRing = 6, LayerRing = 2;
+    void *dhidden[HiddenRing] = {}, *dbranch = nullptr, *dwide[LayerRing] = {}, *dactivated = nullptr, *dqkv[LayerRing] = {};
     float *attention_scratch = nullptr; // dt (arg-max) or delta (softmax)
-    float *token_losses = nullptr, *loss_history = nullptr, *norm_partial = nullptr, *sumsq_partial = nullptr,
+    float *token_losses = nullptr, *loss_history = nullptr, *norm_partial[HiddenRing] = {}, *sumsq_partial = nullptr,
           *logits_fp32 = nullptr, *mean_loss = nullptr, *embedding_partial = nullptr;
     int norm_blocks = 0, sumsq_blocks = 0;
     StepCounters *counters = nullptr;
     TgStepRates *schedule = nullptr;
     int schedule_steps = 0;
     // Muon scratch
-    bf16 *muon_x[2] = {nullptr, nullptr}, *muon_a = nullptr, *muon_b = nullptr;
-    float *muon_sumsq = nullptr;
+    struct MuonFamily { // q|k|v, attention, gate, down, up: the same matrix of every layer
+        int64_t first = 0;
+        int rows = 0, cols = 0;
+        bf16 *x[2] = {nullptr, nullptr}, *a = nullptr, *b = nullptr;
+        float *sumsq = nullptr;
+    };
+    std::vector<MuonFamily> muon;
     // the reference architecture's step in three kernels (reference_step.cu, small_optimizer_kernel); unset: operator by operator
     bool reference_step = false;
     ReferenceStepPlan reference_plan;
@@ -110,13 +133,15 @@ struct Engine {
     double family_ms[FamilyCount] = {};
     int64_t family_launches[FamilyCount] = {};
     int64_t launches = 0, graph_launches = 0;
-    GemmWorkspace gemm_workspace; // this engine's split-K scratch (never shared with another engine or stream)
-    float *simt_scratch = nullptr; // partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
-    cudaGraphExec_t step_graph = nullptr; // one captured training step
-    bool graph_warm = false;
+    Lane lanes[LaneCount];
+    int lane = 0;            // where run() launches
+    bool concurrent = false; // whether work is forked at all
+    std::vector<cudaEvent_t> fork_events;
+    size_t next_fork_event = 0;
+    float *simt_scratch[2] = {nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
+    StepGraph graphs[GraphKinds];
     int forward_batch = 0; // sequences the next forward pass covers (0: the configured batch)
-    uint64_t graph_generation = 0;
-    void drop_graph();
+    void drop_graphs();
 
     explicit Engine(const TgConfigEx &c);
     ~Engine();
@@ -144,6 +169,12 @@ struct Engine {
     int64_t read_activation(int layer, const char *name, float *out, int64_t capacity);
 
   private:
+    struct OnLane { // run() launches on another lane while this lives
+        Engine &e;
+        OnLane(Engine &engine, int l) : e(engine) { e.lane = l; }
+        OnLane(const OnLane &) = delete;
+        ~OnLane() { e.lane = 0; }
+    };
     void initialize();
     void release();
     template <class F> void run(Family f, F &&launch);
@@ -153,7 +184,15 @@ struct Engine {
     void exchange_bucket(int64_t begin, int64_t end, int index);
     void finish_exchange();
     void optimize();
-    void muon_family(int64_t first_offset, int rows, int cols);
+    void muon_family(const MuonFamily &family);
+    bool use_graphs() const { return !profile && !comm && !(config.flags & TG_FLAG_NO_GRAPH); }
+    template <class F> void replay(GraphKind kind, F &&body);
+    cudaEvent_t mark(int on); // an event after everything lane `on` holds
+    void await(int on, cudaEvent_t event);
+    void fork(int from, int to) {
+        if (concurrent)
+            await(to, mark(from));
+    }
     void prepare_reference_step();
     void reference_train_step(bool sample, bool save);
     void one_step(RunMode mode, bool last = true);

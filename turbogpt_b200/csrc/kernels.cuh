@@ -59,7 +59,9 @@ struct NormBackwardArgs {
     int rows, width, blocks;
     const float *stats = nullptr; // [rows][2] from the forward pass (nullptr: recomputed from x)
 };
+// dx and the blocks' sums of the scale and bias gradients in `partial`; then those sums over the blocks.
 void launch_norm_backward(Dtype t, const NormBackwardArgs &a, cudaStream_t s);
+void launch_norm_backward_reduce(const NormBackwardArgs &a, cudaStream_t s);
 int norm_backward_blocks(int rows, int sms);
 
 // ---- positional rotation (reference cuda/attention.cuh:19-30) ----

@@ -436,6 +436,7 @@ int tg_ex_norm_backward(int kind, const void *x, const void *dy, const void *sca
                            residual_in, dx, partial, dscale, kind == TG_NORM_LAYER ? dbias : nullptr, rows, width, blocks,
                            width % 256 == 0 && width <= 1024 ? stats : nullptr};
         launch_norm_backward(Dtype::BF16, a, s);
+        launch_norm_backward_reduce(a, s);
         CHECK_CUDA(cudaFreeAsync(partial, s));
         CHECK_CUDA(cudaGetLastError());
     });
