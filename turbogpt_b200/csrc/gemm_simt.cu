@@ -1,10 +1,12 @@
 // GEMM on CUDA cores: C[m,n] = sum_k A[m,k] * B[n,k] with arbitrary element strides, BF16 or
 // FP32 operands, FP32 accumulation.  It serves the shapes the tensor-core kernel does not take
 // (the reference architecture's 16/48-wide matrices), the FP32 check mode, and is the on-device
-// cross-check of the tcgen05 kernel.  64x64 output tile, 16-deep shared-memory slices, 4x4
-// outputs per thread.
+// cross-check of the tcgen05 kernel.  Two kernels: gemm_simt_kernel takes any strides, sizes and
+// alignments (64x64 output tile, 16-deep shared-memory slices, 4x4 outputs per thread, scalar loads);
+// gemm_simt_wide_kernel takes what its vector loads can reach and every shape of a real model (see there).
 #include "device_utils.cuh"
 #include "kernels.cuh"
+#include <algorithm>
 
 constexpr int TileM = 64, TileN = 64, TileK = 16;
 
@@ -107,6 +109,119 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs g, float *parti
         }
 }
 
+// The same product for aligned operands.  FP32 multiply-adds bound it (128 per clock and SM, 72 TFLOP/s), so the rest has to
+// stay out of their way: 8 x TN outputs per thread (12 or 16 shared-memory words per 32 or 64 multiply-adds), operands
+// as 128-bit loads that are issued a slice ahead and land in the other of two shared-memory buffers, one barrier a slice.
+// TN = 8: 128 x 128 tiles, 256 threads; TN = 4: 64 x 64 tiles, 128 threads, for outputs of too few large tiles.
+// FP32, 2048 x 1024 x 256: 97 -> FIXME us.
+template <class T> struct Quad;
+template <> struct Quad<float> {
+    float4 v;
+    __device__ __forceinline__ float at(int i) const { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+};
+template <> struct Quad<bf16> {
+    uint2 v;
+    __device__ __forceinline__ float at(int i) const {
+        const unsigned w = i < 2 ? v.x : v.y;
+        return __uint_as_float(i % 2 ? w & 0xffff0000u : w << 16);
+    }
+};
+// Rows x TileK elements of an operand, four at a time along its unit stride, through registers into [k][row].
+template <class In, int Rows, int Threads> struct SliceLoader {
+    static constexpr int Count = Rows * TileK / 4 / Threads;
+    Quad<In> quad[Count];
+    __device__ __forceinline__ void fetch(const In *base, int64_t row_stride, int64_t k_stride, int first_row, int rows, int k0, int k_end) {
+#pragma unroll
+        for (int c = 0; c < Count; ++c) {
+            const int i = threadIdx.x + c * Threads;
+            const bool k_major = k_stride == 1;
+            const int row = first_row + (k_major ? i / (TileK / 4) : i % (Rows / 4) * 4), k = k0 + (k_major ? i % (TileK / 4) * 4 : i / (Rows / 4));
+            quad[c] = {};
+            if (row < rows && k < k_end)
+                quad[c].v = *reinterpret_cast<const decltype(quad[c].v) *>(base + row * row_stride + k * k_stride);
+        }
+    }
+    __device__ __forceinline__ void put(float (*tile)[Rows + 4], int64_t k_stride) const {
+#pragma unroll
+        for (int c = 0; c < Count; ++c) {
+            const int i = threadIdx.x + c * Threads;
+            if (k_stride == 1) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    tile[i % (TileK / 4) * 4 + e][i / (TileK / 4)] = quad[c].at(e);
+            } else {
+                *reinterpret_cast<float4 *>(&tile[i / (Rows / 4)][i % (Rows / 4) * 4]) = make_float4(quad[c].at(0), quad[c].at(1), quad[c].at(2), quad[c].at(3));
+            }
+        }
+    }
+};
+template <class In, class Out, int TN>
+__global__ void __launch_bounds__(TN == 8 ? 256 : 128) gemm_simt_wide_kernel(GemmArgs g, float *partials, int slice_k) {
+    constexpr int Side = TN == 8 ? 128 : 64, Threads = TN == 8 ? 256 : 128;
+    __shared__ __align__(16) float as[2][TileK][Side + 4], bs[2][TileK][Side + 4];
+    const int z = partials ? 0 : blockIdx.z;
+    const In *a = (const In *)g.a + z * g.a_batch, *b = (const In *)g.b + z * g.b_batch;
+    const int m0 = blockIdx.y * Side, n0 = blockIdx.x * Side;
+    const int k_begin = partials ? blockIdx.z * slice_k : 0, k_end = partials ? min(g.k, k_begin + slice_k) : g.k;
+    // a warp covers 64 x 32 (TN = 8) or 64 x 16 outputs: 8 threads down, 4 across; a thread's rows and columns come in
+    // runs of four, 32 rows and 4 TN / 2 columns apart, so that its reads are whole 16-byte words without conflicts
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int row = (TN == 8 ? warp % 2 * 64 : 0) + lane / 4 * 4, column = (TN == 8 ? warp / 2 * 32 : warp * 16) + lane % 4 * 4;
+    float acc[8][TN] = {};
+    SliceLoader<In, Side, Threads> next_a, next_b;
+    next_a.fetch(a, g.a_row, g.a_col, m0, g.m, k_begin, k_end);
+    next_b.fetch(b, g.b_row, g.b_col, n0, g.n, k_begin, k_end);
+    next_a.put(as[0], g.a_col);
+    next_b.put(bs[0], g.b_col);
+    __syncthreads();
+    for (int k0 = k_begin, buffer = 0; k0 < k_end; k0 += TileK, buffer ^= 1) {
+        const bool more = k0 + TileK < k_end;
+        if (more) {
+            next_a.fetch(a, g.a_row, g.a_col, m0, g.m, k0 + TileK, k_end);
+            next_b.fetch(b, g.b_row, g.b_col, n0, g.n, k0 + TileK, k_end);
+        }
+#pragma unroll
+        for (int k = 0; k < TileK; ++k) {
+            float av[8], bv[TN];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float4 *>(av + 4 * h) = *reinterpret_cast<const float4 *>(&as[buffer][k][row + 32 * h]);
+#pragma unroll
+            for (int h = 0; h < TN / 4; ++h)
+                *reinterpret_cast<float4 *>(bv + 4 * h) = *reinterpret_cast<const float4 *>(&bs[buffer][k][column + 16 * h]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j)
+                    acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        if (more) {
+            next_a.put(as[buffer ^ 1], g.a_col);
+            next_b.put(bs[buffer ^ 1], g.b_col);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + row + i / 4 * 32 + i % 4;
+        if (m >= g.m)
+            break;
+#pragma unroll
+        for (int j = 0; j < TN; j += 4) {
+            const int n = n0 + column + j / 4 * 16;
+            if (n >= g.n)
+                continue;
+            if (partials) // n is a multiple of 4 here
+                *reinterpret_cast<float4 *>(partials + (int64_t(blockIdx.z) * g.m + m) * g.n + n) =
+                    make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    EpilogueOps<Out>::apply(g, acc[i][j + e], int64_t(m) * g.ldc + n + e, int64_t(m) * g.ldr + n + e, z);
+        }
+    }
+}
+
 // C = the K slices' partial tiles added in slice order (the same bits on every run).
 template <class Out> __global__ void gemm_simt_reduce_kernel(GemmArgs g, const float *partials, int slices) {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, count = int64_t(g.m) * g.n;
@@ -119,40 +234,71 @@ template <class Out> __global__ void gemm_simt_reduce_kernel(GemmArgs g, const f
     EpilogueOps<Out>::apply(g, sum, m * g.ldc + n, m * g.ldr + n, 0);
 }
 
-// A weight gradient of the reference architecture is a 16..96-wide output over tens of thousands of
-// tokens: one or two tiles that would each walk all of K alone.  Such shapes are cut along K.
-int gemm_simt_slices(const GemmArgs &g) {
-    const int64_t tiles = int64_t((g.n + TileN - 1) / TileN) * ((g.m + TileM - 1) / TileM);
-    if (g.batch != 1 || tiles > 32 || g.k < 2048)
-        return 1;
-    const int64_t wanted = (296 + tiles - 1) / tiles, longest = g.k / 64; // at least four 16-deep steps per slice
-    return int(wanted < longest ? wanted : longest);
+// What the vector loads need: unit stride in one dimension of each operand, the other stride, the extent along the unit
+// stride and the base a multiple of four elements; n a multiple of 4.  Below a 64-wide output most of a tile is padding.
+static bool wide_supported(const GemmArgs &g) {
+    const size_t bytes = 4 * dtype_size(g.in);
+    auto operand = [&](const void *p, int64_t row, int64_t col, int rows, int64_t batch) {
+        const bool k_major = col == 1;
+        return (k_major || row == 1) && (k_major ? row : col) % 4 == 0 && (k_major ? g.k : rows) % 4 == 0 && batch % 4 == 0 &&
+               reinterpret_cast<uintptr_t>(p) % bytes == 0;
+    };
+    return g.m >= 64 && g.n >= 64 && g.k >= 16 && g.n % 4 == 0 && operand(g.a, g.a_row, g.a_col, g.m, g.a_batch) &&
+           operand(g.b, g.b_row, g.b_col, g.n, g.b_batch);
+}
+struct SimtPlan {
+    bool wide = false, large = false; // gemm_simt_wide_kernel, with 128 x 128 tiles
+    int slices = 1;
+};
+// The smaller tile costs a quarter more shared-memory reads per product, the larger leaves SMs idle when there are fewer
+// than one per SM.  K is cut where the tiles would not give every SM two blocks (the partial tiles then cost one more pass
+// over the output each), in slices of at least 256 (wide) or 64.
+static SimtPlan simt_plan(const GemmArgs &g) {
+    auto tiles = [&](int side) { return int64_t((g.n + side - 1) / side) * ((g.m + side - 1) / side); };
+    SimtPlan plan;
+    plan.wide = wide_supported(g);
+    plan.large = plan.wide && tiles(128) * g.batch >= 148;
+    const int64_t count = tiles(plan.large ? 128 : 64);
+    if (g.batch != 1)
+        return plan;
+    if (plan.wide) {
+        if (!plan.large && g.k >= 512)
+            plan.slices = int(std::clamp<int64_t>(296 / count, 1, g.k / 256));
+    } else if (count <= 32 && g.k >= 2048) {
+        // A weight gradient of the reference architecture is a 16..96-wide output over tens of thousands of tokens: one or
+        // two tiles that would each walk all of K alone.
+        plan.slices = int(std::min<int64_t>((296 + count - 1) / count, g.k / 64)); // at least four 16-deep steps per slice
+    }
+    return plan;
 }
 size_t gemm_simt_scratch_bytes(const GemmArgs &g) {
-    const int slices = gemm_simt_slices(g);
+    const int slices = simt_plan(g).slices;
     return slices > 1 ? size_t(slices) * g.m * g.n * sizeof(float) : 0;
 }
 
-void launch_gemm_simt(const GemmArgs &g, cudaStream_t s, float *scratch) {
-    const int slices = scratch ? gemm_simt_slices(g) : 1;
+template <class In, class Out> static void launch_simt(const GemmArgs &g, const SimtPlan &plan, float *scratch, cudaStream_t s) {
+    const int slices = scratch ? plan.slices : 1, side = plan.large ? 128 : 64;
     float *partials = slices > 1 ? scratch : nullptr;
     const int slice_k = slices > 1 ? ((g.k + slices - 1) / slices + TileK - 1) / TileK * TileK : 0;
     const int used = slices > 1 ? (g.k + slice_k - 1) / slice_k : 1;
-    dim3 grid((g.n + TileN - 1) / TileN, (g.m + TileM - 1) / TileM, slices > 1 ? used : g.batch);
-    const unsigned reduce_blocks = unsigned((int64_t(g.m) * g.n + 255) / 256);
-    if (g.in == Dtype::BF16 && g.out == Dtype::BF16) {
-        gemm_simt_kernel<bf16, bf16><<<grid, 256, 0, s>>>(g, partials, slice_k);
-        if (partials)
-            gemm_simt_reduce_kernel<bf16><<<reduce_blocks, 256, 0, s>>>(g, partials, used);
-    } else if (g.in == Dtype::BF16 && g.out == Dtype::FP32) {
-        gemm_simt_kernel<bf16, float><<<grid, 256, 0, s>>>(g, partials, slice_k);
-        if (partials)
-            gemm_simt_reduce_kernel<float><<<reduce_blocks, 256, 0, s>>>(g, partials, used);
-    } else if (g.in == Dtype::FP32 && g.out == Dtype::FP32) {
-        gemm_simt_kernel<float, float><<<grid, 256, 0, s>>>(g, partials, slice_k);
-        if (partials)
-            gemm_simt_reduce_kernel<float><<<reduce_blocks, 256, 0, s>>>(g, partials, used);
-    } else {
+    const dim3 grid((g.n + side - 1) / side, (g.m + side - 1) / side, slices > 1 ? used : g.batch);
+    if (plan.large)
+        gemm_simt_wide_kernel<In, Out, 8><<<grid, 256, 0, s>>>(g, partials, slice_k);
+    else if (plan.wide)
+        gemm_simt_wide_kernel<In, Out, 4><<<grid, 128, 0, s>>>(g, partials, slice_k);
+    else
+        gemm_simt_kernel<In, Out><<<grid, 256, 0, s>>>(g, partials, slice_k);
+    if (partials)
+        gemm_simt_reduce_kernel<Out><<<unsigned((int64_t(g.m) * g.n + 255) / 256), 256, 0, s>>>(g, partials, used);
+}
+void launch_gemm_simt(const GemmArgs &g, cudaStream_t s, float *scratch) {
+    const SimtPlan plan = simt_plan(g);
+    if (g.in == Dtype::BF16 && g.out == Dtype::BF16)
+        launch_simt<bf16, bf16>(g, plan, scratch, s);
+    else if (g.in == Dtype::BF16 && g.out == Dtype::FP32)
+        launch_simt<bf16, float>(g, plan, scratch, s);
+    else if (g.in == Dtype::FP32 && g.out == Dtype::FP32)
+        launch_simt<float, float>(g, plan, scratch, s);
+    else
         throw std::runtime_error("GEMM: FP32 operands with BF16 output are not used");
-    }
 }
