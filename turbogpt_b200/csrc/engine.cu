@@ -106,7 +106,13 @@ void Engine::initialize() {
     lanes[0].stream = stream;
     // Profiling times kernels one at a time, and gradient buckets leave in the order the layers finish: both keep one lane.
     concurrent = !profile && c.world == 1 && tensor_cores;
-    for (int l = 1; l < LaneCount && concurrent; ++l)
+    // Above these sizes one product fills the GPU for several rounds of tiles and a second lane has nothing to fill; the step
+    // is then bound by power and the lanes cost what they add.  Measured per step, one lane -> two: 12 layers d 768, 4096
+    // tokens 4.85 -> 4.32 ms, 8192 7.27 -> 7.05, 16384 12.44 -> 12.2, 32768 no difference; 16 layers d 1024, 32768 tokens
+    // 71.2 -> 71.5 ms.  Muon families: 6 layers d 384 1.74 -> 1.58 ms; 12 layers d 768 and 16 layers d 1024 no difference.
+    side_lane = concurrent && int64_t(tokens) * c.width <= int64_t(1) << 24;
+    muon_lanes = concurrent && int64_t(c.base.depth) * c.width * c.width <= int64_t(1) << 22;
+    for (int l = 1; l < (muon_lanes ? LaneCount : side_lane ? 2 : 1); ++l)
         CHECK_CUDA(cudaStreamCreateWithFlags(&lanes[l].stream, cudaStreamNonBlocking));
 
     const int64_t P = layout.count;
@@ -158,22 +164,33 @@ void Engine::initialize() {
     bytes(final_normed, M * W);
     allocate(final_stats, M * 2, false);
     bytes(logits, M * Vocabulary);
-    for (void *&p : dhidden)
-        bytes(p, M * W);
+    // Without a side lane to wait for, the rings are no longer than the chain itself needs.
+    for (int i = 0; i < HiddenRing; ++i)
+        if (i < 2 || side_lane)
+            bytes(dhidden[i], M * W);
+        else
+            dhidden[i] = dhidden[i % 2];
     bytes(dbranch, M * W);
     for (int i = 0; i < LayerRing; ++i) {
-        bytes(dwide[i], M * wide);
-        bytes(dqkv[i], M * 3 * W);
+        if (i < 1 || side_lane) {
+            bytes(dwide[i], M * wide);
+            bytes(dqkv[i], M * 3 * W);
+        } else {
+            dwide[i] = dwide[0], dqkv[i] = dqkv[0];
+        }
     }
     bytes(dactivated, M * Hd);
     allocate(attention_scratch,
              std::max<size_t>(size_t(M) * c.heads, flash_attention_backward_scratch_bytes(c.base.batch, T, c.heads) / sizeof(float)),
              false);
-    for (int l = 0; l < (concurrent ? 2 : 1); ++l) // the lanes of the forward and backward pass
+    for (int l = 0; l < (side_lane ? 2 : 1); ++l) // the lanes of the forward and backward pass
         allocate(simt_scratch[l], SimtScratchBytes / sizeof(float), false);
     norm_blocks = norm_backward_blocks(tokens, sms);
-    for (float *&p : norm_partial)
-        allocate(p, size_t(norm_blocks) * 2 * W, false);
+    for (int i = 0; i < HiddenRing; ++i)
+        if (i < 1 || side_lane)
+            allocate(norm_partial[i], size_t(norm_blocks) * 2 * W, false);
+        else
+            norm_partial[i] = norm_partial[0];
     if (W <= 1024 && tokens >= 4096)
         allocate(embedding_partial, size_t(EmbeddingSlices) * Vocabulary * W, false);
     sumsq_blocks = sms * 8;
@@ -539,7 +556,7 @@ void Engine::backward() {
     const int wide = c.mlp == TG_MLP_SWIGLU ? 2 * Hd : Hd;
     // Nothing in backward waits for a weight gradient or for the sums of a norm's scale and bias gradients: they run on
     // a lane of their own beside the chain of input gradients.
-    const int side = concurrent ? 1 : 0;
+    const int side = side_lane ? 1 : 0;
     auto aside = [&] { // launches go to the side lane, after everything the main lane holds
         if (side)
             fork(0, side);
@@ -651,7 +668,8 @@ void Engine::backward() {
         ++launches; // slices kernel + sum kernel
     exchange_bucket(layout.embedding, layout.embedding + int64_t(Vocabulary) * W, depth + 1);
     finish_exchange();
-    fork(side, 0); // join
+    if (side)
+        fork(side, 0); // join
 }
 
 // ------------------------------------------------------------------------------- optimizer ---
@@ -722,10 +740,10 @@ void Engine::optimize() {
     AdamArgs a{gradient, momentum, variance, weight_high, weight_low, weight_fp32, adam_mode, sumsq_partial,
                sumsq_blocks, schedule, counters, c.base.learning_rate, c.base.beta1, c.base.beta2,
                c.base.weight_decay, c.base.epsilon, c.base.clip, layout.count};
-    const cudaEvent_t norm_ready = concurrent && !muon.empty() ? mark(0) : nullptr;
+    const cudaEvent_t norm_ready = muon_lanes && !muon.empty() ? mark(0) : nullptr;
     run(FOptimizer, [&](cudaStream_t s) { launch_adamw(a, sms, s); });
     // The families are independent chains of small products: each on a lane of its own.
-    const int chains = concurrent ? std::min(int(muon.size()), LaneCount - 1) : 0;
+    const int chains = muon_lanes ? std::min(int(muon.size()), LaneCount - 1) : 0;
     for (int l = 1; l <= chains; ++l)
         await(l, norm_ready);
     for (size_t f = 0; f < muon.size(); ++f) {

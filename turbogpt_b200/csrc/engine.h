@@ -135,7 +135,8 @@ struct Engine {
     int64_t launches = 0, graph_launches = 0;
     Lane lanes[LaneCount];
     int lane = 0;            // where run() launches
-    bool concurrent = false; // whether work is forked at all
+    bool concurrent = false; // whether work may be forked at all
+    bool side_lane = false, muon_lanes = false; // weight gradients beside the chain; the Muon families beside each other
     std::vector<cudaEvent_t> fork_events;
     size_t next_fork_event = 0;
     float *simt_scratch[2] = {nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
