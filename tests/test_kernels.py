@@ -200,3 +200,33 @@ def test_norms_match_torch(rows, width, kind):
         assert max_relative(dbias, bf.grad.numpy()) <= 1e-4
     for a, b in zip(*results):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("batch,context,heads", [(700, 1, 1), (304, 64, 2), (301, 65, 2), (160, 129, 2), (61, 333, 4)])
+def test_attention_with_four_blocks_per_sm(batch, context, heads):
+    """Grids large enough for the one-chain forward kernel, at sequence ends on and off its 64- and 128-row steps."""
+    test_attention_matches_torch(batch, context, heads, 64)
+
+
+@pytest.mark.parametrize("batch", [100, 2])  # 900 blocks of 128 queries: one chain per block; 18: two chains
+def test_attention_forward_when_the_row_maximum_keeps_growing(batch):
+    """Scores that climb by more than 2^8 from step to step: the output accumulator is rescaled between products."""
+    lib = load_library()
+    context, heads = 320, 3
+    g = torch.Generator(device="cuda").manual_seed(7)
+    qkv = torch.randn(batch * context, 3, heads, 64, generator=g, device="cuda")
+    climb = torch.linspace(0, 40, context, device="cuda").repeat(batch)
+    qkv[:, 0, :, 0], qkv[:, 1, :, 0] = 64.0, climb[:, None]  # score ~ 8 * climb: up to 320 above the first keys
+    qkv = qkv.bfloat16().reshape(batch * context, -1)
+    out = torch.empty(batch * context, heads * 64, device="cuda", dtype=torch.bfloat16)
+    lse = torch.empty(batch, heads, context, device="cuda")
+    assert lib.tg_ex_attention_forward(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), batch, context, heads, 64, 1,
+                                       None) == 0, lib.tg_error()
+    torch.cuda.synchronize()
+    q, k, v = qkv.reshape(batch, context, 3, heads, 64).permute(2, 0, 3, 1, 4).double()
+    scores = (q @ k.transpose(-1, -2) / 8).masked_fill(~torch.ones(context, context, dtype=torch.bool, device="cuda").tril(),
+                                                       float("-inf"))
+    expected = (torch.softmax(scores, -1) @ v).transpose(1, 2).reshape(batch * context, -1)
+    # FP32 scores of ~320 carry 2e-5, their exponentials as much; BF16 probabilities and outputs 2^-8 each
+    assert max_relative(out.double().cpu().numpy(), expected.cpu().numpy()) <= 1e-2
+    torch.testing.assert_close(lse.double(), torch.logsumexp(scores, -1), rtol=1e-5, atol=1e-4)

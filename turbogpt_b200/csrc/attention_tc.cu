@@ -41,6 +41,141 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// The steps first_step, first_step + Chains, ... of one online softmax: scores of 64 keys at tmem_s become probabilities
+// (packed over them) for the product that adds to the accumulator at tmem_o.  Returns the number of steps taken.
+template <int Chains>
+__device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile_first, int row, uint32_t tmem_s, uint32_t tmem_o,
+                                             uint32_t s_full, uint32_t p_full, const ForwardParams &p, volatile int *abort_flag,
+                                             float &reference_max, float &running_sum, bool &ok) {
+    const int lane = row % 32, warp_first = tile_first + row - lane, position = tile_first + row;
+    // Probabilities are taken relative to a reference maximum that is only moved (and the output
+    // rescaled) when the true maximum has grown by more than 2^8: values stay inside BF16/FP32 range
+    // and the final division by the row sum, accumulated with the same reference, makes the result exact.
+    int mine = 0; // steps this chain has taken
+    for (int j = first_step; j < steps; j += Chains, ++mine) {
+        ok = mbarrier_wait(s_full, mine & 1, abort_flag, p.counters, 206);
+        if (!ok)
+            break;
+        tcgen05_fence_after();
+        const int key0 = j * KeyStep;
+        const bool diagonal = key0 + KeyStep - 1 > warp_first; // some key of the step lies after some query of the warp
+        if (mine > 0 && !diagonal) {
+            // One pass: exponentials against the reference maximum this chain already has, the row
+            // maximum tracked on the side.  That is exact as long as no row's maximum has grown by
+            // more than 2^8; if one has, nothing has been written yet and the step is redone below.
+            const float offset = reference_max * p.scale_log2;
+            uint32_t packed[32];
+            float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, sum0, sum1;
+            const uint64_t scale2 = float_pair(p.scale_log2, p.scale_log2), offset2 = float_pair(-offset, -offset);
+            uint64_t sum = 0;
+#pragma unroll
+            for (int part = 0; part < 4; ++part) { // 16 keys at a time
+                uint32_t s[16];
+                tmem_load_32x16_async(tmem_s + part * 16, s);
+                tmem_wait_load(s);
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const float x0 = __uint_as_float(s[i]), x1 = __uint_as_float(s[i + 1]);
+                    if (i % 4) // a maximum of three is one instruction
+                        m1 = fmaxf(m1, fmaxf(x0, x1));
+                    else
+                        m0 = fmaxf(m0, fmaxf(x0, x1));
+                    float p0, p1;
+                    split_pair(fma_pair(float_pair(x0, x1), scale2, offset2), p0, p1);
+                    p0 = fast_exp2(p0), p1 = fast_exp2(p1);
+                    sum = add_pair(sum, float_pair(p0, p1));
+                    packed[part * 8 + i / 2] = pack_bf16(p0, p1);
+                }
+            }
+            split_pair(sum, sum0, sum1);
+            const bool fits = (fmaxf(m0, m1) - reference_max) * p.scale_log2 <= 8.f; // false for a -inf reference
+            if (__all_sync(0xffffffffu, fits)) {
+                tmem_store_32x32(tmem_s, packed);
+                tmem_wait_store();
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    mbarrier_arrive(p_full);
+                running_sum += sum0 + sum1;
+                continue;
+            }
+        }
+        float block_max = -CUDART_INF_F;
+        { // first pass over the scores: the row maximum, 32 keys at a time
+            float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t s[32];
+                tmem_load_32x32_async(tmem_s + half * 32, s);
+                tmem_wait_load(s);
+                if (diagonal) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (key0 + half * 32 + i > position)
+                            s[i] = 0xff800000u;
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    m0 = fmaxf(m0, __uint_as_float(s[i]));
+                    m1 = fmaxf(m1, __uint_as_float(s[i + 1]));
+                }
+            }
+            block_max = fmaxf(m0, m1);
+        }
+        const bool grow = (block_max - reference_max) * p.scale_log2 > 8.f; // true for the first unmasked step
+        if (__any_sync(0xffffffffu, grow && reference_max != -CUDART_INF_F)) {
+            // between this chain's products: the scores awaited above were issued after the last one
+            const float correction =
+                grow && reference_max != -CUDART_INF_F ? fast_exp2((reference_max - block_max) * p.scale_log2) : 1.f;
+            running_sum *= correction;
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) { // 32 columns at a time keeps the register count down
+                uint32_t a[32];
+                tmem_load_32x32_async(tmem_o + half * 32, a);
+                tmem_wait_load(a);
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    a[i] = __float_as_uint(__uint_as_float(a[i]) * correction);
+                tmem_store_32x32(tmem_o + half * 32, a);
+            }
+        }
+        if (grow)
+            reference_max = block_max;
+        // a row with nothing unmasked so far (it lies before every key this chain has seen) has
+        // reference_max = -inf: every probability below is exp2(-inf) = 0 with offset 0
+        const float offset = reference_max == -CUDART_INF_F ? 0.f : reference_max * p.scale_log2;
+        float sums[2] = {0.f, 0.f};
+#pragma unroll
+        for (int half = 0; half < 2; ++half) { // second pass: exponentials, 32 keys at a time
+            uint32_t s[32], packed[16];
+            tmem_load_32x32_async(tmem_s + half * 32, s);
+            tmem_wait_load(s);
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                float p0 = fast_exp2(fmaf(__uint_as_float(s[i]), p.scale_log2, -offset));
+                float p1 = fast_exp2(fmaf(__uint_as_float(s[i + 1]), p.scale_log2, -offset));
+                if (diagonal) {
+                    if (key0 + half * 32 + i > position) p0 = 0.f;
+                    if (key0 + half * 32 + i + 1 > position) p1 = 0.f;
+                }
+                sums[0] += p0;
+                sums[1] += p1;
+                packed[i / 2] = pack_bf16(p0, p1);
+            }
+            // the packed half lands on score columns 16 half .. 16 half + 15, which both passes have
+            // finished with (half 1 is read from columns 32 .. 63 before this store is issued)
+            tmem_store_32x16(tmem_s + half * 16, packed);
+        }
+        tmem_wait_store();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0)
+            mbarrier_arrive(p_full);
+        running_sum += sums[0] + sums[1];
+    }
+    return mine;
+}
+
 __global__ void __launch_bounds__(ForwardThreads, 2)
 flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                      ForwardParams p) {
@@ -157,135 +292,12 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const int quarter = warp % 4, chain = (warp - 2) / 4;
         const int row = quarter * 32 + lane;              // query row inside the tile = TMEM lane
         const int position = tile * BlockM + row;          // position inside the sequence
-        const int warp_first = tile * BlockM + quarter * 32;
         const uint32_t lanes = uint32_t(quarter * 32) << 16;
         const uint32_t tmem_s = tmem_s0 + 64 * chain + lanes, tmem_o = tmem_o0 + 64 * chain + lanes;
-        // Probabilities are taken relative to a reference maximum that is only moved (and the output
-        // rescaled) when the true maximum has grown by more than 2^8: values stay inside BF16/FP32 range
-        // and the final division by the row sum, accumulated with the same reference, makes the result exact.
         float reference_max = -CUDART_INF_F, running_sum = 0.f;
         bool ok = true;
-        int mine = 0; // steps this chain has taken
-        for (int j = chain; j < steps; j += 2, ++mine) {
-            ok = mbarrier_wait(s_full0 + 8 * chain, mine & 1, abort_flag, p.counters, 206);
-            if (!ok)
-                break;
-            tcgen05_fence_after();
-            const int key0 = j * KeyStep;
-            const bool diagonal = key0 + KeyStep - 1 > warp_first; // some key of the step lies after some query of the warp
-            if (mine > 0 && !diagonal) {
-                // One pass: exponentials against the reference maximum this chain already has, the row
-                // maximum tracked on the side.  That is exact as long as no row's maximum has grown by
-                // more than 2^8; if one has, nothing has been written yet and the step is redone below.
-                const float offset = reference_max * p.scale_log2;
-                uint32_t packed[32];
-                float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-                for (int part = 0; part < 4; ++part) { // 16 keys at a time
-                    uint32_t s[16];
-                    tmem_load_32x16_async(tmem_s + part * 16, s);
-                    tmem_wait_load(s);
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        const float x0 = __uint_as_float(s[i]), x1 = __uint_as_float(s[i + 1]);
-                        m0 = fmaxf(m0, x0);
-                        m1 = fmaxf(m1, x1);
-                        const float p0 = fast_exp2(fmaf(x0, p.scale_log2, -offset));
-                        const float p1 = fast_exp2(fmaf(x1, p.scale_log2, -offset));
-                        sum0 += p0;
-                        sum1 += p1;
-                        packed[part * 8 + i / 2] = pack_bf16(p0, p1);
-                    }
-                }
-                const bool fits = (fmaxf(m0, m1) - reference_max) * p.scale_log2 <= 8.f; // false for a -inf reference
-                if (__all_sync(0xffffffffu, fits)) {
-                    tmem_store_32x32(tmem_s, packed);
-                    tmem_wait_store();
-                    tcgen05_fence_before();
-                    __syncwarp();
-                    if (lane == 0)
-                        mbarrier_arrive(p_full0 + 8 * chain);
-                    running_sum += sum0 + sum1;
-                    continue;
-                }
-            }
-            float block_max = -CUDART_INF_F;
-            { // first pass over the scores: the row maximum, 32 keys at a time
-                float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F;
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t s[32];
-                    tmem_load_32x32_async(tmem_s + half * 32, s);
-                    tmem_wait_load(s);
-                    if (diagonal) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (key0 + half * 32 + i > position)
-                                s[i] = 0xff800000u;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        m0 = fmaxf(m0, __uint_as_float(s[i]));
-                        m1 = fmaxf(m1, __uint_as_float(s[i + 1]));
-                    }
-                }
-                block_max = fmaxf(m0, m1);
-            }
-            const bool grow = (block_max - reference_max) * p.scale_log2 > 8.f; // true for the first unmasked step
-            if (__any_sync(0xffffffffu, grow && reference_max != -CUDART_INF_F)) {
-                // the accumulator is rescaled only between this chain's products: wait for the last one
-                ok = mbarrier_wait(o_full0 + 8 * chain, (mine - 1) & 1, abort_flag, p.counters, 207);
-                if (!ok)
-                    break;
-                tcgen05_fence_after();
-                const float correction =
-                    grow && reference_max != -CUDART_INF_F ? fast_exp2((reference_max - block_max) * p.scale_log2) : 1.f;
-                running_sum *= correction;
-#pragma unroll 1
-                for (int half = 0; half < 2; ++half) { // 32 columns at a time keeps the register count down
-                    uint32_t a[32];
-                    tmem_load_32x32_async(tmem_o + half * 32, a);
-                    tmem_wait_load(a);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        a[i] = __float_as_uint(__uint_as_float(a[i]) * correction);
-                    tmem_store_32x32(tmem_o + half * 32, a);
-                }
-            }
-            if (grow)
-                reference_max = block_max;
-            // a row with nothing unmasked so far (it lies before every key this chain has seen) has
-            // reference_max = -inf: every probability below is exp2(-inf) = 0 with offset 0
-            const float offset = reference_max == -CUDART_INF_F ? 0.f : reference_max * p.scale_log2;
-            float sums[2] = {0.f, 0.f};
-#pragma unroll
-            for (int half = 0; half < 2; ++half) { // second pass: exponentials, 32 keys at a time
-                uint32_t s[32], packed[16];
-                tmem_load_32x32_async(tmem_s + half * 32, s);
-                tmem_wait_load(s);
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float p0 = fast_exp2(fmaf(__uint_as_float(s[i]), p.scale_log2, -offset));
-                    float p1 = fast_exp2(fmaf(__uint_as_float(s[i + 1]), p.scale_log2, -offset));
-                    if (diagonal) {
-                        if (key0 + half * 32 + i > position) p0 = 0.f;
-                        if (key0 + half * 32 + i + 1 > position) p1 = 0.f;
-                    }
-                    sums[0] += p0;
-                    sums[1] += p1;
-                    packed[i / 2] = pack_bf16(p0, p1);
-                }
-                // the packed half lands on score columns 16 half .. 16 half + 15, which both passes have
-                // finished with (half 1 is read from columns 32 .. 63 before this store is issued)
-                tmem_store_32x16(tmem_s + half * 16, packed);
-            }
-            tmem_wait_store();
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0)
-                mbarrier_arrive(p_full0 + 8 * chain);
-            running_sum += sums[0] + sums[1];
-        }
+        const int mine = softmax_chain<2>(chain, steps, tile * BlockM, row, tmem_s, tmem_o, s_full0 + 8 * chain,
+                                          p_full0 + 8 * chain, p, abort_flag, reference_max, running_sum, ok);
         if (ok && mine > 0)
             ok = mbarrier_wait(o_full0 + 8 * chain, (mine - 1) & 1, abort_flag, p.counters, 208);
         // merge the two chains: each publishes its reference maximum and sum, then takes half of the
@@ -346,6 +358,156 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         tmem_dealloc(tmem_base, ForwardTmemColumns);
 }
 
+// A warp's 32 accumulator rows x 32 columns from tensor memory, scaled, to BF16 in global memory (whole
+// warp; `staging`: 2 KB of shared memory the warp may use; `first_row`: global address of row 0's first column).
+__device__ __forceinline__ void store_accumulator(uint32_t address, uint32_t staging, bf16 *first_row, int64_t row_elements,
+                                                  int valid_rows, float factor, int lane) {
+    uint32_t a[32], packed[16];
+    tmem_load_32x32_async(address, a);
+    tmem_wait_load(a);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        packed[i] = pack_bf16(__uint_as_float(a[2 * i]) * factor, __uint_as_float(a[2 * i + 1]) * factor);
+    store_rows_through_shared(staging, packed, first_row, row_elements * 2, valid_rows, lane);
+}
+
+// One chain per CTA: four softmax warps, and one thread that issues loads and products alike.  128 TMEM columns (64 scores,
+// 64 outputs) and 50 KB of shared memory, so four CTAs share an SM: as many chains in flight as two CTAs of two chains, but a
+// CTA's start (barriers, TMEM, first tiles) and end (stores) hide behind three others instead of one, and a chain's first
+// step, which takes two passes over its scores, comes once per CTA.  What bounds it is the latency of a step's chain:
+// about 1.5 x the time of the exponential unit (64 us at 226 M probabilities) at context 1024.
+constexpr int SingleThreads = 160, SingleTmemColumns = 128;
+constexpr int SingleShared = TileBytes + 2 * 2 * KeyBytes + 1024 + 128; // Q, two slots of K and of V, barriers
+
+__global__ void __launch_bounds__(SingleThreads, 4)
+flash_forward_single_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
+                            ForwardParams p) {
+    extern __shared__ uint8_t raw_shared[];
+    const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
+    uint8_t *aligned = raw_shared + (base - smem_address(raw_shared));
+    uint64_t *barriers = reinterpret_cast<uint64_t *>(aligned + TileBytes + 4 * KeyBytes);
+    const uint32_t q_full = smem_address(barriers), k_full0 = q_full + 8, v_full0 = k_full0 + 16, s_full = v_full0 + 16,
+                   p_full = s_full + 8, o_full = p_full + 8; // 8 barriers
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 8);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const uint32_t smem_q = base, smem_k = base + TileBytes, smem_v = smem_k + 2 * KeyBytes;
+
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int pairs = p.batch * p.heads;
+    const int tile = p.tiles - 1 - int(blockIdx.x / pairs); // long tiles first
+    const int bh = blockIdx.x % pairs, b = bh / p.heads, h = bh % p.heads;
+    const int row0 = b * p.context;
+    const int last_key = min(p.context, (tile + 1) * BlockM);
+    const int steps = (last_key + KeyStep - 1) / KeyStep;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 8; ++i)
+            mbarrier_init(q_full + 8 * i, q_full + 8 * i == p_full ? 4 : 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 4) {
+        if (lane == 0) {
+            prefetch_map(&map_q);
+            prefetch_map(&map_kv);
+        }
+        __syncwarp();
+        tmem_alloc(smem_address(tmem_slot), SingleTmemColumns);
+        tmem_relinquish();
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    grid_launch_dependents(); // the next kernel may set itself up while this one runs; this one holds its tensor memory
+    const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + 64;
+
+    if (warp == 4) {
+        if (elect_one()) {
+            const uint32_t idesc_s = instruction_descriptor(BlockM, KeyStep, 0, 0);
+            const uint32_t idesc_o = instruction_descriptor(BlockM, HeadSize, 0, 1);
+            const uint64_t q_desc = smem_descriptor(smem_q, 16, 1024), k_desc0 = smem_descriptor(smem_k, 16, 1024),
+                           v_desc0 = smem_descriptor(smem_v, 8192, 1024);
+            auto load = [&](int j, int which) { // K (which = 1) or V (which = 2) of step j
+                const uint32_t bar = (which == 1 ? k_full0 : v_full0) + 8 * (j & 1);
+                mbarrier_expect_tx(bar, KeyBytes);
+                tma_load_3d((which == 1 ? smem_k : smem_v) + (j & 1) * KeyBytes, &map_kv, which * p.width + h * HeadSize,
+                            row0 + j * KeyStep, 0, bar);
+            };
+            bool ok = true;
+            auto issue_scores = [&](int j) { // S = Q K_j^T
+                ok = mbarrier_wait(k_full0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, p.counters, 203);
+                if (!ok)
+                    return;
+                tcgen05_fence_after();
+                const uint64_t k_desc = descriptor_at(k_desc0, (j & 1) * KeyBytes);
+#pragma unroll
+                for (int ks = 0; ks < HeadSize / 16; ++ks)
+                    tcgen05_mma_bf16(tmem_s, descriptor_at(q_desc, ks * 32), descriptor_at(k_desc, ks * 32), idesc_s, ks > 0);
+                tcgen05_commit(s_full);
+            };
+            mbarrier_expect_tx(q_full, TileBytes);
+            tma_load_3d(smem_q, &map_q, h * HeadSize, row0 + tile * BlockM, 0, q_full);
+            load(0, 1);
+            if (steps > 1)
+                load(1, 1);
+            load(0, 2);
+            ok = mbarrier_wait(q_full, 0, abort_flag, p.counters, 202);
+            if (ok)
+                issue_scores(0);
+            for (int j = 0; j < steps && ok; ++j) {
+                ok = mbarrier_wait(p_full, j & 1, abort_flag, p.counters, 204) &&
+                     mbarrier_wait(v_full0 + 8 * (j & 1), (j >> 1) & 1, abort_flag, p.counters, 205);
+                if (!ok)
+                    break;
+                tcgen05_fence_after();
+                const uint64_t v_desc = descriptor_at(v_desc0, (j & 1) * KeyBytes);
+#pragma unroll
+                for (int ks = 0; ks < KeyStep / 16; ++ks) // O += P V_j: four 16-key steps
+                    tcgen05_mma_bf16_ts(tmem_o, tmem_s + ks * 8, descriptor_at(v_desc, ks * 2048), idesc_o,
+                                        (j > 0 || ks > 0) ? 1u : 0u);
+                if (j + 1 < steps)
+                    issue_scores(j + 1); // over the probabilities the products above have read
+                // P_j exists, so S_j and the products issued before it (those with V_{j-1}) are complete: their slots are free
+                if (j + 2 < steps)
+                    load(j + 2, 1);
+                if (j + 1 < steps)
+                    load(j + 1, 2);
+            }
+            if (ok)
+                tcgen05_commit(o_full);
+        }
+    } else {
+        const int row = warp * 32 + lane, position = tile * BlockM + row;
+        const uint32_t lanes = uint32_t(warp * 32) << 16;
+        float reference_max = -CUDART_INF_F, running_sum = 0.f;
+        bool ok = true;
+        softmax_chain<1>(0, steps, tile * BlockM, row, tmem_s + lanes, tmem_o + lanes, s_full, p_full, p, abort_flag,
+                         reference_max, running_sum, ok);
+        if (ok)
+            ok = mbarrier_wait(o_full, 0, abort_flag, p.counters, 208);
+        if (__all_sync(0xffffffffu, ok && *abort_flag == 0)) { // the warp stores together or not at all
+            tcgen05_fence_after();
+            // through the Q tile, which no product reads any more: 2 KB per warp
+            const int first = tile * BlockM + warp * 32;
+            bf16 *out = p.out + (int64_t(row0) + first) * p.width + h * HeadSize;
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+                store_accumulator(tmem_o + lanes + half * 32, smem_q + warp * 2048, out + half * 32, p.width, p.context - first,
+                                  1.f / running_sum, lane);
+            if (position < p.context) // natural-log sum-exp of the scaled scores
+                p.lse[(int64_t(b) * p.heads + h) * p.context + position] =
+                    (reference_max * p.scale_log2 + log2f(running_sum)) * 0.6931471805599453f;
+        }
+    }
+    __syncthreads();
+    if (*abort_flag)
+        __nanosleep(2000000);
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 4)
+        tmem_dealloc(tmem_s, SingleTmemColumns);
+}
+
 // ------------------------------------------------------------------------------------------
 // Backward.  Two kernels, both deterministic (no atomics):
 //   dq kernel    : one CTA per 128 query rows, stepping over keys 64 at a time.  S = Q K^T and
@@ -396,19 +558,6 @@ __device__ __forceinline__ uint32_t score_gradient(uint32_t p0, uint32_t p1, uin
                         add_pair(float_pair(__uint_as_float(dp0), __uint_as_float(dp1)), minus_delta)),
                d0, d1);
     return pack_bf16(d0, d1);
-}
-
-// A warp's 32 accumulator rows x 32 columns from tensor memory, scaled, to BF16 in global memory (whole
-// warp; `staging`: 2 KB of shared memory the warp may use; `first_row`: global address of row 0's first column).
-__device__ __forceinline__ void store_accumulator(uint32_t address, uint32_t staging, bf16 *first_row, int64_t row_elements,
-                                                  int valid_rows, float factor, int lane) {
-    uint32_t a[32], packed[16];
-    tmem_load_32x32_async(address, a);
-    tmem_wait_load(a);
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-        packed[i] = pack_bf16(__uint_as_float(a[2 * i]) * factor, __uint_as_float(a[2 * i + 1]) * factor);
-    store_rows_through_shared(staging, packed, first_row, row_elements * 2, valid_rows, lane);
 }
 
 // dq kernel.  64 keys per step.  S = Q K^T is double-buffered in tensor memory and issued two steps
@@ -905,6 +1054,8 @@ void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int 
     if (device < 64 && !configured[device]) {
         CHECK_CUDA(cudaFuncSetAttribute(flash_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         ForwardShared));
+        CHECK_CUDA(cudaFuncSetAttribute(flash_forward_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        SingleShared));
         configured[device] = true;
     }
     const int width = heads * HeadSize;
@@ -917,7 +1068,15 @@ void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int 
     const uint64_t rows = uint64_t(batch) * context;
     CUtensorMap map_q = make_map_bf16(qkv, uint64_t(3) * width, rows, 1, uint64_t(3) * width, 0, HeadSize, BlockM);
     CUtensorMap map_kv = make_map_bf16(qkv, uint64_t(3) * width, rows, 1, uint64_t(3) * width, 0, HeadSize, KeyStep);
-    flash_forward_kernel<<<batch * heads * p.tiles, ForwardThreads, ForwardShared, s>>>(map_q, map_kv, p);
+    // The one-chain kernel needs CTAs enough to fill four places on every SM several times over: a CTA takes twice as long
+    // there, so with few CTAs the longest one decides.  Measured, two chains -> one, at (batch x heads, context): (768, 256)
+    // 41 -> 33 us, (384, 1024) 119 -> 107, (144, 1024) 47.5 -> 43.3, (128, 2048) 128 -> 123, (64, 4096) equal; but
+    // (64, 2048) 65.5 -> 69, (96, 512) 13.5 -> 17 and (32, 4096) 105 -> 120.
+    const int grid = batch * heads * p.tiles, sms = 148;
+    if (grid >= (p.tiles <= 4 ? 3 : 7) * sms)
+        flash_forward_single_kernel<<<grid, SingleThreads, SingleShared, s>>>(map_q, map_kv, p);
+    else
+        flash_forward_kernel<<<grid, ForwardThreads, ForwardShared, s>>>(map_q, map_kv, p);
     CHECK_CUDA(cudaGetLastError());
 }
 
