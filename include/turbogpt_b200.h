@@ -221,8 +221,8 @@ int tg_ex_attention_backward(const void *qkv, const void *out, const void *dout,
  * [rows, width] (cuda/ops.cuh:56-66).  Scale and bias are FP32 values passed as the engine stores
  * them: the high 16 bits as BF16 (`*_high`) and the low 16 bits (`*_low`, uint16) in separate arrays;
  * bias pointers are ignored for RMSNorm.  `stats` (optional, [rows][2] floats) receives every row's
- * mean and 1/sqrt(variance + eps) for the backward pass; it is written for widths 256, 512, 768 and
- * 1024 (the register-resident kernels) and left untouched otherwise. */
+ * mean and 1/sqrt(variance + eps) for the backward pass; it is written for widths from 128 to 1024
+ * (the register-resident kernels) and left untouched otherwise. */
 int tg_ex_norm_forward(int kind, const void *x, const void *scale_high, const void *scale_low, const void *bias_high,
                        const void *bias_low, void *y, float *stats, int rows, int width, void *stream);
 /* Its backward (cuda/ops.cuh:67-80): dx = norm'(dy) rounded to BF16, plus residual_in when not NULL

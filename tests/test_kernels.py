@@ -230,3 +230,11 @@ def test_attention_forward_when_the_row_maximum_keeps_growing(batch):
     # FP32 scores of ~320 carry 2e-5, their exponentials as much; BF16 probabilities and outputs 2^-8 each
     assert max_relative(out.double().cpu().numpy(), expected.cpu().numpy()) <= 1e-2
     torch.testing.assert_close(lse.double(), torch.logsumexp(scores, -1), rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("rows,width", [(37, 128), (515, 136), (300, 248), (129, 264), (2331, 384), (700, 520),
+                                        (260, 1000), (9, 1016)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_norms_at_widths_off_the_register_tile(rows, width, kind):
+    """Widths that fill the last 256 columns of a row partly: same checks, same bounds."""
+    test_norms_match_torch(rows, width, kind)

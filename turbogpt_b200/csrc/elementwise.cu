@@ -256,8 +256,9 @@ __device__ __forceinline__ void unpack8(const Packet<float> &r, float (&v)[8]) {
     v[0] = r.a.x, v[1] = r.a.y, v[2] = r.a.z, v[3] = r.a.w, v[4] = r.b.x, v[5] = r.b.y, v[6] = r.b.z, v[7] = r.b.w;
 }
 
-// Widths of 256..1024 in steps of 256: the row lives in registers (one 128-bit load per 256
-// columns and lane), so x is read once; scale and bias are read once per block into shared memory.
+// Widths up to 1024: the row lives in registers (one 128-bit load per 256 columns and lane), so x is read once; scale
+// and bias are read once per block into shared memory.  Ragged (a width that is no multiple of 256): some lanes have no
+// columns in the last 256; the row's moments take two passes there, as in the kernel for other widths.
 //
 // Per-lane vectors of 8 floats in shared memory are stored as two float4 planes,
 // [v][half][lane][4]: consecutive lanes then touch consecutive 16-byte words and a warp-wide access
@@ -289,8 +290,9 @@ __device__ __forceinline__ void warp_sum2(float &a, float &b) {
 // passes like the FP32 model they are compared with; BF16 rows take one pass over values shifted by
 // the row's first element (exact for the shift, immune to a large common offset), whose two sums
 // share one warp reduction: the row's dependent chain is one shuffle plus one reduction.
-template <class T, int V> __device__ __forceinline__ void row_moments(int kind, const float (&x)[V][8], int width,
-                                                                       float &mean, float &inv) {
+// `tail`: the lane has columns in the last 256 (it holds zeros there otherwise).
+template <class T, int V, bool Ragged>
+__device__ __forceinline__ void row_moments(int kind, const float (&x)[V][8], int width, bool tail, float &mean, float &inv) {
     float sums[4] = {0, 0, 0, 0}, squares[4] = {0, 0, 0, 0};
     if (kind == TG_NORM_RMS) {
 #pragma unroll
@@ -302,7 +304,7 @@ template <class T, int V> __device__ __forceinline__ void row_moments(int kind, 
         inv = rsqrtf(warp_sum((squares[0] + squares[1]) + (squares[2] + squares[3])) / width + 1e-6f);
         return;
     }
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (sizeof(T) == 4 || Ragged) {
 #pragma unroll
         for (int v = 0; v < V; ++v)
 #pragma unroll
@@ -313,7 +315,8 @@ template <class T, int V> __device__ __forceinline__ void row_moments(int kind, 
         for (int v = 0; v < V; ++v)
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                squares[j % 4] += (x[v][j] - mean) * (x[v][j] - mean);
+                if (!Ragged || v + 1 < V || tail)
+                    squares[j % 4] += (x[v][j] - mean) * (x[v][j] - mean);
         inv = rsqrtf(warp_sum((squares[0] + squares[1]) + (squares[2] + squares[3])) / width + 1e-5f);
     } else {
         const float shift = __shfl_sync(0xffffffffu, x[0][0], 0);
@@ -332,22 +335,29 @@ template <class T, int V> __device__ __forceinline__ void row_moments(int kind, 
         inv = rsqrtf(fmaxf(s2 / width - offset * offset, 0.f) + 1e-5f);
     }
 }
-template <class T, int V> __global__ void __launch_bounds__(256, 4) norm_rows_kernel(NormArgs a) {
+template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 4) norm_rows_kernel(NormArgs a) {
     sm100::grid_launch_dependents(); // the next kernel may set itself up while this one runs
     __shared__ __align__(16) float sw[V * 256], sb[V * 256]; // FP32 scale and bias in the plane layout
     const int lane = threadIdx.x % 32, warps = blockDim.x / 32;
-    for (int c = threadIdx.x; c < V * 256; c += blockDim.x) {
+    for (int c = threadIdx.x; c < (Ragged ? a.width : V * 256); c += blockDim.x) {
         sw[plane_of_column(c)] = join_weight(a.scale_high[c], a.scale_low[c]);
         sb[plane_of_column(c)] = a.kind == TG_NORM_LAYER ? join_weight(a.bias_high[c], a.bias_low[c]) : 0.f;
     }
     __syncthreads();
     const int stride = gridDim.x * warps;
     int row = blockIdx.x * warps + threadIdx.x / 32;
+    const bool tail = !Ragged || ((V - 1) * 32 + lane) * 8 < a.width;
     Packet<T> next[V]; // the warp's next row, fetched while the current one is normalised
-    if (row < a.rows)
+    if (Ragged)
+        next[V - 1] = Packet<T>{}; // stays zero in the lanes without a tail
+    auto fetch = [&](int r) {
 #pragma unroll
         for (int k = 0; k < V; ++k)
-            fetch8((const T *)a.x + int64_t(row) * a.width + (k * 32 + lane) * 8, next[k]);
+            if (k + 1 < V || tail)
+                fetch8((const T *)a.x + int64_t(r) * a.width + (k * 32 + lane) * 8, next[k]);
+    };
+    if (row < a.rows)
+        fetch(row);
     for (; row < a.rows; row += stride) {
         T *y = (T *)a.y + int64_t(row) * a.width;
         float v[V][8];
@@ -355,11 +365,9 @@ template <class T, int V> __global__ void __launch_bounds__(256, 4) norm_rows_ke
         for (int k = 0; k < V; ++k)
             unpack8(next[k], v[k]);
         if (row + stride < a.rows)
-#pragma unroll
-            for (int k = 0; k < V; ++k)
-                fetch8((const T *)a.x + int64_t(row + stride) * a.width + (k * 32 + lane) * 8, next[k]);
+            fetch(row + stride);
         float mean, inv;
-        row_moments<T, V>(a.kind, v, a.width, mean, inv);
+        row_moments<T, V, Ragged>(a.kind, v, a.width, tail, mean, inv);
         if (a.stats && lane == 0)
             reinterpret_cast<float2 *>(a.stats)[row] = make_float2(mean, inv); // kept for the backward pass
 #pragma unroll
@@ -370,22 +378,33 @@ template <class T, int V> __global__ void __launch_bounds__(256, 4) norm_rows_ke
 #pragma unroll
             for (int j = 0; j < 8; ++j)
                 out[j] = a.kind == TG_NORM_RMS ? v[k][j] * inv * w[j] : (v[k][j] - mean) * inv * w[j] + b[j];
-            store8(y + (k * 32 + lane) * 8, out);
+            if (k + 1 < V || tail)
+                store8(y + (k * 32 + lane) * 8, out);
         }
     }
 }
-template <class T> static void launch_norm_rows(const NormArgs &a, cudaStream_t s) {
+// Rows in registers: up to 1024 columns, full multiples of 256 or not (the kernel for other widths reads x three times and
+// its per-warp sums with eight-way bank conflicts: a step of 8 layers, d 640, 4096 tokens took 3.02 ms, 2.44 with rows in
+// registers; 6 layers, d 384, 2331 tokens 1.59 and 1.49).  Below 128 most lanes would hold none, and the rows of the 16-wide reference
+// architecture keep the order of additions that its checks were made with.
+static bool rows_in_registers(int width) { return width >= 128 && width <= 1024 && width % 8 == 0; }
+template <class T, int V> static void launch_norm_rows(const NormArgs &a, cudaStream_t s) {
     const int blocks = blocks_for(a.rows, 8, 148 * 4);
-    switch (a.width / 256) {
-    case 1: norm_rows_kernel<T, 1><<<blocks, 256, 0, s>>>(a); break;
-    case 2: norm_rows_kernel<T, 2><<<blocks, 256, 0, s>>>(a); break;
-    case 3: norm_rows_kernel<T, 3><<<blocks, 256, 0, s>>>(a); break;
-    default: norm_rows_kernel<T, 4><<<blocks, 256, 0, s>>>(a); break;
-    }
+    if (a.width % 256)
+        norm_rows_kernel<T, V, true><<<blocks, 256, 0, s>>>(a);
+    else
+        norm_rows_kernel<T, V, false><<<blocks, 256, 0, s>>>(a);
 }
 void launch_norm(Dtype t, const NormArgs &a, cudaStream_t s) {
-    if (a.width % 256 == 0 && a.width <= 1024) {
-        DISPATCH(t, launch_norm_rows<T>(a, s));
+    if (rows_in_registers(a.width)) {
+        DISPATCH(t, {
+            switch ((a.width + 255) / 256) {
+            case 1: launch_norm_rows<T, 1>(a, s); break;
+            case 2: launch_norm_rows<T, 2>(a, s); break;
+            case 3: launch_norm_rows<T, 3>(a, s); break;
+            default: launch_norm_rows<T, 4>(a, s); break;
+            }
+        });
         return;
     }
     DISPATCH(t, (norm_kernel<T><<<blocks_for(a.rows, 8), 256, 0, s>>>(a)));
@@ -477,25 +496,28 @@ __global__ void __launch_bounds__(256) norm_backward_reduce_kernel(const float *
             dbias[c - width] = total;
     }
 }
-// Register-resident variant for widths 256..1024: x, dy and the residual gradient are read once, and
+// Register-resident variant for widths up to 1024: x, dy and the residual gradient are read once, and
 // a warp fetches its next row while it works on the current one.  The row's mean and 1/sigma come
 // from the forward pass when it saved them (`stats`), so the only reduction a row waits for is the
 // pair sum(dz), sum(dz z).  Each warp keeps the scale/bias gradient sums of its rows in its own slice
 // of shared memory (plane layout: a lane owns its words, no conflicts, no atomics); warps are summed
 // in order at the end, blocks in order by the reduce kernel: deterministic.
-template <class T, int V> __global__ void __launch_bounds__(256, 2) norm_backward_rows_kernel(NormBackwardArgs a) {
+template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 2) norm_backward_rows_kernel(NormBackwardArgs a) {
     sm100::grid_launch_dependents(); // the next kernel may set itself up while this one runs
     extern __shared__ float sums[]; // [V * 256] scale, then [warps][2][V * 256] gradient sums, all in the plane layout
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32, warps = blockDim.x / 32;
     float *scale = sums, *mine = sums + V * 256 + warp * 2 * V * 256;
     for (int c = threadIdx.x; c < V * 256; c += blockDim.x)
-        scale[plane_of_column(c)] = join_weight(a.scale_high[c], a.scale_low[c]);
+        scale[plane_of_column(c)] = !Ragged || c < a.width ? join_weight(a.scale_high[c], a.scale_low[c]) : 0.f;
     for (int c = lane; c < 2 * V * 256; c += 32)
         mine[c] = 0.f;
     __syncthreads();
     const bool residual = a.residual_in != nullptr, saved = a.stats != nullptr;
     const int stride = gridDim.x * warps;
+    const bool tail = !Ragged || ((V - 1) * 32 + lane) * 8 < a.width;
     Packet<T> nx[V], ng[V], nr[V];
+    if (Ragged)
+        nx[V - 1] = ng[V - 1] = nr[V - 1] = Packet<T>{}; // stay zero in the lanes without a tail
     float2 nstat = make_float2(0.f, 1.f);
     auto fetch = [&](int row) {
         const int64_t offset = int64_t(row) * a.width;
@@ -503,6 +525,8 @@ template <class T, int V> __global__ void __launch_bounds__(256, 2) norm_backwar
             nstat = reinterpret_cast<const float2 *>(a.stats)[row];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
+            if (v + 1 == V && !tail)
+                continue;
             fetch8((const T *)a.x + offset + (v * 32 + lane) * 8, nx[v]);
             fetch8((const T *)a.dy + offset + (v * 32 + lane) * 8, ng[v]);
             if (residual)
@@ -526,7 +550,7 @@ template <class T, int V> __global__ void __launch_bounds__(256, 2) norm_backwar
         if (row + stride < a.rows)
             fetch(row + stride); // in flight during this row's arithmetic
         if (!saved)
-            row_moments<T, V>(a.kind, x, a.width, mean, inv);
+            row_moments<T, V, Ragged>(a.kind, x, a.width, tail, mean, inv);
         float part_dz[4] = {0, 0, 0, 0}, part_dzz[4] = {0, 0, 0, 0};
 #pragma unroll
         for (int v = 0; v < V; ++v) {
@@ -565,7 +589,8 @@ template <class T, int V> __global__ void __launch_bounds__(256, 2) norm_backwar
                 for (int j = 0; j < 8; ++j)
                     out[j] = res[j] + rounded<T>(out[j]);
             }
-            store8((T *)a.dx + offset + (v * 32 + lane) * 8, out);
+            if (v + 1 < V || tail)
+                store8((T *)a.dx + offset + (v * 32 + lane) * 8, out);
         }
     }
     __syncthreads();
@@ -577,31 +602,32 @@ template <class T, int V> __global__ void __launch_bounds__(256, 2) norm_backwar
         a.partial[int64_t(blockIdx.x) * 2 * a.width + c] = total;
     }
 }
-template <class T, int V> static void launch_norm_backward_rows(const NormBackwardArgs &a, cudaStream_t s) {
-    const size_t shared = size_t(V * 256 + 8 * 2 * a.width) * sizeof(float);
+template <class T, int V, bool Ragged> static void launch_norm_backward_rows(const NormBackwardArgs &a, cudaStream_t s) {
+    const size_t shared = size_t(V * 256 + 8 * 2 * V * 256) * sizeof(float);
     static std::atomic<unsigned long long> configured{0}; // one bit per device; engines on other devices run on other threads
     int device = 0;
     CHECK_CUDA(cudaGetDevice(&device));
     if (shared > 48 * 1024 && (device >= 64 || !(configured.load() >> device & 1))) {
-        CHECK_CUDA(cudaFuncSetAttribute(norm_backward_rows_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CHECK_CUDA(cudaFuncSetAttribute(norm_backward_rows_kernel<T, V, Ragged>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(shared)));
         if (device < 64)
             configured.fetch_or(1ull << device);
     }
-    norm_backward_rows_kernel<T, V><<<a.blocks, 256, shared, s>>>(a);
+    norm_backward_rows_kernel<T, V, Ragged><<<a.blocks, 256, shared, s>>>(a);
 }
 int norm_backward_blocks(int rows, int sms) {
     return blocks_for(rows, 8, int64_t(sms) * 2);
 }
 void launch_norm_backward(Dtype t, const NormBackwardArgs &a, cudaStream_t s) {
     size_t shared = size_t(2) * a.width * sizeof(float);
-    if (a.width % 256 == 0 && a.width <= 1024) {
+    if (rows_in_registers(a.width)) {
         DISPATCH(t, {
-            switch (a.width / 256) {
-            case 1: launch_norm_backward_rows<T, 1>(a, s); break;
-            case 2: launch_norm_backward_rows<T, 2>(a, s); break;
-            case 3: launch_norm_backward_rows<T, 3>(a, s); break;
-            default: launch_norm_backward_rows<T, 4>(a, s); break;
+            const bool ragged = a.width % 256;
+            switch ((a.width + 255) / 256) {
+            case 1: ragged ? launch_norm_backward_rows<T, 1, true>(a, s) : launch_norm_backward_rows<T, 1, false>(a, s); break;
+            case 2: ragged ? launch_norm_backward_rows<T, 2, true>(a, s) : launch_norm_backward_rows<T, 2, false>(a, s); break;
+            case 3: ragged ? launch_norm_backward_rows<T, 3, true>(a, s) : launch_norm_backward_rows<T, 3, false>(a, s); break;
+            default: ragged ? launch_norm_backward_rows<T, 4, true>(a, s) : launch_norm_backward_rows<T, 4, false>(a, s); break;
             }
         });
         return;
