@@ -191,7 +191,7 @@ void Engine::initialize() {
             allocate(norm_partial[i], size_t(norm_blocks) * 2 * W, false);
         else
             norm_partial[i] = norm_partial[0];
-    if (W <= 1024 && tokens >= 4096)
+    if (embedding_backward_sliced(tokens, W))
         allocate(embedding_partial, size_t(EmbeddingSlices) * Vocabulary * W, false);
     sumsq_blocks = sms * 8;
     allocate(sumsq_partial, sumsq_blocks);

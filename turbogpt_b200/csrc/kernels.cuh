@@ -33,6 +33,7 @@ void launch_embedding(Dtype t, const void *table, const uint8_t *x, void *hidden
 // one CTA per byte value scans the tokens in order.
 // `scratch`: EmbeddingSlices x 256 x width floats (nullptr: single-pass kernel for small shapes).
 constexpr int EmbeddingSlices = 8;
+bool embedding_backward_sliced(int tokens, int width); // whether it needs `scratch`
 void launch_embedding_backward(Dtype t, const void *dhidden, const uint8_t *x, float *grad, int tokens,
                                int width, bool accumulate, float *scratch, cudaStream_t s);
 
