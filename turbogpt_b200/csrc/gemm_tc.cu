@@ -650,6 +650,10 @@ struct Schedule {
 // block: the MMA takes bn/2, the shared-memory operand reads (128+bn)/4; a tile adds a fixed drain
 // cost and every split one pass over the FP32 partial tile.  CTA pairs (256-row tiles) are tried
 // first: they halve the B bytes each SM stages per K block.
+// SplitCost: writing partial tiles, the fence, the ticket and reading them back (or a second launch) take 4 to 5 us however
+// small the tiles: 2048 x 256 x 1024 took 12.2 us with K cut in two, 8.5 us uncut; 1024 of these units are about 2 us. Steps: 6 layers d 384, 2331
+// tokens 1.46 -> 1.32 ms, 8 layers d 640, 4096 tokens 2.44 -> 2.33, 12 layers d 768, 4096 tokens 4.31 -> 4.14.
+constexpr int SplitCost = 1000;
 Schedule choose_schedule(const GemmArgs &g, int sms) {
     const bool b_mn = g.b_col != 1;
     const bool second_tensor = g.epilogue != Epilogue::Store; // K is split only for plain stores
@@ -681,7 +685,7 @@ Schedule choose_schedule(const GemmArgs &g, int sms) {
                 if (splits > 1 && (k_blocks + per - 1) / per != splits)
                     continue; // would leave an empty split
                 const long long rounds = (tiles * splits + slots - 1) / slots;
-                const long long time = rounds * ((long long)per * block_cost + bn + (splits > 1 ? splits * bn / 2 : 0));
+                const long long time = rounds * ((long long)per * block_cost + bn + (splits > 1 ? splits * bn / 2 + SplitCost : 0));
                 if (!best.bn || time < best_time)
                     best.bn = bn, best.splits = splits, best.k_blocks_per_split = per, best.pair = unit == 2,
                     best_time = time;
