@@ -646,14 +646,15 @@ struct Schedule {
     int bn = 0, splits = 1, k_blocks_per_split = 0, pair = 0;
 };
 
-// Tile width, K splits and single CTA / CTA pair by a small cost model, in clocks per 64-deep K
+// Tile width, K splits and single CTA / CTA pair by a small cost model, in clocks per 16 of a 64-deep K
 // block: the MMA takes bn/2, the shared-memory operand reads (128+bn)/4; a tile adds a fixed drain
 // cost and every split one pass over the FP32 partial tile.  CTA pairs (256-row tiles) are tried
 // first: they halve the B bytes each SM stages per K block.
-// SplitCost: writing partial tiles, the fence, the ticket and reading them back (or a second launch) take 4 to 5 us however
-// small the tiles: 2048 x 256 x 1024 took 12.2 us with K cut in two, 8.5 us uncut; 1024 of these units are about 2 us. Steps: 6 layers d 384, 2331
-// tokens 1.46 -> 1.32 ms, 8 layers d 640, 4096 tokens 2.44 -> 2.33, 12 layers d 768, 4096 tokens 4.31 -> 4.14.
-constexpr int SplitCost = 1000;
+// SplitCost, in the model's units (four clocks each: 2000 are about 4.3 us): writing partial tiles, the fence, the
+// ticket and reading them back, or a second launch, take 4 to 5 us however small the tiles: 2048 x 256 x 1024 took 12.2 us
+// with K cut in two, 8.5 us uncut.  Steps without the cost, with 1000, 2000 and 4000: 4 layers d 256, 2048 tokens 508, 494,
+// 455, 454 us; 6 layers d 384, 2331 tokens 1.46, 1.32, 1.22, 1.21 ms; 8 layers d 640, 4096 tokens 2.44, 2.33, 2.28, 2.25 ms.
+constexpr int SplitCost = 2000;
 Schedule choose_schedule(const GemmArgs &g, int sms) {
     const bool b_mn = g.b_col != 1;
     const bool second_tensor = g.epilogue != Epilogue::Store; // K is split only for plain stores
