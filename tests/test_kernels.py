@@ -54,6 +54,26 @@ def test_tensor_core_gemm_matches_fp32_product(a_mn, b_mn, m, n, k):
         assert max_relative(simt, expected) <= tolerance
 
 
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("m,n,k", [(129, 72, 72), (4100, 264, 72), (4100, 520, 72), (4100, 776, 72),  # single blocks, tiles 64 to 256 wide
+                                   (4100, 520, 3080), (4100, 776, 3080), (16400, 136, 3080),          # many rounds over a long K: pairs
+                                   (129, 72, 3080), (129, 2056, 3080)])                               # K cut in six, in four
+def test_products_of_every_tile_form_at_their_edges(m, n, k, b_mn):
+    """One shape for each choice of the schedule, with partial tiles in every dimension, against 64 bits: FP32 sums of k exact
+    products, then one BF16 rounding."""
+    lib = load_library()
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, b = (torch.randn(rows, k, generator=g, device="cuda").bfloat16() for rows in (m, n))
+    stored = b.T.contiguous() if b_mn else b
+    c = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+    assert lib.tg_ex_gemm(a.data_ptr(), k, 1, stored.data_ptr(), *((1, n) if b_mn else (k, 1)), c.data_ptr(), n, m, n, k, 0, 1, None) == 0, \
+        lib.tg_error()
+    torch.cuda.synchronize()
+    expected, magnitude = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+    assert ((c.double() - expected).abs() <= k * 2.0 ** -24 * magnitude + 2.0 ** -8 * expected.abs()).all()
+    assert lib.tg_ex_last_device_error(None) == 0
+
+
 def test_split_k_weight_gradient_is_deterministic():
     lib = load_library()
     a, sa, b, sb, expected = operands(768, 768, 16384, True, True, seed=3)

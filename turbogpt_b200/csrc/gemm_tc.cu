@@ -646,7 +646,60 @@ struct Schedule {
     int bn = 0, splits = 1, k_blocks_per_split = 0, pair = 0;
 };
 
-// Tile width, K splits and single CTA / CTA pair by a small cost model, in clocks per 16 of a 64-deep K
+// What a schedule costs, in nanoseconds: launch + rounds of tiles x (64-deep K blocks x block + tile).  Fitted to 832 products
+// of 256 to 32768 tokens and widths 128 to 1024 (activations and input gradients, K-major and MN-major B), each timed with every
+// tile width, single and paired; the model reproduces the times within 5 to 8 % and its choice is 0.3 % slower than the best of
+// each (geometric mean).  A pair's launch costs 0.9 us more and its tiles take longer to hand over, single CTAs read more
+// operand bytes per product: pairs are for many rounds over a long K.  The model before it (MMA and shared-memory clocks, no
+// launch or tile times) chose 8 % slower on average: 4096 x 768 x 2304 17.4 -> 13.9 us, 8192 x 2048 x 512 25.1 -> 18.5,
+// 1024 x 2304 x 768 7.5 -> 6.4, 32768 x 512 x 128 21.9 -> 13.5.  The tile's shape does not change a result: every element
+// adds its products in ascending k.
+struct TileCost {
+    int bn, block, tile;
+};
+constexpr TileCost SingleCost[] = {{256, 342, 1500}, {192, 262, 1280}, {128, 209, 940}, {64, 184, 550}};
+constexpr TileCost PairCost[] = {{256, 284, 2100}, {192, 211, 1900}, {128, 188, 1450}};
+constexpr int SingleLaunch = 3240, PairLaunch = 4100;
+// A K split of n: partial tiles, fence, ticket and read-back by one SM, or from four on a second launch, and the partial tiles'
+// passes through memory.
+constexpr long long split_cost(int splits, int bn, long long outputs) {
+    return splits == 1 ? 0 : 4500 + (splits < 4 ? 20 * bn : 0) + splits * outputs / 1000;
+}
+Schedule product_schedule(const GemmArgs &g, int sms) {
+    const bool b_mn = g.b_col != 1;
+    const bool plain = g.epilogue == Epilogue::Store; // K is split only for plain stores
+    const bool whole_rows = g.epilogue == Epilogue::CrossEntropy; // a tile must hold complete rows
+    const int m_tiles = (g.m + BM - 1) / BM, k_blocks = (g.k + BK - 1) / BK;
+    Schedule best;
+    long long best_time = 0;
+    auto consider = [&](const TileCost &cost, int unit, int launch) {
+        const int bn = cost.bn, slots = sms / unit;
+        if ((bn > 64 && bn - 64 >= g.n) || (whole_rows && bn != 256))
+            return; // a narrower tile already covers N
+        if (unit == 2 && b_mn && bn == 192)
+            return; // each CTA stages bn/2 rows of B: whole 64-row blocks when B is MN-major
+        const long long tiles = (long long)((m_tiles + unit - 1) / unit) * ((g.n + bn - 1) / bn) * g.batch;
+        for (int splits : {1, 2, 3, 4, 6, 8, 12, 16}) {
+            const int per = (k_blocks + splits - 1) / splits;
+            if (splits > 1 && (!plain || k_blocks / splits < 8 || tiles * splits > slots || (k_blocks + per - 1) / per != splits))
+                continue; // the last: would leave an empty split
+            const long long rounds = (tiles * splits + slots - 1) / slots;
+            const long long time = launch + rounds * ((long long)per * cost.block + cost.tile) + split_cost(splits, bn, (long long)g.m * g.n * g.batch);
+            if (!best.bn || time < best_time)
+                best.bn = bn, best.splits = splits, best.k_blocks_per_split = per, best.pair = unit == 2, best_time = time;
+        }
+    };
+    if (m_tiles >= 2 && sms >= 2)
+        for (const TileCost &cost : PairCost)
+            consider(cost, 2, PairLaunch);
+    for (const TileCost &cost : SingleCost)
+        consider(cost, 1, SingleLaunch);
+    return best;
+}
+
+// Weight gradients: FP32 outputs over a long K.  Their schedules were measured in steps rather than alone, where they run beside
+// the chain of input gradients: fewer blocks of longer life leave the chain more of the GPU.
+// Tile width, K splits and single CTA / CTA pair by a cost model in clocks per 16 of a 64-deep K
 // block: the MMA takes bn/2, the shared-memory operand reads (128+bn)/4; a tile adds a fixed drain
 // cost and every split one pass over the FP32 partial tile.  CTA pairs (256-row tiles) are tried
 // first: they halve the B bytes each SM stages per K block.
@@ -660,10 +713,8 @@ struct Schedule {
 // and cut, of 964 shapes the three that this decides: dW 3072 x 768 over 16384 tokens 65.5 and 63.5 us, 768 x 3072 74.1
 // and 70.5, 2560 x 640 61.2 and 57.5; at 12000 tokens whole is faster (49.0 and 50.7) and stays, at 32768 the cut by itself.
 constexpr int SplitCost = 2000, CutWeight = 48, WholeWeight = 49;
-Schedule choose_schedule(const GemmArgs &g, int sms) {
+Schedule weight_gradient_schedule(const GemmArgs &g, int sms) {
     const bool b_mn = g.b_col != 1;
-    const bool second_tensor = g.epilogue != Epilogue::Store; // K is split only for plain stores
-    const bool whole_rows = g.epilogue == Epilogue::CrossEntropy; // a tile must hold complete rows
     const int m_tiles = (g.m + BM - 1) / BM, k_blocks = (g.k + BK - 1) / BK;
     Schedule best;
     long long best_time = 0;
@@ -675,8 +726,6 @@ Schedule choose_schedule(const GemmArgs &g, int sms) {
         for (int bn : {256, 192, 128, 64}) {
             if (bn > 64 && bn - 64 >= g.n)
                 continue; // a narrower tile already covers N
-            if (whole_rows && bn != 256)
-                continue;
             if (unit == 2 && (bn == 64 || (b_mn && bn == 192)))
                 continue; // each CTA stages bn/2 rows of B: whole 64-row blocks when B is MN-major
             const long long tiles = m_units * ((g.n + bn - 1) / bn) * g.batch;
@@ -685,7 +734,7 @@ Schedule choose_schedule(const GemmArgs &g, int sms) {
             const int mma = bn / 2 > (128 + bn) / 4 ? bn / 2 : (128 + bn) / 4;
             const int block_cost = unit == 2 ? mma + 16 : mma * (k_blocks >= 64 ? 9 : 11) / 8 + 16;
             for (int splits : {1, 2, 3, 4, 6, 8, 12, 16}) {
-                if (splits > 1 && (k_blocks / splits < 8 || tiles * splits > slots || second_tensor))
+                if (splits > 1 && (k_blocks / splits < 8 || tiles * splits > slots))
                     continue;
                 const int per = (k_blocks + splits - 1) / splits;
                 if (splits > 1 && (k_blocks + per - 1) / per != splits)
@@ -700,6 +749,9 @@ Schedule choose_schedule(const GemmArgs &g, int sms) {
         }
     }
     return best;
+}
+Schedule choose_schedule(const GemmArgs &g, int sms) {
+    return g.out == Dtype::FP32 && g.epilogue == Epilogue::Store ? weight_gradient_schedule(g, sms) : product_schedule(g, sms);
 }
 
 // Scratch a schedule needs: FP32 partial tiles and one ticket per output tile (none without a K split).
