@@ -387,6 +387,34 @@ def test_graph_replay_is_bit_identical_to_direct_launches():
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("depth,width,batch,context,tied", [
+    (5, 256, 8, 256, 1),   # lanes; pieces of one layer each
+    (9, 128, 2, 333, 0),   # pieces of several layers, the first layers left for the last copy; a head of its own
+    (2, 1024, 5, 4096, 1), # no lanes (20480 x 1024 above 2^24)
+    (2, 128, 2, 128, 1)])  # nothing is worth a piece
+def test_batch_results_leave_early_and_are_those_of_this_call(depth, width, batch, context, tied):
+    """tg_batch copies logits and finished layers' gradients out while the replayed sequence goes on: with other inputs, and
+    other weights, in every call, nothing of the call before may be copied.  Launched directly in one lane, bit for bit."""
+    rng = np.random.default_rng(depth)
+    inputs = rng.integers(0, 256, (6, 2, batch, context), dtype=np.uint8)
+    results = []
+    for flags in (0, bridge.FLAG_NO_GRAPH | bridge.FLAG_PROFILE):
+        ex = ConfigEx.gpt(Config(depth=depth, context=context, batch=batch), width, width // 64, flags=flags)
+        ex.tied = tied
+        with Native(ex) as engine:
+            w = rng.standard_normal(engine.count).astype(np.float32) * .05 if not results else w
+            outputs = []
+            for i, (x, y) in enumerate(inputs):
+                if i in (0, 4):
+                    engine.set_weights(w * (1 + i))
+                outputs += engine.batch(x, y)
+                if i == 2:
+                    outputs += [engine.batch(x, y, backward=False)[0], engine.predict(x[0])]
+            results.append(outputs)
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_predict_runs_one_sequence_and_matches_the_batched_forward():
     """tg_predict covers one sequence (the reference replicates the context over the batch and reads
     the first copy); its logits are those of the batched forward on the replicated context."""
