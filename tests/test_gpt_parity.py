@@ -195,6 +195,32 @@ def test_cuda_core_products_and_attention_at_tile_edges_fp32(depth, width, heads
     np.testing.assert_allclose(losses, expected_losses, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("width,heads,context,batch", [
+    (64, 1, 65, 1),    # K of four slices, one for each group of threads; a second row of tiles with one row
+    (128, 2, 37, 5),   # eight slices
+    (320, 5, 64, 2),   # twenty
+    (512, 8, 200, 4)]) # K cut over blocks in the second product of the MLP
+def test_fp32_products_against_64_bits(width, heads, context, batch):
+    """The FP32 engine's own activations, through its projections in 64 bits: sums of K products, each rounded once."""
+    arch, model, w, x, y = fixture(1, width, heads, context, batch, True)
+    ex = ConfigEx.gpt(Config(depth=1, context=context, batch=batch, clip=0), width, heads, precision=bridge.PRECISION_FP32)
+    layout = bridge.parameter_layout(ex)
+
+    def matrix(rows, cols):
+        offset = next(o for o, r, c in layout[1:] if (r, c) == (rows, cols))
+        return w[offset:offset + rows * cols].reshape(rows, cols).astype(np.float64)
+
+    with Native(ex) as engine:
+        engine.set_weights(w)
+        engine.batch(x, y)
+        read = lambda name, layer=0: engine.activation(layer, name).reshape(batch * context, -1).astype(np.float64)
+        normed, qkv, middle, activated = read("normed1"), read("qkv"), read("middle"), read("activated")
+        final = read("final_x", -1)
+    for left, weights, added, got in ((normed, matrix(3 * width, width), 0., qkv), (activated, matrix(width, 4 * width), middle, final)):
+        bound = 2.0 ** -24 * (weights.shape[1] * (np.abs(left) @ np.abs(weights).T) + 2 * np.abs(got))
+        assert (np.abs(left @ weights.T + added - got) <= bound).all()
+
+
 def lanes_against_one(depth, width, batch, context, optimizer, precision=bridge.PRECISION_BF16):
     heads = width // 64
     data = np.random.default_rng(5).integers(0, 256, 1 << 15, dtype=np.uint8)

@@ -3,10 +3,12 @@
 // (the reference architecture's 16/48-wide matrices), the FP32 check mode, and is the on-device
 // cross-check of the tcgen05 kernel.  Two kernels: gemm_simt_kernel takes any strides, sizes and
 // alignments (64x64 output tile, 16-deep shared-memory slices, 4x4 outputs per thread, scalar loads);
-// gemm_simt_wide_kernel takes what its vector loads can reach and every shape of a real model (see there).
+// gemm_simt_wide_kernel (BF16 operands) and gemm_fp32_kernel (FP32) take what 16-byte pieces can reach and every shape of
+// a real model (see there).
 #include "device_utils.cuh"
 #include "kernels.cuh"
 #include <algorithm>
+#include <type_traits>
 
 constexpr int TileM = 64, TileN = 64, TileK = 16;
 
@@ -113,7 +115,6 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs g, float *parti
 // stay out of their way: 8 x TN outputs per thread (12 or 16 shared-memory words per 32 or 64 multiply-adds), operands
 // as 128-bit loads that are issued a slice ahead and land in the other of two shared-memory buffers, one barrier a slice.
 // TN = 8: 128 x 128 tiles, 256 threads; TN = 4: 64 x 64 tiles, 128 threads, for outputs of too few large tiles.
-// FP32, 2048 x 1024 x 256: 97 -> 46 us (23 TFLOP/s).
 template <class T> struct Quad;
 template <> struct Quad<float> {
     float4 v;
@@ -222,6 +223,140 @@ __global__ void __launch_bounds__(TN == 8 ? 256 : 128) gemm_simt_wide_kernel(Gem
     }
 }
 
+// FP32 operands of the same alignment.  128 multiply-adds per clock and SM bound it; next come the operand reads from shared
+// memory: they return 128 bytes per clock, so 8 x 4 outputs per thread (12 words for 32 multiply-adds) leave a third of the
+// multiply-add rate unused, 8 x 8 (16 for 64) just none.  64 x 64 tiles of 64 threads are two warps, too few to hide their own
+// latencies on an SM that holds one to four tiles, so FP32Groups groups of 64 threads each take every fourth slice of K, with
+// buffers and a barrier of their own, and their sums are added through shared memory in group order.
+// Against the kernel for BF16 operands, which took these before: the 51 products of 4 layers d 256 over 2048 tokens 2230 -> 1720 us
+// (that evaluation 2.52 -> 2.37 ms), 6 layers d 512 over 4096 tokens 19.9 -> 16.3 ms; eight groups in one block per SM instead of two
+// blocks of four measured 5 % slower.  Sums are shorter too: gradients 1.7 to 2.3e-7 from 64 bits instead of 3.0 to 4.6e-7.
+// Slices come by cp.async as they lie in memory: [row][k] where K is the unit stride (read as pairs of k), else [k][row].
+constexpr int FP32Side = 64, FP32Groups = 4, FP32Stages = 2, FP32PitchK = TileK + 4, FP32PitchRow = FP32Side + 4;
+constexpr int FP32Slice = FP32Side * FP32PitchK; // floats of one operand's slice; the [k][row] form needs less
+constexpr int FP32Shared = FP32Groups * FP32Stages * 2 * FP32Slice * int(sizeof(float));
+static_assert(TileK * FP32PitchRow <= FP32Slice && FP32Groups * FP32Side * FP32PitchRow * int(sizeof(float)) <= FP32Shared, "");
+
+// Outside the operand nothing is read; the address given is then its first one.
+__device__ __forceinline__ void copy16_or_zeros(float *to, const float *from, const float *operand, bool inside) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(to))), "l"(inside ? from : operand), "r"(inside ? 16 : 0)
+                 : "memory");
+}
+// The 16-byte pieces of an operand's slices that one of 64 threads copies: four a slice, sixteen rows (K-major) or four k apart.
+template <bool KMajor> struct SliceCopier {
+    static constexpr int Pieces = FP32Side * TileK / 4 / 64;
+    const float *operand, *source; // the operand; the first piece of the next slice
+    int64_t apart, advance;
+    int row, k, rows_left, shared_at; // of the first piece
+    __device__ __forceinline__ SliceCopier(const float *base, int64_t row_stride, int64_t k_stride, int first_row, int rows, int first_k, int thread)
+        : operand(base) {
+        row = KMajor ? thread / (TileK / 4) : thread % (FP32Side / 4) * 4;
+        const int in_slice = KMajor ? thread % (TileK / 4) * 4 : thread / (FP32Side / 4);
+        k = first_k + in_slice, rows_left = rows - first_row - row;
+        source = base + (first_row + row) * row_stride + k * k_stride;
+        apart = KMajor ? 16 * row_stride : 4 * k_stride;
+        advance = TileK * FP32Groups * k_stride;
+        shared_at = KMajor ? row * FP32PitchK + in_slice : in_slice * FP32PitchRow + row;
+    }
+    __device__ __forceinline__ void copy(float *slice, int k_end) {
+        const float *from = source;
+#pragma unroll
+        for (int c = 0; c < Pieces; ++c, from += apart)
+            copy16_or_zeros(slice + shared_at + c * (KMajor ? 16 * FP32PitchK : 4 * FP32PitchRow), from, operand,
+                            KMajor ? 16 * c < rows_left && k < k_end : rows_left > 0 && k + 4 * c < k_end);
+        source += advance, k += TileK * FP32Groups;
+    }
+};
+// A thread's eight rows (or columns) of a tile, by its place 0..7: as the reads want them, without bank conflicts.
+template <bool KMajor> __device__ __forceinline__ int fp32_row(int place, int i) {
+    return KMajor ? place + 8 * i : i / 4 * 32 + place * 4 + i % 4;
+}
+template <bool KMajor> __device__ __forceinline__ void read_pair(const float *slice, int place, int k, float (&v)[2][8]) { // k and k + 1
+    if constexpr (KMajor) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 u = *reinterpret_cast<const float2 *>(slice + fp32_row<true>(place, i) * FP32PitchK + k);
+            v[0][i] = u.x, v[1][i] = u.y;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float4 *>(v[e] + 4 * h) = *reinterpret_cast<const float4 *>(slice + (k + e) * FP32PitchRow + h * 32 + place * 4);
+    }
+}
+template <bool AK, bool BK>
+__global__ void __launch_bounds__(64 * FP32Groups, 2) gemm_fp32_kernel(GemmArgs g, float *partials, int slice_k) {
+    extern __shared__ __align__(16) float shared[];
+    const int z = partials ? 0 : blockIdx.z;
+    const float *a = (const float *)g.a + z * g.a_batch, *b = (const float *)g.b + z * g.b_batch;
+    const int m0 = blockIdx.y * FP32Side, n0 = blockIdx.x * FP32Side;
+    const int k_begin = partials ? blockIdx.z * slice_k : 0, k_end = partials ? min(g.k, k_begin + slice_k) : g.k;
+    const int group = threadIdx.x / 64, thread = threadIdx.x % 64;
+    const int down = thread % 32 / 4, across = thread / 32 * 4 + thread % 4; // 8 x 8 threads, a warp 8 x 4
+    float *buffers = shared + group * FP32Stages * 2 * FP32Slice;
+    const int slices = (k_end - k_begin + TileK - 1) / TileK;
+    SliceCopier<AK> copy_a(a, g.a_row, g.a_col, m0, g.m, k_begin + group * TileK, thread);
+    SliceCopier<BK> copy_b(b, g.b_row, g.b_col, n0, g.n, k_begin + group * TileK, thread);
+    auto fetch = [&](int stage) { // the group's next slice
+        float *to = buffers + stage * 2 * FP32Slice;
+        copy_a.copy(to, k_end);
+        copy_b.copy(to + FP32Slice, k_end);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[8][8] = {};
+    if (group < slices)
+        fetch(0);
+    for (int s = group, stage = 0; s < slices; s += FP32Groups, stage ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + group) : "memory"); // the slice has landed, and the other stage has been read
+        if (s + FP32Groups < slices)
+            fetch(stage ^ 1);
+        const float *as = buffers + stage * 2 * FP32Slice, *bs = as + FP32Slice;
+#pragma unroll
+        for (int k = 0; k < TileK; k += 2) {
+            float av[2][8], bv[2][8];
+            read_pair<AK>(as, down, k, av);
+            read_pair<BK>(bs, across, k, bv);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        acc[i][j] = fmaf(av[e][i], bv[e][j], acc[i][j]);
+        }
+    }
+    __syncthreads(); // every group's buffers have been read: they now take the sums
+    float *sums = shared + group * FP32Side * FP32PitchRow;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            sums[fp32_row<AK>(down, i) * FP32PitchRow + fp32_row<BK>(across, j)] = acc[i][j];
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < FP32Side * FP32Side / 4 / (64 * FP32Groups); ++c) {
+        const int i = threadIdx.x + c * 64 * FP32Groups, row = i / (FP32Side / 4), column = i % (FP32Side / 4) * 4;
+        const int m = m0 + row, n = n0 + column;
+        if (m >= g.m || n >= g.n) // n is a multiple of 4 here
+            continue;
+        float v[4] = {};
+#pragma unroll
+        for (int k = 0; k < FP32Groups; ++k) {
+            const float4 u = *reinterpret_cast<const float4 *>(shared + (k * FP32Side + row) * FP32PitchRow + column);
+            v[0] += u.x, v[1] += u.y, v[2] += u.z, v[3] += u.w;
+        }
+        if (partials)
+            *reinterpret_cast<float4 *>(partials + (int64_t(blockIdx.z) * g.m + m) * g.n + n) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                EpilogueOps<float>::apply(g, v[e], int64_t(m) * g.ldc + n + e, int64_t(m) * g.ldr + n + e, z);
+    }
+}
+
 // C = the K slices' partial tiles added in slice order (the same bits on every run).
 template <class Out> __global__ void gemm_simt_reduce_kernel(GemmArgs g, const float *partials, int slices) {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, count = int64_t(g.m) * g.n;
@@ -250,14 +385,14 @@ struct SimtPlan {
     bool wide = false, large = false; // gemm_simt_wide_kernel, with 128 x 128 tiles
     int slices = 1;
 };
-// The smaller tile costs a quarter more shared-memory reads per product, the larger leaves SMs idle when there are fewer
+// BF16: the smaller tile costs a quarter more shared-memory reads per product, the larger leaves SMs idle when there are fewer
 // than one per SM.  K is cut where the tiles would not give every SM two blocks (the partial tiles then cost one more pass
 // over the output each), in slices of at least 256 (wide) or 64.
 static SimtPlan simt_plan(const GemmArgs &g) {
     auto tiles = [&](int side) { return int64_t((g.n + side - 1) / side) * ((g.m + side - 1) / side); };
     SimtPlan plan;
     plan.wide = wide_supported(g);
-    plan.large = plan.wide && tiles(128) * g.batch >= 148;
+    plan.large = plan.wide && g.in == Dtype::BF16 && tiles(128) * g.batch >= 148;
     const int64_t count = tiles(plan.large ? 128 : 64);
     if (g.batch != 1)
         return plan;
@@ -276,18 +411,31 @@ size_t gemm_simt_scratch_bytes(const GemmArgs &g) {
     return slices > 1 ? size_t(slices) * g.m * g.n * sizeof(float) : 0;
 }
 
+static void launch_fp32(const GemmArgs &g, dim3 grid, float *partials, int slice_k, cudaStream_t s) {
+    auto launch = [&](auto kernel) {
+        CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FP32Shared));
+        kernel<<<grid, 64 * FP32Groups, FP32Shared, s>>>(g, partials, slice_k);
+    };
+    const bool ak = g.a_col == 1, bk = g.b_col == 1;
+    if (ak)
+        bk ? launch(gemm_fp32_kernel<true, true>) : launch(gemm_fp32_kernel<true, false>);
+    else
+        bk ? launch(gemm_fp32_kernel<false, true>) : launch(gemm_fp32_kernel<false, false>);
+}
 template <class In, class Out> static void launch_simt(const GemmArgs &g, const SimtPlan &plan, float *scratch, cudaStream_t s) {
     const int slices = scratch ? plan.slices : 1, side = plan.large ? 128 : 64;
     float *partials = slices > 1 ? scratch : nullptr;
     const int slice_k = slices > 1 ? ((g.k + slices - 1) / slices + TileK - 1) / TileK * TileK : 0;
     const int used = slices > 1 ? (g.k + slice_k - 1) / slice_k : 1;
     const dim3 grid((g.n + side - 1) / side, (g.m + side - 1) / side, slices > 1 ? used : g.batch);
-    if (plan.large)
-        gemm_simt_wide_kernel<In, Out, 8><<<grid, 256, 0, s>>>(g, partials, slice_k);
-    else if (plan.wide)
-        gemm_simt_wide_kernel<In, Out, 4><<<grid, 128, 0, s>>>(g, partials, slice_k);
-    else
+    if (!plan.wide)
         gemm_simt_kernel<In, Out><<<grid, 256, 0, s>>>(g, partials, slice_k);
+    else if constexpr (std::is_same_v<In, float>)
+        launch_fp32(g, grid, partials, slice_k, s);
+    else if (plan.large)
+        gemm_simt_wide_kernel<In, Out, 8><<<grid, 256, 0, s>>>(g, partials, slice_k);
+    else
+        gemm_simt_wide_kernel<In, Out, 4><<<grid, 128, 0, s>>>(g, partials, slice_k);
     if (partials)
         gemm_simt_reduce_kernel<Out><<<unsigned((int64_t(g.m) * g.n + 255) / 256), 256, 0, s>>>(g, partials, used);
 }
