@@ -82,6 +82,14 @@ def test_step_matches_the_operator_path(depth, context, batch):
                 np.testing.assert_allclose(got[part], expected[part], atol=2e-6, rtol=2e-5)
 
 
+@pytest.mark.parametrize("depth,context,batch", [
+    (2, 80, 2), (2, 96, 150), (3, 100, 4),  # 5, 6 (two rounds) and 7 row tiles of a block: teams of three, of two and of two
+    (3, 16, 149 * 2 + 1), (16, 32, 3)])     # two and three row tiles: the weight gradients beside the next layer (two rounds), and not
+def test_teams_of_two_and_three_warps_per_row_tile(depth, context, batch):
+    """The same bounds as everywhere."""
+    test_step_matches_the_operator_path(depth, context, batch)
+
+
 @pytest.mark.parametrize("depth,context,batch", [(4, 4, 16), (2, 5, 7), (8, 8, 2001)])
 def test_graph_direct_and_streamed_steps_are_the_same(depth, context, batch):
     """Replayed graphs, direct launches and steps fed from host bytes leave bit-identical weights."""

@@ -3,8 +3,8 @@
 //
 // What bounds it: a token's whole step is 52 k multiply-adds over matrices of 16 columns, so as separate
 // kernels (one per operator, ~150 launches) a step is launch latency and half-empty tiles: 1.43 ms at depth 4,
-// context 4, batch 2880, and 0.86 ms at batch 16 (now 49 and 35 us with reduction and update: the latency of the chain of
-// dependent products, at 5 warps per SM and 1).  Here a block takes whole sequences (up to 128 tokens) through
+// context 4, batch 2880, and 0.86 ms at batch 16 (now 49 and 33 us with reduction and update: the latency of the chain of
+// dependent products, at three warps for every 16 tokens; 50 and 37 us with one).  Here a block takes whole sequences (up to 128 tokens) through
 // every layer and back: each warp keeps its 16 tokens' residual stream in registers, the weights sit in shared
 // memory once, and only k and v (forward) and the attention gradients (backward) pass between warps.
 //
@@ -30,7 +30,7 @@ namespace {
 constexpr int Width = 16, Heads = 4, Hidden = 48;
 constexpr int StepWarps = 16, StepThreads = StepWarps * 32;
 constexpr int HeadTiles = Vocabulary / 16 / StepWarps; // 16-column groups of logits per warp
-constexpr int MaxRows = 128;                 // tokens of one block's tile: 16 per warp
+constexpr int MaxRows = 128, MaxRowTiles = MaxRows / 16; // tokens of one block's tile: 16 per warp
 constexpr int LayerParameters = 4 * Width * Width + 3 * Hidden * Width + 2 * Width;
 constexpr int OffQkv = Width, OffAttention = OffQkv + 3 * Width * Width, OffMlpNorm = OffAttention + Width * Width,
               OffGate = OffMlpNorm + Width, OffDown = OffGate + 2 * Hidden * Width; // inside a layer; gate and up are adjacent
@@ -42,8 +42,10 @@ constexpr int Layer0 = Vocabulary * Width;   // after the embedding
 constexpr int RowsQkv = 0, RowsAttention = 48, RowsWide = 64, RowsDown = 160, LayerRows = 208; // down: 3 panels of 16 rows
 constexpr int PitchWide = 208, PitchHidden = 112, PitchQkv = 112, PitchWidth = 48, PitchLogits = 528;
 constexpr int StageBytesPerRow = PitchWide + PitchHidden + PitchQkv + 5 * PitchWidth;
+constexpr int MaxShared = 232448;
 struct StepShared {
     int weights, scales, rope, bytes, saved_x, saved_middle, saved_top, selected, exchange, dy, dt_gate, norm_sums, row_sums, stage, total;
+    bool overlap; // two stages: a layer's weight gradients are taken by the warps without rows while the others are at the next layer
     __host__ __device__ StepShared(int depth, int rows, int context) {
         int at = 0;
         auto take = [&](int n) {
@@ -62,13 +64,16 @@ struct StepShared {
         exchange = take(rows * PitchQkv);
         dy = take(rows * 32);
         dt_gate = take(rows * Heads * 8);
-        norm_sums = take(StepWarps * 2 * Width * 4);
+        norm_sums = take(StepWarps * 2 * Width * 4); // of every second layer in its second half: at most eight warps own rows
         row_sums = take(rows * StepWarps * 8);
         stage = take(rows * StageBytesPerRow);
+        // up to two row tiles ten warps or more have no part in them
+        overlap = rows <= 32 && at + rows * StageBytesPerRow <= MaxShared;
+        if (overlap)
+            take(rows * StageBytesPerRow);
         total = at;
     }
 };
-constexpr int MaxShared = 232448;
 
 struct StepParams {
     const uint8_t *data; // resident corpus to sample from, or nullptr: x and y hold the batch
@@ -264,11 +269,22 @@ __device__ __forceinline__ void save_tile(void *base, int columns, int first_col
 struct Four {
     float v[4];
 };
-__device__ __forceinline__ Four load_four(const void *p, bool keep = true) { // zeros unless `keep`
-    uint2 u = *static_cast<const uint2 *>(p);
-    if (!keep)
-        u = make_uint2(0u, 0u);
+// From shared memory.  Written out so that a load never waits for a condition on its use: as plain loads the compiler put them
+// behind the condition, and the gradients' gather loop took 1730 clocks instead of 950 (680 in pairs).
+__device__ __forceinline__ Four load_four(const void *p) {
+    uint2 u;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(u.x), "=r"(u.y) : "r"(smem_address(p)) : "memory");
     return {{__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u)}};
+}
+__device__ __forceinline__ float2 load_pair(const void *p) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_address(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ int load_byte(const void *p) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(smem_address(p)) : "memory");
+    return int(v);
 }
 __device__ __forceinline__ float dot_four(const Four &a, const Four &b) {
     float s = 0.f;
@@ -346,10 +362,27 @@ __device__ __forceinline__ void weight_gradient(float *out, int columns, uint32_
     add_gradient(out, columns, acc, accumulate, lane);
 }
 
+// A tile's 16 rows belong to one warp, its owner; the warps that own none help: one or two more per tile take a share of its
+// products (a third of the MLP's columns, parts of q, k and v), which otherwise follow one another in one warp, a chain of
+// dependent instructions that leaves the SM idle.  The shares of a sum meet in shared memory and are added in a fixed order.
+// [from, to) of the three 16-column groups that a member of a team of two or three takes: of the MLP, of q, k and v going
+// forward, and when they are recomputed going back (while the owner is at the norm and the attention projection).
+struct Share {
+    int from, to;
+};
+__device__ __forceinline__ Share mlp_share_of(int team, int member) {
+    return team == 3 ? Share{member, member + 1} : member ? Share{2, 3} : Share{0, 2};
+}
+__device__ __forceinline__ Share qkv_share_of(int team, int member) {
+    return team == 3 ? Share{member, member + 1} : member ? Share{1, 3} : Share{0, 1};
+}
+__device__ __forceinline__ Share qkv_back_share_of(int team, int member) {
+    return member == 0 ? Share{0, 0} : member == 2 ? Share{2, 3} : Share{0, team == 3 ? 2 : 3};
+}
+
 // The kernel's code is kept short (loops are rolled, one call site for the weight gradients): a block's warps run it once
 // per layer with little to overlap, and unrolled it was bound by instruction fetch (4.4 of 9 cycles per instruction).
-// Sixteen warps although eight own rows at most: the head and the weight gradients are shared by all (8 warps: 3 % faster
-// at one or two tiles per SM, 3 % slower at many).
+// Sixteen warps although eight own rows at most: the head and the weight gradients are shared by all, the layers by teams.
 template <bool Save> // also write the activations to p.saved
 __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __grid_constant__ StepParams p) {
     extern __shared__ __align__(16) uint8_t shared[];
@@ -373,6 +406,29 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
     for (int i = threadIdx.x; i < p.context; i += StepThreads)
         reinterpret_cast<float2 *>(shared + at.rope)[i] = p.rope[i];
     grid_dependency_wait(); // the weights and the step count of the update before this step
+
+    // ---- a tile's bytes and the embeddings of its tokens (into the attention gradients' memory), one thread per row ----
+    auto fetch_tokens = [&](int tile) {
+        const int r = threadIdx.x, first_sequence = tile * p.sequences, valid = min(p.sequences, p.batch - first_sequence) * p.context;
+        if (r >= p.rows)
+            return;
+        int x = 0, y = 0;
+        if (r < valid) {
+            if (p.data) { // endpoint = lo + hash(seed + step * batch + sequence) % (size - lo), see sample_kernel
+                const int64_t lo = p.context > 8 ? p.context : 8;
+                const uint64_t seed = p.seed + uint64_t(p.counters->step) * uint64_t(p.batch) + uint64_t(first_sequence + r / p.context);
+                const uint8_t *source = p.data + lo + (long long)(hash_u64(seed) % uint64_t(p.data_size - lo)) - p.context + r % p.context;
+                x = source[0], y = source[1];
+            } else {
+                x = p.x[int64_t(first_sequence) * p.context + r], y = p.y[int64_t(first_sequence) * p.context + r];
+            }
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+                copy_async<16>(base + at.dy + r * 32 + half * 16, p.weight_high + x * Width + half * 8);
+        }
+        xs[r] = uint8_t(x), ys[r] = uint8_t(y);
+    };
+    fetch_tokens(blockIdx.x);
 
     // ---- weights to shared memory; they are awaited before the first product ----
     const int final_norm = Layer0 + p.depth * LayerParameters, head = final_norm + Width, head_rows = p.depth * LayerRows;
@@ -411,8 +467,33 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
         scales[i] = join_weight(p.weight_high[from + i % Width], p.weight_low[from + i % Width]);
     }
 
-    const int row_tiles = p.rows / 16, row0 = warp * 16;
-    const bool mine = warp < row_tiles; // the warp owns 16 rows of the tile
+    const int row_tiles = p.rows / 16, team = min(3, StepWarps / row_tiles); // at most 8 row tiles: two or three
+    int own = warp % row_tiles, member = warp / row_tiles; // the warp's 16 rows, and its place in the team at them
+    asm volatile("" : "+r"(own), "+r"(member));            // kept, not divided out again at every use
+    const int row0 = own * 16;
+    const bool mine = member == 0, active = member < team; // the warp owns the rows; it has a share in them
+    const Share mlp_share = mlp_share_of(team, member), qkv_share = qkv_share_of(team, member), qkv_back_share = qkv_back_share_of(team, member);
+    auto team_barrier = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + own), "r"(32 * team) : "memory"); };
+    // 32 bytes per lane and helper in the memory of the head's row sums: the helper's share of a sum, or the owner's gradient for it
+    auto helper_slot = [&](int helper) { return reinterpret_cast<float4 *>(shared + at.row_sums + ((own * 2 + helper - 1) * 32 + lane) * 32); };
+    auto add_shares = [&](Tile &v) {
+#pragma unroll 1
+        for (int helper = 1; helper < team; ++helper) {
+            const float4 a = helper_slot(helper)[0], b = helper_slot(helper)[1];
+            v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w, v[4] += b.x, v[5] += b.y, v[6] += b.z, v[7] += b.w;
+        }
+    };
+    auto hand_in = [&](const Tile &v) {
+        helper_slot(member)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        helper_slot(member)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    };
+    auto hand_out = [&](const Tile &v) { // the owner's rows, rounded
+        uint32_t packed[4];
+        pack_tile(v, packed);
+#pragma unroll 1
+        for (int helper = 1; helper < team; ++helper)
+            *reinterpret_cast<uint4 *>(helper_slot(helper)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    };
     // rows g and g + 8: position inside the sequence and the sequence's first row
     int start[2], position[2];
 #pragma unroll
@@ -427,23 +508,9 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
         const int first_sequence = tile * p.sequences, count = min(p.sequences, p.batch - first_sequence);
         const int valid = count * p.context; // rows of the tile that hold tokens
         const int64_t token0 = int64_t(first_sequence) * p.context;
-        __syncthreads(); // the previous tile has been read (first tile: nothing)
-        if (p.data) { // endpoint = lo + hash(seed + step * batch + sequence) % (size - lo), see sample_kernel
-            const int64_t lo = p.context > 8 ? p.context : 8;
-            const uint64_t step_seed = p.seed + uint64_t(p.counters->step) * uint64_t(p.batch);
-            long long *endpoints = reinterpret_cast<long long *>(stage);
-            for (int s = threadIdx.x; s < count; s += StepThreads)
-                endpoints[s] = lo + (long long)(hash_u64(step_seed + uint64_t(first_sequence + s)) % uint64_t(p.data_size - lo));
-            __syncthreads();
-            for (int r = threadIdx.x; r < p.rows; r += StepThreads) {
-                const uint8_t *source = p.data + (r < valid ? endpoints[r / p.context] - p.context + r % p.context : 0);
-                xs[r] = source[0], ys[r] = source[1];
-            }
-        } else {
-            for (int r = threadIdx.x; r < p.rows; r += StepThreads) {
-                xs[r] = r < valid ? p.x[token0 + r] : 0;
-                ys[r] = r < valid ? p.y[token0 + r] : 0;
-            }
+        if (accumulate) {
+            __syncthreads(); // the previous tile has been read
+            fetch_tokens(tile);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
@@ -454,14 +521,14 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             for (int r = 0; r < 2; ++r) {
                 if (row0 + g + 8 * r >= valid) // stays zero: an infinite weight that no token reads must not reach the sums
                     continue;
-                const uint32_t *row = reinterpret_cast<const uint32_t *>(p.weight_high + int(xs[row0 + g + 8 * r]) * Width);
+                const uint32_t *row = reinterpret_cast<const uint32_t *>(shared + at.dy + (row0 + g + 8 * r) * 32);
                 const uint32_t a = row[t], b = row[4 + t];
                 x[2 * r] = __uint_as_float(a << 16), x[2 * r + 1] = __uint_as_float(a & 0xffff0000u);
                 x[4 + 2 * r] = __uint_as_float(b << 16), x[5 + 2 * r] = __uint_as_float(b & 0xffff0000u);
             }
         }
-        auto saved_slot = [&](int offset, int l) { return reinterpret_cast<uint4 *>(shared + offset) + (l * row_tiles + warp) * 32 + lane; };
-        auto top_slot = [&](int l) { return reinterpret_cast<float2 *>(shared + at.saved_top) + (l * row_tiles + warp) * 32 + lane; };
+        auto saved_slot = [&](int offset, int l) { return reinterpret_cast<uint4 *>(shared + offset) + (l * row_tiles + own) * 32 + lane; };
+        auto top_slot = [&](int l) { return reinterpret_cast<float2 *>(shared + at.saved_top) + (l * row_tiles + own) * 32 + lane; };
         auto keep = [&](int offset, int l, const Tile &v) {
             uint32_t packed[4];
             pack_tile(v, packed);
@@ -471,13 +538,13 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             if constexpr (Save)
                 save_tile(to, columns, column, heads, v, token0 + row0, valid - row0, g, t);
         };
-        // normed1 and the rotated q, k, v of a layer from its input, the latter to `buffer` [row][48]
-        auto project_qkv = [&](int l, uint32_t panel, const Tile &input, Tile &normed, uint8_t *buffer) {
+        // normed1 of a layer and its rotated q, k, v (those in `share`) from its input, the latter to `buffer` [row][48]
+        auto project_qkv = [&](int l, uint32_t panel, const Tile &input, Tile &normed, uint8_t *buffer, const Share &share) {
             rms_norm(input, Scale(scales + 2 * l * Width, t), normed);
             uint32_t a[4];
             pack_tile(normed, a);
 #pragma unroll 1
-            for (int m = 0; m < 3; ++m) {
+            for (int m = share.from; m < share.to; ++m) {
                 Tile y = {};
                 multiply(y, a, panel, RowsQkv + 16 * m, lane);
                 round_tile(y);
@@ -495,19 +562,24 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             // k and v of consecutive layers alternate between two buffers: one barrier a layer (the second lies in the stage)
             uint8_t *buffer = l % 2 ? stage : shared + at.exchange;
             const uint32_t panel = weights + l * LayerRows * 32;
-            if (mine) {
+            if (mine)
                 keep(at.saved_x, l, x);
-                Tile normed;
-                project_qkv(l, panel, x, normed, buffer);
-                save(p.saved.layer[l].x, Width, 0, false, x);
-                save(p.saved.layer[l].normed1, Width, 0, false, normed);
+            if (active) {
+                team_barrier();
+                Tile input, normed;
+                unpack_tile(*saved_slot(at.saved_x, l), input);
+                project_qkv(l, panel, input, normed, buffer, qkv_share);
+                if (mine) {
+                    save(p.saved.layer[l].x, Width, 0, false, x);
+                    save(p.saved.layer[l].normed1, Width, 0, false, normed);
+                }
             }
             __syncthreads();
-            if (!mine)
+            if (!active)
                 continue;
-            Tile attended;
             uint32_t a[4];
-            {
+            if (mine) {
+                Tile attended;
                 Four q[2];
                 float top[2];
                 int best[2];
@@ -517,38 +589,49 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                     top[r] = -CUDART_INF_F, best[r] = start[r];
                 }
 #pragma unroll 1
-                for (int j = 0; j <= longest; ++j)
+                for (int j = 0; j <= longest; j += 2) {
+                    Four k[2][2];
 #pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const int key = start[r] + min(j, position[r]); // the row's own key again once past it: no change
-                        const float score = dot_four(q[r], load_four(buffer + key * PitchQkv + 32 + 8 * t));
-                        if (score > top[r]) // the first key wins ties
-                            top[r] = score, best[r] = key;
-                    }
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) // the row's own key again once past it: no change
+                            k[u][r] = load_four(buffer + (start[r] + min(j + u, position[r])) * PitchQkv + 32 + 8 * t);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const float score = dot_four(q[r], k[u][r]);
+                            if (score > top[r]) // the first key wins ties
+                                top[r] = score, best[r] = start[r] + min(j + u, position[r]);
+                        }
+                }
+                const Four v[2] = {load_four(buffer + best[0] * PitchQkv + 64 + 8 * t), load_four(buffer + best[1] * PitchQkv + 64 + 8 * t)};
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float gate = gelu(top[r]);
-                    const Four v = load_four(buffer + best[r] * PitchQkv + 64 + 8 * t);
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
-                        attended[(c >> 1) * 4 + 2 * r + (c & 1)] = v.v[c] * gate; // rounded when packed
+                        attended[(c >> 1) * 4 + 2 * r + (c & 1)] = v[r].v[c] * gate; // rounded when packed
                     shared[at.selected + (l * p.rows + row0 + g + 8 * r) * Heads + t] = uint8_t(best[r]);
                 }
                 *top_slot(l) = make_float2(top[0], top[1]);
+                pack_tile(attended, a);
+                Tile branch = {};
+                multiply(branch, a, panel, RowsAttention, lane);
+                add_branch(x, branch); // middle
+                keep(at.saved_middle, l, x);
+                save(p.saved.layer[l].attended, Width, 0, true, attended);
+                save(p.saved.layer[l].middle, Width, 0, false, x);
             }
-            pack_tile(attended, a);
-            Tile branch = {};
-            multiply(branch, a, panel, RowsAttention, lane);
-            add_branch(x, branch); // middle
-            keep(at.saved_middle, l, x);
-            save(p.saved.layer[l].attended, Width, 0, true, attended);
-            save(p.saved.layer[l].middle, Width, 0, false, x);
-            Tile normed, down = {};
-            rms_norm(x, Scale(scales + (2 * l + 1) * Width, t), normed);
-            save(p.saved.layer[l].normed2, Width, 0, false, normed);
+            team_barrier();
+            Tile middle, normed, down = {};
+            unpack_tile(*saved_slot(at.saved_middle, l), middle);
+            rms_norm(middle, Scale(scales + (2 * l + 1) * Width, t), normed);
+            if (mine)
+                save(p.saved.layer[l].normed2, Width, 0, false, normed);
             pack_tile(normed, a);
 #pragma unroll 1
-            for (int m = 0; m < 3; ++m) {
+            for (int m = mlp_share.from; m < mlp_share.to; ++m) {
                 Tile gate = {}, up = {};
                 multiply(gate, a, panel, RowsWide + 16 * m, lane);
                 multiply(up, a, panel, RowsWide + Hidden + 16 * m, lane);
@@ -558,7 +641,13 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                 pack_tile(up, h);
                 multiply(down, h, panel, RowsDown + 16 * m, lane);
             }
-            add_branch(x, down);
+            if (!mine)
+                hand_in(down);
+            team_barrier();
+            if (mine) {
+                add_shares(down);
+                add_branch(x, down);
+            }
         }
 
         // ---- head and loss: every warp takes its share of the 256 columns, for all rows ----
@@ -658,42 +747,78 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                 multiply_transposed(dnormed, a, weights, head_rows + 16 * m, lane);
             }
             round_tile(dnormed);
-            rms_norm_backward(x, dnormed, final_scale, nullptr, x, norm_sums + warp * 2 * Width, lane);
+            rms_norm_backward(x, dnormed, final_scale, nullptr, x, norm_sums + (p.depth % 2 * MaxRowTiles + own) * 2 * Width, lane);
         }
-        auto sum_norm = [&](int which, int offset) { // 16 lanes: a norm's scale gradient over the warps, in order
+        auto sum_norm = [&](int half, int which, int offset) { // 16 lanes: a norm's scale gradient over the warps, in order
             float total = 0.f;
             for (int w = 0; w < row_tiles; ++w)
-                total += norm_sums[(w * 2 + which) * Width + lane];
+                total += norm_sums[((half * MaxRowTiles + w) * 2 + which) * Width + lane];
             partial[offset + lane] = accumulate ? partial[offset + lane] + total : total;
         };
 #pragma unroll 1
         for (int job = warp; job < 16; job += StepWarps)
             weight_gradient(partial + head + 16 * job * Width, Width, stage_base + s_logits + 32 * job, PitchLogits, stage_base + s_final,
                             PitchWidth, p.rows, accumulate, lane);
+        if (mine)
+            hand_out(x); // the row sums have been read
         __syncthreads();
         if (warp == StepWarps - 1 && lane < Width)
-            sum_norm(0, final_norm); // before the next barrier but one overwrites the sums
+            sum_norm(p.depth % 2, 0, final_norm);
 
         // ---- backward ----
-        for (int l = p.depth - 1; l >= 0; --l) {
-            uint8_t *exchange = shared + at.exchange;
+        const int first_free = at.overlap ? team * row_tiles : 0, stage_apart = at.overlap ? p.rows * StageBytesPerRow : 0;
+        for (int l = p.depth - 1; l >= -1; --l) {
+            // the 13 weight-gradient tiles of 16 x 16 and two norm scales of the layer that has just been staged
+            if (l + 1 < p.depth && warp >= first_free) {
+                const int layer0 = Layer0 + (l + 1) * LayerParameters;
+                const uint32_t from = stage_base + (l + 1) % 2 * stage_apart;
+#pragma unroll 1
+                for (int job = warp - first_free; job < 15; job += StepWarps - first_free) {
+                    if (job >= 13) {
+                        if (lane < Width)
+                            sum_norm((l + 1) % 2, job - 13, layer0 + (job == 13 ? 0 : OffMlpNorm));
+                        continue;
+                    }
+                    int to = OffGate + 16 * job * Width, columns = Width, dy_at = s_wide + 32 * job, dy_pitch = PitchWide, x_at = s_normed2,
+                        x_pitch = PitchWidth;
+                    if (job >= 6) // down: columns 16 (job - 6) of [16][48]
+                        to = OffDown + 16 * (job - 6), columns = Hidden, dy_at = s_dh, dy_pitch = PitchWidth, x_at = s_hidden + 32 * (job - 6),
+                        x_pitch = PitchHidden;
+                    if (job >= 9)
+                        to = OffQkv + 16 * (job - 9) * Width, columns = Width, dy_at = s_qkv + 32 * (job - 9), dy_pitch = PitchQkv, x_at = s_normed1,
+                        x_pitch = PitchWidth;
+                    if (job == 12)
+                        to = OffAttention, dy_at = s_dh2, dy_pitch = PitchWidth, x_at = s_attended;
+                    weight_gradient(partial + layer0 + to, columns, from + dy_at, dy_pitch, from + x_at, x_pitch, p.rows, accumulate, lane);
+                }
+            }
+            if (!at.overlap && l + 1 < p.depth)
+                __syncthreads();
+            if (l < 0)
+                break;
+            uint8_t *const stage = shared + at.stage + l % 2 * stage_apart, *exchange = shared + at.exchange;
             const uint8_t *selected = shared + at.selected + l * p.rows * Heads;
             const uint32_t panel = weights + l * LayerRows * 32;
             Tile input, dq;
             Four dy[2];
-            if (mine) {
+            if (active) {
                 Tile middle, normed;
                 uint32_t a[4], dh[4];
                 unpack_tile(*saved_slot(at.saved_middle, l), middle);
                 const Scale scale(scales + (2 * l + 1) * Width, t);
                 rms_norm(middle, scale, normed);
                 pack_tile(normed, a);
-                put_tile(stage + s_normed2 + row0 * PitchWidth, PitchWidth, normed, g, t);
-                put_tile(stage + s_dh + row0 * PitchWidth, PitchWidth, x, g, t);
-                pack_tile(x, dh);
+                if (mine) {
+                    put_tile(stage + s_normed2 + row0 * PitchWidth, PitchWidth, normed, g, t);
+                    put_tile(stage + s_dh + row0 * PitchWidth, PitchWidth, x, g, t);
+                    pack_tile(x, dh);
+                } else {
+                    const uint4 u = *reinterpret_cast<const uint4 *>(helper_slot(member));
+                    dh[0] = u.x, dh[1] = u.y, dh[2] = u.z, dh[3] = u.w;
+                }
                 Tile branch = {};
 #pragma unroll 1
-                for (int m = 0; m < 3; ++m) {
+                for (int m = mlp_share.from; m < mlp_share.to; ++m) {
                     Tile gate = {}, up = {}, dout = {};
                     multiply(gate, a, panel, RowsWide + 16 * m, lane);
                     multiply(up, a, panel, RowsWide + Hidden + 16 * m, lane);
@@ -709,38 +834,51 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                     pack_tile(up, d);
                     multiply_transposed(branch, d, panel, RowsWide + Hidden + 16 * m, lane);
                 }
-                round_tile(branch);
-                rms_norm_backward(middle, branch, scale, &x, x, norm_sums + (warp * 2 + 1) * Width, lane);
-                put_tile(stage + s_dh2 + row0 * PitchWidth, PitchWidth, x, g, t);
-                // gradient of the attended values: the lane's head t of rows g and g + 8
-                pack_tile(x, a);
-                Tile dattended = {};
-                multiply_transposed(dattended, a, panel, RowsAttention, lane);
-                round_tile(dattended);
-                put_heads(shared + at.dy + row0 * 32, 32, dattended, g, t);
+                if (!mine)
+                    hand_in(branch);
+                team_barrier();
+                if (mine) {
+                    add_shares(branch);
+                    round_tile(branch);
+                    rms_norm_backward(middle, branch, scale, &x, x, norm_sums + ((l % 2 * MaxRowTiles + own) * 2 + 1) * Width, lane);
+                    put_tile(stage + s_dh2 + row0 * PitchWidth, PitchWidth, x, g, t);
+                    // gradient of the attended values: the lane's head t of rows g and g + 8
+                    pack_tile(x, a);
+                    Tile dattended = {};
+                    multiply_transposed(dattended, a, panel, RowsAttention, lane);
+                    round_tile(dattended);
+                    put_heads(shared + at.dy + row0 * 32, 32, dattended, g, t);
 #pragma unroll
-                for (int r = 0; r < 2; ++r)
-                    dy[r] = {{dattended[2 * r], dattended[2 * r + 1], dattended[4 + 2 * r], dattended[5 + 2 * r]}};
+                    for (int r = 0; r < 2; ++r)
+                        dy[r] = {{dattended[2 * r], dattended[2 * r + 1], dattended[4 + 2 * r], dattended[5 + 2 * r]}};
+                }
                 unpack_tile(*saved_slot(at.saved_x, l), input);
-                project_qkv(l, panel, input, normed, exchange);
-                put_tile(stage + s_normed1 + row0 * PitchWidth, PitchWidth, normed, g, t);
+                if (qkv_back_share.to) {
+                    project_qkv(l, panel, input, normed, exchange, qkv_back_share);
+                    if (qkv_back_share.from == 0)
+                        put_tile(stage + s_normed1 + row0 * PitchWidth, PitchWidth, normed, g, t);
+                }
             }
             __syncthreads();
             if (mine) {
-                const float2 top = *top_slot(l);
+                const float2 top = load_pair(top_slot(l));
                 Tile attended;
+                Four k[2], v[2];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const int row = row0 + g + 8 * r, key = selected[row * Heads + t];
+                    const uint8_t *key = exchange + load_byte(selected + (row0 + g + 8 * r) * Heads + t) * PitchQkv + 8 * t;
+                    k[r] = load_four(key + 32), v[r] = load_four(key + 64);
+                }
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
                     const float score = r ? top.y : top.x, gate = gelu(score);
-                    const Four v = load_four(exchange + key * PitchQkv + 64 + 8 * t), k = load_four(exchange + key * PitchQkv + 32 + 8 * t);
-                    const float dt = dot_four(dy[r], v) * gelu_derivative(score);
-                    dt_gate[row * Heads + t] = make_float2(dt, gate);
+                    const float dt = dot_four(dy[r], v[r]) * gelu_derivative(score);
+                    dt_gate[(row0 + g + 8 * r) * Heads + t] = make_float2(dt, gate);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const int i = (c >> 1) * 4 + 2 * r + (c & 1);
-                        attended[i] = v.v[c] * gate;
-                        dq[i] = dt * k.v[c];
+                        attended[i] = v[r].v[c] * gate;
+                        dq[i] = dt * k[r].v[c];
                     }
                 }
                 round_tile(dq);
@@ -750,20 +888,32 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             if (mine) {
                 Tile dk = {}, dv = {};
 #pragma unroll 1
-                for (int j = 0; j < furthest; ++j) // a key gathers from the queries that selected it; of the others it takes zeros
+                for (int j = 0; j < furthest; j += 2) { // a key gathers from the queries that selected it; of the others it takes zeros
+                    // (every load of the pair is issued before the first is used)
+                    Four q[2][2], d[2][2];
+                    float2 w[2][2];
+                    bool chosen[2][2];
 #pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const int row = row0 + g + 8 * r, last = min(row + p.context - 1 - position[r], p.rows - 1), query = min(row + j, last);
-                        const bool chosen = row + j <= last && selected[query * Heads + t] == row;
-                        const float2 w = dt_gate[query * Heads + t];
-                        const float dt = chosen ? w.x : 0.f, gate = chosen ? w.y : 0.f;
-                        const Four q = load_four(exchange + query * PitchQkv + 8 * t, chosen), d = load_four(shared + at.dy + query * 32 + 8 * t, chosen);
+                    for (int u = 0; u < 2; ++u)
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const int i = (c >> 1) * 4 + 2 * r + (c & 1);
-                            dk[i] += dt * q.v[c], dv[i] += d.v[c] * gate;
+                        for (int r = 0; r < 2; ++r) {
+                            const int row = row0 + g + 8 * r, last = min(row + p.context - 1 - position[r], p.rows - 1), query = min(row + j + u, last);
+                            q[u][r] = load_four(exchange + query * PitchQkv + 8 * t), d[u][r] = load_four(shared + at.dy + query * 32 + 8 * t);
+                            w[u][r] = load_pair(dt_gate + query * Heads + t);
+                            chosen[u][r] = (row + j + u <= last) & (load_byte(selected + query * Heads + t) == row);
                         }
-                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const float dt = chosen[u][r] ? w[u][r].x : 0.f, gate = chosen[u][r] ? w[u][r].y : 0.f;
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                const int i = (c >> 1) * 4 + 2 * r + (c & 1);
+                                dk[i] += dt * (chosen[u][r] ? q[u][r].v[c] : 0.f), dv[i] += (chosen[u][r] ? d[u][r].v[c] : 0.f) * gate;
+                            }
+                        }
+                }
                 round_tile(dk);
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
@@ -784,37 +934,16 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                 pack_tile(dv, a);
                 multiply_transposed(branch, a, panel, RowsQkv + 32, lane);
                 round_tile(branch);
-                rms_norm_backward(input, branch, Scale(scales + 2 * l * Width, t), &x, x, norm_sums + warp * 2 * Width, lane);
-            }
-            __syncthreads();
-            // the layer's 13 weight-gradient tiles of 16 x 16 and two norm scales
-            const int layer0 = Layer0 + l * LayerParameters;
-#pragma unroll 1
-            for (int job = warp; job < 15; job += StepWarps) {
-                if (job >= 13) {
-                    if (lane < Width)
-                        sum_norm(job - 13, layer0 + (job == 13 ? 0 : OffMlpNorm));
-                    continue;
-                }
-                int to = OffGate + 16 * job * Width, columns = Width, dy_at = s_wide + 32 * job, dy_pitch = PitchWide, x_at = s_normed2,
-                    x_pitch = PitchWidth;
-                if (job >= 6) // down: columns 16 (job - 6) of [16][48]
-                    to = OffDown + 16 * (job - 6), columns = Hidden, dy_at = s_dh, dy_pitch = PitchWidth, x_at = s_hidden + 32 * (job - 6),
-                    x_pitch = PitchHidden;
-                if (job >= 9)
-                    to = OffQkv + 16 * (job - 9) * Width, columns = Width, dy_at = s_qkv + 32 * (job - 9), dy_pitch = PitchQkv, x_at = s_normed1,
-                    x_pitch = PitchWidth;
-                if (job == 12)
-                    to = OffAttention, dy_at = s_dh2, dy_pitch = PitchWidth, x_at = s_attended;
-                weight_gradient(partial + layer0 + to, columns, stage_base + dy_at, dy_pitch, stage_base + x_at, x_pitch, p.rows, accumulate, lane);
+                rms_norm_backward(input, branch, Scale(scales + 2 * l * Width, t), &x, x, norm_sums + (l % 2 * MaxRowTiles + own) * 2 * Width, lane);
+                hand_out(x);
             }
             __syncthreads();
         }
 
         // ---- embedding gradient: one-hot(x)^T dh, the one-hot operand built in registers ----
         bool finite = true;
-        if (mine) {
-            put_tile(stage + s_dh + row0 * PitchWidth, PitchWidth, x, g, t);
+        if (mine) { // (the first layer's stage may still be read)
+            put_tile(stage + stage_apart + s_dh + row0 * PitchWidth, PitchWidth, x, g, t);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 finite = finite && isfinite(x[i]);
@@ -826,12 +955,12 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
 #pragma unroll 1
                 for (int r = 0; r < valid; ++r)
                     if (xs[r] == i / Width)
-                        total += __bfloat162float(reinterpret_cast<const bf16 *>(stage + s_dh + r * PitchWidth)[i % Width]);
+                        total += __bfloat162float(reinterpret_cast<const bf16 *>(stage + stage_apart + s_dh + r * PitchWidth)[i % Width]);
                 partial[i] = accumulate ? partial[i] + total : total;
             }
             continue;
         }
-        const uint32_t b_lane = stage_base + s_dh + (((lane >> 3) & 1) * 8 + (lane & 7)) * PitchWidth + (lane >> 4) * 16;
+        const uint32_t b_lane = stage_base + stage_apart + s_dh + (((lane >> 3) & 1) * 8 + (lane & 7)) * PitchWidth + (lane >> 4) * 16;
 #pragma unroll 1
         for (int job = warp; job < 16; job += StepWarps) {
             Tile acc = {};
