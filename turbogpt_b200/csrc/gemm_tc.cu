@@ -13,8 +13,8 @@
 //
 // Epilogue: four warps share each 32-lane quarter of tensor memory and take every fourth
 // 32-column chunk.  A lane owns one output row: it reads its accumulator chunk (tcgen05.ld),
-// optionally combines it with the same chunk of a second tensor read straight from global memory
-// (residual, saved GELU derivative, or the Newton-Schulz operand) and writes 32-byte pieces with
+// optionally combines it with the same chunk of a second tensor read straight from global memory, the first one
+// before the products are done (residual, saved GELU derivative, or the Newton-Schulz operand), and writes 32-byte pieces with
 // 256-bit stores.
 //
 // Weight-gradient GEMMs have few output tiles and a very long K; they are split along K and each
@@ -322,13 +322,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             long long t = w / p.splits;
             const int nt = int(t % n_tiles), mt = int(t / n_tiles % m_units) * Unit + int(rank),
                       z = int(t / n_tiles / m_units);
+            const long long row = (long long)mt * BM + quarter * 32 + lane;
+            constexpr int Pieces = OutFp32 ? 4 : 2; // 32-byte pieces per 32-column chunk row
+            constexpr int PieceColumns = 32 / Pieces;
+            uint32_t rv[has_r ? Pieces : 1][8];
+            auto fetch_second = [&](int c) { // the second tensor's part of a chunk
+                const int column = nt * p.bn + c * 32;
+                if (!has_r || row >= p.m)
+                    return;
+                const char *src = (const char *)p.r + (z * p.r_batch + row * p.ldr + column) * (OutFp32 ? 4 : 2);
+#pragma unroll
+                for (int g = 0; g < Pieces; ++g)
+                    if (column + g * PieceColumns < p.n)
+                        load_global32(src + g * 32, rv[g], p.wide && column + (g + 1) * PieceColumns <= p.n,
+                                      column + g * PieceColumns + PieceColumns / 2 < p.n);
+            };
+            if (share * 32 < p.bn)
+                fetch_second(share); // on its way while the products are awaited (steps of short products 1 to 1.6 % faster)
             bool ready = mbarrier_wait(tfull0 + 8 * buffer, buffer_phase, abort_flag, p.counters, 104);
             if (p.splits > 1 || whole_rows) // the warps meet at named barriers below: leave together or not at all
                 ready = epilogue_all(ready);
             if (!ready)
                 break;
             tcgen05_fence_after();
-            const long long row = (long long)mt * BM + quarter * 32 + lane;
             const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + buffer * MaxBN;
             const int tile_columns = min(p.bn, p.n - nt * p.bn);
             const int chunks = (tile_columns + 31) / 32;
@@ -404,21 +420,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
             } else if (p.splits == 1) {
                 const bool row_ok = row < p.m;
-                const long long c_row = z * p.c_batch + row * p.ldc, r_row = z * p.r_batch + row * p.ldr;
+                const long long c_row = z * p.c_batch + row * p.ldc;
                 auto process = [&](uint32_t (&acc)[32], int c) {
                     const int column = nt * p.bn + c * 32;
-                    // Second tensor for this chunk: issue the global loads before waiting on TMEM.
-                    constexpr int Pieces = OutFp32 ? 4 : 2; // 32-byte pieces per 32-column chunk row
-                    constexpr int PieceColumns = 32 / Pieces;
-                    uint32_t rv[has_r ? Pieces : 1][8];
-                    if (has_r && row_ok) {
-                        const char *src = (const char *)p.r + (r_row + column) * (OutFp32 ? 4 : 2);
-#pragma unroll
-                        for (int g = 0; g < Pieces; ++g)
-                            if (column + g * PieceColumns < p.n)
-                                load_global32(src + g * 32, rv[g], p.wide && column + (g + 1) * PieceColumns <= p.n,
-                                              column + g * PieceColumns + PieceColumns / 2 < p.n);
-                    }
                     tmem_wait_load(acc);
                     if (!row_ok)
                         return;
@@ -486,6 +490,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 for (int c = share; c < chunks; c += Shares) {
                     uint32_t acc[32];
                     tmem_load_32x32_async(taddr + c * 32, acc);
+                    if (c != share)
+                        fetch_second(c);
                     process(acc, c);
                 }
                 tcgen05_fence_before();
