@@ -5,6 +5,7 @@
 #include "device_utils.cuh"
 #include "kernels.cuh"
 #include "sm100.cuh"
+#include <algorithm>
 
 // Fixed-order partial sums of squares: block b covers a contiguous slice.
 __global__ void __launch_bounds__(256) sum_squares_kernel(const float *gradient, int64_t count, float *partial) {
@@ -207,23 +208,42 @@ __global__ void __launch_bounds__(256) muon_prepare_transpose_kernel(MuonPrepare
     const int64_t size = int64_t(a.rows) * a.cols, base = matrix * a.stride;
     const int tiles_across = a.cols / MuonTile, tiles = (a.rows / MuonTile) * tiles_across;
     float squares = 0;
+    // A thread's two groups of eight columns of a tile (rows 32 apart) are fetched while the tile before is worked on: as plain
+    // loads, each waiting for the stores before it, a tile cost two round trips to memory.
+    constexpr int Items = MuonTile * 8 / 256;
+    const int rr = threadIdx.x / 8, chunk = threadIdx.x % 8;
+    float next_g[Items][8], next_m[Items][8];
+    auto place = [&](int t, int i) { return base + int64_t(t / tiles_across * MuonTile + rr + 32 * i) * a.cols + t % tiles_across * MuonTile + chunk * 8; };
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int i = 0; i < Items; ++i) {
+            load8(a.gradient + place(t, i), next_g[i]);
+            load8(a.momentum + place(t, i), next_m[i]);
+        }
+    };
+    if (int(blockIdx.x) < tiles)
+        fetch(blockIdx.x);
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int r0 = t / tiles_across * MuonTile, c0 = t % tiles_across * MuonTile;
-        for (int item = threadIdx.x; item < MuonTile * 8; item += blockDim.x) { // (row, group of 8 columns)
-            const int rr = item / 8, chunk = item % 8;
-            const int64_t at = base + int64_t(r0 + rr) * a.cols + c0 + chunk * 8;
-            float g[8], m[8];
-            load8(a.gradient + at, g);
-            load8(a.momentum + at, m);
+        float g[Items][8], m[Items][8];
+#pragma unroll
+        for (int i = 0; i < Items; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                g[i][j] = next_g[i][j], m[i][j] = next_m[i][j];
+        if (t + int(gridDim.x) < tiles)
+            fetch(t + gridDim.x);
+#pragma unroll
+        for (int i = 0; i < Items; ++i) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                g[j] *= clip;
-                m[j] += (1 - mu) * (g[j] - m[j]);
-                const bf16 u = __float2bfloat16_rn(g[j] + mu * (m[j] - g[j]));
-                tile[(chunk * 8 + j) * MuonTilePitch + rr] = u;
+                g[i][j] *= clip;
+                m[i][j] += (1 - mu) * (g[i][j] - m[i][j]);
+                const bf16 u = __float2bfloat16_rn(g[i][j] + mu * (m[i][j] - g[i][j]));
+                tile[(chunk * 8 + j) * MuonTilePitch + rr + 32 * i] = u;
                 squares += __bfloat162float(u) * __bfloat162float(u);
             }
-            store8(a.momentum + at, m);
+            store8(a.momentum + place(t, i), m[i]);
         }
         __syncthreads();
         for (int item = threadIdx.x; item < MuonTile * 8; item += blockDim.x) { // (column, group of 8 rows)
@@ -277,12 +297,6 @@ __global__ void __launch_bounds__(256) muon_normalize_vector_kernel(bf16 *x, con
             v[j] /= norm;
         store8(x + matrix * per_matrix + i, v);
     }
-}
-void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, cudaStream_t s) {
-    if (per_matrix % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0)
-        muon_normalize_vector_kernel<<<dim3(MuonBlocks, batch), 256, 0, s>>>(x, sumsq, per_matrix);
-    else
-        muon_normalize_kernel<<<dim3(MuonBlocks, batch), 256, 0, s>>>(x, sumsq, per_matrix);
 }
 // All Newton-Schulz iterations of one small matrix (the reference architecture's 16 x 16 .. 16 x 48) in one
 // block's shared memory, with the roundings of the three-GEMM form: BF16 operands, FP32 sums over ascending k,
@@ -431,8 +445,20 @@ __global__ void __launch_bounds__(256) muon_apply_transpose_kernel(MuonApplyArgs
         __syncthreads();
     }
 }
+// Blocks per matrix of a stage that leaves no partial sums: eight per SM over all matrices, as far as there are 64 x 64 tiles (four
+// thousand elements) for them.  With MuonBlocks of them a block of six 1536 x 384 matrices took four tiles one after another.
+static int muon_blocks(int64_t size, int batch) {
+    return int(std::max<int64_t>(1, std::min<int64_t>(size / (MuonTile * MuonTile), std::max(148 * 8 / batch, MuonBlocks))));
+}
+void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, cudaStream_t s) {
+    const dim3 grid(muon_blocks(per_matrix, batch), batch);
+    if (per_matrix % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0)
+        muon_normalize_vector_kernel<<<grid, 256, 0, s>>>(x, sumsq, per_matrix);
+    else
+        muon_normalize_kernel<<<grid, 256, 0, s>>>(x, sumsq, per_matrix);
+}
 void launch_muon_apply(const MuonApplyArgs &a, cudaStream_t s) {
-    const dim3 grid(MuonBlocks, a.batch);
+    const dim3 grid(muon_blocks(int64_t(a.rows) * a.cols, a.batch), a.batch);
     const bool aligned = a.stride % 8 == 0 && reinterpret_cast<uintptr_t>(a.weight_high) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(a.weight_low) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(a.weight_fp32) % 32 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0;
