@@ -161,7 +161,6 @@ flash_backward_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __gr
         return it;
     };
 
-    grid_launch_dependents(); // the next kernel may set itself up while this one runs
     if (threadIdx.x == 32) {
         prefetch_map(&map_qkv128);
         prefetch_map(&map_qkv64);
@@ -195,6 +194,7 @@ flash_backward_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __gr
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_launch_dependents(); // the next kernel may set itself up while this one runs; this one holds its tensor memory
     const uint32_t tmem_base = *tmem_slot;
     // S^T buffers at 0 and 64 (a warp's packed P^T goes to the first 16 columns of its own 32), dP^T at 128 and 192,
     // dV at 256, dK at 320, dQ buffers at 384 and 448

@@ -236,7 +236,6 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     const int last_key = min(p.context, (tile + 1) * BlockM);
     const int steps = (last_key + KeyStep - 1) / KeyStep; // causal: keys 0 .. last_key - 1, 64 per step
 
-    grid_launch_dependents(); // the next kernel may set itself up while this one runs
     if (threadIdx.x == 0) {
         mbarrier_init(q_full, 1);
         for (int s = 0; s < ForwardRing; ++s) {
@@ -260,6 +259,7 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_launch_dependents(); // the next kernel may set itself up while this one runs; this one holds its tensor memory
     const uint32_t tmem_base = *tmem_slot;
     // chain c: scores of its steps at 64 c (the probabilities pack into the first 32 of those columns),
     // its output accumulator at 128 + 64 c
@@ -640,7 +640,6 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_con
     const int last_key = min(p.context, (tile + 1) * BlockM); // keys 0..last_key-1 can be attended
     const int blocks = (last_key + DqStep - 1) / DqStep;
 
-    grid_launch_dependents(); // the next kernel may set itself up while this one runs
     if (threadIdx.x == 0) {
         mbarrier_init(qdo_full, 1);
         for (int s = 0; s < DqRing; ++s) {
@@ -663,6 +662,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_con
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_launch_dependents(); // the next kernel may set itself up while this one runs; this one holds its tensor memory
     const uint32_t tmem_base = *tmem_slot;
     // S buffers at 0 and 64 (a half's packed dS goes to the first 16 columns of its own 32), dP at 128, dQ at 192
     const uint32_t tmem_dp = tmem_base + 128, tmem_dq = tmem_base + 192;
@@ -877,7 +877,6 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_co
     const int first_block = tile * (BlockN / DkvStep), query_blocks = (p.context + DkvStep - 1) / DkvStep;
     const int blocks = query_blocks - first_block; // query blocks first_block .. query_blocks-1
 
-    grid_launch_dependents(); // the next kernel may set itself up while this one runs
     if (threadIdx.x == 0) {
         mbarrier_init(kv_full, 1);
         for (int s = 0; s < DkvRing; ++s) {
@@ -899,6 +898,7 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_co
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_launch_dependents(); // the next kernel may set itself up while this one runs; this one holds its tensor memory
     const uint32_t tmem_base = *tmem_slot;
     // S^T at 0 (a half's packed P^T goes to the first 16 columns of its own 32), dP^T at 64 (dS^T likewise);
     // dV at 128, dK at 192

@@ -36,12 +36,17 @@ using namespace sm100;
 namespace {
 constexpr int BM = 128, BK = 64, MaxBN = 256, MaxStages = 8;
 constexpr int StageABytes = BM * BK * 2;
-constexpr int EpilogueWarps = 16;
-constexpr int Threads = 64 + 32 * EpilogueWarps; // warp 0: TMA, warp 1: MMA, then the epilogue warps
+constexpr int threads_of(int epilogue_warps) { return 64 + 32 * epilogue_warps; } // warp 0: TMA, warp 1: MMA, then the epilogue warps
 constexpr int ControlBytes = 512;   // barriers, TMEM slot, flags
 constexpr int RowScratchBytes = 2 * 4 * BM * 4; // CrossEntropy: row maxima and row sums of the four column shares
 constexpr int MaxShared = 232448 - 1024; // 227 KB less the runtime's own reservation
-constexpr int TmemColumns = 512;
+// A batched product of at most one tile per SM, up to 128 columns wide, runs in half an SM: eight epilogue warps, one accumulator of
+// its own width, and a ring of half the shared memory.  Those are Muon's Newton-Schulz products where the families' run beside each
+// other on four lanes: 108 to 144 blocks each, one to an SM, kept waiting for one another (6 layers d 384: 4 steps 5400 -> 5150 us,
+// the same bits; two blocks to an SM above one tile per SM measured level).  Products in a chain of their own stay with the deep
+// ring: tg_predict of 12 layers d 768 takes 838 us with halves, 735 without.  Every kernel that takes tensor memory lets its
+// dependents launch only once it holds it, so none can wait for columns that a kernel waiting for it holds.
+constexpr int HalfShared = 113 * 1024;
 
 struct TcParams {
     int m, n, k, batch;
@@ -50,6 +55,7 @@ struct TcParams {
     int splits, k_blocks_per_split;
     int epilogue, out_fp32;
     int stages;             // depth of the operand ring
+    int tmem_columns;
     int wide;               // C, C2 and R rows are 32-byte aligned: 256-bit epilogue accesses
     int reduce_later;       // K splits only write their partial tiles; splitk_reduce_kernel adds them afterwards
     void *c, *c2;
@@ -95,13 +101,14 @@ __device__ __forceinline__ void store_group(const TcParams &p, float (&v)[8], lo
     store8((bf16 *)p.c + ci, v);
 }
 
-// AND of a predicate over the 512 epilogue threads (named barrier 1).
-__device__ __forceinline__ bool epilogue_all(bool ok) {
+// The epilogue threads meet (named barrier 1), with the AND of a predicate over them.
+template <int Warps> __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * Warps) : "memory"); }
+template <int Warps> __device__ __forceinline__ bool epilogue_all(bool ok) {
     uint32_t result;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 512, p;\n\t"
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\t"
                  "selp.u32 %0, 1, 0, q;\n\t}"
                  : "=r"(result)
-                 : "r"(uint32_t(ok))
+                 : "r"(uint32_t(ok)), "n"(32 * Warps)
                  : "memory");
     return result != 0;
 }
@@ -135,8 +142,8 @@ __device__ __forceinline__ void store_global32(void *p, const uint32_t (&r)[8], 
 // cta_group::2 MMAs issued by the pair's first CTA.  Each CTA stages its own 128 rows of A and half
 // of the B tile (the tensor core reads the other half from the partner's shared memory), so a
 // K block costs each SM 16 KB + BN/2 x 128 B instead of 16 KB + BN x 128 B and the ring is deeper.
-template <int Kind, bool OutFp32, bool Pair>
-__global__ void __launch_bounds__(Threads, 1)
+template <int Kind, bool OutFp32, bool Pair, int EpilogueWarps>
+__global__ void __launch_bounds__(threads_of(EpilogueWarps), EpilogueWarps == 8 ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcParams p) {
     extern __shared__ uint8_t raw_shared[];
     const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
@@ -170,10 +177,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     if (warp == 1) {
         if constexpr (Pair) {
-            tmem_alloc_pair(smem_address(tmem_slot), TmemColumns);
+            tmem_alloc_pair(smem_address(tmem_slot), p.tmem_columns);
             tmem_relinquish_pair();
         } else {
-            tmem_alloc(smem_address(tmem_slot), TmemColumns);
+            tmem_alloc(smem_address(tmem_slot), p.tmem_columns);
             tmem_relinquish();
         }
     }
@@ -307,8 +314,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else {
-        // ---------------- epilogue: 16 warps; warps q, q+4, q+8, q+12 share TMEM lanes 32q..32q+31 and
-        // take every fourth 32-column chunk.  Four warps per scheduler hide one another's TMEM,
+        // ---------------- epilogue: 16 (8) warps; warps q, q+4, .. share TMEM lanes 32q..32q+31 and
+        // take every fourth (second) 32-column chunk.  Four warps per scheduler hide one another's TMEM,
         // ALU, SFU and global-load latencies (the epilogue math is a dependent chain per element).
         constexpr int Shares = EpilogueWarps / 4;
         const int quarter = warp % 4, share = (warp - 2) / 4;
@@ -341,7 +348,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 fetch_second(share); // on its way while the products are awaited (steps of short products 1 to 1.6 % faster)
             bool ready = mbarrier_wait(tfull0 + 8 * buffer, buffer_phase, abort_flag, p.counters, 104);
             if (p.splits > 1 || whole_rows) // the warps meet at named barriers below: leave together or not at all
-                ready = epilogue_all(ready);
+                ready = epilogue_all<EpilogueWarps>(ready);
             if (!ready)
                 break;
             tcgen05_fence_after();
@@ -383,7 +390,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     picked = column == target ? v[j] : picked;
                 }
                 row_high[share * BM + local] = high;
-                asm volatile("bar.sync 1, 512;" ::: "memory");
+                epilogue_barrier<EpilogueWarps>();
                 high = fmaxf(fmaxf(row_high[local], row_high[BM + local]), fmaxf(row_high[2 * BM + local], row_high[3 * BM + local]));
                 float sum = 0.f;
 #pragma unroll
@@ -392,7 +399,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     sum += v[j];
                 }
                 row_sum[share * BM + local] = sum;
-                asm volatile("bar.sync 1, 512;" ::: "memory");
+                epilogue_barrier<EpilogueWarps>();
                 sum = ((row_sum[local] + row_sum[BM + local]) + row_sum[2 * BM + local]) + row_sum[3 * BM + local];
                 if (row_ok) {
                     if (target / 32 % Shares == share)
@@ -534,7 +541,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 // Ticket: the split that arrives last reduces the tile in split order.
                 __threadfence();
-                asm volatile("bar.sync 1, 512;" ::: "memory");
+                epilogue_barrier<EpilogueWarps>();
                 if (threadIdx.x == 64) {
                     unsigned ticket = atomicAdd(&p.tickets[t * Unit + rank], 1u);
                     int last = ticket == unsigned(p.splits - 1);
@@ -542,7 +549,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         p.tickets[t * Unit + rank] = 0; // ready for the next launch
                     last_split_flag[0] = last;
                 }
-                asm volatile("bar.sync 1, 512;" ::: "memory");
+                epilogue_barrier<EpilogueWarps>();
                 if (last_split_flag[0]) {
                     __threadfence();
                     for (int chunk = share; chunk < p.bn / 32; chunk += Shares) {
@@ -575,7 +582,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         }
                     }
                 }
-                asm volatile("bar.sync 1, 512;" ::: "memory"); // last_split_flag is reused next tile
+                epilogue_barrier<EpilogueWarps>(); // last_split_flag is reused next tile
             }
             if (++buffer == 2) {
                 buffer = 0;
@@ -594,10 +601,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if constexpr (Pair) {
         cluster_sync_all(); // neither CTA's tensor or shared memory is released while the other may touch it
         if (warp == 1)
-            tmem_dealloc_pair(tmem_base, TmemColumns);
+            tmem_dealloc_pair(tmem_base, p.tmem_columns);
     } else {
         if (warp == 1)
-            tmem_dealloc(tmem_base, TmemColumns);
+            tmem_dealloc(tmem_base, p.tmem_columns);
     }
 }
 
@@ -823,7 +830,10 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
     const int bn_local = p.bn / unit;
     const int stage_bytes = StageABytes + bn_local * BK * 2;
     const int row_scratch = g.epilogue == Epilogue::CrossEntropy ? RowScratchBytes : 0;
-    p.stages = (MaxShared - 1024 - ControlBytes - row_scratch) / stage_bytes;
+    const bool half = g.batch > 1 && !p.out_fp32 && (g.epilogue == Epilogue::Store || g.epilogue == Epilogue::Axpby) && !sc.pair &&
+                      sc.bn <= 128 && tiles * p.splits <= sms;
+    p.tmem_columns = half ? sc.bn : 2 * MaxBN;
+    p.stages = ((half ? HalfShared : MaxShared) - 1024 - ControlBytes - row_scratch) / stage_bytes;
     if (p.stages > MaxStages)
         p.stages = MaxStages;
     const int shared = p.stages * stage_bytes + ControlBytes + row_scratch + 1024;
@@ -863,7 +873,7 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
             }
         }
         cudaLaunchConfig_t config{};
-        config.gridDim = dim3(grid), config.blockDim = dim3(Threads);
+        config.gridDim = dim3(grid), config.blockDim = dim3(threads_of(half ? 8 : 16));
         config.dynamicSmemBytes = shared, config.stream = s;
         cudaLaunchAttribute attributes[2]{};
         attributes[0].id = cudaLaunchAttributeClusterDimension;
@@ -878,22 +888,26 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
         constexpr bool P = decltype(pair_tag)::value;
         if (p.out_fp32) {
             if (g.epilogue == Epilogue::Axpby)
-                launch(gemm_tc_kernel<int(Epilogue::Axpby), true, P>);
+                launch(gemm_tc_kernel<int(Epilogue::Axpby), true, P, 16>);
             else
-                launch(gemm_tc_kernel<int(Epilogue::Store), true, P>);
+                launch(gemm_tc_kernel<int(Epilogue::Store), true, P, 16>);
         } else {
             switch (g.epilogue) {
-            case Epilogue::Store: launch(gemm_tc_kernel<int(Epilogue::Store), false, P>); break;
-            case Epilogue::Residual: launch(gemm_tc_kernel<int(Epilogue::Residual), false, P>); break;
-            case Epilogue::GeluDual: launch(gemm_tc_kernel<int(Epilogue::GeluDual), false, P>); break;
-            case Epilogue::GeluGrad: launch(gemm_tc_kernel<int(Epilogue::GeluGrad), false, P>); break;
-            case Epilogue::Axpby: launch(gemm_tc_kernel<int(Epilogue::Axpby), false, P>); break;
-            case Epilogue::CrossEntropy: launch(gemm_tc_kernel<int(Epilogue::CrossEntropy), false, P>); break;
+            case Epilogue::Store: launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16>); break;
+            case Epilogue::Residual: launch(gemm_tc_kernel<int(Epilogue::Residual), false, P, 16>); break;
+            case Epilogue::GeluDual: launch(gemm_tc_kernel<int(Epilogue::GeluDual), false, P, 16>); break;
+            case Epilogue::GeluGrad: launch(gemm_tc_kernel<int(Epilogue::GeluGrad), false, P, 16>); break;
+            case Epilogue::Axpby: launch(gemm_tc_kernel<int(Epilogue::Axpby), false, P, 16>); break;
+            case Epilogue::CrossEntropy: launch(gemm_tc_kernel<int(Epilogue::CrossEntropy), false, P, 16>); break;
             }
         }
     };
     if (sc.pair)
         launch_kind(std::true_type{});
+    else if (half && g.epilogue == Epilogue::Store)
+        launch(gemm_tc_kernel<int(Epilogue::Store), false, false, 8>);
+    else if (half)
+        launch(gemm_tc_kernel<int(Epilogue::Axpby), false, false, 8>);
     else
         launch_kind(std::false_type{});
     CHECK_CUDA(cudaGetLastError());
