@@ -83,11 +83,34 @@ def test_step_matches_the_operator_path(depth, context, batch):
 
 
 @pytest.mark.parametrize("depth,context,batch", [
-    (2, 80, 2), (2, 96, 150), (3, 100, 4),  # 5, 6 (two rounds) and 7 row tiles of a block: teams of three, of two and of two
-    (3, 16, 149 * 2 + 1), (16, 32, 3)])     # two and three row tiles: the weight gradients beside the next layer (two rounds), and not
-def test_teams_of_two_and_three_warps_per_row_tile(depth, context, batch):
+    (2, 80, 2), (2, 96, 150), (3, 100, 4),       # 5, 6 (two rounds) and 7 row tiles of a block: no helpers
+    (3, 16, 149 * 2 + 1), (16, 32, 3),           # 3 and 2: helpers, and the weight gradients beside the next layer
+    (16, 32, 150), (16, 16, 500), (12, 16, 800)])  # 2, 2 and 3, in two rounds: gradients added to the first tile's as they come
+def test_tiles_with_helpers_and_without(depth, context, batch):
     """The same bounds as everywhere."""
     test_step_matches_the_operator_path(depth, context, batch)
+
+
+def test_no_bit_of_a_token_depends_on_the_tile_it_is_in():
+    """15 sequences over 15, 8, 5, 3, 2 and 1 blocks: 1, 2 and 3 row tiles of a block, with helpers, 5 and 8 without, in one
+    or two rounds.  Activations are a token's own; and as every byte occurs once, so is its embedding's gradient.
+    (60 batches: sums in another order flip about one BF16 rounding in 30000.)"""
+    rng = np.random.default_rng(11)
+    inputs = [(rng.permutation(256)[:240].astype(np.uint8).reshape(15, 16), rng.integers(0, 256, (15, 16), dtype=np.uint8))
+              for _ in range(60)]
+    results = []
+    for blocks in (15, 8, 5, 3, 2, 1):
+        ex = ConfigEx.reference(Config(depth=4, context=16, batch=15, blocks=blocks, clip=0))
+        w, outputs = bridge.initialize_weights(ex) * 8, []  # branches of the residual stream's own size
+        with Native(ex) as engine:
+            for x, y in inputs:
+                engine.set_weights(w)
+                engine.train_batch(x, y)
+                outputs += [engine.activation(-1, "final_x"), engine.optimizer_state()[0][:4096]]
+        results.append(outputs)
+    assert np.count_nonzero(results[0][-1]) > 3000
+    for other in results[1:]:
+        assert sum(np.count_nonzero(a != b) for a, b in zip(results[0], other)) == 0
 
 
 @pytest.mark.parametrize("depth,context,batch", [(4, 4, 16), (2, 5, 7), (8, 8, 2001)])

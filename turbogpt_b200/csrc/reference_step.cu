@@ -3,8 +3,8 @@
 //
 // What bounds it: a token's whole step is 52 k multiply-adds over matrices of 16 columns, so as separate
 // kernels (one per operator, ~150 launches) a step is launch latency and half-empty tiles: 1.43 ms at depth 4,
-// context 4, batch 2880, and 0.86 ms at batch 16 (now 49 and 33 us with reduction and update: the latency of the chain of
-// dependent products, at three warps for every 16 tokens; 50 and 37 us with one).  Here a block takes whole sequences (up to 128 tokens) through
+// context 4, batch 2880, and 0.86 ms at batch 16 (now 49 and 31 us with reduction and update: the latency of the chain of
+// dependent products).  Here a block takes whole sequences (up to 128 tokens) through
 // every layer and back: each warp keeps its 16 tokens' residual stream in registers, the weights sit in shared
 // memory once, and only k and v (forward) and the attention gradients (backward) pass between warps.
 //
@@ -43,6 +43,7 @@ constexpr int RowsQkv = 0, RowsAttention = 48, RowsWide = 64, RowsDown = 160, La
 constexpr int PitchWide = 208, PitchHidden = 112, PitchQkv = 112, PitchWidth = 48, PitchLogits = 528;
 constexpr int StageBytesPerRow = PitchWide + PitchHidden + PitchQkv + 5 * PitchWidth;
 constexpr int MaxShared = 232448;
+constexpr int TeamRows = 48; // rows of the largest tile whose owners have helpers: see below
 struct StepShared {
     int weights, scales, rope, bytes, saved_x, saved_middle, saved_top, selected, exchange, dy, dt_gate, norm_sums, row_sums, stage, total;
     bool overlap; // two stages: a layer's weight gradients are taken by the warps without rows while the others are at the next layer
@@ -67,8 +68,8 @@ struct StepShared {
         norm_sums = take(StepWarps * 2 * Width * 4); // of every second layer in its second half: at most eight warps own rows
         row_sums = take(rows * StepWarps * 8);
         stage = take(rows * StageBytesPerRow);
-        // up to two row tiles ten warps or more have no part in them
-        overlap = rows <= 32 && at + rows * StageBytesPerRow <= MaxShared;
+        // up to three row tiles seven warps or more have no part in them
+        overlap = rows <= TeamRows && at + rows * StageBytesPerRow <= MaxShared;
         if (overlap)
             take(rows * StageBytesPerRow);
         total = at;
@@ -362,28 +363,25 @@ __device__ __forceinline__ void weight_gradient(float *out, int columns, uint32_
     add_gradient(out, columns, acc, accumulate, lane);
 }
 
-// A tile's 16 rows belong to one warp, its owner; the warps that own none help: one or two more per tile take a share of its
-// products (a third of the MLP's columns, parts of q, k and v), which otherwise follow one another in one warp, a chain of
-// dependent instructions that leaves the SM idle.  The shares of a sum meet in shared memory and are added in a fixed order.
-// [from, to) of the three 16-column groups that a member of a team of two or three takes: of the MLP, of q, k and v going
-// forward, and when they are recomputed going back (while the owner is at the norm and the attention projection).
-struct Share {
+// A tile's 16 rows belong to one warp, its owner.  In tiles of up to TeamRows rows two other warps help each owner and take a third
+// of its products each (of the MLP's columns, of q, k and v), which otherwise follow one another in one warp, a chain of dependent
+// instructions that leaves the SM idle; the warps that are left take the weight gradients of a layer beside the next one.  Where the
+// line lies, us a step without and with: 16 rows, depth 4 35.8 and 30.9; 32 rows, context 4 40.2 and 36.4, depth 16 239 and 214;
+// 48 rows, context 4 41.3 and 39.2, depth 8 64.2 and 60.2; 64 rows, context 16 47.3 and 48.1, context 64 68.1 and 71.1; 80 rows,
+// where one warp is left for the gradients, 49.5 and 60.8.
+// What a helper hands over are factors, never a part of a sum: the owner multiplies them into its one accumulator in the order of
+// the columns, so that no bit depends on the tile.
+struct Share { // [from, to) of the three 16-column groups that a warp takes: of the MLP, and of q, k and v going forward
     int from, to;
 };
-__device__ __forceinline__ Share mlp_share_of(int team, int member) {
-    return team == 3 ? Share{member, member + 1} : member ? Share{2, 3} : Share{0, 2};
-}
-__device__ __forceinline__ Share qkv_share_of(int team, int member) {
-    return team == 3 ? Share{member, member + 1} : member ? Share{1, 3} : Share{0, 1};
-}
-__device__ __forceinline__ Share qkv_back_share_of(int team, int member) {
-    return member == 0 ? Share{0, 0} : member == 2 ? Share{2, 3} : Share{0, team == 3 ? 2 : 3};
-}
+// Of q, k and v when they are recomputed going back, while the owner is at the norm and the attention projection.
+__device__ __forceinline__ Share qkv_back_share_of(int member) { return member == 0 ? Share{0, 0} : member == 1 ? Share{0, 2} : Share{2, 3}; }
 
 // The kernel's code is kept short (loops are rolled, one call site for the weight gradients): a block's warps run it once
 // per layer with little to overlap, and unrolled it was bound by instruction fetch (4.4 of 9 cycles per instruction).
 // Sixteen warps although eight own rows at most: the head and the weight gradients are shared by all, the layers by teams.
-template <bool Save> // also write the activations to p.saved
+// Save: also write the activations to p.saved.  Teams: see TeamRows.
+template <bool Save, bool Teams>
 __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __grid_constant__ StepParams p) {
     extern __shared__ __align__(16) uint8_t shared[];
     const StepShared at(p.depth, p.rows, p.context);
@@ -393,7 +391,7 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
     const float2 *rope = reinterpret_cast<const float2 *>(shared + at.rope);
     uint8_t *xs = shared + at.bytes, *ys = xs + p.rows;
     float2 *dt_gate = reinterpret_cast<float2 *>(shared + at.dt_gate);
-    float *norm_sums = reinterpret_cast<float *>(shared + at.norm_sums); // [warp][two norms][16]
+    float *norm_sums = reinterpret_cast<float *>(shared + at.norm_sums); // [layer's parity][row tile][two norms][16]
     float2 *row_sums = reinterpret_cast<float2 *>(shared + at.row_sums); // [row][warp]: maximum, sum of exponentials
     uint8_t *stage = shared + at.stage;
     const int s_wide = 0, s_hidden = s_wide + p.rows * PitchWide, s_qkv = s_hidden + p.rows * PitchHidden,
@@ -467,32 +465,43 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
         scales[i] = join_weight(p.weight_high[from + i % Width], p.weight_low[from + i % Width]);
     }
 
-    const int row_tiles = p.rows / 16, team = min(3, StepWarps / row_tiles); // at most 8 row tiles: two or three
-    int own = warp % row_tiles, member = warp / row_tiles; // the warp's 16 rows, and its place in the team at them
-    asm volatile("" : "+r"(own), "+r"(member));            // kept, not divided out again at every use
+    constexpr int Team = Teams ? 3 : 1;
+    const int row_tiles = p.rows / 16;
+    int own = Teams ? warp % row_tiles : warp, member = Teams ? warp / row_tiles : 0; // the warp's 16 rows, its place in the team at them
+    asm volatile("" : "+r"(own), "+r"(member));                                       // kept, not divided out again at every use
     const int row0 = own * 16;
-    const bool mine = member == 0, active = member < team; // the warp owns the rows; it has a share in them
-    const Share mlp_share = mlp_share_of(team, member), qkv_share = qkv_share_of(team, member), qkv_back_share = qkv_back_share_of(team, member);
-    auto team_barrier = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + own), "r"(32 * team) : "memory"); };
-    // 32 bytes per lane and helper in the memory of the head's row sums: the helper's share of a sum, or the owner's gradient for it
-    auto helper_slot = [&](int helper) { return reinterpret_cast<float4 *>(shared + at.row_sums + ((own * 2 + helper - 1) * 32 + lane) * 32); };
-    auto add_shares = [&](Tile &v) {
-#pragma unroll 1
-        for (int helper = 1; helper < team; ++helper) {
-            const float4 a = helper_slot(helper)[0], b = helper_slot(helper)[1];
-            v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w, v[4] += b.x, v[5] += b.y, v[6] += b.z, v[7] += b.w;
+    const bool mine = Teams ? member == 0 : own < row_tiles, active = Teams ? member < Team : mine; // owns the rows; has a share in them
+    const Share share = Teams ? Share{member, member + 1} : Share{0, 3}, qkv_back_share = Teams ? qkv_back_share_of(member) : share;
+    auto team_barrier = [&] {
+        if constexpr (Teams)
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + own), "n"(32 * Team) : "memory");
+    };
+    // The owner's rows as the helpers read them, after it has put them there.
+    auto as_kept = [&](const uint4 *slot, const Tile &owners, Tile &v) {
+        if constexpr (Teams) {
+            unpack_tile(*slot, v);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = owners[i];
         }
     };
-    auto hand_in = [&](const Tile &v) {
-        helper_slot(member)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        helper_slot(member)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    // 32 bytes per lane and helper in the memory of the head's row sums: two packed tiles, the helper's or, going back, first the
+    // owner's gradient for it
+    auto helper_slot = [&](int helper) { return reinterpret_cast<uint4 *>(shared + at.row_sums + ((own * 2 + helper - 1) * 32 + lane) * 32); };
+    auto hand_in = [&](int which, const uint32_t (&v)[4]) { helper_slot(member)[which] = make_uint4(v[0], v[1], v[2], v[3]); };
+    auto handed_in = [&](int helper, int which, uint32_t (&v)[4]) {
+        const uint4 u = helper_slot(helper)[which];
+        v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w;
     };
     auto hand_out = [&](const Tile &v) { // the owner's rows, rounded
-        uint32_t packed[4];
-        pack_tile(v, packed);
-#pragma unroll 1
-        for (int helper = 1; helper < team; ++helper)
-            *reinterpret_cast<uint4 *>(helper_slot(helper)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        if constexpr (Teams) {
+            uint32_t packed[4];
+            pack_tile(v, packed);
+#pragma unroll
+            for (int helper = 1; helper < Team; ++helper)
+                helper_slot(helper)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        }
     };
     // rows g and g + 8: position inside the sequence and the sequence's first row
     int start[2], position[2];
@@ -567,8 +576,8 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             if (active) {
                 team_barrier();
                 Tile input, normed;
-                unpack_tile(*saved_slot(at.saved_x, l), input);
-                project_qkv(l, panel, input, normed, buffer, qkv_share);
+                as_kept(saved_slot(at.saved_x, l), x, input);
+                project_qkv(l, panel, input, normed, buffer, share);
                 if (mine) {
                     save(p.saved.layer[l].x, Width, 0, false, x);
                     save(p.saved.layer[l].normed1, Width, 0, false, normed);
@@ -625,13 +634,13 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             }
             team_barrier();
             Tile middle, normed, down = {};
-            unpack_tile(*saved_slot(at.saved_middle, l), middle);
+            as_kept(saved_slot(at.saved_middle, l), x, middle);
             rms_norm(middle, Scale(scales + (2 * l + 1) * Width, t), normed);
             if (mine)
                 save(p.saved.layer[l].normed2, Width, 0, false, normed);
             pack_tile(normed, a);
 #pragma unroll 1
-            for (int m = mlp_share.from; m < mlp_share.to; ++m) {
+            for (int m = share.from; m < share.to; ++m) {
                 Tile gate = {}, up = {};
                 multiply(gate, a, panel, RowsWide + 16 * m, lane);
                 multiply(up, a, panel, RowsWide + Hidden + 16 * m, lane);
@@ -639,13 +648,19 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                 save(p.saved.layer[l].activated, Hidden, 16 * m, false, up);
                 uint32_t h[4];
                 pack_tile(up, h);
-                multiply(down, h, panel, RowsDown + 16 * m, lane);
+                if (mine)
+                    multiply(down, h, panel, RowsDown + 16 * m, lane);
+                else
+                    hand_in(0, h);
             }
-            if (!mine)
-                hand_in(down);
             team_barrier();
             if (mine) {
-                add_shares(down);
+#pragma unroll
+                for (int helper = 1; helper < Team; ++helper) {
+                    uint32_t h[4];
+                    handed_in(helper, 0, h);
+                    multiply(down, h, panel, RowsDown + 16 * helper, lane);
+                }
                 add_branch(x, down);
             }
         }
@@ -766,7 +781,8 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
             sum_norm(p.depth % 2, 0, final_norm);
 
         // ---- backward ----
-        const int first_free = at.overlap ? team * row_tiles : 0, stage_apart = at.overlap ? p.rows * StageBytesPerRow : 0;
+        const bool overlap = Teams && at.overlap;
+        const int first_free = overlap ? Team * row_tiles : 0, stage_apart = overlap ? p.rows * StageBytesPerRow : 0;
         for (int l = p.depth - 1; l >= -1; --l) {
             // the 13 weight-gradient tiles of 16 x 16 and two norm scales of the layer that has just been staged
             if (l + 1 < p.depth && warp >= first_free) {
@@ -792,7 +808,7 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                     weight_gradient(partial + layer0 + to, columns, from + dy_at, dy_pitch, from + x_at, x_pitch, p.rows, accumulate, lane);
                 }
             }
-            if (!at.overlap && l + 1 < p.depth)
+            if (!overlap && l + 1 < p.depth)
                 __syncthreads();
             if (l < 0)
                 break;
@@ -813,12 +829,15 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                     put_tile(stage + s_dh + row0 * PitchWidth, PitchWidth, x, g, t);
                     pack_tile(x, dh);
                 } else {
-                    const uint4 u = *reinterpret_cast<const uint4 *>(helper_slot(member));
-                    dh[0] = u.x, dh[1] = u.y, dh[2] = u.z, dh[3] = u.w;
+                    handed_in(member, 0, dh);
                 }
                 Tile branch = {};
+                auto into_branch = [&](int m, const uint32_t (&dgate)[4], const uint32_t (&dup)[4]) {
+                    multiply_transposed(branch, dgate, panel, RowsWide + 16 * m, lane);
+                    multiply_transposed(branch, dup, panel, RowsWide + Hidden + 16 * m, lane);
+                };
 #pragma unroll 1
-                for (int m = mlp_share.from; m < mlp_share.to; ++m) {
+                for (int m = share.from; m < share.to; ++m) {
                     Tile gate = {}, up = {}, dout = {};
                     multiply(gate, a, panel, RowsWide + 16 * m, lane);
                     multiply(up, a, panel, RowsWide + Hidden + 16 * m, lane);
@@ -828,17 +847,23 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
                     put_tile(stage + s_hidden + row0 * PitchHidden + 32 * m, PitchHidden, activated, g, t);
                     put_tile(stage + s_wide + row0 * PitchWide + 32 * m, PitchWide, gate, g, t);
                     put_tile(stage + s_wide + row0 * PitchWide + 2 * Hidden + 32 * m, PitchWide, up, g, t);
-                    uint32_t d[4];
-                    pack_tile(gate, d);
-                    multiply_transposed(branch, d, panel, RowsWide + 16 * m, lane);
-                    pack_tile(up, d);
-                    multiply_transposed(branch, d, panel, RowsWide + Hidden + 16 * m, lane);
+                    uint32_t dgate[4], dup[4];
+                    pack_tile(gate, dgate);
+                    pack_tile(up, dup);
+                    if (mine)
+                        into_branch(m, dgate, dup);
+                    else
+                        hand_in(0, dgate), hand_in(1, dup);
                 }
-                if (!mine)
-                    hand_in(branch);
                 team_barrier();
                 if (mine) {
-                    add_shares(branch);
+#pragma unroll
+                    for (int helper = 1; helper < Team; ++helper) {
+                        uint32_t dgate[4], dup[4];
+                        handed_in(helper, 0, dgate);
+                        handed_in(helper, 1, dup);
+                        into_branch(helper, dgate, dup);
+                    }
                     round_tile(branch);
                     rms_norm_backward(middle, branch, scale, &x, x, norm_sums + ((l % 2 * MaxRowTiles + own) * 2 + 1) * Width, lane);
                     put_tile(stage + s_dh2 + row0 * PitchWidth, PitchWidth, x, g, t);
@@ -1094,7 +1119,8 @@ void launch_reference_step(const ReferenceStepArgs &a, const ReferenceStepPlan &
     if (a.save)
         p.saved = *a.save;
     const int shared = StepShared(a.depth, plan.rows, a.context).total;
-    auto *kernel = a.save ? reference_step_kernel<true> : reference_step_kernel<false>;
+    auto *kernel = plan.rows <= TeamRows ? a.save ? reference_step_kernel<true, true> : reference_step_kernel<false, true>
+                                         : a.save ? reference_step_kernel<true, false> : reference_step_kernel<false, false>;
     CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MaxShared));
     // Launched programmatically: each kernel's set-up overlaps the tail of the one before it.
     cudaLaunchAttribute attribute{};
