@@ -190,6 +190,10 @@ int tg_ex_selftest_bounded_wait(Engine *engine, double limit_ms);
  * cuda/mma.cuh:77-108 and cuda/ops.cuh:30-55,83-109.  out_fp32: C is float, else BF16. */
 int tg_ex_gemm(const void *a, int64_t a_row, int64_t a_col, const void *b, int64_t b_row, int64_t b_col,
                void *c, int64_t ldc, int m, int n, int k, int out_fp32, int tensor_cores, void *stream);
+/* Diagnostic: how tg_ex_gemm runs a product on the tensor cores of a GPU with `sms` SMs.  schedule[3]: columns of a tile,
+ * parts that K is cut into, whether two CTAs share a tile of 256 rows (else one takes 128).  Touches no device. */
+int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_col, int64_t ldc, int m, int n, int k, int out_fp32,
+                        int sms, int32_t *schedule);
 /* No counterpart in the reference (its engine allocates everything in tg_create).  Weight gradient
  * dw[out, in] (FP32) = dy[tokens, out]^T x[tokens, in] (BF16, row-major, device pointers) for callers
  * that must not allocate device memory when they need it — a process whose memory pool already owns

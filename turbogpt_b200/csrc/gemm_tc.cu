@@ -662,7 +662,9 @@ struct Schedule {
 // What a schedule costs, in nanoseconds: launch + rounds of tiles x (64-deep K blocks x block + tile).  Fitted to 832 products
 // of 256 to 32768 tokens and widths 128 to 1024 (activations and input gradients, K-major and MN-major B), each timed with every
 // tile width, single and paired; the model reproduces the times within 5 to 8 % and its choice is 0.3 % slower than the best of
-// each (geometric mean).  A pair's launch costs 0.9 us more and its tiles take longer to hand over, single CTAs read more
+// each (geometric mean).  The costs below for rows off the cache lines are fitted to 824 more, of odd multiples of eight: without
+// them the choice was 1.6 % slower than the best of each and in the worst cases took wide single tiles where pairs of them, which
+// stage fewer lines, were a third faster; with them 0.9 %.  A pair's launch costs 0.9 us more and its tiles take longer to hand over, single CTAs read more
 // operand bytes per product: pairs are for many rounds over a long K.  The model before it (MMA and shared-memory clocks, no
 // launch or tile times) chose 8 % slower on average: 4096 x 768 x 2304 17.4 -> 13.9 us, 8192 x 2048 x 512 25.1 -> 18.5,
 // 1024 x 2304 x 768 7.5 -> 6.4, 32768 x 512 x 128 21.9 -> 13.5.  The tile's shape does not change a result: every element
@@ -673,6 +675,10 @@ struct TileCost {
 constexpr TileCost SingleCost[] = {{256, 342, 1500}, {192, 262, 1280}, {128, 209, 940}, {64, 184, 550}};
 constexpr TileCost PairCost[] = {{256, 284, 2100}, {192, 211, 1900}, {128, 188, 1450}};
 constexpr int SingleLaunch = 3240, PairLaunch = 4100;
+// Rows that do not start on a cache line take two of them for one, and those off a 32-byte sector five sectors for four: picoseconds
+// per 128-byte line of an operand and 64-deep K block (the first is hidden where a pair stages half of B).  Rows of C off a sector
+// are written in parts: nanoseconds per tile column.
+constexpr int LineCost = 140, SectorCost = 500, RaggedStoreCost = 4;
 // A K split of n: partial tiles, fence, ticket and read-back by one SM, or from four on a second launch, and the partial tiles'
 // passes through memory.
 constexpr long long split_cost(int splits, int bn, long long outputs) {
@@ -683,30 +689,45 @@ Schedule product_schedule(const GemmArgs &g, int sms) {
     const bool plain = g.epilogue == Epilogue::Store; // K is split only for plain stores
     const bool whole_rows = g.epilogue == Epilogue::CrossEntropy; // a tile must hold complete rows
     const int m_tiles = (g.m + BM - 1) / BM, k_blocks = (g.k + BK - 1) / BK;
+    const int64_t a_pitch = g.a_col == 1 ? g.a_row : g.a_col, b_pitch = b_mn ? g.b_col : g.b_row; // elements of two bytes
+    auto lines_off = [&](int bytes, int b_rows) { return (a_pitch * 2 % bytes ? BM : 0) + (b_pitch * 2 % bytes ? b_rows : 0); };
     Schedule best;
     long long best_time = 0;
-    auto consider = [&](const TileCost &cost, int unit, int launch) {
+    // `splits_allowed`: 0 for any number of them, at the costs of aligned rows; otherwise that many, at the operands' own costs.
+    auto consider = [&](const TileCost &cost, int unit, int launch, int splits_allowed) {
         const int bn = cost.bn, slots = sms / unit;
         if ((bn > 64 && bn - 64 >= g.n) || (whole_rows && bn != 256))
             return; // a narrower tile already covers N
         if (unit == 2 && b_mn && bn == 192)
             return; // each CTA stages bn/2 rows of B: whole 64-row blocks when B is MN-major
+        int block = cost.block, tile = cost.tile;
+        if (splits_allowed) {
+            block += ((unit == 1 ? LineCost * lines_off(128, bn) : 0) + SectorCost * lines_off(32, bn / unit)) / 1000;
+            tile += g.ldc * int(dtype_size(g.out)) % 32 ? RaggedStoreCost * bn : 0;
+        }
         const long long tiles = (long long)((m_tiles + unit - 1) / unit) * ((g.n + bn - 1) / bn) * g.batch;
         for (int splits : {1, 2, 3, 4, 6, 8, 12, 16}) {
             const int per = (k_blocks + splits - 1) / splits;
             if (splits > 1 && (!plain || k_blocks / splits < 8 || tiles * splits > slots || (k_blocks + per - 1) / per != splits))
                 continue; // the last: would leave an empty split
+            if (splits_allowed && splits != splits_allowed)
+                continue;
             const long long rounds = (tiles * splits + slots - 1) / slots;
-            const long long time = launch + rounds * ((long long)per * cost.block + cost.tile) + split_cost(splits, bn, (long long)g.m * g.n * g.batch);
+            const long long time = launch + rounds * ((long long)per * block + tile) + split_cost(splits, bn, (long long)g.m * g.n * g.batch);
             if (!best.bn || time < best_time)
                 best.bn = bn, best.splits = splits, best.k_blocks_per_split = per, best.pair = unit == 2, best_time = time;
         }
     };
-    if (m_tiles >= 2 && sms >= 2)
-        for (const TileCost &cost : PairCost)
-            consider(cost, 2, PairLaunch);
-    for (const TileCost &cost : SingleCost)
-        consider(cost, 1, SingleLaunch);
+    auto consider_all = [&](int splits_allowed) {
+        best = {};
+        if (m_tiles >= 2 && sms >= 2)
+            for (const TileCost &cost : PairCost)
+                consider(cost, 2, PairLaunch, splits_allowed);
+        for (const TileCost &cost : SingleCost)
+            consider(cost, 1, SingleLaunch, splits_allowed);
+    };
+    consider_all(0); // how often K is cut decides the order of the sums: the alignment of the rows has no say in it
+    consider_all(best.splits);
     return best;
 }
 
@@ -1019,6 +1040,10 @@ static __device__ __align__(256) unsigned char static_scratch[StaticErrorOffset 
 void *static_scratch_address[64] = {}; // per device, filled on first use
 } // namespace
 
+GemmSchedule gemm_tc_schedule(const GemmArgs &g, int sms) {
+    const Schedule sc = choose_schedule(g, sms);
+    return {sc.bn, sc.splits, sc.pair};
+}
 size_t gemm_tc_static_scratch_bytes() { return StaticPartialBytes; }
 
 void launch_weight_gradient_static(const void *dy, const void *x, float *dw, int out, int in, int tokens,

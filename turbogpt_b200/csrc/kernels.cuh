@@ -199,6 +199,10 @@ void release_gemm_workspace(GemmWorkspace &w);
 int launch_gemm_tc(const GemmArgs &g, int sms, StepCounters *counters, cudaStream_t s,
                     GemmWorkspace *workspace = nullptr);
 int gemm_tc_shared_bytes();
+struct GemmSchedule {
+    int tile_columns, splits, pair;
+};
+GemmSchedule gemm_tc_schedule(const GemmArgs &g, int sms); // what launch_gemm_tc runs; touches no device
 int gemm_tc_take_device_error(cudaStream_t s);
 // Weight gradient dW[out, in] = dy^T x whose split-K scratch is a fixed array inside the library:
 // allocates nothing (see gemm_tc.cu).  Throws when the shape needs more scratch than the array holds.

@@ -306,6 +306,18 @@ int tg_ex_gemm(const void *a, int64_t a_row, int64_t a_col, const void *b, int64
         CHECK_CUDA(cudaGetLastError());
     });
 }
+int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_col, int64_t ldc, int m, int n, int k, int out_fp32,
+                        int sms, int32_t *schedule) {
+    return guarded([&] {
+        GemmArgs g;
+        g.a_row = a_row, g.a_col = a_col, g.b_row = b_row, g.b_col = b_col, g.ldc = ldc;
+        g.m = m, g.n = n, g.k = k, g.out = out_fp32 ? Dtype::FP32 : Dtype::BF16;
+        if (!schedule || sms < 1 || !gemm_tc_supported(g))
+            throw std::runtime_error("GEMM shape or layout is outside the tensor-core kernel's range");
+        const GemmSchedule s = gemm_tc_schedule(g, sms);
+        schedule[0] = s.tile_columns, schedule[1] = s.splits, schedule[2] = s.pair;
+    });
+}
 int tg_ex_head_cross_entropy(const void *x, const void *head, const uint8_t *targets, float *losses, void *dlogits,
                              int rows, int width, float scale, void *stream) {
     return guarded([&] {
