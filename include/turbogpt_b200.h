@@ -190,10 +190,18 @@ int tg_ex_selftest_bounded_wait(Engine *engine, double limit_ms);
  * cuda/mma.cuh:77-108 and cuda/ops.cuh:30-55,83-109.  out_fp32: C is float, else BF16. */
 int tg_ex_gemm(const void *a, int64_t a_row, int64_t a_col, const void *b, int64_t b_row, int64_t b_col,
                void *c, int64_t ldc, int m, int n, int k, int out_fp32, int tensor_cores, void *stream);
-/* Diagnostic: how tg_ex_gemm runs a product on the tensor cores of a GPU with `sms` SMs.  schedule[3]: columns of a tile,
- * parts that K is cut into, whether two CTAs share a tile of 256 rows (else one takes 128).  Touches no device. */
-int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_col, int64_t ldc, int m, int n, int k, int out_fp32,
-                        int sms, int32_t *schedule);
+/* C_z[M,N] = A_z . B_z^T, or alpha A_z . B_z^T + beta R_z where r is not NULL (R laid out as C), for z < batch; BF16, on the
+ * tensor cores, element strides as in tg_ex_gemm and between the matrices of a batch.  These are the products of Muon's
+ * Newton-Schulz iterations (cuda/optim.cuh:60-106).  beside_others: others run on the GPU at the same time, so a product of few
+ * tiles takes half of an SM for each (the same results). */
+int tg_ex_gemm_batched(const void *a, int64_t a_row, int64_t a_col, int64_t a_batch, const void *b, int64_t b_row, int64_t b_col,
+                       int64_t b_batch, void *c, int64_t ldc, int64_t c_batch, const void *r, float alpha, float beta, int m, int n,
+                       int k, int batch, int beside_others, void *stream);
+/* Diagnostic: how tg_ex_gemm (batch 1) and tg_ex_gemm_batched run a product on the tensor cores of a GPU with `sms` SMs.
+ * schedule[4]: columns of a tile, parts that K is cut into, whether two CTAs share a tile of 256 rows (else one takes 128),
+ * whether a tile takes half an SM.  Touches no device. */
+int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_col, int64_t ldc, int m, int n, int k, int batch,
+                        int out_fp32, int beside_others, int sms, int32_t *schedule);
 /* No counterpart in the reference (its engine allocates everything in tg_create).  Weight gradient
  * dw[out, in] (FP32) = dy[tokens, out]^T x[tokens, in] (BF16, row-major, device pointers) for callers
  * that must not allocate device memory when they need it — a process whose memory pool already owns

@@ -6,11 +6,17 @@ import pytest
 SMS = 148
 
 
-def schedule(library, m, n, k, b_mn=False, out_fp32=False, ldc=None):
-    plan = (C.c_int32 * 3)()
-    b = (1, n) if b_mn else (k, 1)
-    assert library.tg_ex_gemm_schedule(k, 1, *b, ldc or n, m, n, k, int(out_fp32), SMS, plan) == 0, library.tg_error()
+def schedule(library, m, n, k, b_mn=False, batch=1, beside_others=False, pitch=lambda x: x):
+    """(tile columns, K splits, CTA pair, half an SM)"""
+    plan = (C.c_int32 * 4)()
+    b = (1, pitch(n)) if b_mn else (pitch(k), 1)
+    assert library.tg_ex_gemm_schedule(pitch(k), 1, *b, pitch(n), m, n, k, batch, 0, int(beside_others), SMS, plan) == 0, \
+        library.tg_error()
     return tuple(plan)
+
+
+def whole_lines(elements):
+    return (elements + 63) // 64 * 64
 
 
 # Measured us: the form that costs of aligned rows choose, and the fastest.
@@ -24,12 +30,8 @@ def schedule(library, m, n, k, b_mn=False, out_fp32=False, ldc=None):
     (9158, 3104, 440, False, (256, 1, 0), (256, 1, 1)),   # 43.2, 35.8
     (1425, 1480, 3536, True, (128, 1, 0), (128, 1, 1))])  # 23.3, 18.9
 def test_rows_off_the_cache_lines_are_priced(library, m, n, k, b_mn, aligned_choice, fastest):
-    assert schedule(library, m, n, k, b_mn) == fastest
-    plan = (C.c_int32 * 3)()  # the same product with rows padded to whole cache lines
-    pad = lambda x: (x + 63) // 64 * 64
-    b = (1, pad(n)) if b_mn else (pad(k), 1)
-    assert library.tg_ex_gemm_schedule(pad(k), 1, *b, pad(n), m, n, k, 0, SMS, plan) == 0
-    assert tuple(plan) == aligned_choice
+    assert schedule(library, m, n, k, b_mn)[:3] == fastest
+    assert schedule(library, m, n, k, b_mn, pitch=whole_lines)[:3] == aligned_choice
 
 
 def test_alignment_has_no_say_in_how_often_k_is_cut(library):
@@ -37,16 +39,30 @@ def test_alignment_has_no_say_in_how_often_k_is_cut(library):
     for m in (16, 100, 260, 445, 1140, 5000):
         for n in range(72, 1500, 88):
             for k in range(520, 8000, 504):
-                plan = (C.c_int32 * 3)()
-                pad = lambda x: (x + 63) // 64 * 64
-                assert library.tg_ex_gemm_schedule(pad(k), 1, pad(k), 1, pad(n), m, n, k, 0, SMS, plan) == 0
-                assert schedule(library, m, n, k)[1] == plan[1]
-                cut += plan[1] > 1
+                splits = schedule(library, m, n, k)[1]
+                assert splits == schedule(library, m, n, k, pitch=whole_lines)[1]
+                cut += splits > 1
     assert cut > 100
 
 
+@pytest.mark.parametrize("depth,width", [(6, 384), (3, 320), (2, 1024), (4, 768)])  # the last two: a rank's share of 16 and 12 layers
+def test_half_an_sm_only_beside_others(library, depth, width):
+    """The products of Muon's square and wide matrices: A = X X^T, A A, and B X.  A chain that has the GPU to itself (data
+    parallelism, a profiled engine, a large model) keeps the deep ring."""
+    halves = 0
+    for n in (width, 3 * width, 4 * width):
+        for m, columns, k, b_mn in ((width, width, n, False), (width, width, width, True), (width, n, width, True)):
+            alone = schedule(library, m, columns, k, b_mn, depth)
+            beside = schedule(library, m, columns, k, b_mn, depth, True)
+            assert alone[3] == 0 and beside[:3] == alone[:3]
+            assert not beside[3] or (beside[0] <= 128 and not beside[2])
+            halves += beside[3]
+    assert halves >= 6
+    assert schedule(library, width, width, width, True, 1, True)[3] == 0  # one matrix is no batch
+
+
 def test_what_the_kernel_does_not_take_is_refused(library):
-    plan = (C.c_int32 * 3)()
+    plan = (C.c_int32 * 4)()
     for a_col, n, k in ((1, 60, 64), (1, 68, 64), (1, 64, 32), (2, 64, 64)):
-        assert library.tg_ex_gemm_schedule(k, a_col, k, 1, n, 128, n, k, 0, SMS, plan) < 0
+        assert library.tg_ex_gemm_schedule(k, a_col, k, 1, n, 128, n, k, 1, 0, 0, SMS, plan) < 0
         assert b"outside the tensor-core" in library.tg_error()

@@ -1,5 +1,7 @@
 """Kernel-level GPU checks through the C-ABI microbenchmark entry points: the tcgen05 GEMM in
 all operand layouts against an FP32 product, attention and cross-entropy against plain PyTorch."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -71,6 +73,48 @@ def test_products_of_every_tile_form_at_their_edges(m, n, k, b_mn):
     torch.cuda.synchronize()
     expected, magnitude = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
     assert ((c.double() - expected).abs() <= k * 2.0 ** -24 * magnitude + 2.0 ** -8 * expected.abs()).all()
+    assert lib.tg_ex_last_device_error(None) == 0
+
+
+@pytest.mark.parametrize("m,n,k,b_mn", [
+    *((m, n, k, b_mn) for k in (64, 72, 192, 320, 1544)  # shorter than the ring of half an SM, as long, round after round
+      for m, n, b_mn in ((320, 320, False), (320, 320, True), (129, 72, True), (64, 64, False),  # 64 columns, four stages
+                         (320, 1928, False), (320, 1928, True))),                                # 128 columns, three stages
+    (129, 72, 3080, True), (320, 320, 3080, False)])                                             # K cut in six, in four
+def test_batched_products_in_half_an_sm(m, n, k, b_mn):
+    """Partial tiles in every dimension against 64 bits, both epilogues; two such products run at once, so that blocks of both
+    share SMs; and with an SM for each tile, bit for bit."""
+    lib, batch = load_library(), 3
+    plan = (ctypes.c_int32 * 4)()
+    assert lib.tg_ex_gemm_schedule(k, 1, *((1, n) if b_mn else (k, 1)), n, m, n, k, batch, 0, 1, 148, plan) == 0 and plan[3] == 1
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, b, r = (torch.randn(batch, *shape, generator=g, device="cuda").bfloat16() for shape in ((m, k), (n, k), (m, n)))
+    stored = b.transpose(1, 2).contiguous() if b_mn else b
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+
+    def product(out, second, beside, stream):
+        assert lib.tg_ex_gemm_batched(a.data_ptr(), k, 1, m * k, stored.data_ptr(), *((1, n) if b_mn else (k, 1)), n * k,
+                                      out.data_ptr(), n, m * n, second, 2.0315, -4.775, m, n, k, batch, beside,
+                                      stream.cuda_stream) == 0, lib.tg_error()
+
+    plain, scaled = ([torch.full((batch, m, n), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(9)] for _ in range(2))
+    torch.cuda.synchronize()
+    for p, s in zip(plain[:8], scaled[:8]):
+        product(p, None, 1, streams[0])
+        product(s, r.data_ptr(), 1, streams[1])
+    product(plain[8], None, 0, streams[0])
+    product(scaled[8], r.data_ptr(), 0, streams[1])
+    torch.cuda.synchronize()
+    exact, magnitude = a.double() @ b.double().transpose(1, 2), a.double().abs() @ b.double().abs().transpose(1, 2)
+    # FP32 sums of k exact products, then for the second form two FP32 roundings of either term, and one to BF16
+    bound = k * 2.0 ** -24 * magnitude
+    assert ((plain[0].double() - exact).abs() <= bound + 2.0 ** -8 * exact.abs()).all()
+    expected = 2.0315 * exact - 4.775 * r.double()
+    assert ((scaled[0].double() - expected).abs() <=
+            2.0315 * bound + 2.0 ** -22 * (2.0315 * exact.abs() + 4.775 * r.double().abs()) + 2.0 ** -8 * expected.abs()).all()
+    for p, s in zip(plain[1:], scaled[1:]):
+        assert torch.equal(p, plain[0]) and torch.equal(s, scaled[0])
     assert lib.tg_ex_last_device_error(None) == 0
 
 

@@ -738,7 +738,7 @@ void Engine::muon_family(const MuonFamily &family) {
         x2.out = Dtype::BF16;
         for (GemmArgs *g : {&a, &b, &x2}) {
             run(FMuon, [&](cudaStream_t s) {
-                g->in = Dtype::BF16;
+                g->in = Dtype::BF16, g->beside_others = muon_lanes;
                 if (tensor_cores && gemm_tc_supported(*g))
                     launches += launch_gemm_tc(*g, sms, counters, s, &lanes[lane].workspace) - 1;
                 else

@@ -40,11 +40,12 @@ constexpr int threads_of(int epilogue_warps) { return 64 + 32 * epilogue_warps; 
 constexpr int ControlBytes = 512;   // barriers, TMEM slot, flags
 constexpr int RowScratchBytes = 2 * 4 * BM * 4; // CrossEntropy: row maxima and row sums of the four column shares
 constexpr int MaxShared = 232448 - 1024; // 227 KB less the runtime's own reservation
-// A batched product of at most one tile per SM, up to 128 columns wide, runs in half an SM: eight epilogue warps, one accumulator of
-// its own width, and a ring of half the shared memory.  Those are Muon's Newton-Schulz products where the families' run beside each
-// other on four lanes: 108 to 144 blocks each, one to an SM, kept waiting for one another (6 layers d 384: 4 steps 5400 -> 5150 us,
-// the same bits; two blocks to an SM above one tile per SM measured level).  Products in a chain of their own stay with the deep
-// ring: tg_predict of 12 layers d 768 takes 838 us with halves, 735 without.  Every kernel that takes tensor memory lets its
+// Where the caller says that others run beside it (GemmArgs::beside_others), a batched product of at most one tile per SM, up to 128
+// columns wide, runs in half an SM: eight epilogue warps, one accumulator of its own width, and a ring of half the shared memory.
+// Those are Muon's Newton-Schulz products when the families' chains run beside each other on four lanes: of 60 in a step of 6 layers
+// d 384 the 45 of 128 columns, 108 blocks each, which as whole SMs are kept waiting for one another (4 steps 5400 -> 5150 us, the
+// same bits; two blocks to an SM above one tile per SM measured level).  Products in a chain of their own, a sharded or profiled
+// optimizer's among them, keep the deep ring: tg_predict of 12 layers d 768 takes 838 us with halves, 735 without.  Every kernel that takes tensor memory lets its
 // dependents launch only once it holds it, so none can wait for columns that a kernel waiting for it holds.
 constexpr int HalfShared = 113 * 1024;
 
@@ -788,6 +789,12 @@ Schedule choose_schedule(const GemmArgs &g, int sms) {
     return g.out == Dtype::FP32 && g.epilogue == Epilogue::Store ? weight_gradient_schedule(g, sms) : product_schedule(g, sms);
 }
 
+bool half_an_sm(const GemmArgs &g, const Schedule &sc, int sms) {
+    const long long tiles = (long long)((g.m + BM - 1) / BM) * ((g.n + sc.bn - 1) / sc.bn) * g.batch;
+    return g.beside_others && g.batch > 1 && g.out == Dtype::BF16 && (g.epilogue == Epilogue::Store || g.epilogue == Epilogue::Axpby) &&
+           !sc.pair && sc.bn <= 128 && tiles * sc.splits <= sms;
+}
+
 // Scratch a schedule needs: FP32 partial tiles and one ticket per output tile (none without a K split).
 struct ScratchNeed {
     size_t partial_bytes = 0, tickets = 0;
@@ -851,8 +858,7 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
     const int bn_local = p.bn / unit;
     const int stage_bytes = StageABytes + bn_local * BK * 2;
     const int row_scratch = g.epilogue == Epilogue::CrossEntropy ? RowScratchBytes : 0;
-    const bool half = g.batch > 1 && !p.out_fp32 && (g.epilogue == Epilogue::Store || g.epilogue == Epilogue::Axpby) && !sc.pair &&
-                      sc.bn <= 128 && tiles * p.splits <= sms;
+    const bool half = half_an_sm(g, sc, sms);
     p.tmem_columns = half ? sc.bn : 2 * MaxBN;
     p.stages = ((half ? HalfShared : MaxShared) - 1024 - ControlBytes - row_scratch) / stage_bytes;
     if (p.stages > MaxStages)
@@ -1042,7 +1048,7 @@ void *static_scratch_address[64] = {}; // per device, filled on first use
 
 GemmSchedule gemm_tc_schedule(const GemmArgs &g, int sms) {
     const Schedule sc = choose_schedule(g, sms);
-    return {sc.bn, sc.splits, sc.pair};
+    return {sc.bn, sc.splits, sc.pair, half_an_sm(g, sc, sms)};
 }
 size_t gemm_tc_static_scratch_bytes() { return StaticPartialBytes; }
 

@@ -176,6 +176,7 @@ struct GemmArgs {
     float alpha = 1.f, beta = 0.f;
     int batch = 1;           // batched over z with element strides below
     int64_t a_batch = 0, b_batch = 0, c_batch = 0, r_batch = 0;
+    bool beside_others = false; // other lanes' products run at the same time: leave them half of an SM where that is enough
 };
 // `scratch`: gemm_simt_scratch_bytes(g) bytes for shapes that are cut along K (small outputs over a long K,
 // partial tiles added in a fixed order); nullptr: never cut.
@@ -200,7 +201,7 @@ int launch_gemm_tc(const GemmArgs &g, int sms, StepCounters *counters, cudaStrea
                     GemmWorkspace *workspace = nullptr);
 int gemm_tc_shared_bytes();
 struct GemmSchedule {
-    int tile_columns, splits, pair;
+    int tile_columns, splits, pair, half_an_sm;
 };
 GemmSchedule gemm_tc_schedule(const GemmArgs &g, int sms); // what launch_gemm_tc runs; touches no device
 int gemm_tc_take_device_error(cudaStream_t s);

@@ -306,16 +306,32 @@ int tg_ex_gemm(const void *a, int64_t a_row, int64_t a_col, const void *b, int64
         CHECK_CUDA(cudaGetLastError());
     });
 }
-int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_col, int64_t ldc, int m, int n, int k, int out_fp32,
-                        int sms, int32_t *schedule) {
+int tg_ex_gemm_batched(const void *a, int64_t a_row, int64_t a_col, int64_t a_batch, const void *b, int64_t b_row, int64_t b_col,
+                       int64_t b_batch, void *c, int64_t ldc, int64_t c_batch, const void *r, float alpha, float beta, int m, int n,
+                       int k, int batch, int beside_others, void *stream) {
+    return guarded([&] {
+        require_sm100();
+        GemmArgs g;
+        g.a = a, g.a_row = a_row, g.a_col = a_col, g.a_batch = a_batch, g.b = b, g.b_row = b_row, g.b_col = b_col, g.b_batch = b_batch;
+        g.c = c, g.ldc = ldc, g.c_batch = c_batch, g.m = m, g.n = n, g.k = k, g.batch = batch, g.beside_others = beside_others;
+        if (r)
+            g.epilogue = Epilogue::Axpby, g.r = r, g.ldr = ldc, g.r_batch = c_batch, g.alpha = alpha, g.beta = beta;
+        if (batch < 1 || !gemm_tc_supported(g))
+            throw std::runtime_error("GEMM shape or layout is outside the tensor-core kernel's range");
+        launch_gemm_tc(g, device_sms(), nullptr, static_cast<cudaStream_t>(stream));
+        CHECK_CUDA(cudaGetLastError());
+    });
+}
+int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_col, int64_t ldc, int m, int n, int k, int batch,
+                        int out_fp32, int beside_others, int sms, int32_t *schedule) {
     return guarded([&] {
         GemmArgs g;
         g.a_row = a_row, g.a_col = a_col, g.b_row = b_row, g.b_col = b_col, g.ldc = ldc;
-        g.m = m, g.n = n, g.k = k, g.out = out_fp32 ? Dtype::FP32 : Dtype::BF16;
-        if (!schedule || sms < 1 || !gemm_tc_supported(g))
+        g.m = m, g.n = n, g.k = k, g.batch = batch, g.out = out_fp32 ? Dtype::FP32 : Dtype::BF16, g.beside_others = beside_others;
+        if (!schedule || sms < 1 || batch < 1 || !gemm_tc_supported(g))
             throw std::runtime_error("GEMM shape or layout is outside the tensor-core kernel's range");
         const GemmSchedule s = gemm_tc_schedule(g, sms);
-        schedule[0] = s.tile_columns, schedule[1] = s.splits, schedule[2] = s.pair;
+        schedule[0] = s.tile_columns, schedule[1] = s.splits, schedule[2] = s.pair, schedule[3] = s.half_an_sm;
     });
 }
 int tg_ex_head_cross_entropy(const void *x, const void *head, const uint8_t *targets, float *losses, void *dlogits,
