@@ -268,6 +268,7 @@ void Engine::initialize() {
         if (c.flags & TG_FLAG_BF16_GRADIENT_EXCHANGE)
             allocate(gradient_bf16, P, false);
     }
+    copies.create(layout, depth, !comm); // under data parallelism the gradients are added up over the ranks after the pass
     CHECK_CUDA(cudaStreamSynchronize(stream));
 }
 
@@ -307,14 +308,7 @@ void Engine::release() {
             cudaStreamSynchronize(l.stream);
     for (cudaEvent_t ev : fork_events)
         cudaEventDestroy(ev);
-    if (forward_done)
-        cudaEventDestroy(forward_done);
-    for (const GradientPiece &piece : gradient_pieces)
-        cudaEventDestroy(piece.ready);
-    if (copy_stream) {
-        cudaStreamSynchronize(copy_stream);
-        cudaStreamDestroy(copy_stream);
-    }
+    copies.destroy();
     for (auto &t : timed) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
@@ -678,7 +672,7 @@ void Engine::backward() {
         if (side)
             layer_done[l] = mark(side);
         if (announce_gradients)
-            for (const GradientPiece &piece : gradient_pieces)
+            for (const BatchCopies::Piece &piece : copies.pieces)
                 if (piece.layer == l)
                     announce(piece.ready, side);
         int64_t layer_end = l + 1 < depth ? layout.layers[l + 1].attention_norm : layout.final_norm;
@@ -819,8 +813,8 @@ void Engine::one_step(RunMode mode, bool last) {
     }
     if (mode != RunMode::OptimizerOnly) {
         forward(mode != RunMode::Evaluate, mode != RunMode::Train && logits_fp32 != nullptr);
-        if (forward_done && (mode == RunMode::Gradients || mode == RunMode::Evaluate))
-            announce(forward_done, 0);
+        if (mode == RunMode::Gradients)
+            announce(copies.forward_done, 0);
         if (mode == RunMode::Evaluate)
             return;
         if (mode == RunMode::Train)
@@ -953,46 +947,34 @@ float Engine::train_mean_loss(int steps) {
     return float(sum / config.base.context);
 }
 
-// The results of tg_batch leave while the GPU is at work: the logits during the backward pass, the gradients in pieces of two
-// megabytes or more as their layers are finished (not under data parallelism, where they are added up over the ranks afterwards).
-// 15 MB into ordinary memory take 0.65 ms, longer than a small model's step: 4 layers d 256, 2048 tokens 1.28 -> 1.17 ms, in FP32
-// 3.2 -> 2.54 ms, into pinned arrays 0.74 -> 0.59 ms.
-void Engine::prepare_copies() {
-    constexpr int64_t Least = 1 << 19; // floats
-    auto event = [](cudaEvent_t &e) { CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); };
-    event(forward_done);
-    int64_t end = layout.count;
-    for (int l = config.base.depth - 1; l >= 0 && !comm; --l) {
-        const int64_t begin = layout.layers[l].attention_norm;
-        if (end - begin < Least)
-            continue;
-        gradient_pieces.push_back({l, begin, nullptr});
-        event(gradient_pieces.back().ready);
-        end = begin;
-    }
-    CHECK_CUDA(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking)); // last: it says that all is there
-}
-
 // Has the kernel map the pages of a result before the copy into it needs them (a caller's fresh array has none: 0.28 ms of page
-// faults for 15 MB), on the host while the GPU computes.  Contents are left alone; where the call is not known or the memory is not
-// ordinary host memory, nothing happens and the copy takes the faults itself.
+// faults for 15 MB), on the host while the GPU computes.  Contents are left alone; where the call is not known, the copy takes the
+// faults itself.  Memory that CUDA knows has its pages: the walk over them cost pinned arrays 1.0 of 8.8 ms (12 layers d 768, 4096
+// tokens).  Both arrays are mapped before the first copy, which in ordinary memory holds the host until it is done: with the
+// gradients' pages after the logits' copy, fresh arrays take up to 5 % longer, mapped ones up to 7 % less.
 static void map_pages(void *p, size_t bytes) {
 #ifdef MADV_POPULATE_WRITE
+    if (!p)
+        return;
+    cudaPointerAttributes known{};
+    CHECK_CUDA(cudaPointerGetAttributes(&known, p));
     const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE)), begin = (reinterpret_cast<uintptr_t>(p) + page - 1) / page * page,
                     end = (reinterpret_cast<uintptr_t>(p) + bytes) / page * page;
-    if (p && begin < end)
+    if (known.type == cudaMemoryTypeUnregistered && begin < end)
         (void)madvise(reinterpret_cast<void *>(begin), end - begin, MADV_POPULATE_WRITE);
 #endif
 }
 
+// With gradients, the results leave while the GPU is at work: the logits during the backward pass, the gradients in pieces of two
+// megabytes or more as their layers are finished.  15 MB into ordinary memory take 0.65 ms, longer than a small model's step: 4 layers
+// d 256, 2048 tokens 1.29 -> 1.21 ms, in FP32 3.2 -> 2.4 ms, into pinned arrays 0.73 -> 0.57 ms.
 void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, float *gradient_out,
                    float *per_position) {
     set_device();
     const int B = config.base.batch, T = config.base.context;
+    std::vector<float> losses(tokens); // here, so that it cannot throw between the first copy into the caller's arrays and the wait for it
     if (!logits_fp32)
         allocate(logits_fp32, size_t(tokens) * Vocabulary, false);
-    if (!copy_stream)
-        prepare_copies();
     CHECK_CUDA(cudaMemcpyAsync(x, bx, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemcpyAsync(y, by, tokens, cudaMemcpyHostToDevice, stream));
     replay(gradient_out ? GraphGradients : GraphEvaluate,
@@ -1000,22 +982,24 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
     const size_t logit_bytes = size_t(tokens) * Vocabulary * 4;
     map_pages(logits_out, logit_bytes);
     map_pages(gradient_out, size_t(layout.count) * 4);
-    if (logits_out) { // beside the backward pass
-        CHECK_CUDA(cudaStreamWaitEvent(copy_stream, forward_done, 0));
-        CHECK_CUDA(cudaMemcpyAsync(logits_out, logits_fp32, logit_bytes, cudaMemcpyDeviceToHost, copy_stream));
+    if (logits_out) {
+        if (gradient_out) // beside the backward pass
+            CHECK_CUDA(cudaStreamWaitEvent(copies.stream, copies.forward_done, 0));
+        CHECK_CUDA(cudaMemcpyAsync(logits_out, logits_fp32, logit_bytes, cudaMemcpyDeviceToHost, gradient_out ? copies.stream : stream));
     }
     if (gradient_out) { // the layers as they are finished, last first, then what is left
         int64_t left = layout.count;
-        for (const GradientPiece &piece : gradient_pieces) {
-            CHECK_CUDA(cudaStreamWaitEvent(copy_stream, piece.ready, 0));
-            CHECK_CUDA(cudaMemcpyAsync(gradient_out + piece.begin, gradient + piece.begin, (left - piece.begin) * 4, cudaMemcpyDeviceToHost, copy_stream));
+        for (const BatchCopies::Piece &piece : copies.pieces) {
+            CHECK_CUDA(cudaStreamWaitEvent(copies.stream, piece.ready, 0));
+            CHECK_CUDA(cudaMemcpyAsync(gradient_out + piece.begin, gradient + piece.begin, (left - piece.begin) * 4, cudaMemcpyDeviceToHost,
+                                       copies.stream));
             left = piece.begin;
         }
         CHECK_CUDA(cudaMemcpyAsync(gradient_out, gradient, left * 4, cudaMemcpyDeviceToHost, stream));
     }
-    std::vector<float> losses(tokens);
     CHECK_CUDA(cudaMemcpyAsync(losses.data(), token_losses, size_t(tokens) * 4, cudaMemcpyDeviceToHost, stream));
-    CHECK_CUDA(cudaStreamSynchronize(copy_stream)); // a pinned array's copy returns before it is done
+    if (gradient_out)
+        CHECK_CUDA(cudaStreamSynchronize(copies.stream)); // a pinned array's copy returns before it is done
     CHECK_CUDA(cudaStreamSynchronize(stream));
     flush_profile();
     check_device_error();

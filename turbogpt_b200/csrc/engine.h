@@ -1,6 +1,7 @@
 // The training engine behind the C ABI: device arena, the kernel sequence of one step
 // (forward, loss, backward, gradient exchange, optimizer) and its evaluation modes.
 #pragma once
+#include "batch_copies.h"
 #include "kernels.cuh"
 #include <memory>
 #include <string>
@@ -140,15 +141,7 @@ struct Engine {
     std::vector<cudaEvent_t> fork_events; // as many as a backward pass marks: none is recorded again before its last wait
     size_t next_fork_event = 0;
     float *simt_scratch[2] = {nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
-    // What tg_batch's results leave by, made with its first call: see prepare_copies.
-    struct GradientPiece { // `gradient` from `begin` to the piece before it, or the end: complete after the backward pass of `layer`
-        int layer;
-        int64_t begin;
-        cudaEvent_t ready;
-    };
-    cudaStream_t copy_stream = nullptr;
-    cudaEvent_t forward_done = nullptr;
-    std::vector<GradientPiece> gradient_pieces;
+    BatchCopies copies; // of tg_batch's results
     bool announce_gradients = false;
     StepGraph graphs[GraphKinds];
     int forward_batch = 0; // sequences the next forward pass covers (0: the configured batch)
@@ -199,7 +192,6 @@ struct Engine {
     bool use_graphs() const { return !profile && !comm && !(config.flags & TG_FLAG_NO_GRAPH); }
     template <class F> void replay(GraphKind kind, F &&body);
     void announce(cudaEvent_t event, int on);
-    void prepare_copies();
     cudaEvent_t mark(int on); // an event after everything lane `on` holds
     void await(int on, cudaEvent_t event);
     void fork(int from, int to) {
