@@ -709,7 +709,7 @@ void Engine::muon_family(const MuonFamily &family) {
     MuonPrepareArgs prep{gradient + first_offset, momentum + first_offset, family.x[0], family.sumsq, sumsq_partial,
                          sumsq_blocks, schedule, counters, c.base.momentum, c.base.clip, rows, cols, depth, stride};
     run(FMuon, [&](cudaStream_t s) { launch_muon_prepare(prep, s); });
-    run(FMuon, [&](cudaStream_t s) { launch_muon_normalize(family.x[0], family.sumsq, per, depth, s); });
+    run(FMuon, [&](cudaStream_t s) { launch_muon_normalize(family.x[0], family.sumsq, per, depth, sms, s); });
     bf16 *cur = family.x[0] + first * per, *nxt = family.x[1] + first * per;
     bf16 *a_buffer = family.a + int64_t(first) * r * r, *b_buffer = family.b + int64_t(first) * r * r;
     const bool small = muon_newton_schulz_small_supported(r, n); // the reference architecture: one launch, in place
@@ -751,7 +751,7 @@ void Engine::muon_family(const MuonFamily &family) {
     MuonApplyArgs apply{all, weight_high + first_offset, weight_low + first_offset,
                         weight_fp32 ? weight_fp32 + first_offset : nullptr, schedule, counters, c.base.muon_lr,
                         c.base.weight_decay, rows, cols, depth, stride};
-    run(FMuon, [&](cudaStream_t s) { launch_muon_apply(apply, s); });
+    run(FMuon, [&](cudaStream_t s) { launch_muon_apply(apply, sms, s); });
 }
 
 void Engine::optimize() {

@@ -276,7 +276,7 @@ struct MuonPrepareArgs { // momentum, Nesterov direction, BF16 cast (+ transpose
     int64_t stride;      // elements between consecutive matrices of the batch in the flat arrays
 };
 void launch_muon_prepare(const MuonPrepareArgs &a, cudaStream_t s);
-void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, cudaStream_t s);
+void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, int sms, cudaStream_t s);
 // `matrices` consecutive [r, n] BF16 matrices (r <= n), orthogonalised in place by `steps` Newton-Schulz iterations.
 bool muon_newton_schulz_small_supported(int r, int n);
 void launch_muon_newton_schulz_small(bf16 *x, int r, int n, int steps, int matrices, cudaStream_t s);
@@ -291,7 +291,7 @@ struct MuonApplyArgs {
     int rows, cols, batch;
     int64_t stride;
 };
-void launch_muon_apply(const MuonApplyArgs &a, cudaStream_t s);
+void launch_muon_apply(const MuonApplyArgs &a, int sms, cudaStream_t s);
 void launch_advance(StepCounters *counters, cudaStream_t s);
 // AdamW, Muon and the advance of the step counters in one kernel, for models whose hidden matrices are at most 16 x 48
 // (or 48 x 16): one warp orthogonalises one matrix in registers.

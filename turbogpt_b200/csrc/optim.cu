@@ -447,18 +447,18 @@ __global__ void __launch_bounds__(256) muon_apply_transpose_kernel(MuonApplyArgs
 }
 // Blocks per matrix of a stage that leaves no partial sums: eight per SM over all matrices, as far as there are 64 x 64 tiles (four
 // thousand elements) for them.  With MuonBlocks of them a block of six 1536 x 384 matrices took four tiles one after another.
-static int muon_blocks(int64_t size, int batch) {
-    return int(std::max<int64_t>(1, std::min<int64_t>(size / (MuonTile * MuonTile), std::max(148 * 8 / batch, MuonBlocks))));
+static int muon_blocks(int64_t size, int batch, int sms) {
+    return int(std::max<int64_t>(1, std::min<int64_t>(size / (MuonTile * MuonTile), std::max(sms * 8 / batch, MuonBlocks))));
 }
-void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, cudaStream_t s) {
-    const dim3 grid(muon_blocks(per_matrix, batch), batch);
+void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, int sms, cudaStream_t s) {
+    const dim3 grid(muon_blocks(per_matrix, batch, sms), batch);
     if (per_matrix % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0)
         muon_normalize_vector_kernel<<<grid, 256, 0, s>>>(x, sumsq, per_matrix);
     else
         muon_normalize_kernel<<<grid, 256, 0, s>>>(x, sumsq, per_matrix);
 }
-void launch_muon_apply(const MuonApplyArgs &a, cudaStream_t s) {
-    const dim3 grid(muon_blocks(int64_t(a.rows) * a.cols, a.batch), a.batch);
+void launch_muon_apply(const MuonApplyArgs &a, int sms, cudaStream_t s) {
+    const dim3 grid(muon_blocks(int64_t(a.rows) * a.cols, a.batch, sms), a.batch);
     const bool aligned = a.stride % 8 == 0 && reinterpret_cast<uintptr_t>(a.weight_high) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(a.weight_low) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(a.weight_fp32) % 32 == 0 && reinterpret_cast<uintptr_t>(a.x) % 16 == 0;
