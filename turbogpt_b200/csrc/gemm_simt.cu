@@ -111,16 +111,11 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs g, float *parti
         }
 }
 
-// The same product for aligned operands.  FP32 multiply-adds bound it (128 per clock and SM, 72 TFLOP/s), so the rest has to
+// The same product for aligned BF16 operands.  FP32 multiply-adds bound it (128 per clock and SM, 72 TFLOP/s), so the rest has to
 // stay out of their way: 8 x TN outputs per thread (12 or 16 shared-memory words per 32 or 64 multiply-adds), operands
-// as 128-bit loads that are issued a slice ahead and land in the other of two shared-memory buffers, one barrier a slice.
+// as 64-bit loads that are issued a slice ahead and land in the other of two shared-memory buffers, one barrier a slice.
 // TN = 8: 128 x 128 tiles, 256 threads; TN = 4: 64 x 64 tiles, 128 threads, for outputs of too few large tiles.
-template <class T> struct Quad;
-template <> struct Quad<float> {
-    float4 v;
-    __device__ __forceinline__ float at(int i) const { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
-};
-template <> struct Quad<bf16> {
+struct Quad {
     uint2 v;
     __device__ __forceinline__ float at(int i) const {
         const unsigned w = i < 2 ? v.x : v.y;
@@ -128,10 +123,10 @@ template <> struct Quad<bf16> {
     }
 };
 // Rows x TileK elements of an operand, four at a time along its unit stride, through registers into [k][row].
-template <class In, int Rows, int Threads> struct SliceLoader {
+template <int Rows, int Threads> struct SliceLoader {
     static constexpr int Count = Rows * TileK / 4 / Threads;
-    Quad<In> quad[Count];
-    __device__ __forceinline__ void fetch(const In *base, int64_t row_stride, int64_t k_stride, int first_row, int rows, int k0, int k_end) {
+    Quad quad[Count];
+    __device__ __forceinline__ void fetch(const bf16 *base, int64_t row_stride, int64_t k_stride, int first_row, int rows, int k0, int k_end) {
 #pragma unroll
         for (int c = 0; c < Count; ++c) {
             const int i = threadIdx.x + c * Threads;
@@ -139,7 +134,7 @@ template <class In, int Rows, int Threads> struct SliceLoader {
             const int row = first_row + (k_major ? i / (TileK / 4) : i % (Rows / 4) * 4), k = k0 + (k_major ? i % (TileK / 4) * 4 : i / (Rows / 4));
             quad[c] = {};
             if (row < rows && k < k_end)
-                quad[c].v = *reinterpret_cast<const decltype(quad[c].v) *>(base + row * row_stride + k * k_stride);
+                quad[c].v = *reinterpret_cast<const uint2 *>(base + row * row_stride + k * k_stride);
         }
     }
     __device__ __forceinline__ void put(float (*tile)[Rows + 4], int64_t k_stride) const {
@@ -156,12 +151,12 @@ template <class In, int Rows, int Threads> struct SliceLoader {
         }
     }
 };
-template <class In, class Out, int TN>
+template <class Out, int TN>
 __global__ void __launch_bounds__(TN == 8 ? 256 : 128) gemm_simt_wide_kernel(GemmArgs g, float *partials, int slice_k) {
     constexpr int Side = TN == 8 ? 128 : 64, Threads = TN == 8 ? 256 : 128;
     __shared__ __align__(16) float as[2][TileK][Side + 4], bs[2][TileK][Side + 4];
     const int z = partials ? 0 : blockIdx.z;
-    const In *a = (const In *)g.a + z * g.a_batch, *b = (const In *)g.b + z * g.b_batch;
+    const bf16 *a = (const bf16 *)g.a + z * g.a_batch, *b = (const bf16 *)g.b + z * g.b_batch;
     const int m0 = blockIdx.y * Side, n0 = blockIdx.x * Side;
     const int k_begin = partials ? blockIdx.z * slice_k : 0, k_end = partials ? min(g.k, k_begin + slice_k) : g.k;
     // a warp covers 64 x 32 (TN = 8) or 64 x 16 outputs: 8 threads down, 4 across; a thread's rows and columns come in
@@ -169,7 +164,7 @@ __global__ void __launch_bounds__(TN == 8 ? 256 : 128) gemm_simt_wide_kernel(Gem
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int row = (TN == 8 ? warp % 2 * 64 : 0) + lane / 4 * 4, column = (TN == 8 ? warp / 2 * 32 : warp * 16) + lane % 4 * 4;
     float acc[8][TN] = {};
-    SliceLoader<In, Side, Threads> next_a, next_b;
+    SliceLoader<Side, Threads> next_a, next_b;
     next_a.fetch(a, g.a_row, g.a_col, m0, g.m, k_begin, k_end);
     next_b.fetch(b, g.b_row, g.b_col, n0, g.n, k_begin, k_end);
     next_a.put(as[0], g.a_col);
@@ -370,7 +365,8 @@ template <class Out> __global__ void gemm_simt_reduce_kernel(GemmArgs g, const f
 }
 
 // What the vector loads need: unit stride in one dimension of each operand, the other stride, the extent along the unit
-// stride and the base a multiple of four elements; n a multiple of 4.  Below a 64-wide output most of a tile is padding.
+// stride and the base a multiple of four elements; n a multiple of 4.  Below a 64-wide output most of a tile is padding.  The
+// FP32 kernel has the three layouts that a layer needs: activations, input gradients, weight gradients.
 static bool wide_supported(const GemmArgs &g) {
     const size_t bytes = 4 * dtype_size(g.in);
     auto operand = [&](const void *p, int64_t row, int64_t col, int rows, int64_t batch) {
@@ -378,11 +374,13 @@ static bool wide_supported(const GemmArgs &g) {
         return (k_major || row == 1) && (k_major ? row : col) % 4 == 0 && (k_major ? g.k : rows) % 4 == 0 && batch % 4 == 0 &&
                reinterpret_cast<uintptr_t>(p) % bytes == 0;
     };
+    if (g.in == Dtype::FP32 && g.a_col != 1 && g.b_col == 1)
+        return false;
     return g.m >= 64 && g.n >= 64 && g.k >= 16 && g.n % 4 == 0 && operand(g.a, g.a_row, g.a_col, g.m, g.a_batch) &&
            operand(g.b, g.b_row, g.b_col, g.n, g.b_batch);
 }
 struct SimtPlan {
-    bool wide = false, large = false; // gemm_simt_wide_kernel, with 128 x 128 tiles
+    bool wide = false, large = false; // gemm_simt_wide_kernel (FP32: gemm_fp32_kernel), with 128 x 128 tiles
     int slices = 1;
 };
 // BF16: the smaller tile costs a quarter more shared-memory reads per product, the larger leaves SMs idle when there are fewer
@@ -416,11 +414,12 @@ static void launch_fp32(const GemmArgs &g, dim3 grid, float *partials, int slice
         CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FP32Shared));
         kernel<<<grid, 64 * FP32Groups, FP32Shared, s>>>(g, partials, slice_k);
     };
-    const bool ak = g.a_col == 1, bk = g.b_col == 1;
-    if (ak)
-        bk ? launch(gemm_fp32_kernel<true, true>) : launch(gemm_fp32_kernel<true, false>);
+    if (g.a_col != 1)
+        launch(gemm_fp32_kernel<false, false>);
+    else if (g.b_col != 1)
+        launch(gemm_fp32_kernel<true, false>);
     else
-        bk ? launch(gemm_fp32_kernel<false, true>) : launch(gemm_fp32_kernel<false, false>);
+        launch(gemm_fp32_kernel<true, true>);
 }
 template <class In, class Out> static void launch_simt(const GemmArgs &g, const SimtPlan &plan, float *scratch, cudaStream_t s) {
     const int slices = scratch ? plan.slices : 1, side = plan.large ? 128 : 64;
@@ -433,9 +432,9 @@ template <class In, class Out> static void launch_simt(const GemmArgs &g, const 
     else if constexpr (std::is_same_v<In, float>)
         launch_fp32(g, grid, partials, slice_k, s);
     else if (plan.large)
-        gemm_simt_wide_kernel<In, Out, 8><<<grid, 256, 0, s>>>(g, partials, slice_k);
+        gemm_simt_wide_kernel<Out, 8><<<grid, 256, 0, s>>>(g, partials, slice_k);
     else
-        gemm_simt_wide_kernel<In, Out, 4><<<grid, 128, 0, s>>>(g, partials, slice_k);
+        gemm_simt_wide_kernel<Out, 4><<<grid, 128, 0, s>>>(g, partials, slice_k);
     if (partials)
         gemm_simt_reduce_kernel<Out><<<unsigned((int64_t(g.m) * g.n + 255) / 256), 256, 0, s>>>(g, partials, used);
 }
