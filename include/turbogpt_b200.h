@@ -167,6 +167,10 @@ int tg_ex_train_batch(Engine *engine, const uint8_t *x, const uint8_t *y, float 
  * names: up to `capacity` pointers to static strings; returns the number of families. */
 int tg_ex_profile(Engine *engine, const char **names, double *milliseconds, int64_t *launches,
                   int capacity, int reset);
+/* Diagnostic: how the reference architecture's training step cuts its batch on a GPU with `sms` SMs.  plan[5]: tokens of a tile
+ * (in groups of 16), tiles, blocks that take them in turn, whether other warps help a tile's own, whether weight gradients run
+ * beside the next layer.  < 0 where the step runs operator by operator.  Touches no device. */
+int tg_ex_reference_step_plan(const TgConfigEx *config, int sms, int32_t *plan);
 /* Number of kernels this library launched on the engine's stream since creation. */
 int64_t tg_ex_launch_count(Engine *engine);
 /* Diagnostic: copies an activation saved by the last forward pass (tg_batch / tg_train keep them for

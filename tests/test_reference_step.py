@@ -82,12 +82,16 @@ def test_step_matches_the_operator_path(depth, context, batch):
                 np.testing.assert_allclose(got[part], expected[part], atol=2e-6, rtol=2e-5)
 
 
-@pytest.mark.parametrize("depth,context,batch", [
-    (2, 80, 2), (2, 96, 150), (3, 100, 4),       # 5, 6 (two rounds) and 7 row tiles of a block: no helpers
-    (3, 16, 149 * 2 + 1), (16, 32, 3),           # 3 and 2: helpers, and the weight gradients beside the next layer
-    (16, 32, 150), (16, 16, 500), (12, 16, 800)])  # 2, 2 and 3, in two rounds: gradients added to the first tile's as they come
-def test_tiles_with_helpers_and_without(depth, context, batch):
+@pytest.mark.parametrize("depth,context,batch,row_tiles,rounds,helpers,overlap", [
+    (2, 80, 2, 5, 1, 0, 0), (2, 96, 150, 6, 2, 0, 0), (3, 100, 4, 7, 1, 0, 0),
+    (3, 16, 149 * 2 + 1, 3, 1, 1, 1), (16, 32, 3, 2, 1, 1, 1), (16, 48, 3, 3, 1, 1, 0),
+    (16, 32, 150, 2, 2, 1, 1), (16, 16, 500, 2, 2, 1, 1), (12, 16, 800, 3, 2, 1, 1)])  # gradients added to the first tile's
+def test_tiles_with_helpers_and_without(depth, context, batch, row_tiles, rounds, helpers, overlap):
     """The same bounds as everywhere."""
+    ex, plan = ConfigEx.reference(Config(depth=depth, context=context, batch=batch)), (C.c_int32 * 5)()
+    assert bridge.load_library().tg_ex_reference_step_plan(C.byref(ex), 148, plan) == 0
+    rows, tiles, blocks, *form = plan
+    assert (rows // 16, -(-tiles // blocks), *form) == (row_tiles, rounds, helpers, overlap)
     test_step_matches_the_operator_path(depth, context, batch)
 
 

@@ -172,6 +172,7 @@ def load_library() -> C.CDLL:
     lib.tg_ex_selftest_bounded_wait.argtypes = [P, C.c_double]
     lib.tg_ex_launch_count.argtypes = [P]
     lib.tg_ex_launch_count.restype = I64
+    lib.tg_ex_reference_step_plan.argtypes = [C.POINTER(ConfigEx), I, P]
     lib.tg_ex_read_activation.argtypes = [P, I, C.c_char_p, P, I64]
     lib.tg_ex_read_activation.restype = I64
     lib.tg_ex_gemm.argtypes = [P, I64, I64, P, I64, I64, P, I64, I, I, I, I, I, P]
@@ -193,7 +194,7 @@ EXPORTS = ('error create destroy parameter_count blocks shared_bytes set_weights
            'set_optimizer_state memory set_data train get_training_losses training_versions pipeline_stats '
            'onecycle_point set_onecycle batch predict optimizer_test synchronize').split()
 EXTENSIONS = ('reference_config gpt_config parameter_count parameter_layout initialize_weights config_digest save_checkpoint load_checkpoint nccl_unique_id '
-              'stream sample train_mean_loss train_batch profile launch_count read_activation selftest_bounded_wait gemm gemm_batched gemm_schedule weight_gradient_static last_device_error attention_forward attention_backward '
+              'stream sample train_mean_loss train_batch profile reference_step_plan launch_count read_activation selftest_bounded_wait gemm gemm_batched gemm_schedule weight_gradient_static last_device_error attention_forward attention_backward '
               'norm_forward norm_backward cross_entropy head_cross_entropy').split()
 
 

@@ -223,6 +223,7 @@ struct ReferenceStepPlan { // how a batch is cut into tiles, and the scratch tha
     int sequences = 0, rows = 0, tiles = 0; // per tile: whole sequences, their tokens in groups of 16
     int blocks = 0, gradient_blocks = 0;    // of the step and reduce kernels
     int64_t partial_stride = 0;             // floats per block of gradient sums
+    bool helpers = false, overlap = false;  // warps that help a row tile's owner; weight gradients beside the next layer
 };
 struct ReferenceStepArgs {
     const uint8_t *data; // corpus to sample the batch from (as launch_sample does for world 1); nullptr: x and y hold it

@@ -1105,6 +1105,8 @@ ReferenceStepPlan reference_step_plan(const TgConfigEx &c, int sms) {
     const int count = Layer0 + c.base.depth * LayerParameters + Width + Vocabulary * Width;
     plan.gradient_blocks = (count + ReduceParameters - 1) / ReduceParameters;
     plan.partial_stride = int64_t(plan.gradient_blocks) * ReduceParameters;
+    plan.helpers = plan.rows <= TeamRows;
+    plan.overlap = StepShared(c.base.depth, plan.rows, c.base.context).overlap;
     return plan;
 }
 
@@ -1119,8 +1121,8 @@ void launch_reference_step(const ReferenceStepArgs &a, const ReferenceStepPlan &
     if (a.save)
         p.saved = *a.save;
     const int shared = StepShared(a.depth, plan.rows, a.context).total;
-    auto *kernel = plan.rows <= TeamRows ? a.save ? reference_step_kernel<true, true> : reference_step_kernel<false, true>
-                                         : a.save ? reference_step_kernel<true, false> : reference_step_kernel<false, false>;
+    auto *kernel = plan.helpers ? a.save ? reference_step_kernel<true, true> : reference_step_kernel<false, true>
+                                : a.save ? reference_step_kernel<true, false> : reference_step_kernel<false, false>;
     CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MaxShared));
     // Launched programmatically: each kernel's set-up overlaps the tail of the one before it.
     cudaLaunchAttribute attribute{};

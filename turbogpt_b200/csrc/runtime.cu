@@ -334,6 +334,17 @@ int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_c
         schedule[0] = s.tile_columns, schedule[1] = s.splits, schedule[2] = s.pair, schedule[3] = s.half_an_sm;
     });
 }
+int tg_ex_reference_step_plan(const TgConfigEx *config, int sms, int32_t *plan) {
+    return guarded([&] {
+        if (!config || !plan || sms < 1)
+            throw std::runtime_error("Missing configuration");
+        validate_config(*config);
+        if (!reference_step_supported(*config))
+            throw std::runtime_error("This configuration trains operator by operator");
+        const ReferenceStepPlan p = reference_step_plan(*config, sms);
+        plan[0] = p.rows, plan[1] = p.tiles, plan[2] = p.blocks, plan[3] = p.helpers, plan[4] = p.overlap;
+    });
+}
 int tg_ex_head_cross_entropy(const void *x, const void *head, const uint8_t *targets, float *losses, void *dlogits,
                              int rows, int width, float scale, void *stream) {
     return guarded([&] {
