@@ -56,23 +56,53 @@ def test_tensor_core_gemm_matches_fp32_product(a_mn, b_mn, m, n, k):
         assert max_relative(simt, expected) <= tolerance
 
 
+# (tile columns, K splits, CTA pair) with K-major and with MN-major B, and how many rounds of tiles a block takes on 148 SMs.
+TILE_FORMS = [
+    ((129, 72, 72), (64, 1, 0), (64, 1, 0), 1), ((4100, 264, 72), (128, 1, 0), (128, 1, 0), 1),
+    ((4100, 520, 72), (192, 1, 0), (192, 1, 0), 1), ((4100, 776, 72), (256, 1, 0), (256, 1, 0), 1),
+    ((20000, 72, 72), (64, 1, 0), (64, 1, 0), 3), ((20000, 72, 200), (128, 1, 0), (128, 1, 0), 2),
+    ((9000, 520, 72), (192, 1, 0), (192, 1, 0), 2), ((33000, 200, 72), (256, 1, 0), (256, 1, 0), 2),
+    ((4100, 264, 1032), (128, 1, 1), (128, 1, 1), 1), ((2050, 1544, 520), (256, 1, 1), (256, 1, 1), 1),
+    ((4100, 520, 3080), (192, 1, 1), (256, 1, 1), 1), ((4100, 776, 3080), (256, 1, 1), (256, 1, 1), 1),
+    ((16400, 136, 3080), (192, 1, 1), (192, 1, 0), 1),
+    ((20000, 72, 1032), (128, 1, 1), (128, 1, 1), 2), ((33000, 200, 520), (256, 1, 1), (256, 1, 1), 2),
+    ((129, 72, 3080), (64, 6, 0), (64, 6, 0), 1), ((129, 2056, 3080), (128, 4, 0), (128, 4, 0), 1),
+    ((2305, 272, 8008), (192, 3, 1), (128, 2, 1), 1)]  # the last of two or three blocks adds their parts itself
+
+
+def test_tile_forms_are_what_the_schedule_chooses():
+    for (m, n, k), *forms, rounds in TILE_FORMS:
+        for b_mn, form in enumerate(forms):
+            plan = (ctypes.c_int32 * 4)()
+            assert load_library().tg_ex_gemm_schedule(k, 1, *((1, n) if b_mn else (k, 1)), n, m, n, k, 1, 0, 0, 148, plan) == 0
+            assert tuple(plan)[:3] == form, (m, n, k, b_mn)
+            columns, splits, pair = form
+            tiles = -(-m // (256 if pair else 128)) * -(-n // columns) * splits
+            assert -(-tiles // (74 if pair else 148)) == rounds
+
+
 @pytest.mark.parametrize("b_mn", [False, True])
-@pytest.mark.parametrize("m,n,k", [(129, 72, 72), (4100, 264, 72), (4100, 520, 72), (4100, 776, 72),  # single blocks, tiles 64 to 256 wide
-                                   (4100, 520, 3080), (4100, 776, 3080), (16400, 136, 3080),          # many rounds over a long K: pairs
-                                   (129, 72, 3080), (129, 2056, 3080)])                               # K cut in six, in four
+@pytest.mark.parametrize("m,n,k", [form[0] for form in TILE_FORMS])
 def test_products_of_every_tile_form_at_their_edges(m, n, k, b_mn):
-    """One shape for each choice of the schedule, with partial tiles in every dimension, against 64 bits: FP32 sums of k exact
-    products, then one BF16 rounding."""
+    """The choices of the schedule, with partial tiles in every dimension, against 64 bits: FP32 sums of k exact products, then one
+    BF16 rounding; and with a second tensor (never with K cut), two FP32 roundings of either term before it."""
     lib = load_library()
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     a, b = (torch.randn(rows, k, generator=g, device="cuda").bfloat16() for rows in (m, n))
     stored = b.T.contiguous() if b_mn else b
-    c = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
-    assert lib.tg_ex_gemm(a.data_ptr(), k, 1, stored.data_ptr(), *((1, n) if b_mn else (k, 1)), c.data_ptr(), n, m, n, k, 0, 1, None) == 0, \
-        lib.tg_error()
+    c, scaled = (torch.empty(m, n, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    r = torch.randn(m, n, generator=g, device="cuda").bfloat16()
+    strides = (1, n) if b_mn else (k, 1)
+    assert lib.tg_ex_gemm(a.data_ptr(), k, 1, stored.data_ptr(), *strides, c.data_ptr(), n, m, n, k, 0, 1, None) == 0, lib.tg_error()
+    assert lib.tg_ex_gemm_batched(a.data_ptr(), k, 1, 0, stored.data_ptr(), *strides, 0, scaled.data_ptr(), n, 0, r.data_ptr(), .5, 3.,
+                                  m, n, k, 1, 0, None) == 0, lib.tg_error()
     torch.cuda.synchronize()
     expected, magnitude = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
-    assert ((c.double() - expected).abs() <= k * 2.0 ** -24 * magnitude + 2.0 ** -8 * expected.abs()).all()
+    bound = k * 2.0 ** -24 * magnitude
+    assert ((c.double() - expected).abs() <= bound + 2.0 ** -8 * expected.abs()).all()
+    second = .5 * expected + 3. * r.double()
+    assert ((scaled.double() - second).abs() <=
+            .5 * bound + 2.0 ** -22 * (.5 * expected.abs() + 3. * r.double().abs()) + 2.0 ** -8 * second.abs()).all()
     assert lib.tg_ex_last_device_error(None) == 0
 
 
