@@ -415,7 +415,8 @@ def test_graph_replay_is_bit_identical_to_direct_launches():
 
 @pytest.mark.parametrize("depth,width,batch,context,tied", [
     (5, 256, 8, 256, 1),   # lanes; pieces of one layer each
-    (9, 128, 2, 333, 0),   # pieces of several layers, the first layers left for the last copy; a head of its own
+    (9, 128, 2, 333, 0),   # pieces of three layers, nothing but the embedding left for the last copy; a head of its own
+    (8, 128, 2, 333, 0), (10, 128, 2, 100, 1),  # and two layers, one layer left for it
     (2, 1024, 5, 4096, 1), # no lanes (20480 x 1024 above 2^24)
     (2, 128, 2, 128, 1)])  # nothing is worth a piece
 def test_batch_results_leave_early_and_are_those_of_this_call(depth, width, batch, context, tied):
