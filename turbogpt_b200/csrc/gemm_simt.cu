@@ -219,13 +219,16 @@ __global__ void __launch_bounds__(TN == 8 ? 256 : 128) gemm_simt_wide_kernel(Gem
 }
 
 // FP32 operands of the same alignment.  128 multiply-adds per clock and SM bound it; next come the operand reads from shared
-// memory: they return 128 bytes per clock, so 8 x 4 outputs per thread (12 words for 32 multiply-adds) leave a third of the
-// multiply-add rate unused, 8 x 8 (16 for 64) just none.  64 x 64 tiles of 64 threads are two warps, too few to hide their own
+// memory: they return 128 bytes per clock, so with 8 x 4 outputs per thread (12 words for 32 multiply-adds) they take half as
+// long again as the multiply-adds, with 8 x 8 (16 for 64) exactly as long.  What is left is how well the two overlap and the last
+// round of tiles: 2048 x 768 x 256 is 384 tiles for the 296 that fit at once.  64 x 64 tiles of 64 threads are two warps, too few to hide their own
 // latencies on an SM that holds one to four tiles, so FP32Groups groups of 64 threads each take every fourth slice of K, with
 // buffers and a barrier of their own, and their sums are added through shared memory in group order.
 // Against the kernel for BF16 operands, which took these before: the 51 products of 4 layers d 256 over 2048 tokens 2230 -> 1720 us
 // (that evaluation 2.52 -> 2.37 ms), 6 layers d 512 over 4096 tokens 19.9 -> 16.3 ms; eight groups in one block per SM instead of two
-// blocks of four measured 5 % slower.  Sums are shorter too: gradients 1.7 to 2.3e-7 from 64 bits instead of 3.0 to 4.6e-7.
+// blocks of four measured 5 % slower.  128 registers for two blocks spill 56 bytes (activations) and 96 (input gradients); one block
+// without spills is 2 to 3 % slower from 2000 tokens on (steps of 2 layers d 1024, 16384 tokens 70.9 and 73.2 ms), 4 to 6 % faster where
+// the tiles are fewer than the SMs (4 layers d 256, one sequence of 256 tokens 428 and 402 us).  Sums are shorter too: gradients 1.7 to 2.3e-7 from 64 bits instead of 3.0 to 4.6e-7.
 // Slices come by cp.async as they lie in memory: [row][k] where K is the unit stride (read as pairs of k), else [k][row].
 constexpr int FP32Side = 64, FP32Groups = 4, FP32Stages = 2, FP32PitchK = TileK + 4, FP32PitchRow = FP32Side + 4;
 constexpr int FP32Slice = FP32Side * FP32PitchK; // floats of one operand's slice; the [k][row] form needs less

@@ -446,7 +446,8 @@ __global__ void __launch_bounds__(256) muon_apply_transpose_kernel(MuonApplyArgs
     }
 }
 // Blocks per matrix of a stage that leaves no partial sums: eight per SM over all matrices, as far as there are 64 x 64 tiles (four
-// thousand elements) for them.  With MuonBlocks of them a block of six 1536 x 384 matrices took four tiles one after another.
+// thousand elements) for them.  With MuonBlocks of them a block of six 1536 x 384 matrices took four tiles one after another: eight
+// optimizer steps of 8 layers d 512 7.17 -> 6.74 ms, 4 layers d 1024 16.6 -> 15.7, 6 layers d 384 level.
 static int muon_blocks(int64_t size, int batch, int sms) {
     return int(std::max<int64_t>(1, std::min<int64_t>(size / (MuonTile * MuonTile), std::max(sms * 8 / batch, MuonBlocks))));
 }
