@@ -508,6 +508,8 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
             run(FActivation, [&](cudaStream_t s) { launch_swiglu(act, a.wide, a.activated, M, Hd, s); });
         } else {
             up.n = Hd, up.ldc = Hd, up.epilogue = Epilogue::GeluDual, up.c2 = a.activated;
+            if (!want_gradient) // the derivative is for the backward pass
+                up.epilogue = Epilogue::Gelu, up.c = a.activated, up.c2 = nullptr;
             gemm(FGemmForward, up);
         }
         GemmArgs down;

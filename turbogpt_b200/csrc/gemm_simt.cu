@@ -31,6 +31,9 @@ template <class Out> struct EpilogueOps {
             ((Out *)g.c2 + z * g.c_batch)[c_index] = from_float<Out>(gelu(pre));
             break;
         }
+        case Epilogue::Gelu:
+            c[c_index] = from_float<Out>(gelu(rounded<Out>(value)));
+            break;
         case Epilogue::GeluGrad: {
             const Out *r = (const Out *)g.r + z * g.r_batch;
             c[c_index] = from_float<Out>(rounded<Out>(value) * to_float(r[r_index]));

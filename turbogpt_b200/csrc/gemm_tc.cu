@@ -68,21 +68,46 @@ struct TcParams {
     StepCounters *counters;
 };
 
+// Two BF16 values of a word as a pair of FP32 ones (the lower half first), and back.
+__device__ __forceinline__ uint64_t unpack_pair(uint32_t packed) {
+    return float_pair(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u));
+}
+__device__ __forceinline__ uint32_t pack_pair(uint64_t v) {
+    float lo, hi;
+    split_pair(v, lo, hi);
+    return pack_bf16(lo, hi);
+}
+__device__ __forceinline__ uint64_t both(float v) { return float_pair(v, v); }
+
+// gelu(x) = x Phi(x) and gelu'(x) = Phi(x) + x phi(x) of two BF16 values, as BF16.
 // Phi(x) = 0.5 (1 + erf(x / sqrt 2)) by Abramowitz & Stegun 7.1.26 (|error| < 3e-7) with every
 // constant folded: t = 1 / (1 + p |x| / sqrt 2), e = 2^(-x^2 log2(e) / 2), tail = 0.5 erfc = poly(t) t e.
-// Two SFU operations (rcp, ex2) and nine FMA-pipe operations; the exponential also gives the
-// Gaussian density of the derivative.
-__device__ __forceinline__ void gelu_terms(float x, float &cdf, float &density) {
-    float t, e;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.23164189f, fabsf(x), 1.f)));
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-0.72134752f * x * x));
-    float poly = fmaf(t, 0.5307027145f, -0.7265760135f);
-    poly = fmaf(t, poly, 0.7107068705f);
-    poly = fmaf(t, poly, -0.142248368f);
-    poly = fmaf(t, poly, 0.127414796f);
-    const float tail = poly * t * e;
-    cdf = x >= 0.f ? 1.f - tail : tail;
-    density = 0.3989422804014327f * e; // exp(-x^2/2) / sqrt(2 pi)
+// Two SFU operations (rcp, ex2) per value; the exponential also gives the Gaussian density of the derivative.  Issue slots bound
+// this epilogue: in pairs it takes 14 instructions a value, one value at a time 25.
+template <bool Derivative>
+__device__ __forceinline__ void gelu_pair(uint32_t packed, uint32_t &activated, uint32_t &derivative) {
+    const uint64_t x = unpack_pair(packed), magnitude = unpack_pair(packed & 0x7fff7fffu);
+    float d0, d1, q0, q1, t0, t1, e0, e1;
+    split_pair(fma_pair(both(0.23164189f), magnitude, both(1.f)), d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
+    split_pair(mul_pair(mul_pair(both(-0.72134752f), x), x), q0, q1);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(q0));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(q1));
+    const uint64_t t = float_pair(t0, t1), e = float_pair(e0, e1);
+    uint64_t poly = fma_pair(t, both(0.5307027145f), both(-0.7265760135f));
+    poly = fma_pair(t, poly, both(0.7107068705f));
+    poly = fma_pair(t, poly, both(-0.142248368f));
+    poly = fma_pair(t, poly, both(0.127414796f));
+    const uint64_t tail = mul_pair(mul_pair(poly, t), e), rest = fma_pair(tail, both(-1.f), both(1.f));
+    float x0, x1, a0, a1, b0, b1;
+    split_pair(x, x0, x1);
+    split_pair(tail, a0, a1);
+    split_pair(rest, b0, b1);
+    const uint64_t cdf = float_pair(x0 >= 0.f ? b0 : a0, x1 >= 0.f ? b1 : a1);
+    activated = pack_pair(mul_pair(x, cdf));
+    if (Derivative)
+        derivative = pack_pair(fma_pair(x, mul_pair(both(0.3989422804014327f), e), cdf)); // exp(-x^2/2) / sqrt(2 pi)
 }
 
 // Direct global store of eight consecutive outputs (split-K reduction path only).
@@ -112,6 +137,28 @@ template <int Warps> __device__ __forceinline__ bool epilogue_all(bool ok) {
                  : "r"(uint32_t(ok)), "n"(32 * Warps)
                  : "memory");
     return result != 0;
+}
+
+// Where a work item lies: the K splits of a tile follow one another, tiles run along n first, matrices of a batch last.  In 32 bits
+// (a tile has at least 8192 outputs: 2^31 of them do not fit any memory): 64-bit divisions cost every warp some 500 instructions an item.
+struct Item {
+    int split, tile, nt, mt, z;
+};
+__device__ __forceinline__ Item locate(const TcParams &p, int work, int n_tiles, int m_units, int unit, int rank) {
+    Item i;
+    i.split = 0, i.tile = work, i.z = 0;
+    if (p.splits > 1) {
+        i.tile = work / p.splits;
+        i.split = work - i.tile * p.splits;
+    }
+    int m = i.tile / n_tiles;
+    i.nt = i.tile - m * n_tiles;
+    if (p.batch > 1) {
+        i.z = m / m_units;
+        m -= i.z * m_units;
+    }
+    i.mt = m * unit + rank;
+    return i;
 }
 
 // 32 bytes to or from global memory: one 256-bit access when `wide` (32-byte aligned), else two
@@ -200,30 +247,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int m_tiles = ((p.m + BM * Unit - 1) / (BM * Unit)) * Unit, n_tiles = (p.n + p.bn - 1) / p.bn;
     const int k_blocks = (p.k + BK - 1) / BK;
     const int m_units = m_tiles / Unit;
-    const long long work_items = (long long)m_units * n_tiles * p.batch * p.splits;
-    const long long first_item = blockIdx.x / Unit, item_stride = gridDim.x / Unit;
+    const int work_items = m_units * n_tiles * p.batch * p.splits;
+    const int first_item = int(blockIdx.x) / Unit, item_stride = int(gridDim.x) / Unit;
     const uint32_t stage_tx = stage_bytes * Unit; // bytes landing for one stage in both CTAs
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (elect_one()) {
+            // Both CTAs' bytes are counted on the first CTA's barrier, armed by that CTA.
+            const uint32_t landed0 = Pair ? cluster_address(full0, 0) : full0;
+            // A K-major operand comes as one box of 64 K-elements, an MN-major one as boxes of 64 rows of the tile.
+            const int a_dx = p.a_mn ? 0 : BK, a_dy = p.a_mn ? BK : 0, b_dx = p.b_mn ? 0 : BK, b_dy = p.b_mn ? BK : 0;
+            const int b_boxes = p.b_mn ? bn_local / 64 : 1;
             int stage = 0;
             uint32_t phase = 0;
-            for (long long w = first_item; w < work_items; w += item_stride) {
-                const int split = int(w % p.splits);
-                long long t = w / p.splits;
-                const int nt = int(t % n_tiles), mt = int(t / n_tiles % m_units) * Unit + int(rank),
-                      z = int(t / n_tiles / m_units);
-                const int kb0 = split * p.k_blocks_per_split;
+            for (int w = first_item; w < work_items; w += item_stride) {
+                const Item item = locate(p, w, n_tiles, m_units, Unit, int(rank));
+                const int kb0 = item.split * p.k_blocks_per_split;
                 const int kb1 = min(k_blocks, kb0 + p.k_blocks_per_split);
+                const int m_first = item.mt * BM, n_first = item.nt * p.bn + int(rank) * bn_local, z = item.z;
+                int ax = p.a_mn ? m_first : kb0 * BK, ay = p.a_mn ? kb0 * BK : m_first;
+                int bx = p.b_mn ? n_first : kb0 * BK, by = p.b_mn ? kb0 * BK : n_first;
                 bool ok = true;
-                for (int kb = kb0; kb < kb1 && ok; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     ok = mbarrier_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, p.counters, 101);
                     if (!ok)
                         break;
-                    const uint32_t sa = base + stage * stage_bytes, sb = sa + StageABytes;
-                    // Both CTAs' bytes are counted on the first CTA's barrier, armed by that CTA.
-                    const uint32_t bar = Pair ? cluster_address(full0 + 8 * stage, 0) : full0 + 8 * stage;
+                    const uint32_t sa = base + stage * stage_bytes, sb = sa + StageABytes, bar = landed0 + 8 * stage;
                     if (rank == 0)
                         mbarrier_expect_tx(full0 + 8 * stage, stage_tx);
                     auto load = [&](uint32_t dst, const CUtensorMap *map, int x, int y) {
@@ -232,19 +282,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         else
                             tma_load_3d(dst, map, x, y, z, bar);
                     };
-                    const int n_first = nt * p.bn + int(rank) * bn_local;
-                    if (!p.a_mn) {
-                        load(sa, &map_a, kb * BK, mt * BM);
-                    } else {
-                        for (int j = 0; j < BM / 64; ++j)
-                            load(sa + j * 64 * BK * 2, &map_a, mt * BM + j * 64, kb * BK);
-                    }
-                    if (!p.b_mn) {
-                        load(sb, &map_b, kb * BK, n_first);
-                    } else {
-                        for (int j = 0; j < bn_local / 64; ++j)
-                            load(sb + j * 64 * BK * 2, &map_b, n_first + j * 64, kb * BK);
-                    }
+                    load(sa, &map_a, ax, ay);
+                    if (p.a_mn)
+                        load(sa + 64 * BK * 2, &map_a, ax + 64, ay);
+                    load(sb, &map_b, bx, by);
+                    for (int j = 1; j < b_boxes; ++j)
+                        load(sb + j * 64 * BK * 2, &map_b, bx + j * 64, by);
+                    ax += a_dx, ay += a_dy, bx += b_dx, by += b_dy;
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
@@ -261,12 +305,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // Per 16-element K step inside a stage: 32 bytes along a K-major row, or 16 rows of
             // 128 bytes for an MN-major operand.
             const uint32_t a_step = p.a_mn ? 16 * 128 : 32, b_step = p.b_mn ? 16 * 128 : 32;
-            const uint32_t a_lbo = p.a_mn ? 64 * BK * 2 : 16, b_lbo = p.b_mn ? 64 * BK * 2 : 16;
+            // the first stage's descriptors; the products only move them along
+            const uint64_t a_desc = smem_descriptor(base, p.a_mn ? 64 * BK * 2 : 16, 1024),
+                           b_desc = smem_descriptor(base + StageABytes, p.b_mn ? 64 * BK * 2 : 16, 1024);
+            auto commit = [](uint32_t bar) { // arrives once the products issued so far are done, in both CTAs of a pair
+                if constexpr (Pair)
+                    tcgen05_commit_both(bar);
+                else
+                    tcgen05_commit(bar);
+            };
             int stage = 0, buffer = 0;
             uint32_t phase = 0, buffer_phase = 0;
-            for (long long w = first_item; w < work_items; w += item_stride) {
-                const int split = int(w % p.splits);
-                const int kb0 = split * p.k_blocks_per_split;
+            for (int w = first_item; w < work_items; w += item_stride) {
+                const int kb0 = p.splits > 1 ? w % p.splits * p.k_blocks_per_split : 0;
                 const int kb1 = min(k_blocks, kb0 + p.k_blocks_per_split);
                 if (!mbarrier_wait(tempty0 + 8 * buffer, buffer_phase ^ 1, abort_flag, p.counters, 102))
                     break;
@@ -278,23 +329,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (!ok)
                         break;
                     tcgen05_fence_after();
-                    const uint32_t sa = base + stage * stage_bytes, sb = sa + StageABytes;
+                    const uint64_t da = descriptor_at(a_desc, stage * stage_bytes), db = descriptor_at(b_desc, stage * stage_bytes);
 #pragma unroll
                     for (int ks = 0; ks < BK / 16; ++ks) {
-                        uint64_t da = smem_descriptor(sa + ks * a_step, a_lbo, 1024);
-                        uint64_t db = smem_descriptor(sb + ks * b_step, b_lbo, 1024);
+                        const uint64_t dak = descriptor_at(da, ks * a_step), dbk = descriptor_at(db, ks * b_step);
                         if constexpr (Pair)
-                            tcgen05_mma_bf16_pair(accumulator, da, db, instruction, (kb > kb0 || ks > 0) ? 1u : 0u);
+                            tcgen05_mma_bf16_pair(accumulator, dak, dbk, instruction, (kb > kb0 || ks > 0) ? 1u : 0u);
                         else
-                            tcgen05_mma_bf16(accumulator, da, db, instruction, (kb > kb0 || ks > 0) ? 1u : 0u);
+                            tcgen05_mma_bf16(accumulator, dak, dbk, instruction, (kb > kb0 || ks > 0) ? 1u : 0u);
                     }
-                    // frees the stage (in both CTAs) once these MMAs have read it
-                    if constexpr (Pair) {
-                        tcgen05_commit_pair(cluster_address(empty0 + 8 * stage, 0));
-                        tcgen05_commit_pair(cluster_address(empty0 + 8 * stage, 1));
-                    } else {
-                        tcgen05_commit(empty0 + 8 * stage);
-                    }
+                    commit(empty0 + 8 * stage); // frees the stage once these products have read it
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
@@ -302,12 +346,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 if (!ok)
                     break;
-                if constexpr (Pair) { // accumulator complete, in both CTAs' tensor memory
-                    tcgen05_commit_pair(cluster_address(tfull0 + 8 * buffer, 0));
-                    tcgen05_commit_pair(cluster_address(tfull0 + 8 * buffer, 1));
-                } else {
-                    tcgen05_commit(tfull0 + 8 * buffer);
-                }
+                commit(tfull0 + 8 * buffer); // the accumulator is complete
                 if (++buffer == 2) {
                     buffer = 0;
                     buffer_phase ^= 1;
@@ -323,30 +362,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         constexpr bool has_r = Kind == int(Epilogue::Residual) || Kind == int(Epilogue::GeluGrad) ||
                                Kind == int(Epilogue::Axpby);
         constexpr bool whole_rows = Kind == int(Epilogue::CrossEntropy); // the sixteen warps meet per tile
+        constexpr int Pieces = OutFp32 ? 4 : 2; // 32-byte pieces per 32-column chunk row
+        constexpr int PieceColumns = 32 / Pieces;
+        auto row_of = [&](const Item &item) { return (long long)item.mt * BM + quarter * 32 + lane; };
+        auto fetch_second = [&](const Item &item, int c, uint32_t (&rv)[has_r ? Pieces : 1][8]) { // the second tensor's part of a chunk
+            const int column = item.nt * p.bn + c * 32;
+            const long long row = row_of(item);
+            if (!has_r || row >= p.m)
+                return;
+            const char *src = (const char *)p.r + (item.z * p.r_batch + row * p.ldr + column) * (OutFp32 ? 4 : 2);
+#pragma unroll
+            for (int g = 0; g < Pieces; ++g)
+                if (column + g * PieceColumns < p.n)
+                    load_global32(src + g * 32, rv[g], p.wide && column + (g + 1) * PieceColumns <= p.n,
+                                  column + g * PieceColumns + PieceColumns / 2 < p.n);
+        };
+        // The second tensor's chunk is fetched one chunk ahead, over the end of a tile too: where products are short the
+        // accumulators are ready before the epilogue gets to them, and nothing else would hide these loads.
+        uint32_t rv[has_r ? Pieces : 1][8];
+        auto item_of = [&](int w) { return locate(p, w, n_tiles, m_units, Unit, int(rank)); };
+        if (has_r && first_item < work_items && share * 32 < p.bn)
+            fetch_second(item_of(first_item), share, rv);
         int buffer = 0;
         uint32_t buffer_phase = 0;
-        for (long long w = first_item; w < work_items; w += item_stride) {
-            const int split = int(w % p.splits);
-            long long t = w / p.splits;
-            const int nt = int(t % n_tiles), mt = int(t / n_tiles % m_units) * Unit + int(rank),
-                      z = int(t / n_tiles / m_units);
-            const long long row = (long long)mt * BM + quarter * 32 + lane;
-            constexpr int Pieces = OutFp32 ? 4 : 2; // 32-byte pieces per 32-column chunk row
-            constexpr int PieceColumns = 32 / Pieces;
-            uint32_t rv[has_r ? Pieces : 1][8];
-            auto fetch_second = [&](int c) { // the second tensor's part of a chunk
-                const int column = nt * p.bn + c * 32;
-                if (!has_r || row >= p.m)
-                    return;
-                const char *src = (const char *)p.r + (z * p.r_batch + row * p.ldr + column) * (OutFp32 ? 4 : 2);
-#pragma unroll
-                for (int g = 0; g < Pieces; ++g)
-                    if (column + g * PieceColumns < p.n)
-                        load_global32(src + g * 32, rv[g], p.wide && column + (g + 1) * PieceColumns <= p.n,
-                                      column + g * PieceColumns + PieceColumns / 2 < p.n);
-            };
-            if (share * 32 < p.bn)
-                fetch_second(share); // on its way while the products are awaited (steps of short products 1 to 1.6 % faster)
+        for (int w = first_item; w < work_items; w += item_stride) {
+            const Item item = item_of(w);
+            const int nt = item.nt, mt = item.mt, z = item.z, split = item.split;
+            const long long row = row_of(item);
             bool ready = mbarrier_wait(tfull0 + 8 * buffer, buffer_phase, abort_flag, p.counters, 104);
             if (p.splits > 1 || whole_rows) // the warps meet at named barriers below: leave together or not at all
                 ready = epilogue_all<EpilogueWarps>(ready);
@@ -426,89 +468,100 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         }
                     }
                 }
-            } else if (p.splits == 1) {
+            } else if (Kind != int(Epilogue::Store) || p.splits == 1) {
                 const bool row_ok = row < p.m;
                 const long long c_row = z * p.c_batch + row * p.ldc;
-                auto process = [&](uint32_t (&acc)[32], int c) {
-                    const int column = nt * p.bn + c * 32;
-                    tmem_wait_load(acc);
-                    if (!row_ok)
-                        return;
-                    char *dst = (char *)p.c + (c_row + column) * (OutFp32 ? 4 : 2);
-#pragma unroll
-                    for (int g = 0; g < Pieces; ++g) {
-                        if (column + g * PieceColumns >= p.n)
-                            break;
-                        const bool whole = p.wide && column + (g + 1) * PieceColumns <= p.n;
-                        uint32_t out[8];
-                        if constexpr (OutFp32) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                float v = __uint_as_float(acc[g * 8 + j]);
-                                if (has_r) // Axpby on FP32
-                                    v = p.alpha * v + p.beta * __uint_as_float(rv[g][j]);
-                                out[j] = __float_as_uint(v);
-                            }
-                        } else {
-                            float v[16], r[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                v[j] = __uint_as_float(acc[g * 16 + j]);
-                            if (has_r) {
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) {
-                                    r[2 * j] = __uint_as_float(rv[g][j] << 16);
-                                    r[2 * j + 1] = __uint_as_float(rv[g][j] & 0xffff0000u);
-                                }
-                            }
-                            if constexpr (Kind == int(Epilogue::Residual)) {
-#pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    v[j] = rounded<bf16>(v[j]) + r[j];
-                            } else if constexpr (Kind == int(Epilogue::GeluDual)) {
-                                uint32_t activated[8];
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) { // v becomes gelu'(pre), `activated` gelu(pre)
-                                    float cdf0, cdf1, den0, den1;
-                                    const float x0 = rounded<bf16>(v[2 * j]), x1 = rounded<bf16>(v[2 * j + 1]);
-                                    gelu_terms(x0, cdf0, den0);
-                                    gelu_terms(x1, cdf1, den1);
-                                    activated[j] = pack_bf16(x0 * cdf0, x1 * cdf1);
-                                    v[2 * j] = fmaf(x0, den0, cdf0);
-                                    v[2 * j + 1] = fmaf(x1, den1, cdf1);
-                                }
-                                store_global32((char *)p.c2 + (c_row + column) * 2 + g * 32, activated, whole,
-                                               column + g * 16 + 8 < p.n);
-                            } else if constexpr (Kind == int(Epilogue::GeluGrad)) {
-#pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    v[j] = rounded<bf16>(v[j]) * r[j];
-                            } else if constexpr (Kind == int(Epilogue::Axpby)) {
-#pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    v[j] = p.alpha * v[j] + p.beta * r[j];
-                            }
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                out[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
-                        }
-                        store_global32(dst + g * 32, out, whole, column + g * PieceColumns + PieceColumns / 2 < p.n);
+                auto release = [&] { // the accumulator is in registers: the tile after the next may overwrite it
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if constexpr (Pair)
+                            mbarrier_arrive_cluster(cluster_address(tempty0 + 8 * buffer, 0));
+                        else
+                            mbarrier_arrive(tempty0 + 8 * buffer);
                     }
                 };
+                auto process = [&](const uint32_t *acc, int c, int g) { // one 32-byte piece of a chunk, from its accumulator columns
+                    const int column = nt * p.bn + c * 32 + g * PieceColumns;
+                    if (!row_ok || column >= p.n)
+                        return;
+                    const bool whole = p.wide && column + PieceColumns <= p.n, second = column + PieceColumns / 2 < p.n;
+                    uint32_t out[8];
+                    if constexpr (OutFp32) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            float v = __uint_as_float(acc[j]);
+                            if (has_r) // Axpby on FP32
+                                v = p.alpha * v + p.beta * __uint_as_float(rv[g][j]);
+                            out[j] = __float_as_uint(v);
+                        }
+                    } else if constexpr (Kind == int(Epilogue::Axpby)) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            out[j] = pack_bf16(p.alpha * __uint_as_float(acc[2 * j]) + p.beta * __uint_as_float(rv[g][j] << 16),
+                                               p.alpha * __uint_as_float(acc[2 * j + 1]) + p.beta * __uint_as_float(rv[g][j] & 0xffff0000u));
+                    } else {
+                        uint32_t activated[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) { // two columns at a time
+                            const uint32_t sum = pack_bf16(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+                            if constexpr (Kind == int(Epilogue::Residual))
+                                out[j] = pack_pair(add_pair(unpack_pair(sum), unpack_pair(rv[g][j])));
+                            else if constexpr (Kind == int(Epilogue::GeluGrad))
+                                out[j] = pack_pair(mul_pair(unpack_pair(sum), unpack_pair(rv[g][j])));
+                            else if constexpr (Kind == int(Epilogue::GeluDual))
+                                gelu_pair<true>(sum, activated[j], out[j]); // out: gelu'(pre)
+                            else if constexpr (Kind == int(Epilogue::Gelu))
+                                gelu_pair<false>(sum, out[j], activated[j]);
+                            else
+                                out[j] = sum;
+                        }
+                        if constexpr (Kind == int(Epilogue::GeluDual))
+                            store_global32((char *)p.c2 + (c_row + column) * 2, activated, whole, second);
+                    }
+                    store_global32((char *)p.c + (c_row + column) * (OutFp32 ? 4 : 2), out, whole, second);
+                };
                 for (int c = share; c < chunks; c += Shares) {
-                    uint32_t acc[32];
-                    tmem_load_32x32_async(taddr + c * 32, acc);
-                    if (c != share)
-                        fetch_second(c);
-                    process(acc, c);
+                    const bool last = c + Shares >= chunks;
+                    auto fetch_next = [&](uint32_t (&to)[has_r ? Pieces : 1][8]) {
+                        if (!last)
+                            fetch_second(item, c + Shares, to);
+                        else if (w + item_stride < work_items)
+                            fetch_second(item_of(w + item_stride), share, to);
+                    };
+                    if constexpr (has_r && !OutFp32) { // half a chunk's accumulator at a time: two halves, and twice the second tensor, would spill
+                        uint32_t acc[16], ahead[Pieces][8];
+                        tmem_load_32x16_async(taddr + c * 32, acc);
+                        fetch_next(ahead);
+                        tmem_wait_load(acc);
+                        process(acc, c, 0);
+                        tmem_load_32x16_async(taddr + c * 32 + 16, acc);
+                        tmem_wait_load(acc);
+                        if (last)
+                            release();
+                        process(acc, c, 1);
+#pragma unroll
+                        for (int g = 0; g < Pieces; ++g)
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                rv[g][j] = ahead[g][j];
+                    } else {
+                        uint32_t acc[32];
+                        tmem_load_32x32_async(taddr + c * 32, acc);
+                        tmem_wait_load(acc);
+                        if (last)
+                            release();
+#pragma unroll
+                        for (int g = 0; g < Pieces; ++g)
+                            process(acc + g * PieceColumns, c, g);
+                        if (has_r) // four pieces in flight beside four in use would not fit the registers
+                            fetch_next(rv);
+                    }
                 }
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    if constexpr (Pair)
-                        mbarrier_arrive_cluster(cluster_address(tempty0 + 8 * buffer, 0));
-                    else
-                        mbarrier_arrive(tempty0 + 8 * buffer);
+                if (share >= chunks) { // no chunk of this tile, perhaps one of the next
+                    release();
+                    if (has_r && w + item_stride < work_items && share * 32 < p.bn)
+                        fetch_second(item_of(w + item_stride), share, rv);
                 }
             } else {
                 // Partial tile to the workspace (padded to whole tiles, so no bounds checks).  A 32 x 32
@@ -544,10 +597,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 __threadfence();
                 epilogue_barrier<EpilogueWarps>();
                 if (threadIdx.x == 64) {
-                    unsigned ticket = atomicAdd(&p.tickets[t * Unit + rank], 1u);
+                    unsigned ticket = atomicAdd(&p.tickets[item.tile * Unit + rank], 1u);
                     int last = ticket == unsigned(p.splits - 1);
                     if (last)
-                        p.tickets[t * Unit + rank] = 0; // ready for the next launch
+                        p.tickets[item.tile * Unit + rank] = 0; // ready for the next launch
                     last_split_flag[0] = last;
                 }
                 epilogue_barrier<EpilogueWarps>();
@@ -923,6 +976,7 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
             case Epilogue::Store: launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16>); break;
             case Epilogue::Residual: launch(gemm_tc_kernel<int(Epilogue::Residual), false, P, 16>); break;
             case Epilogue::GeluDual: launch(gemm_tc_kernel<int(Epilogue::GeluDual), false, P, 16>); break;
+            case Epilogue::Gelu: launch(gemm_tc_kernel<int(Epilogue::Gelu), false, P, 16>); break;
             case Epilogue::GeluGrad: launch(gemm_tc_kernel<int(Epilogue::GeluGrad), false, P, 16>); break;
             case Epilogue::Axpby: launch(gemm_tc_kernel<int(Epilogue::Axpby), false, P, 16>); break;
             case Epilogue::CrossEntropy: launch(gemm_tc_kernel<int(Epilogue::CrossEntropy), false, P, 16>); break;

@@ -359,10 +359,10 @@ __device__ __forceinline__ void tcgen05_mma_bf16_pair(uint32_t d_tmem, uint64_t 
                  "l"(a_desc), "l"(b_desc), "r"(instruction), "r"(accumulate)
                  : "memory");
 }
-// Arrives on one mbarrier (a shared::cluster address, in either CTA) when the pair's MMAs issued so
-// far have completed.
-__device__ __forceinline__ void tcgen05_commit_pair(uint32_t cluster_bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
+// Arrives on the mbarrier at this shared-memory address in both CTAs of the pair when the pair's MMAs issued so far have completed.
+__device__ __forceinline__ void tcgen05_commit_both(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"(uint16_t(3))
                  : "memory");
 }
 
