@@ -112,19 +112,11 @@ __device__ __forceinline__ void gelu_pair(uint32_t packed, uint32_t &activated, 
 
 // Direct global store of eight consecutive outputs (split-K reduction path only).
 __device__ __forceinline__ void store_group(const TcParams &p, float (&v)[8], long long row, int col, int z) {
-    const long long ci = z * p.c_batch + row * p.ldc + col, ri = z * p.r_batch + row * p.ldr + col;
-    if (p.out_fp32) {
-        if (p.epilogue == int(Epilogue::Axpby)) {
-            float r[8];
-            load8((const float *)p.r + ri, r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                v[j] = p.alpha * v[j] + p.beta * r[j];
-        }
+    const long long ci = z * p.c_batch + row * p.ldc + col;
+    if (p.out_fp32)
         store8((float *)p.c + ci, v);
-        return;
-    }
-    store8((bf16 *)p.c + ci, v);
+    else
+        store8((bf16 *)p.c + ci, v);
 }
 
 // The epilogue threads meet (named barrier 1), with the AND of a predicate over them.
@@ -161,6 +153,20 @@ __device__ __forceinline__ Item locate(const TcParams &p, int work, int n_tiles,
     return i;
 }
 
+// Two neighbouring lanes hold a row each, eight words (32 bytes) at `low` and eight at `high`: afterwards `low` is the even lane's row
+// and `high` the odd lane's, the first 32 bytes of them in the even lane and the second in the odd one.  A warp's 256-bit access then
+// touches 16 pieces of 64 bytes.  With lane = row, 32 pieces of 32 bytes, stores run at 18 B/clk and SM and loads at 32 where the
+// paths from and to L2 carry 32 and 64; measured 3710 and 2050 clocks for a 128 x 256 tile's stores, 2060 and 1060 for loads.  As much
+// as the pairs gives whole lines: four lanes exchanged through twice the shuffles stored no faster.
+__device__ __forceinline__ void exchange_rows(uint32_t *low, uint32_t *high, bool odd) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? low[j] : high[j], 1);
+        low[j] = odd ? got : low[j];
+        high[j] = odd ? high[j] : got;
+    }
+}
+
 // 32 bytes to or from global memory: one 256-bit access when `wide` (32-byte aligned), else two
 // 128-bit accesses; `second` says whether the upper half is inside the tensor.
 __device__ __forceinline__ void load_global32(const void *p, uint32_t (&r)[8], bool wide, bool second) {
@@ -175,7 +181,7 @@ __device__ __forceinline__ void load_global32(const void *p, uint32_t (&r)[8], b
         r[0] = a.x, r[1] = a.y, r[2] = a.z, r[3] = a.w, r[4] = b.x, r[5] = b.y, r[6] = b.z, r[7] = b.w;
     }
 }
-__device__ __forceinline__ void store_global32(void *p, const uint32_t (&r)[8], bool wide, bool second) {
+__device__ __forceinline__ void store_global32(void *p, const uint32_t *r, bool wide, bool second) {
     if (wide) {
         asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]),
                      "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -362,24 +368,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         constexpr bool has_r = Kind == int(Epilogue::Residual) || Kind == int(Epilogue::GeluGrad) ||
                                Kind == int(Epilogue::Axpby);
         constexpr bool whole_rows = Kind == int(Epilogue::CrossEntropy); // the sixteen warps meet per tile
-        constexpr int Pieces = OutFp32 ? 4 : 2; // 32-byte pieces per 32-column chunk row
-        constexpr int PieceColumns = 32 / Pieces;
-        auto row_of = [&](const Item &item) { return (long long)item.mt * BM + quarter * 32 + lane; };
-        auto fetch_second = [&](const Item &item, int c, uint32_t (&rv)[has_r ? Pieces : 1][8]) { // the second tensor's part of a chunk
-            const int column = item.nt * p.bn + c * 32;
+        // A lane drains its own row of tensor memory, and stores (and reads of the second tensor) half of its own and half of its
+        // neighbour's: see exchange_rows.
+        const bool odd = lane & 1;
+        auto row_of = [&](const Item &item) { return (long long)item.mt * BM + quarter * 32 + (lane & ~1); }; // the pair's first row
+        auto fetch_second = [&](const Item &item, int c, uint32_t (&rv)[2][8]) { // the second tensor's part of a chunk
+            const int column = item.nt * p.bn + c * 32 + (odd ? 16 : 0);
             const long long row = row_of(item);
-            if (!has_r || row >= p.m)
+            if (!has_r || column >= p.n)
                 return;
-            const char *src = (const char *)p.r + (item.z * p.r_batch + row * p.ldr + column) * (OutFp32 ? 4 : 2);
+            const bf16 *src = (const bf16 *)p.r + item.z * p.r_batch + row * p.ldr + column;
 #pragma unroll
-            for (int g = 0; g < Pieces; ++g)
-                if (column + g * PieceColumns < p.n)
-                    load_global32(src + g * 32, rv[g], p.wide && column + (g + 1) * PieceColumns <= p.n,
-                                  column + g * PieceColumns + PieceColumns / 2 < p.n);
+            for (int g = 0; g < 2; ++g)
+                if (row + g < p.m)
+                    load_global32(src + g * p.ldr, rv[g], p.wide && column + 16 <= p.n, column + 8 < p.n);
         };
         // The second tensor's chunk is fetched one chunk ahead, over the end of a tile too: where products are short the
         // accumulators are ready before the epilogue gets to them, and nothing else would hide these loads.
-        uint32_t rv[has_r ? Pieces : 1][8];
+        uint32_t rv[2][8];
         auto item_of = [&](int w) { return locate(p, w, n_tiles, m_units, Unit, int(rank)); };
         if (has_r && first_item < work_items && share * 32 < p.bn)
             fetch_second(item_of(first_item), share, rv);
@@ -388,7 +394,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int w = first_item; w < work_items; w += item_stride) {
             const Item item = item_of(w);
             const int nt = item.nt, mt = item.mt, z = item.z, split = item.split;
-            const long long row = row_of(item);
             bool ready = mbarrier_wait(tfull0 + 8 * buffer, buffer_phase, abort_flag, p.counters, 104);
             if (p.splits > 1 || whole_rows) // the warps meet at named barriers below: leave together or not at all
                 ready = epilogue_all<EpilogueWarps>(ready);
@@ -423,6 +428,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     else
                         mbarrier_arrive(tempty0 + 8 * buffer);
                 }
+                const long long row = (long long)mt * BM + local;
                 const bool row_ok = row < p.m;
                 const int target = row_ok ? static_cast<const uint8_t *>(p.r)[row] : 0;
                 float high = v[0], picked = 0.f;
@@ -469,8 +475,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
             } else if (Kind != int(Epilogue::Store) || p.splits == 1) {
-                const bool row_ok = row < p.m;
-                const long long c_row = z * p.c_batch + row * p.ldc;
+                const long long row = row_of(item), c_row = z * p.c_batch + row * p.ldc;
                 auto release = [&] { // the accumulator is in registers: the tile after the next may overwrite it
                     tcgen05_fence_before();
                     __syncwarp();
@@ -481,81 +486,95 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             mbarrier_arrive(tempty0 + 8 * buffer);
                     }
                 };
-                auto process = [&](const uint32_t *acc, int c, int g) { // one 32-byte piece of a chunk, from its accumulator columns
-                    const int column = nt * p.bn + c * 32 + g * PieceColumns;
-                    if (!row_ok || column >= p.n)
-                        return;
-                    const bool whole = p.wide && column + PieceColumns <= p.n, second = column + PieceColumns / 2 < p.n;
-                    uint32_t out[8];
-                    if constexpr (OutFp32) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            float v = __uint_as_float(acc[j]);
-                            if (has_r) // Axpby on FP32
-                                v = p.alpha * v + p.beta * __uint_as_float(rv[g][j]);
-                            out[j] = __float_as_uint(v);
-                        }
-                    } else if constexpr (Kind == int(Epilogue::Axpby)) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            out[j] = pack_bf16(p.alpha * __uint_as_float(acc[2 * j]) + p.beta * __uint_as_float(rv[g][j] << 16),
-                                               p.alpha * __uint_as_float(acc[2 * j + 1]) + p.beta * __uint_as_float(rv[g][j] & 0xffff0000u));
-                    } else {
-                        uint32_t activated[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) { // two columns at a time
-                            const uint32_t sum = pack_bf16(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
-                            if constexpr (Kind == int(Epilogue::Residual))
-                                out[j] = pack_pair(add_pair(unpack_pair(sum), unpack_pair(rv[g][j])));
-                            else if constexpr (Kind == int(Epilogue::GeluGrad))
-                                out[j] = pack_pair(mul_pair(unpack_pair(sum), unpack_pair(rv[g][j])));
-                            else if constexpr (Kind == int(Epilogue::GeluDual))
-                                gelu_pair<true>(sum, activated[j], out[j]); // out: gelu'(pre)
-                            else if constexpr (Kind == int(Epilogue::Gelu))
-                                gelu_pair<false>(sum, out[j], activated[j]);
-                            else
-                                out[j] = sum;
-                        }
-                        if constexpr (Kind == int(Epilogue::GeluDual))
-                            store_global32((char *)p.c2 + (c_row + column) * 2, activated, whole, second);
-                    }
-                    store_global32((char *)p.c + (c_row + column) * (OutFp32 ? 4 : 2), out, whole, second);
-                };
                 for (int c = share; c < chunks; c += Shares) {
                     const bool last = c + Shares >= chunks;
-                    auto fetch_next = [&](uint32_t (&to)[has_r ? Pieces : 1][8]) {
-                        if (!last)
-                            fetch_second(item, c + Shares, to);
-                        else if (w + item_stride < work_items)
-                            fetch_second(item_of(w + item_stride), share, to);
-                    };
-                    if constexpr (has_r && !OutFp32) { // half a chunk's accumulator at a time: two halves, and twice the second tensor, would spill
-                        uint32_t acc[16], ahead[Pieces][8];
-                        tmem_load_32x16_async(taddr + c * 32, acc);
-                        fetch_next(ahead);
-                        tmem_wait_load(acc);
-                        process(acc, c, 0);
-                        tmem_load_32x16_async(taddr + c * 32 + 16, acc);
-                        tmem_wait_load(acc);
-                        if (last)
-                            release();
-                        process(acc, c, 1);
-#pragma unroll
-                        for (int g = 0; g < Pieces; ++g)
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                rv[g][j] = ahead[g][j];
-                    } else {
+                    const int chunk_column = nt * p.bn + c * 32;
+                    if constexpr (OutFp32) {
                         uint32_t acc[32];
                         tmem_load_32x32_async(taddr + c * 32, acc);
                         tmem_wait_load(acc);
                         if (last)
                             release();
 #pragma unroll
-                        for (int g = 0; g < Pieces; ++g)
-                            process(acc + g * PieceColumns, c, g);
-                        if (has_r) // four pieces in flight beside four in use would not fit the registers
-                            fetch_next(rv);
+                        for (int half = 0; half < 2; ++half) {
+                            exchange_rows(acc + half * 16, acc + half * 16 + 8, odd);
+                            const int column = chunk_column + half * 16 + (odd ? 8 : 0);
+#pragma unroll
+                            for (int g = 0; g < 2; ++g)
+                                if (row + g < p.m && column < p.n)
+                                    store_global32((float *)p.c + c_row + g * p.ldc + column, acc + half * 16 + g * 8, p.wide, true);
+                        }
+                    } else {
+                        // the chunk's row as BF16: sums of the products, for Axpby the results
+                        uint32_t v[16], ahead[2][8];
+                        if constexpr (has_r) {
+                            if constexpr (Kind == int(Epilogue::Axpby))
+                                exchange_rows(rv[0], rv[1], odd); // to lane = row
+#pragma unroll
+                            for (int half = 0; half < 2; ++half) { // 16 columns at a time: 32, and twice the second tensor, would spill
+                                uint32_t acc[16];
+                                tmem_load_32x16_async(taddr + c * 32 + half * 16, acc);
+                                if (half == 0) {
+                                    if (!last)
+                                        fetch_second(item, c + Shares, ahead);
+                                    else if (w + item_stride < work_items)
+                                        fetch_second(item_of(w + item_stride), share, ahead);
+                                }
+                                tmem_wait_load(acc);
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) {
+                                    const float s0 = __uint_as_float(acc[2 * j]), s1 = __uint_as_float(acc[2 * j + 1]);
+                                    if constexpr (Kind == int(Epilogue::Axpby))
+                                        v[half * 8 + j] = pack_bf16(p.alpha * s0 + p.beta * __uint_as_float(rv[half][j] << 16),
+                                                                    p.alpha * s1 + p.beta * __uint_as_float(rv[half][j] & 0xffff0000u));
+                                    else
+                                        v[half * 8 + j] = pack_bf16(s0, s1);
+                                }
+                            }
+                        } else {
+                            uint32_t acc[32];
+                            tmem_load_32x32_async(taddr + c * 32, acc);
+                            tmem_wait_load(acc);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                v[j] = pack_bf16(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+                        }
+                        if (last)
+                            release();
+                        exchange_rows(v, v + 8, odd);
+                        const int column = chunk_column + (odd ? 16 : 0);
+                        const bool whole = p.wide && column + 16 <= p.n, second = column + 8 < p.n;
+#pragma unroll
+                        for (int g = 0; g < 2; ++g) {
+                            uint32_t out[8], activated[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) { // two columns at a time
+                                const uint32_t sum = v[g * 8 + j];
+                                if constexpr (Kind == int(Epilogue::Residual))
+                                    out[j] = pack_pair(add_pair(unpack_pair(sum), unpack_pair(rv[g][j])));
+                                else if constexpr (Kind == int(Epilogue::GeluGrad))
+                                    out[j] = pack_pair(mul_pair(unpack_pair(sum), unpack_pair(rv[g][j])));
+                                else if constexpr (Kind == int(Epilogue::GeluDual))
+                                    gelu_pair<true>(sum, activated[j], out[j]); // out: gelu'(pre)
+                                else if constexpr (Kind == int(Epilogue::Gelu))
+                                    gelu_pair<false>(sum, out[j], activated[j]);
+                                else
+                                    out[j] = sum;
+                            }
+                            if (row + g < p.m && column < p.n) {
+                                const long long at = c_row + g * p.ldc + column;
+                                store_global32((bf16 *)p.c + at, out, whole, second);
+                                if constexpr (Kind == int(Epilogue::GeluDual))
+                                    store_global32((bf16 *)p.c2 + at, activated, whole, second);
+                            }
+                        }
+                        if constexpr (has_r) {
+#pragma unroll
+                            for (int g = 0; g < 2; ++g)
+#pragma unroll
+                                for (int j = 0; j < 8; ++j)
+                                    rv[g][j] = ahead[g][j];
+                        }
                     }
                 }
                 if (share >= chunks) { // no chunk of this tile, perhaps one of the next
@@ -605,6 +624,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 epilogue_barrier<EpilogueWarps>();
                 if (last_split_flag[0]) {
+                    const long long row = (long long)mt * BM + quarter * 32 + lane;
                     __threadfence();
                     for (int chunk = share; chunk < p.bn / 32; chunk += Shares) {
                         const int column = nt * p.bn + chunk * 32;
@@ -967,10 +987,7 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
     auto launch_kind = [&](auto pair_tag) {
         constexpr bool P = decltype(pair_tag)::value;
         if (p.out_fp32) {
-            if (g.epilogue == Epilogue::Axpby)
-                launch(gemm_tc_kernel<int(Epilogue::Axpby), true, P, 16>);
-            else
-                launch(gemm_tc_kernel<int(Epilogue::Store), true, P, 16>);
+            launch(gemm_tc_kernel<int(Epilogue::Store), true, P, 16>);
         } else {
             switch (g.epilogue) {
             case Epilogue::Store: launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16>); break;
@@ -1026,7 +1043,7 @@ bool gemm_tc_supported(const GemmArgs &g) {
         return false;
     if (g.a_batch % 8 || g.b_batch % 8 || g.c_batch % 8 || g.r_batch % 8)
         return false;
-    if (g.out == Dtype::FP32 && !(g.epilogue == Epilogue::Store || g.epilogue == Epilogue::Axpby))
+    if (g.out == Dtype::FP32 && g.epilogue != Epilogue::Store)
         return false;
     return true;
 }
