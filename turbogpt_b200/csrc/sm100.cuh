@@ -326,9 +326,11 @@ __device__ __forceinline__ uint32_t cluster_address(uint32_t local_address, uint
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrive on an mbarrier of another CTA of the cluster.
+// Arrive on an mbarrier of another CTA of the cluster.  Relaxed: what the arrival tells the other side (accumulator columns
+// have been read) is ordered by tcgen05_fence_before(); with release semantics the thread would first wait until all of its stores to
+// global memory have been performed.
 __device__ __forceinline__ void mbarrier_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // Tile load into this CTA's shared memory whose completion is counted on an mbarrier that may live
 // in the pair's other CTA (`cluster_bar` is a shared::cluster address).
