@@ -403,6 +403,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + buffer * MaxBN;
             const int tile_columns = min(p.bn, p.n - nt * p.bn);
             const int chunks = (tile_columns + 31) / 32;
+            auto release = [&] { // the accumulator has been read: the products of the tile after the next may overwrite it
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if constexpr (Pair)
+                        mbarrier_arrive_cluster(cluster_address(tempty0 + 8 * buffer, 0));
+                    else
+                        mbarrier_arrive(tempty0 + 8 * buffer);
+                }
+            };
             if constexpr (whole_rows) {
                 // One 256-column tile holds whole rows of logits.  A thread owns row `row` in the 32-column chunks
                 // `share` and `share + 4`; the four shares of a row exchange their maxima and sums through shared
@@ -410,82 +420,78 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 float *row_high = reinterpret_cast<float *>(aligned + p.stages * stage_bytes + ControlBytes);
                 float *row_sum = row_high + Shares * BM;
                 const int local = quarter * 32 + lane;
-                float v[64];
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t acc[32];
-                    tmem_load_32x32_async(taddr + (share + half * Shares) * 32, acc);
-                    tmem_wait_load(acc);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        v[half * 32 + j] = __uint_as_float(acc[j]);
-                }
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) { // the accumulator is in registers: the next tile's products may overwrite it
-                    if constexpr (Pair)
-                        mbarrier_arrive_cluster(cluster_address(tempty0 + 8 * buffer, 0));
-                    else
-                        mbarrier_arrive(tempty0 + 8 * buffer);
-                }
                 const long long row = (long long)mt * BM + local;
-                const bool row_ok = row < p.m;
-                const int target = row_ok ? static_cast<const uint8_t *>(p.r)[row] : 0;
-                float high = v[0], picked = 0.f;
+                const int target = row < p.m ? static_cast<const uint8_t *>(p.r)[row] : 0;
+                // Three passes over the thread's 64 columns, 16 at a time; the exponentials replace the logits in tensor memory.  With
+                // the 64 columns in registers the epilogue of a tile took 16000 clocks (unrolled code that runs once, and 250 bytes
+                // of spills), like this 8900.
+                auto first_column = [&](int piece) { return (share + piece / 2 * Shares) * 32 + piece % 2 * 16; };
+                float high = -CUDART_INF_F, picked = 0.f;
+#pragma unroll 1
+                for (int piece = 0; piece < 4; ++piece) {
+                    uint32_t v[16];
+                    tmem_load_32x16_async(taddr + first_column(piece), v);
+                    const int at = target - first_column(piece);
+                    tmem_wait_load(v);
 #pragma unroll
-                for (int j = 0; j < 64; ++j) {
-                    high = fmaxf(high, v[j]);
-                    const int column = (share + (j / 32) * Shares) * 32 + j % 32;
-                    picked = column == target ? v[j] : picked;
+                    for (int j = 0; j < 16; ++j) {
+                        high = fmaxf(high, __uint_as_float(v[j]));
+                        picked = j == at ? __uint_as_float(v[j]) : picked;
+                    }
                 }
                 row_high[share * BM + local] = high;
                 epilogue_barrier<EpilogueWarps>();
                 high = fmaxf(fmaxf(row_high[local], row_high[BM + local]), fmaxf(row_high[2 * BM + local], row_high[3 * BM + local]));
                 float sum = 0.f;
+#pragma unroll 1
+                for (int piece = 0; piece < 4; ++piece) {
+                    uint32_t v[16];
+                    tmem_load_32x16_async(taddr + first_column(piece), v);
+                    tmem_wait_load(v);
 #pragma unroll
-                for (int j = 0; j < 64; ++j) {
-                    v[j] = expf(v[j] - high);
-                    sum += v[j];
+                    for (int j = 0; j < 16; ++j) {
+                        const float e = expf(__uint_as_float(v[j]) - high);
+                        sum += e;
+                        v[j] = __float_as_uint(e);
+                    }
+                    tmem_store_32x16(taddr + first_column(piece), v);
                 }
+                tmem_wait_store();
                 row_sum[share * BM + local] = sum;
                 epilogue_barrier<EpilogueWarps>();
                 sum = ((row_sum[local] + row_sum[BM + local]) + row_sum[2 * BM + local]) + row_sum[3 * BM + local];
-                if (row_ok) {
-                    if (target / 32 % Shares == share)
-                        static_cast<float *>(p.c2)[row] = high + logf(sum) - picked;
-                    if (p.c) {
-                        const float inverse = 1.f / sum;
+                if (row < p.m && target / 32 % Shares == share)
+                    static_cast<float *>(p.c2)[row] = high + logf(sum) - picked;
+                if (p.c) {
+                    const float inverse = 1.f / sum;
+#pragma unroll 1
+                    for (int half = 0; half < 2; ++half) {
+                        uint32_t out[16];
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            const int column = (share + half * Shares) * 32;
-                            char *dst = (char *)p.c + (row * p.ldc + column) * 2;
+                        for (int g = 0; g < 2; ++g) {
+                            const int column = first_column(half * 2 + g), at = target - column;
+                            uint32_t v[16];
+                            tmem_load_32x16_async(taddr + column, v);
+                            tmem_wait_load(v);
 #pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                uint32_t out[8];
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) {
-                                    const int e = half * 32 + g * 16 + 2 * j;
-                                    const float a = (v[e] * inverse - (column + g * 16 + 2 * j == target ? 1.f : 0.f)) * p.alpha;
-                                    const float b = (v[e + 1] * inverse - (column + g * 16 + 2 * j + 1 == target ? 1.f : 0.f)) * p.alpha;
-                                    out[j] = pack_bf16(a, b);
-                                }
-                                store_global32(dst + g * 32, out, p.wide, true);
+                            for (int j = 0; j < 8; ++j) {
+                                const float a = (__uint_as_float(v[2 * j]) * inverse - (2 * j == at ? 1.f : 0.f)) * p.alpha;
+                                const float b = (__uint_as_float(v[2 * j + 1]) * inverse - (2 * j + 1 == at ? 1.f : 0.f)) * p.alpha;
+                                out[g * 8 + j] = pack_bf16(a, b);
                             }
                         }
+                        exchange_rows(out, out + 8, odd);
+                        const long long row0 = row_of(item);
+                        bf16 *dst = (bf16 *)p.c + row0 * p.ldc + first_column(half * 2) + (odd ? 16 : 0);
+#pragma unroll
+                        for (int g = 0; g < 2; ++g)
+                            if (row0 + g < p.m)
+                                store_global32(dst + g * p.ldc, out + g * 8, p.wide, true);
                     }
                 }
+                release();
             } else if (Kind != int(Epilogue::Store) || p.splits == 1) {
                 const long long row = row_of(item), c_row = z * p.c_batch + row * p.ldc;
-                auto release = [&] { // the accumulator is in registers: the tile after the next may overwrite it
-                    tcgen05_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if constexpr (Pair)
-                            mbarrier_arrive_cluster(cluster_address(tempty0 + 8 * buffer, 0));
-                        else
-                            mbarrier_arrive(tempty0 + 8 * buffer);
-                    }
-                };
                 for (int c = share; c < chunks; c += Shares) {
                     const bool last = c + Shares >= chunks;
                     const int chunk_column = nt * p.bn + c * 32;
