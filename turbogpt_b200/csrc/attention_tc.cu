@@ -746,31 +746,41 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_con
         const bool valid = position < p.context, ragged = warp_first + 31 >= p.context;
         const int64_t padded = int64_t(p.tiles) * BlockM, stat = bh * padded + position;
         const float lse2 = valid ? p.lse[(int64_t(b) * p.heads + h) * p.context + position] * 1.4426950408889634f : 0.f;
-        // delta = rowsum(dO * O) for this thread's query: O from global memory, dO from the tile the TMA
-        // warp loaded (row r of a 128-byte-swizzled tile keeps its 16-byte chunk c at position c ^ (r % 8)).
+        // delta = rowsum(dO * O): O from global memory, dO from the tile the TMA warp loaded (row r of a 128-byte-swizzled tile
+        // keeps its 16-byte chunk c at position c ^ (r % 8)).  Eight lanes take a row, so that a load covers four whole rows
+        // and the sums are short; with a lane to a row the block's start took DELTA_FIGURES.
         float delta = 0.f;
         bool ok = true;
         {
+            const int group = lane / 8, chunk = lane % 8; // row 4 i + group of the warp's 32, 16 bytes at `chunk`
             uint4 o[8];
-            if (valid) {
-                const uint4 *source = reinterpret_cast<const uint4 *>(p.out + (int64_t(row0) + position) * p.width + h * HeadSize);
+            const bf16 *source = p.out + (int64_t(row0) + warp_first + group) * p.width + h * HeadSize + chunk * 8;
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    o[c] = source[c];
+            for (int i = 0; i < 8; ++i) {
+                o[i] = make_uint4(0, 0, 0, 0);
+                if (warp_first + 4 * i + group < p.context)
+                    o[i] = *reinterpret_cast<const uint4 *>(source + int64_t(4 * i) * p.width);
             }
             ok = mbarrier_wait(qdo_full, 0, abort_flag, p.counters, 308);
-            if (ok && valid) {
-                const uint4 *tile_row = reinterpret_cast<const uint4 *>(aligned + TileBytes + row * 128);
+            const uint32_t tile_rows = smem_do + quarter * 32 * 128;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 g = tile_row[c ^ (row & 7)];
-                    const unsigned a4[4] = {o[c].x, o[c].y, o[c].z, o[c].w}, b4[4] = {g.x, g.y, g.z, g.w};
+            for (int i = 0; i < 8 && ok; ++i) {
+                const int r = 4 * i + group;
+                const uint4 g = load_shared16(tile_rows + r * 128 + ((chunk ^ (r & 7)) << 4));
+                const unsigned a4[4] = {o[i].x, o[i].y, o[i].z, o[i].w}, b4[4] = {g.x, g.y, g.z, g.w};
+                float sum = 0.f;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        delta += __uint_as_float(a4[i] << 16) * __uint_as_float(b4[i] << 16) +
-                                 __uint_as_float(a4[i] & 0xffff0000u) * __uint_as_float(b4[i] & 0xffff0000u);
-                }
+                for (int k = 0; k < 4; ++k)
+                    sum += __uint_as_float(a4[k] << 16) * __uint_as_float(b4[k] << 16) +
+                           __uint_as_float(a4[k] & 0xffff0000u) * __uint_as_float(b4[k] & 0xffff0000u);
+#pragma unroll
+                for (int k = 1; k < 8; k <<= 1)
+                    sum += __shfl_xor_sync(0xffffffffu, sum, k);
+                const float mine = __shfl_sync(0xffffffffu, sum, (lane & 3) * 8); // row 4 i + lane % 4
+                delta = lane / 4 == i ? mine : delta;
             }
+            if (!valid)
+                delta = 0.f;
             if (ok && half == 0) { // rows past the end of the sequence hold zeros
                 p.statistics[stat] = -lse2;
                 p.statistics[pairs * padded + stat] = -delta;
