@@ -466,7 +466,7 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
     const bool layer_norm = c.norm == TG_NORM_LAYER;
     auto norm = [&](const void *in, int64_t scale, int64_t bias, void *out, float *stats) {
         NormArgs a{c.norm, in, weight_high + scale, layer_norm ? weight_high + bias : nullptr, weight_low + scale,
-                   layer_norm ? weight_low + bias : nullptr, out, M, W, stats};
+                   layer_norm ? weight_low + bias : nullptr, out, M, W, stats, true}; // the embedding, at least, lies between them and the optimizer
         run(FNorm, [&](cudaStream_t s) { launch_norm(act, a, s); });
     };
     run(FEmbedding, [&](cudaStream_t s) { launch_embedding(act, weight(layout.embedding), x, layers[0].x, M, W, s); });
@@ -599,7 +599,7 @@ void Engine::backward() {
     auto norm_back = [&](const void *xin, const void *dy, int64_t scale, int64_t bias, const void *residual,
                          void *dx, const float *stats) {
         NormBackwardArgs a{c.norm, xin, dy, weight_high + scale, weight_low + scale, residual, dx, norm_partial[norms++ % HiddenRing],
-                           gradient + scale, layer_norm ? gradient + bias : nullptr, M, W, norm_blocks, stats};
+                           gradient + scale, layer_norm ? gradient + bias : nullptr, M, W, norm_blocks, stats, true};
         run(FNormBackward, [&](cudaStream_t s) { launch_norm_backward(act, a, s); });
         const OnLane on = aside();
         run(FNormBackward, [&](cudaStream_t s) { launch_norm_backward_reduce(a, s); });

@@ -46,6 +46,8 @@ struct NormArgs {
     void *y;
     int rows, width;
     float *stats = nullptr; // optional [rows][2]: mean and 1/sqrt(variance + eps) of every row, for the backward pass
+    // The scale and bias were written before the kernel that precedes this one in the stream began: they may be read while it runs.
+    bool settled = false;
 };
 void launch_norm(Dtype t, const NormArgs &a, cudaStream_t s);
 struct NormBackwardArgs {
@@ -59,6 +61,7 @@ struct NormBackwardArgs {
     float *dscale, *dbias;   // outputs (overwritten); dbias nullptr for RMSNorm
     int rows, width, blocks;
     const float *stats = nullptr; // [rows][2] from the forward pass (nullptr: recomputed from x)
+    bool settled = false; // as in NormArgs
 };
 // dx and the blocks' sums of the scale and bias gradients in `partial`; then those sums over the blocks.
 void launch_norm_backward(Dtype t, const NormBackwardArgs &a, cudaStream_t s);

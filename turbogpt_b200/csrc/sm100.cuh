@@ -56,6 +56,18 @@ inline CUtensorMap make_map_bf16(const void *base, uint64_t inner, uint64_t oute
 }
 
 #ifdef __CUDACC__
+// Launches a kernel that sets itself up while the one before it in the stream runs: it calls grid_dependency_wait() before it touches
+// what that one wrote.
+template <class... Parameters, class... Arguments>
+inline void launch_overlapping(void (*kernel)(Parameters...), int grid, int block, size_t shared, cudaStream_t s, const Arguments &...arguments) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid), config.blockDim = dim3(block), config.dynamicSmemBytes = shared, config.stream = s;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute, config.numAttrs = 1;
+    CHECK_CUDA(cudaLaunchKernelEx(&config, kernel, Parameters(arguments)...));
+}
 // ------------------------------------------------------------------ device ------------------
 __device__ __forceinline__ uint32_t smem_address(const void *p) {
     return uint32_t(__cvta_generic_to_shared(p));
