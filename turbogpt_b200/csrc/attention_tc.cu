@@ -22,10 +22,12 @@ namespace {
 constexpr int BlockM = 128, BlockN = 128, HeadSize = 64;
 constexpr int TileBytes = 128 * HeadSize * 2; // 16 KB: a Q, K or V tile
 constexpr int KeyStep = 64, KeyBytes = KeyStep * HeadSize * 2; // the forward pass takes 64 keys (8 KB of K, of V) per step
-constexpr int ForwardRing = 4;                                 // shared-memory ring of (K, V) steps
 constexpr int ForwardThreads = 320;                            // warp 0 TMA, warp 1 MMA, 8 softmax warps
-constexpr int ForwardShared = TileBytes + ForwardRing * 2 * KeyBytes + 2048 + 1024 + 256; // Q, ring, merge buffer
-constexpr int ForwardTmemColumns = 256; // per chain: 64 score columns, 64 output columns
+// By the score buffers of a chain: steps in the shared-memory ring of (K, V), bytes (Q, ring, merge buffer), tensor memory columns
+// (64 to a score buffer, 64 to a chain's output).
+constexpr int forward_ring(int buffers) { return 4 * buffers; }
+constexpr int forward_shared(int buffers) { return TileBytes + forward_ring(buffers) * 2 * KeyBytes + 2048 + 1024 + 256; }
+constexpr int forward_columns(int buffers) { return 256 * buffers; }
 
 struct ForwardParams {
     bf16 *out;
@@ -60,9 +62,11 @@ __device__ __forceinline__ uint64_t unpack_pair(uint32_t packed) {
 // (packed over them) for the product that adds to the accumulator at tmem_o.  Returns the number of steps taken.
 // One chain: the scores of the second step are at tmem_o when the first begins, and the reference maximum is taken over both
 // (the probability of a maximum is 1, without a rounding error: two chains have two such); `sums.rounded` is kept too.
-template <int Chains>
-__device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile_first, int row, uint32_t tmem_s, uint32_t tmem_o,
-                                             uint32_t s_full, uint32_t p_full, const ForwardParams &p, volatile int *abort_flag,
+// Two buffers: the scores of every second step are 128 columns further, with a barrier two further; a product with V may then be
+// under way (`o_full` counts them) when the next scores are ready.
+template <int Chains, int Buffers>
+__device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile_first, int row, uint32_t tmem_s0, uint32_t tmem_o,
+                                             uint32_t s_full, uint32_t p_full, uint32_t o_full, const ForwardParams &p, volatile int *abort_flag,
                                              float &reference_max, RowSums &sums, bool &ok) {
     constexpr bool Rounded = Chains == 1;
     const int lane = row % 32, warp_first = tile_first + row - lane, position = tile_first + row;
@@ -71,7 +75,9 @@ __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile
     // and the final division by the row sum, accumulated with the same reference, makes the result exact.
     int mine = 0; // steps this chain has taken
     for (int j = first_step; j < steps; j += Chains, ++mine) {
-        ok = mbarrier_wait(s_full, mine & 1, abort_flag, p.counters, 206);
+        const int buffer = Buffers == 2 ? mine & 1 : 0;
+        const uint32_t tmem_s = tmem_s0 + 128 * buffer;
+        ok = mbarrier_wait(s_full + 16 * buffer, (Buffers == 2 ? mine >> 1 : mine) & 1, abort_flag, p.counters, 206);
         if (!ok)
             break;
         tcgen05_fence_after();
@@ -114,7 +120,7 @@ __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0)
-                    mbarrier_arrive(p_full);
+                    mbarrier_arrive(p_full + 16 * buffer);
                 if (Rounded)
                     sums.pair = add_pair(sums.pair, sum), sums.rounded = add_pair(sums.rounded, rounded);
                 else
@@ -150,7 +156,14 @@ __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile
         }
         const bool grow = (block_max - reference_max) * p.scale_log2 > 8.f; // true for the first unmasked step
         if (__any_sync(0xffffffffu, grow && reference_max != -CUDART_INF_F)) {
-            // between this chain's products: the scores awaited above were issued after the last one
+            // between this chain's products: with one buffer the scores awaited above were issued after the last one, with two after
+            // the last but one
+            if (Buffers == 2 && mine > 0) {
+                ok = mbarrier_wait(o_full, (mine - 1) & 1, abort_flag, p.counters, 207);
+                if (!ok)
+                    break;
+                tcgen05_fence_after();
+            }
             const float correction =
                 grow && reference_max != -CUDART_INF_F ? fast_exp2((reference_max - block_max) * p.scale_log2) : 1.f;
             if (Rounded) {
@@ -204,7 +217,7 @@ __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0)
-            mbarrier_arrive(p_full);
+            mbarrier_arrive(p_full + 16 * buffer);
         if (Rounded)
             sums.pair = add_pair(sums.pair, float_pair(sum0, sum1)), sums.rounded = add_pair(sums.rounded, rounded);
         else
@@ -213,17 +226,19 @@ __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile
     return mine;
 }
 
-__global__ void __launch_bounds__(ForwardThreads, 2)
+template <int Buffers>
+__global__ void __launch_bounds__(ForwardThreads, Buffers == 2 ? 1 : 2)
 flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                      ForwardParams p) {
+    constexpr int Ring = forward_ring(Buffers);
     extern __shared__ uint8_t raw_shared[];
     const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
     uint8_t *aligned = raw_shared + (base - smem_address(raw_shared));
-    float *exchange = reinterpret_cast<float *>(aligned + TileBytes + ForwardRing * 2 * KeyBytes); // [2 chains][max | sum][128 rows]
+    float *exchange = reinterpret_cast<float *>(aligned + TileBytes + Ring * 2 * KeyBytes); // [2 chains][max | sum][128 rows]
     uint64_t *barriers = reinterpret_cast<uint64_t *>(exchange + 4 * BlockM);
-    const uint32_t q_full = smem_address(barriers), kv_full0 = q_full + 8, kv_empty0 = kv_full0 + 8 * ForwardRing,
-                   s_full0 = kv_empty0 + 8 * ForwardRing, p_full0 = s_full0 + 16, o_full0 = p_full0 + 16;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 1 + 2 * ForwardRing + 6);
+    const uint32_t q_full = smem_address(barriers), kv_full0 = q_full + 8, kv_empty0 = kv_full0 + 8 * Ring,
+                   s_full0 = kv_empty0 + 8 * Ring, p_full0 = s_full0 + 16 * Buffers, o_full0 = p_full0 + 16 * Buffers;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 1 + 2 * Ring + 2 + 4 * Buffers);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const uint32_t smem_q = base, smem_kv = base + TileBytes;
 
@@ -238,40 +253,43 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
     if (threadIdx.x == 0) {
         mbarrier_init(q_full, 1);
-        for (int s = 0; s < ForwardRing; ++s) {
+        for (int s = 0; s < Ring; ++s) {
             mbarrier_init(kv_full0 + 8 * s, 1);
             mbarrier_init(kv_empty0 + 8 * s, 1);
         }
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < 2 * Buffers; ++c) {
             mbarrier_init(s_full0 + 8 * c, 1);
             mbarrier_init(p_full0 + 8 * c, 4);
-            mbarrier_init(o_full0 + 8 * c, 1);
         }
+        for (int c = 0; c < 2; ++c)
+            mbarrier_init(o_full0 + 8 * c, 1);
         *abort_flag = 0;
         fence_barrier_init();
         prefetch_map(&map_q);
         prefetch_map(&map_kv);
     }
     if (warp == 1) {
-        tmem_alloc(smem_address(tmem_slot), ForwardTmemColumns);
+        tmem_alloc(smem_address(tmem_slot), forward_columns(Buffers));
         tmem_relinquish();
     }
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
     grid_launch_dependents(); // the next kernel may set itself up while this one runs; this one holds its tensor memory
+    if (Buffers == 2)
+        grid_dependency_wait(); // and this one did so while the one before it ran
     const uint32_t tmem_base = *tmem_slot;
-    // chain c: scores of its steps at 64 c (the probabilities pack into the first 32 of those columns),
-    // its output accumulator at 128 + 64 c
-    const uint32_t tmem_s0 = tmem_base, tmem_o0 = tmem_base + 128;
+    // chain c: scores of its steps at 64 c, with two buffers and at 128 + 64 c in turn (the probabilities pack into the first 32 of
+    // those columns), its output accumulator behind them
+    const uint32_t tmem_s0 = tmem_base, tmem_o0 = tmem_base + 128 * Buffers;
 
     if (warp == 0) {
         if (elect_one()) {
             mbarrier_expect_tx(q_full, TileBytes);
             tma_load_3d(smem_q, &map_q, h * HeadSize, row0 + tile * BlockM, 0, q_full);
             for (int j = 0; j < steps; ++j) {
-                const int ring = j % ForwardRing;
-                if (!mbarrier_wait(kv_empty0 + 8 * ring, ((j / ForwardRing) & 1) ^ 1, abort_flag, p.counters, 201))
+                const int ring = j % Ring;
+                if (!mbarrier_wait(kv_empty0 + 8 * ring, ((j / Ring) & 1) ^ 1, abort_flag, p.counters, 201))
                     break;
                 const uint32_t bar = kv_full0 + 8 * ring, dst = smem_kv + ring * 2 * KeyBytes;
                 mbarrier_expect_tx(bar, 2 * KeyBytes);
@@ -287,39 +305,37 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                            v_desc0 = smem_descriptor(smem_kv + KeyBytes, 8192, 1024);
             bool ok = mbarrier_wait(q_full, 0, abort_flag, p.counters, 202);
             int issued = 0;
-            auto issue_scores = [&]() { // S = Q K_j^T into the buffer of chain j % 2
-                const int ring = issued % ForwardRing, chain = issued & 1;
-                ok = mbarrier_wait(kv_full0 + 8 * ring, (issued / ForwardRing) & 1, abort_flag, p.counters, 203);
+            auto issue_scores = [&]() { // S = Q K_j^T into a buffer of chain j % 2
+                const int ring = issued % Ring, buffer = issued % (2 * Buffers);
+                ok = mbarrier_wait(kv_full0 + 8 * ring, (issued / Ring) & 1, abort_flag, p.counters, 203);
                 if (!ok)
                     return;
                 tcgen05_fence_after();
                 const uint64_t k_desc = descriptor_at(k_desc0, ring * 2 * KeyBytes);
 #pragma unroll
                 for (int ks = 0; ks < HeadSize / 16; ++ks)
-                    tcgen05_mma_bf16(tmem_s0 + 64 * chain, descriptor_at(q_desc, ks * 32), descriptor_at(k_desc, ks * 32),
+                    tcgen05_mma_bf16(tmem_s0 + 64 * buffer, descriptor_at(q_desc, ks * 32), descriptor_at(k_desc, ks * 32),
                                      idesc_s, ks > 0);
-                tcgen05_commit(s_full0 + 8 * chain);
+                tcgen05_commit(s_full0 + 8 * buffer);
                 ++issued;
             };
-            if (ok)
-                issue_scores();
-            if (ok && steps > 1)
+            while (ok && issued < min(steps, 2 * Buffers))
                 issue_scores();
             for (int j = 0; j < steps && ok; ++j) {
-                const int chain = j & 1, ring = j % ForwardRing;
-                ok = mbarrier_wait(p_full0 + 8 * chain, (j >> 1) & 1, abort_flag, p.counters, 204);
+                const int chain = j & 1, ring = j % Ring;
+                ok = mbarrier_wait(p_full0 + 8 * (j % (2 * Buffers)), (j / (2 * Buffers)) & 1, abort_flag, p.counters, 204);
                 if (!ok)
                     break;
                 tcgen05_fence_after();
                 const uint64_t v_desc = descriptor_at(v_desc0, ring * 2 * KeyBytes);
 #pragma unroll
                 for (int ks = 0; ks < KeyStep / 16; ++ks) // O_chain += P V_j: four 16-key steps
-                    tcgen05_mma_bf16_ts(tmem_o0 + 64 * chain, tmem_s0 + 64 * chain + ks * 8,
+                    tcgen05_mma_bf16_ts(tmem_o0 + 64 * chain, tmem_s0 + 64 * (j % (2 * Buffers)) + ks * 8,
                                         descriptor_at(v_desc, ks * 2048), idesc_o, (j > 1 || ks > 0) ? 1u : 0u);
                 tcgen05_commit(o_full0 + 8 * chain);
                 tcgen05_commit(kv_empty0 + 8 * ring); // K_j and V_j are no longer read
                 if (issued < steps)
-                    issue_scores(); // step j + 2 reuses this chain's buffer: issued after the products that read it
+                    issue_scores(); // step j + 2 Buffers takes this step's buffer: issued after the products that read it
             }
         }
     } else {
@@ -334,9 +350,11 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         float reference_max = -CUDART_INF_F;
         RowSums sums;
         bool ok = true;
-        const int mine = softmax_chain<2>(chain, steps, tile * BlockM, row, tmem_s, tmem_o, s_full0 + 8 * chain,
-                                          p_full0 + 8 * chain, p, abort_flag, reference_max, sums, ok);
+        const int mine = softmax_chain<2, Buffers>(chain, steps, tile * BlockM, row, tmem_s, tmem_o, s_full0 + 8 * chain, p_full0 + 8 * chain,
+                                                   o_full0 + 8 * chain, p, abort_flag, reference_max, sums, ok);
         const float running_sum = sums.sum;
+        if (Buffers == 2 && ok && mine > 1) // up to two products may be under way: a phase is awaited by its parity, so each in turn
+            ok = mbarrier_wait(o_full0 + 8 * chain, mine & 1, abort_flag, p.counters, 208);
         if (ok && mine > 0)
             ok = mbarrier_wait(o_full0 + 8 * chain, (mine - 1) & 1, abort_flag, p.counters, 208);
         // merge the two chains: each publishes its reference maximum and sum, then takes half of the
@@ -394,7 +412,7 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     tcgen05_fence_before();
     __syncthreads();
     if (warp == 1)
-        tmem_dealloc(tmem_base, ForwardTmemColumns);
+        tmem_dealloc(tmem_base, forward_columns(Buffers));
 }
 
 // A warp's 32 accumulator rows x 32 columns from tensor memory, scaled, to BF16 in global memory (whole
@@ -531,7 +549,7 @@ flash_forward_single_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         float reference_max = -CUDART_INF_F;
         RowSums sums;
         bool ok = true;
-        softmax_chain<1>(0, steps, tile * BlockM, row, tmem_s + lanes, tmem_o + lanes, s_full, p_full, p, abort_flag,
+        softmax_chain<1, 1>(0, steps, tile * BlockM, row, tmem_s + lanes, tmem_o + lanes, s_full, p_full, o_full, p, abort_flag,
                          reference_max, sums, ok);
         if (ok)
             ok = mbarrier_wait(o_full, 0, abort_flag, p.counters, 208);
@@ -1112,8 +1130,8 @@ void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int 
     int device = 0;
     CHECK_CUDA(cudaGetDevice(&device));
     if (device < 64 && !configured[device]) {
-        CHECK_CUDA(cudaFuncSetAttribute(flash_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        ForwardShared));
+        CHECK_CUDA(cudaFuncSetAttribute(flash_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, forward_shared(1)));
+        CHECK_CUDA(cudaFuncSetAttribute(flash_forward_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, forward_shared(2)));
         CHECK_CUDA(cudaFuncSetAttribute(flash_forward_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         SingleShared));
         configured[device] = true;
@@ -1136,8 +1154,10 @@ void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int 
     const int grid = batch * heads * p.tiles, sms = 148;
     if (grid >= (p.tiles <= 4 ? 3 : 7) * sms)
         flash_forward_single_kernel<<<grid, SingleThreads, SingleShared, s>>>(map_q, map_kv, p);
-    else
-        flash_forward_kernel<<<grid, ForwardThreads, ForwardShared, s>>>(map_q, map_kv, p);
+    else if (grid > sms) // a block alone on its SM takes the tensor memory of two: its chains' next scores are ready when they get to them
+        flash_forward_kernel<1><<<grid, ForwardThreads, forward_shared(1), s>>>(map_q, map_kv, p);
+    else // 12 heads, context 1024 (96 blocks): tg_predict 670 -> 657 us, set up during the products before it 646
+        launch_overlapping(flash_forward_kernel<2>, grid, ForwardThreads, forward_shared(2), s, map_q, map_kv, p);
     CHECK_CUDA(cudaGetLastError());
 }
 
