@@ -5,6 +5,7 @@
 // (sampling seed, schedule point, loss-history row) read from device-resident counters.
 #include "engine.h"
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <dlfcn.h>
@@ -13,6 +14,7 @@
 #include <unistd.h>
 #include <type_traits>
 
+constexpr int64_t TwoSideLanes = int64_t(1) << 22; // token x columns up to which weight gradients have two lanes
 constexpr size_t SimtScratchBytes = size_t(6) << 20; // bounds gemm_simt_scratch_bytes for every shape it cuts
 
 const char *const family_names[FamilyCount] = {
@@ -114,9 +116,15 @@ void Engine::initialize() {
     // is then bound by power and the lanes cost what they add.  Measured per step, one lane -> two: 12 layers d 768, 4096
     // tokens 4.85 -> 4.32 ms, 8192 7.27 -> 7.05, 16384 12.44 -> 12.2, 32768 no difference; 16 layers d 1024, 32768 tokens
     // 71.2 -> 71.5 ms.  Muon families: 6 layers d 384 1.74 -> 1.58 ms; 12 layers d 768 and 16 layers d 1024 no difference.
-    side_lane = concurrent && int64_t(tokens) * c.width <= int64_t(1) << 24;
+    // With one lane of weight gradients that lane was as long as the chain (4 layers d 256, 2048 tokens: 48 us a layer each, four gradients
+    // of 10 us on 4 to 16 SMs one after another), and nothing that shortened the chain showed.  One lane -> two: that step 394 -> 384 us,
+    // with attention's backward pass in one launch 401 -> 361; 6 layers d 384, 2331 tokens with Muon 1219 -> 1141 us; 8 layers d 512, 4096 tokens 2206 -> 2189,
+    // 12 layers d 768, 4096 tokens 1 %, 8192 tokens level; 8 layers d 640, 8192 tokens and 14 layers d 960, 8192 tokens 0.2 and 0.7 % slower.  Three: slower
+    // than two everywhere (361 -> 369 us).
+    const int64_t work = int64_t(tokens) * c.width;
+    side_lanes = !concurrent || work > int64_t(1) << 24 ? 0 : work > TwoSideLanes ? 1 : 2;
     muon_lanes = concurrent && c.hidden_optimizer == TG_HIDDEN_MUON && int64_t(c.base.depth) * c.width * c.width <= int64_t(1) << 22;
-    for (int l = 1; l < (muon_lanes ? LaneCount : side_lane ? 2 : 1); ++l)
+    for (int l = 1; l < (muon_lanes ? LaneCount : 1 + side_lanes); ++l)
         CHECK_CUDA(cudaStreamCreateWithFlags(&lanes[l].stream, cudaStreamNonBlocking));
 
     const int64_t P = layout.count;
@@ -177,17 +185,17 @@ void Engine::initialize() {
         for (size_t i = 0; i < std::size(slots); ++i)
             slots[i] = reinterpret_cast<std::remove_reference_t<decltype(slots[i])>>(raw + i % distinct * bytes_each);
     };
-    ring(dhidden, side_lane ? HiddenRing : 2, M * W * e);
+    ring(dhidden, side_lanes ? HiddenRing : 2, M * W * e);
     bytes(dbranch, M * W);
-    ring(dwide, side_lane ? LayerRing : 1, M * wide * e);
-    ring(dqkv, side_lane ? LayerRing : 1, M * 3 * W * e);
+    ring(dwide, side_lanes ? LayerRing : 1, M * wide * e);
+    ring(dqkv, side_lanes ? LayerRing : 1, M * 3 * W * e);
     bytes(dactivated, M * Hd);
     allocate(attention_scratch,
              std::max<size_t>(size_t(M) * c.heads, flash_attention_backward_scratch_bytes(c.base.batch, T, c.heads) / sizeof(float)),
              false);
-    ring(simt_scratch, side_lane ? 2 : 1, SimtScratchBytes); // the lanes of the forward and backward pass
+    ring(simt_scratch, 1 + side_lanes, SimtScratchBytes); // the lanes of the forward and backward pass
     norm_blocks = norm_backward_blocks(tokens, sms);
-    ring(norm_partial, side_lane ? HiddenRing : 1, size_t(norm_blocks) * 2 * W * sizeof(float));
+    ring(norm_partial, side_lanes ? HiddenRing : 1, size_t(norm_blocks) * 2 * W * sizeof(float));
     if (embedding_backward_sliced(tokens, W))
         allocate(embedding_partial, size_t(EmbeddingSlices) * Vocabulary * W, false);
     sumsq_blocks = sms * 8;
@@ -572,13 +580,25 @@ void Engine::backward() {
     const bool layer_norm = c.norm == TG_NORM_LAYER;
     const int wide = c.mlp == TG_MLP_SWIGLU ? 2 * Hd : Hd;
     // Nothing in backward waits for a weight gradient or for the sums of a norm's scale and bias gradients: they run on
-    // a lane of their own beside the chain of input gradients.
-    const int side = side_lane ? 1 : 0;
+    // lanes of their own (1 .. side_lanes) beside the chain of input gradients.
     next_fork_event = 0;
-    auto aside = [&] { // launches go to the side lane, after everything the main lane holds
+    int asides = 0;
+    auto aside = [&] { // launches go to the side lanes in turn, after everything the main lane holds
+        const int side = side_lanes ? 1 + asides++ % side_lanes : 0;
         if (side)
             fork(0, side);
         return OnLane(*this, side);
+    };
+    using SideMarks = std::array<cudaEvent_t, 2>; // after everything the side lanes hold
+    auto mark_sides = [&] {
+        SideMarks marks{};
+        for (int k = 0; k < side_lanes; ++k)
+            marks[k] = mark(1 + k);
+        return marks;
+    };
+    auto await_sides = [&](const SideMarks &marks) {
+        for (int k = 0; k < side_lanes; ++k)
+            await(0, marks[k]);
     };
     // dW[out, in] = dy^T x: both operands are read "MN-major" (tokens are the contraction).
     auto weight_grad = [&](const void *dy, int out, const void *xin, int in, int64_t offset) {
@@ -625,11 +645,11 @@ void Engine::backward() {
     else
         exchange_bucket(layout.final_norm, layout.final_norm + (layer_norm ? 2 : 1) * W, depth);
 
-    std::vector<cudaEvent_t> layer_done(depth); // the side lane's end of each layer
-    const cudaEvent_t head_done = side ? mark(side) : nullptr;
+    std::vector<SideMarks> layer_done(depth); // the side lanes' end of each layer
+    const SideMarks head_done = mark_sides();
     for (int l = depth - 1; l >= 0; --l) {
-        if (side && l + 2 < depth)
-            await(0, layer_done[l + 2]); // its buffers are about to be written again
+        if (l + 2 < depth)
+            await_sides(layer_done[l + 2]); // its buffers are about to be written again
         void *dwide = this->dwide[l % LayerRing], *dqkv = this->dqkv[l % LayerRing];
         LayerActivations &a = layers[l];
         const LayerOffsets &p = layout.layers[l];
@@ -671,17 +691,18 @@ void Engine::backward() {
         gemm(FGemmInputGrad, input_grad(dqkv, 3 * W, p.qkv, W, dbranch));
         norm_back(a.x, dbranch, p.attention_norm, p.attention_norm_bias, dh(), dh_next(), a.stats1);
         ++hidden;
-        if (side)
-            layer_done[l] = mark(side);
+        layer_done[l] = mark_sides();
         if (announce_gradients)
             for (const BatchCopies::Piece &piece : copies.pieces)
-                if (piece.layer == l)
-                    announce(piece.ready, side);
+                if (piece.layer == l) {
+                    if (side_lanes == 2)
+                        fork(2, 1);
+                    announce(piece.ready, side_lanes ? 1 : 0);
+                }
         int64_t layer_end = l + 1 < depth ? layout.layers[l + 1].attention_norm : layout.final_norm;
         exchange_bucket(p.attention_norm, layer_end, l);
     }
-    if (side)
-        await(0, head_done); // a tied head's gradient is added to
+    await_sides(head_done); // a tied head's gradient is added to
     run(FEmbeddingBackward, [&](cudaStream_t s) {
         launch_embedding_backward(act, dh(), x, gradient + layout.embedding, M, W, c.tied != 0, embedding_partial,
                                   s);
@@ -690,7 +711,7 @@ void Engine::backward() {
         ++launches; // slices kernel + sum kernel
     exchange_bucket(layout.embedding, layout.embedding + int64_t(Vocabulary) * W, depth + 1);
     finish_exchange();
-    if (side)
+    for (int side = 1; side <= side_lanes; ++side)
         fork(side, 0); // join
 }
 

@@ -137,10 +137,11 @@ struct Engine {
     Lane lanes[LaneCount];
     int lane = 0;            // where run() launches
     bool concurrent = false; // whether work may be forked at all
-    bool side_lane = false, muon_lanes = false; // weight gradients beside the chain; the Muon families beside each other
+    int side_lanes = 0;      // lanes of weight gradients beside the chain
+    bool muon_lanes = false; // the Muon families beside each other
     std::vector<cudaEvent_t> fork_events; // as many as a backward pass marks: none is recorded again before its last wait
     size_t next_fork_event = 0;
-    float *simt_scratch[2] = {nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
+    float *simt_scratch[3] = {nullptr, nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
     BatchCopies copies; // of tg_batch's results
     bool announce_gradients = false;
     StepGraph graphs[GraphKinds];
