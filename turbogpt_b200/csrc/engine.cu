@@ -677,9 +677,8 @@ void Engine::backward() {
             SoftmaxAttentionBackwardArgs at{a.qkv, a.attended, dbranch, a.lse, attention_scratch, dqkv, B, T, W, H};
             run(FAttentionBackward, [&](cudaStream_t s) {
                 if (tensor_cores && act == Dtype::BF16 && flash_attention_supported(W, H)) {
-                    launch_flash_attention_backward(a.qkv, a.attended, dbranch, a.lse, attention_scratch, dqkv, B, T, H,
-                                                    counters, s);
-                    ++launches; // dq kernel + dk/dv kernel
+                    launches += launch_flash_attention_backward(a.qkv, a.attended, dbranch, a.lse, attention_scratch, dqkv, B, T, H,
+                                                                counters, s) - 1;
                 } else {
                     launch_softmax_attention_backward(act, at, s);
                 }

@@ -116,7 +116,8 @@ void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int 
 // `scratch`: flash_attention_backward_scratch_bytes() bytes; the dq kernel fills it with every query's lse
 // (base 2) and rowsum(dout * out) for the dk/dv kernel.
 size_t flash_attention_backward_scratch_bytes(int batch, int context, int heads);
-void launch_flash_attention_backward(const void *qkv, const void *out, const void *dout, const float *lse,
+// Returns the number of kernels it launched.
+int launch_flash_attention_backward(const void *qkv, const void *out, const void *dout, const float *lse,
                                      float *scratch, void *dqkv, int batch, int context, int heads,
                                      StepCounters *counters, cudaStream_t s);
 
