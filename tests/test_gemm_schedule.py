@@ -34,6 +34,16 @@ def test_rows_off_the_cache_lines_are_priced(library, m, n, k, b_mn, aligned_cho
     assert schedule(library, m, n, k, b_mn, pitch=whole_lines)[:3] == aligned_choice
 
 
+# Measured us: the form that the costs for any N choose, and the fastest.
+@pytest.mark.parametrize("m,n,k,b_mn,fastest", [
+    (32768, 768, 768, False, (192, 1, 1)),    # 41.0, 34.6
+    (32768, 768, 768, True, (256, 1, 1)),     # 40.9, 36.2
+    (8192, 1536, 384, False, (256, 1, 1)),    # 12.4, 10.7
+    (4096, 3072, 768, False, (256, 1, 1))])   # 18.0, 15.9
+def test_outputs_of_whole_blocks_have_costs_of_their_own(library, m, n, k, b_mn, fastest):
+    assert schedule(library, m, n, k, b_mn)[:3] == fastest
+
+
 def test_alignment_has_no_say_in_how_often_k_is_cut(library):
     cut = 0
     for m in (16, 100, 260, 445, 1140, 5000):

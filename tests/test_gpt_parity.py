@@ -259,6 +259,11 @@ def test_lanes_change_nothing_on_either_side_of_their_limits(depth, width, batch
     lanes_against_one(depth, width, batch, context, optimizer)
 
 
+@pytest.mark.parametrize("tokens", [(4, 2048), (1, 8193)])  # x 512: at 2^22, and above
+def test_one_and_two_lanes_of_weight_gradients_change_nothing(tokens):
+    lanes_against_one(3, 512, *tokens, bridge.HIDDEN_ADAMW)
+
+
 @pytest.mark.parametrize("optimizer", [bridge.HIDDEN_ADAMW, bridge.HIDDEN_MUON])
 def test_lanes_change_nothing_in_fp32(optimizer):
     """FP32 engines have the lanes too: products on CUDA cores, each lane's K slices in scratch of its own."""
@@ -471,3 +476,35 @@ def test_ragged_context_on_the_tensor_core_path(context, batch):
     assert relative(logits, target) <= 1e-2
     assert relative(gradients, expected_grad) <= 1e-2
     np.testing.assert_allclose(losses, expected_losses, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("width,hidden,context,batch", [(128, 192, 77, 5), (192, 1000, 128, 3), (256, 1024, 1024, 1), (320, 3208, 333, 9)])
+def test_evaluation_keeps_the_bits_of_a_call_with_gradients(width, hidden, context, batch):
+    """Without gradients the MLP's epilogue stores GELU alone, not its derivative: the same logits, losses and activations."""
+    rng = np.random.default_rng(width)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    with Native(ConfigEx.gpt(Config(depth=3, context=context, batch=batch), width, width // 64, hidden)) as engine:
+        engine.set_weights(rng.standard_normal(engine.count).astype(np.float32) * .05)
+        for _ in range(3):  # launched directly, captured, replayed
+            logits, _, losses = engine.batch(x, y)
+            kept = engine.read_activation(2, "activated")
+            alone, _, losses_alone = engine.batch(x, y, backward=False)
+            np.testing.assert_array_equal(alone, logits)
+            np.testing.assert_array_equal(losses_alone, losses)
+            np.testing.assert_array_equal(engine.read_activation(2, "activated"), kept)
+
+
+def test_norms_overlap_up_to_a_row_per_warp():
+    """4736 rows: norms start during the product before them; with one sequence more they do not.  The same bits."""
+    context, batch = 148, 33
+    rng = np.random.default_rng(9)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    results, w = [], None
+    for sequences in (batch - 1, batch):
+        with Native(ConfigEx.gpt(Config(depth=3, context=context, batch=sequences), 128, 2)) as engine:
+            w = rng.standard_normal(engine.count).astype(np.float32) * .05 if w is None else w
+            engine.set_weights(w)
+            for _ in range(3):
+                logits = engine.batch(x[:sequences], y[:sequences], backward=False)[0]
+            results.append(logits)
+    np.testing.assert_array_equal(results[0], results[1][:batch - 1])

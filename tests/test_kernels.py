@@ -157,6 +157,27 @@ def test_split_k_weight_gradient_is_deterministic():
         np.testing.assert_array_equal(first, gemm(lib, a, sa, b, sb, 768, 768, 16384, True, True))
 
 
+@pytest.mark.parametrize("m,n,k,plan", [
+    (768, 768, 3007, (128, 4, 1)), (768, 768, 3009, (64, 1, 0)),  # 47 and 48 K blocks
+    (136, 72, 8192, (64, 16, 0)), (1000, 776, 8100, (64, 1, 0)), (1288, 1160, 8192, (128, 1, 0)),
+    (776, 776, 8193, (128, 3, 0))])                               # 129 K blocks
+def test_weight_gradients_of_one_round(m, n, k, plan):
+    """The schedule's limits, partial tiles in every dimension, FP32 sums of k exact products against 64 bits; and without allocation."""
+    lib = load_library()
+    chosen = (ctypes.c_int32 * 4)()
+    assert lib.tg_ex_gemm_schedule(1, m, 1, n, n, m, n, k, 1, 1, 0, 148, chosen) == 0
+    assert tuple(chosen)[:3] == plan, tuple(chosen)
+    g = torch.Generator(device="cuda").manual_seed(k)
+    dy, x = (torch.randn(k, columns, generator=g, device="cuda").bfloat16() for columns in (m, n))
+    dw, static = (torch.full((m, n), float("nan"), device="cuda") for _ in range(2))
+    assert lib.tg_ex_gemm(dy.data_ptr(), 1, m, x.data_ptr(), 1, n, dw.data_ptr(), n, m, n, k, 1, 1, None) == 0, lib.tg_error()
+    assert lib.tg_ex_weight_gradient_static(dy.data_ptr(), x.data_ptr(), static.data_ptr(), m, n, k, None) == 0, lib.tg_error()
+    torch.cuda.synchronize()
+    bound = k * 2.0 ** -24 * (dy.double().abs().T @ x.double().abs())
+    assert ((dw.double() - dy.double().T @ x.double()).abs() <= bound).all()
+    assert torch.equal(dw, static)
+
+
 def test_cross_entropy_matches_torch():
     lib = load_library()
     rows = 4096 + 3
@@ -300,6 +321,38 @@ def test_norms_match_torch(rows, width, kind):
 def test_attention_with_four_blocks_per_sm(batch, context, heads):
     """Grids large enough for the one-chain forward kernel, at sequence ends on and off its 64- and 128-row steps."""
     test_attention_matches_torch(batch, context, heads, 64)
+
+
+def attention(qkv, dout, batch, context, heads):
+    lib, tokens = load_library(), batch * context
+    out = torch.full((tokens, heads * 64), float("nan"), device="cuda", dtype=torch.bfloat16)
+    lse, dqkv = torch.full((batch, heads, context), float("nan"), device="cuda"), torch.full_like(qkv, float("nan"))
+    assert lib.tg_ex_attention_forward(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), batch, context, heads, 64, 1, None) == 0, lib.tg_error()
+    assert lib.tg_ex_attention_backward(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(), batch, context,
+                                        heads, 64, 1, None) == 0, lib.tg_error()
+    torch.cuda.synchronize()
+    assert lib.tg_ex_last_device_error(None) == 0
+    return out, lse, dqkv
+
+
+@pytest.mark.parametrize("context,heads", [(1, 4), (64, 3), (65, 4), (128, 37), (129, 3), (333, 4), (1000, 2), (1024, 4), (1025, 2)])
+def test_attention_with_a_block_per_sm_keeps_the_bits(context, heads):
+    """Up to 148 blocks the forward chains have two score buffers and dQ runs beside dK and dV (that up to context 1024); with more
+    blocks of the same sequences neither.  Sequences do not know of one another: the same bits."""
+    tiles = -(-context // 128) * heads
+    few, many = 148 // tiles, 149 // tiles + 2
+    assert few * tiles <= 148 < many * tiles < 3 * 148  # below the one-chain kernel
+    g = torch.Generator(device="cuda").manual_seed(context)
+    qkv = torch.randn(many * context, heads * 192, generator=g, device="cuda").bfloat16()
+    dout = torch.randn(many * context, heads * 64, generator=g, device="cuda").bfloat16()
+    large = attention(qkv, dout, many, context, heads)
+    small = attention(qkv[:few * context], dout[:few * context], few, context, heads)
+    for a, b in zip(small, large):
+        assert torch.isfinite(b).all() and torch.equal(a, b[:len(a)])
+
+
+def test_attention_forward_of_one_buffer_when_the_row_maximum_keeps_growing():
+    test_attention_forward_when_the_row_maximum_keeps_growing(30)  # 270 blocks: two chains of one score buffer each
 
 
 @pytest.mark.parametrize("batch", [100, 2])  # 900 blocks of 128 queries: one chain per block; 18: two chains

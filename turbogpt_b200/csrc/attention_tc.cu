@@ -12,7 +12,7 @@
 // exponentials the other waits for its scores or hands its probabilities to the MMA thread; the
 // chains never wait for each other and are merged once at the end.  An accumulator is rescaled only
 // when its row maximum has grown by more than 2^8.  Two CTAs share an SM (256 TMEM columns and 84 KB
-// of shared memory each).
+// of shared memory each); in grids of up to one CTA per SM a chain has two score buffers and the ring eight slots.
 #include "device_utils.cuh"
 #include "sm100.cuh"
 

@@ -12,10 +12,12 @@
 // index), which covers y = x W^T, dx = dy W and dW = dy^T x on row-major tensors without transposes.
 //
 // Epilogue: four warps share each 32-lane quarter of tensor memory and take every fourth
-// 32-column chunk.  A lane owns one output row: it reads its accumulator chunk (tcgen05.ld),
-// optionally combines it with the same chunk of a second tensor read straight from global memory, the first one
-// before the products are done (residual, saved GELU derivative, or the Newton-Schulz operand), and writes 32-byte pieces with
-// 256-bit stores.
+// 32-column chunk.  A lane reads its row's accumulator chunk (tcgen05.ld), exchanges half of it with its neighbour (so that a
+// 256-bit access covers 16 rows instead of 32), optionally combines it with the same part of a second tensor read straight from global
+// memory one chunk ahead (residual, saved GELU derivative, or the Newton-Schulz operand), and stores.  Over a short K the epilogue
+// is as long as the products or longer: clocks of a 128 x 256 tile inside the 12-layer step, where K 768 takes the tensor pipe 6144: GELU with
+// its derivative 8000 (11700 with a lane to a row, one value at a time, and a pair's warps awaiting their stores), GELU gradient
+// 7500 (11800), plain 3100 (7200).  Over a long K the products take their 512 clocks a 64-deep block of a 256 x 256 tile (8192^3: 513).
 //
 // Weight-gradient GEMMs have few output tiles and a very long K; they are split along K and each
 // split writes an FP32 partial tile to a workspace.  With two or three splits the last one to finish
@@ -689,8 +691,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // C = the K splits' partial tiles added in split order, for schedules with four or more splits: there the last
-// arriver of a tile would pull every partial tile through one SM (1 MB per CTA at eight splits: 24 000 clocks
-// at the SM's L2 read rate, as long as the products themselves); this kernel spreads the same additions, in the
+// arriver of a tile would pull every partial tile through one SM (1 MB per CTA at eight splits: 24 000 clocks,
+// as long as the products themselves); this kernel spreads the same additions, in the
 // same order, over the whole GPU.  One block per 32 x 32 chunk of the padded output (a chunk is stored column
 // by column, see the kernel above); rows go out whole through a padded shared-memory tile.
 template <bool OutFp32>
