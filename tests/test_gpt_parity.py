@@ -487,11 +487,11 @@ def test_evaluation_keeps_the_bits_of_a_call_with_gradients(width, hidden, conte
         engine.set_weights(rng.standard_normal(engine.count).astype(np.float32) * .05)
         for _ in range(3):  # launched directly, captured, replayed
             logits, _, losses = engine.batch(x, y)
-            kept = engine.read_activation(2, "activated")
+            kept = engine.activation(2, "activated")
             alone, _, losses_alone = engine.batch(x, y, backward=False)
             np.testing.assert_array_equal(alone, logits)
             np.testing.assert_array_equal(losses_alone, losses)
-            np.testing.assert_array_equal(engine.read_activation(2, "activated"), kept)
+            np.testing.assert_array_equal(engine.activation(2, "activated"), kept)
 
 
 def test_norms_overlap_up_to_a_row_per_warp():
