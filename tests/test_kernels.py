@@ -323,32 +323,42 @@ def test_attention_with_four_blocks_per_sm(batch, context, heads):
     test_attention_matches_torch(batch, context, heads, 64)
 
 
-def attention(qkv, dout, batch, context, heads):
-    lib, tokens = load_library(), batch * context
-    out = torch.full((tokens, heads * 64), float("nan"), device="cuda", dtype=torch.bfloat16)
-    lse, dqkv = torch.full((batch, heads, context), float("nan"), device="cuda"), torch.full_like(qkv, float("nan"))
+def attention_forward(qkv, batch, context, heads):
+    lib = load_library()
+    out = torch.full((batch * context, heads * 64), float("nan"), device="cuda", dtype=torch.bfloat16)
+    lse = torch.full((batch, heads, context), float("nan"), device="cuda")
     assert lib.tg_ex_attention_forward(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), batch, context, heads, 64, 1, None) == 0, lib.tg_error()
+    return out, lse
+
+
+def attention_backward(qkv, out, dout, lse, batch, context, heads):
+    lib, dqkv = load_library(), torch.full_like(qkv, float("nan"))
     assert lib.tg_ex_attention_backward(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(), batch, context,
                                         heads, 64, 1, None) == 0, lib.tg_error()
     torch.cuda.synchronize()
     assert lib.tg_ex_last_device_error(None) == 0
-    return out, lse, dqkv
+    return dqkv
 
 
-@pytest.mark.parametrize("context,heads", [(1, 4), (64, 3), (65, 4), (128, 37), (129, 3), (333, 4), (1000, 2), (1024, 4), (1025, 2)])
-def test_attention_with_a_block_per_sm_keeps_the_bits(context, heads):
-    """Up to 148 blocks the forward chains have two score buffers and dQ runs beside dK and dV (that up to context 1024); with more
-    blocks of the same sequences neither.  Sequences do not know of one another: the same bits."""
+@pytest.mark.parametrize("context,heads", [(1, 4), (64, 3), (65, 4), (128, 37), (129, 3), (333, 4), (512, 3), (513, 3), (1000, 2), (1024, 4),
+                                           (1025, 2)])
+def test_attention_of_small_grids_keeps_the_bits(context, heads):
+    """Up to 148 blocks the forward chains have two score buffers, with more one; dQ runs beside dK and dV up to three blocks an SM,
+    seven where a sequence has four tiles at most, and context 1024, then before them.  Sequences do not know of one another: the same bits."""
     tiles = -(-context // 128) * heads
-    few, many = 148 // tiles, 149 // tiles + 2
-    assert few * tiles <= 148 < many * tiles < 3 * 148  # below the one-chain kernel
+    few, some, many = 148 // tiles, 149 // tiles + 2, (7 if context <= 512 else 3) * 148 // tiles + 1
+    assert few * tiles <= 148 < some * tiles < 3 * 148 < many * tiles  # `some`: below the one-chain kernel
     g = torch.Generator(device="cuda").manual_seed(context)
     qkv = torch.randn(many * context, heads * 192, generator=g, device="cuda").bfloat16()
     dout = torch.randn(many * context, heads * 64, generator=g, device="cuda").bfloat16()
-    large = attention(qkv, dout, many, context, heads)
-    small = attention(qkv[:few * context], dout[:few * context], few, context, heads)
-    for a, b in zip(small, large):
+    for a, b in zip(attention_forward(qkv[:few * context], few, context, heads), attention_forward(qkv[:some * context], some, context, heads)):
         assert torch.isfinite(b).all() and torch.equal(a, b[:len(a)])
+    out, lse = attention_forward(qkv, many, context, heads)
+    large = attention_backward(qkv, out, dout, lse, many, context, heads)
+    assert torch.isfinite(large).all()
+    for n in (few, many - 1):
+        rows = n * context
+        assert torch.equal(attention_backward(qkv[:rows], out[:rows], dout[:rows], lse[:n], n, context, heads), large[:rows])
 
 
 def test_attention_forward_of_one_buffer_when_the_row_maximum_keeps_growing():

@@ -900,7 +900,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_con
 constexpr int DkvStep = 64, DkvStepBytes = DkvStep * HeadSize * 2, DkvRing = 4;
 constexpr int DkvShared = 2 * TileBytes + DkvRing * 2 * DkvStepBytes + DkvRing * 128 * 4 + 1024 + 256; // K, V, ring of (Q, dO), statistics
 
-// Beside the dq kernel instead of after it: a block computes the statistics of its queries itself, for contexts up to this.
+// Beside the dq kernel instead of after it: a block computes the statistics of its queries itself, for contexts up to this (8 KB).
 constexpr int OwnStatistics = 1024;
 constexpr int DkvOwnShared = 2 * TileBytes + DkvRing * 2 * DkvStepBytes + 2 * OwnStatistics * 4 + 1024 + 256;
 
@@ -1168,11 +1168,12 @@ flash_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_co
     dkv_block<false>(map_qkv128, map_qkv64, map_do64, p, blockIdx.x);
 }
 
-// Both at once, where all of their blocks find room: the first half of the grid takes tiles of queries, the second tiles of keys.
+// Both at once: the first half of the grid takes tiles of queries, the second tiles of keys.
 constexpr int BothShared = DqShared > DkvOwnShared ? DqShared : DkvOwnShared;
 __global__ void __launch_bounds__(BackwardThreads, 2)
 flash_both_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_constant__ CUtensorMap map_qkv64,
                   const __grid_constant__ CUtensorMap map_do128, const __grid_constant__ CUtensorMap map_do64, BackwardParams p) {
+    grid_dependency_wait(); // launched so that it starts while the kernel before it runs
     const int half = gridDim.x / 2;
     if (int(blockIdx.x) < half)
         dq_block<false>(map_qkv128, map_qkv64, map_do128, p, blockIdx.x);
@@ -1254,11 +1255,13 @@ int launch_flash_attention_backward(const void *qkv, const void *out, const void
     CUtensorMap do64 = make_map_bf16(dout, width, rows, 1, width, 0, HeadSize, DkvStep);
     const int grid = batch * heads * p.tiles;
     CUtensorMap qkv64 = make_map_bf16(qkv, uint64_t(3) * width, rows, 1, uint64_t(3) * width, 0, HeadSize, DqStep);
-    // Where all blocks of both kernels find room at once (two to an SM) they run beside each other; what that costs is the statistics of a
-    // block's queries, once a key tile.  One after the other -> both: (32, 256) 18.5 -> 10.3 us, (42, 333) 22.6 -> 17.0, (12, 1024) 37.0 -> 26.7.
-    const bool both = grid <= 148 && p.tiles * BlockM <= OwnStatistics;
+    // Both kernels' blocks in one launch, where filling and draining the GPU twice costs more than what it takes: a block of keys computes the
+    // statistics of its queries itself, once a key tile.  One after the other -> at once, at (batch x heads, context): (32, 256) 18.5 -> 10.3 us,
+    // (12, 1024) 37.0 -> 26.7, (160, 256) 30.6 -> 23.6, (48, 1024) 50.0 -> 45.7, slower from (96, 1024) 84.9 -> 88.1 on; with up to
+    // four tiles a sequence the statistics cost less: (500, 128) 30.8 -> 26.4, (240, 333) 53.2 -> 49.8, (480, 256) 63.0 -> 59.6.
+    const bool both = p.tiles * BlockM <= OwnStatistics && grid <= (p.tiles <= 4 ? 7 : 3) * 148;
     if (both) {
-        flash_both_kernel<<<2 * grid, BackwardThreads, BothShared, s>>>(qkv128, qkv64, do128, do64, p);
+        launch_overlapping(flash_both_kernel, 2 * grid, BackwardThreads, BothShared, s, qkv128, qkv64, do128, do64, p);
     } else {
         flash_dq_kernel<<<grid, BackwardThreads, DqShared, s>>>(qkv128, qkv64, do128, p); // also writes the statistics
         flash_dkv_kernel<<<grid, BackwardThreads, DkvShared, s>>>(qkv128, qkv64, do64, p);
