@@ -874,6 +874,16 @@ Schedule weight_gradient_schedule(const GemmArgs &g, int sms) {
     }
     return best;
 }
+Schedule choose_schedule(const GemmArgs &g, int sms) {
+    return g.out == Dtype::FP32 && g.epilogue == Epilogue::Store ? weight_gradient_schedule(g, sms) : product_schedule(g, sms);
+}
+
+bool half_an_sm(const GemmArgs &g, const Schedule &sc, int sms) {
+    const long long tiles = (long long)((g.m + BM - 1) / BM) * ((g.n + sc.bn - 1) / sc.bn) * g.batch;
+    return g.beside_others && g.batch > 1 && g.out == Dtype::BF16 && (g.epilogue == Epilogue::Store || g.epilogue == Epilogue::Axpby) &&
+           !sc.pair && sc.bn <= 128 && tiles * sc.splits <= sms;
+}
+
 // Scratch a schedule needs: FP32 partial tiles and one ticket per output tile (none without a K split).
 struct ScratchNeed {
     size_t partial_bytes = 0, tickets = 0;
@@ -886,41 +896,6 @@ ScratchNeed scratch_need(const GemmArgs &g, const Schedule &sc) {
     const int n_tiles = (g.n + sc.bn - 1) / sc.bn;
     return {size_t(sc.splits) * g.batch * padded_m_tiles * BM * n_tiles * sc.bn * sizeof(float),
             size_t(padded_m_tiles) * n_tiles * g.batch};
-}
-
-constexpr size_t StaticPartialBytes = size_t(16) << 20; // of tg_ex_weight_gradient_static: FP32 partial tiles
-// Weight gradients over 3072 to 8192 tokens whose tiles of some width fit the GPU in one round: single CTAs of the narrowest such
-// width, K uncut.  Timed alone, 768 x 768 x 4096 takes 16.3 us cut in four and 12.3 like this, 1536 x 384 x 4096 16.4 and 12.3, 1024 x 1024 x 8192 26.7
-// and 21.3; 8 layers d 512, 4096 tokens 2189 -> 2117 us a step, 12 layers d 768, 4096 tokens 0.9 %, 8 layers d 640, 8192 tokens 0.7 %.  Over fewer
-// tokens it is faster alone too (2048: 9.2 -> 7.8 us), but there the step is its chain of input gradients, and more blocks are more in its way
-// (4 layers d 256, 2048 tokens 360 -> 370 us); over more, few tiles leave SMs idle and K is cut.  What needs more scratch than
-// tg_ex_weight_gradient_static has keeps the schedule that says so.
-Schedule one_round_weight_gradient(const GemmArgs &g, int sms, const Schedule &otherwise) {
-    if (scratch_need(g, otherwise).partial_bytes > StaticPartialBytes)
-        return otherwise;
-    const int m_tiles = (g.m + BM - 1) / BM, k_blocks = (g.k + BK - 1) / BK;
-    for (int bn : {64, 128, 192, 256}) {
-        const long long tiles = (long long)m_tiles * ((g.n + bn - 1) / bn) * g.batch;
-        if (tiles > sms)
-            continue;
-        if (k_blocks > 64 && tiles * 3 < sms * 2)
-            break;
-        Schedule sc;
-        sc.bn = bn, sc.k_blocks_per_split = k_blocks;
-        return sc;
-    }
-    return otherwise;
-}
-Schedule choose_schedule(const GemmArgs &g, int sms) {
-    if (g.out == Dtype::FP32 && g.epilogue == Epilogue::Store && (g.k + BK - 1) / BK >= 48 && (g.k + BK - 1) / BK <= 128)
-        return one_round_weight_gradient(g, sms, weight_gradient_schedule(g, sms));
-    return g.out == Dtype::FP32 && g.epilogue == Epilogue::Store ? weight_gradient_schedule(g, sms) : product_schedule(g, sms);
-}
-
-bool half_an_sm(const GemmArgs &g, const Schedule &sc, int sms) {
-    const long long tiles = (long long)((g.m + BM - 1) / BM) * ((g.n + sc.bn - 1) / sc.bn) * g.batch;
-    return g.beside_others && g.batch > 1 && g.out == Dtype::BF16 && (g.epilogue == Epilogue::Store || g.epilogue == Epilogue::Axpby) &&
-           !sc.pair && sc.bn <= 128 && tiles * sc.splits <= sms;
 }
 
 // Stand-alone calls (tg_ex_gemm) share one workspace per device, grown on demand.
@@ -1151,6 +1126,7 @@ void launch_with(const GemmArgs &g, const Schedule &sc, int sms, StepCounters *c
 // for the same shape, so the results are bit-identical to it.
 // ------------------------------------------------------------------------------------------
 namespace {
+constexpr size_t StaticPartialBytes = size_t(16) << 20; // 16 MiB of FP32 partial tiles
 constexpr int StaticTickets = 1024;                      // output tiles
 constexpr size_t StaticErrorOffset = StaticPartialBytes + StaticTickets * sizeof(unsigned);
 static __device__ __align__(256) unsigned char static_scratch[StaticErrorOffset + 256];
