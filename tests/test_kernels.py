@@ -157,27 +157,6 @@ def test_split_k_weight_gradient_is_deterministic():
         np.testing.assert_array_equal(first, gemm(lib, a, sa, b, sb, 768, 768, 16384, True, True))
 
 
-@pytest.mark.parametrize("m,n,k,plan", [
-    (768, 768, 3007, (128, 4, 1)), (768, 768, 3009, (64, 1, 0)),  # 47 and 48 K blocks
-    (136, 72, 8192, (64, 16, 0)), (1000, 776, 8100, (64, 1, 0)), (1288, 1160, 8192, (128, 1, 0)),
-    (776, 776, 8193, (128, 3, 0))])                               # 129 K blocks
-def test_weight_gradients_of_one_round(m, n, k, plan):
-    """The schedule's limits, partial tiles in every dimension, FP32 sums of k exact products against 64 bits; and without allocation."""
-    lib = load_library()
-    chosen = (ctypes.c_int32 * 4)()
-    assert lib.tg_ex_gemm_schedule(1, m, 1, n, n, m, n, k, 1, 1, 0, 148, chosen) == 0
-    assert tuple(chosen)[:3] == plan, tuple(chosen)
-    g = torch.Generator(device="cuda").manual_seed(k)
-    dy, x = (torch.randn(k, columns, generator=g, device="cuda").bfloat16() for columns in (m, n))
-    dw, static = (torch.full((m, n), float("nan"), device="cuda") for _ in range(2))
-    assert lib.tg_ex_gemm(dy.data_ptr(), 1, m, x.data_ptr(), 1, n, dw.data_ptr(), n, m, n, k, 1, 1, None) == 0, lib.tg_error()
-    assert lib.tg_ex_weight_gradient_static(dy.data_ptr(), x.data_ptr(), static.data_ptr(), m, n, k, None) == 0, lib.tg_error()
-    torch.cuda.synchronize()
-    bound = k * 2.0 ** -24 * (dy.double().abs().T @ x.double().abs())
-    assert ((dw.double() - dy.double().T @ x.double()).abs() <= bound).all()
-    assert torch.equal(dw, static)
-
-
 def test_cross_entropy_matches_torch():
     lib = load_library()
     rows = 4096 + 3
