@@ -340,6 +340,34 @@ def test_attention_of_small_grids_keeps_the_bits(context, heads):
         assert torch.equal(attention_backward(qkv[:rows], out[:rows], dout[:rows], lse[:n], n, context, heads), large[:rows])
 
 
+@pytest.mark.parametrize("batch,context,heads", [(5, 1, 3), (2, 333, 3), (1, 1024, 2), (300, 129, 2), (2, 1100, 3)])
+def test_attention_backward_adds_the_products_of_output_and_gradient_in_their_order(batch, context, heads):
+    """delta = rowsum(dO * O) is one FP32 accumulator over pairs of products, in dQ's kernel and in dK and dV's, in one launch (the first
+    three) and in two.  A row holds 2^34 and, further on, -2^34 among integers up to 6: what precedes the latter is rounded away, what
+    follows stays.  Probabilities are 1 and dP 0, every other sum is exact: the gradients are equal."""
+    g = torch.Generator(device="cuda").manual_seed(context)
+    rows = batch * context
+    small = torch.randint(-3, 4, (rows, heads, 32, 2), generator=g, device="cuda").float()
+    o, do = small, torch.ones_like(small)
+    first = torch.randint(0, 31, (rows, heads, 1), generator=g, device="cuda")
+    second = first + 1 + (torch.rand(rows, heads, 1, generator=g, device="cuda") * (31 - first)).long()
+    for at, sign in ((first, 1.), (second, -1.)):
+        o[..., 0].scatter_(2, at, 2. ** 17)
+        do[..., 0].scatter_(2, at, sign * 2. ** 17)
+        o[..., 1].scatter_(2, at, 0.)
+    pairs = (o.double() * do.double()).sum(-1)
+    delta = (pairs * (torch.arange(32, device="cuda") > second)).sum(-1).view(batch, context, heads, 1).transpose(1, 2)
+    q, k, v = torch.zeros(3, rows, heads, 64, device="cuda")
+    q[..., :32] = torch.randint(-2, 3, (rows, heads, 32), generator=g, device="cuda")  # Q K^T = 0
+    k[..., 32:] = torch.randint(-2, 3, (rows, heads, 32), generator=g, device="cuda")
+    qkv, lse = torch.stack([q, k, v], 1).bfloat16().view(rows, -1), torch.zeros(batch, heads, context, device="cuda")
+    dqkv = attention_backward(qkv, o.bfloat16().view(rows, -1), do.bfloat16().view(rows, -1), lse, batch, context, heads)
+    got_q, got_k, _ = dqkv.view(batch, context, 3, heads, 64).permute(2, 0, 3, 1, 4)
+    q, k = (t.double().view(batch, context, heads, 64).transpose(1, 2) for t in (q, k))
+    assert torch.equal(got_q, (-delta / 8 * k.cumsum(2)).bfloat16())
+    assert torch.equal(got_k, (-delta / 8 * q).flip(2).cumsum(2).flip(2).bfloat16())
+
+
 def test_attention_forward_of_one_buffer_when_the_row_maximum_keeps_growing():
     test_attention_forward_when_the_row_maximum_keeps_growing(30)  # 270 blocks: two chains of one score buffer each
 

@@ -628,28 +628,45 @@ __device__ __forceinline__ uint32_t score_gradient(uint32_t p0, uint32_t p1, uin
     return pack_bf16(d0, d1);
 }
 
-// delta = rowsum(dO * O) of a warp's 32 rows, lane = row.  Eight lanes take a row, so that a load covers four whole rows and the sums
-// are short (a lane to a row took 32 lines to a load and one long chain).  `gradient(r, chunk)`: 16 bytes of dO's row r.
+// delta = rowsum(dO * O) of a warp's 32 rows, lane = row.  Eight lanes take a row, so that a load covers four whole rows (a lane to a row
+// took 32 lines to a load).  A row's 32 sums of two neighbouring products are then brought together in one lane and added in the row's
+// order: dQ and dK keep the bits of one accumulator per row.  `gradient(r, chunk)`: 16 bytes of dO's row r.
 template <class Gradient>
 __device__ __forceinline__ float output_dot_gradient(const uint4 (&o)[8], int lane, Gradient gradient) {
     const int group = lane / 8, chunk = lane % 8;
-    float delta = 0.f;
+    float sums[8][4]; // of row 4 i + group, this lane's chunk
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const uint4 g = gradient(4 * i + group, chunk);
         const unsigned a4[4] = {o[i].x, o[i].y, o[i].z, o[i].w}, b4[4] = {g.x, g.y, g.z, g.w};
-        float sum = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            sum += __uint_as_float(a4[k] << 16) * __uint_as_float(b4[k] << 16) +
-                   __uint_as_float(a4[k] & 0xffff0000u) * __uint_as_float(b4[k] & 0xffff0000u);
-#pragma unroll
-        for (int k = 1; k < 8; k <<= 1)
-            sum += __shfl_xor_sync(0xffffffffu, sum, k);
-        const float mine = __shfl_sync(0xffffffffu, sum, (lane & 3) * 8); // row 4 i + lane % 4
-        delta = lane / 4 == i ? mine : delta;
+            sums[i][k] = __uint_as_float(a4[k] << 16) * __uint_as_float(b4[k] << 16) +
+                         __uint_as_float(a4[k] & 0xffff0000u) * __uint_as_float(b4[k] & 0xffff0000u);
     }
-    return delta;
+    // The eight lanes of a group exchange rows for chunks: afterwards sums[c] is chunk c of row 4 (lane % 8) + group.
+#pragma unroll
+    for (int bit = 4; bit > 0; bit >>= 1) {
+        const bool upper = chunk & bit;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i & bit)
+                continue;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float got = __shfl_xor_sync(0xffffffffu, upper ? sums[i][k] : sums[i | bit][k], bit);
+                sums[i][k] = upper ? got : sums[i][k];
+                sums[i | bit][k] = upper ? sums[i | bit][k] : got;
+            }
+        }
+    }
+    float delta = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            delta += sums[c][k];
+    return __shfl_sync(0xffffffffu, delta, (lane & 3) * 8 + lane / 4);
 }
 // Row 4 i + lane / 8 of the 32 rows at `rows`, 16 bytes at lane % 8, for i = 0 .. 7; zeros from row `valid` on.
 __device__ __forceinline__ void load_four_rows_at_a_time(const bf16 *rows, int64_t row_elements, int valid, int lane, uint4 (&v)[8]) {
