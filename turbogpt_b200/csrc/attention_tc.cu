@@ -63,10 +63,14 @@ __device__ __forceinline__ uint64_t unpack_pair(uint32_t packed) {
 // One chain: the scores of the second step are at tmem_o when the first begins, and the reference maximum is taken over both
 // (the probability of a maximum is 1, without a rounding error: two chains have two such); `sums.rounded` is kept too.
 // Two buffers: the scores of every second step are 128 columns further, with a barrier two further; a product with V may then be
-// under way (`o_full` counts them) when the next scores are ready.
+// under way when the next scores are ready.
+// Step n's product has ended when `s_full` of step n + Buffers completes: those scores take its buffer, and where no such step follows
+// the barrier completes all the same.  No other wait is for a product: a wait knows a phase by its parity alone, so a thread has to see
+// every phase of a barrier before the next can begin, as it does here (a step begins with this wait, and ends with the arrival
+// that the product, and with it the next phase, needs).
 template <int Chains, int Buffers>
 __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile_first, int row, uint32_t tmem_s0, uint32_t tmem_o,
-                                             uint32_t s_full, uint32_t p_full, uint32_t o_full, const ForwardParams &p, volatile int *abort_flag,
+                                             uint32_t s_full, uint32_t p_full, const ForwardParams &p, volatile int *abort_flag,
                                              float &reference_max, RowSums &sums, bool &ok) {
     constexpr bool Rounded = Chains == 1;
     const int lane = row % 32, warp_first = tile_first + row - lane, position = tile_first + row;
@@ -156,10 +160,9 @@ __device__ __forceinline__ int softmax_chain(int first_step, int steps, int tile
         }
         const bool grow = (block_max - reference_max) * p.scale_log2 > 8.f; // true for the first unmasked step
         if (__any_sync(0xffffffffu, grow && reference_max != -CUDART_INF_F)) {
-            // between this chain's products: with one buffer the scores awaited above were issued after the last one, with two after
-            // the last but one
+            // between this chain's products: with one buffer the scores awaited above came after the last one, with two the next ones do
             if (Buffers == 2 && mine > 0) {
-                ok = mbarrier_wait(o_full, (mine - 1) & 1, abort_flag, p.counters, 207);
+                ok = mbarrier_wait(s_full + 16 * (buffer ^ 1), ((mine + 1) >> 1) & 1, abort_flag, p.counters, 207);
                 if (!ok)
                     break;
                 tcgen05_fence_after();
@@ -237,8 +240,8 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     float *exchange = reinterpret_cast<float *>(aligned + TileBytes + Ring * 2 * KeyBytes); // [2 chains][max | sum][128 rows]
     uint64_t *barriers = reinterpret_cast<uint64_t *>(exchange + 4 * BlockM);
     const uint32_t q_full = smem_address(barriers), kv_full0 = q_full + 8, kv_empty0 = kv_full0 + 8 * Ring,
-                   s_full0 = kv_empty0 + 8 * Ring, p_full0 = s_full0 + 16 * Buffers, o_full0 = p_full0 + 16 * Buffers;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 1 + 2 * Ring + 2 + 4 * Buffers);
+                   s_full0 = kv_empty0 + 8 * Ring, p_full0 = s_full0 + 16 * Buffers;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 1 + 2 * Ring + 4 * Buffers);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const uint32_t smem_q = base, smem_kv = base + TileBytes;
 
@@ -261,8 +264,6 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             mbarrier_init(s_full0 + 8 * c, 1);
             mbarrier_init(p_full0 + 8 * c, 4);
         }
-        for (int c = 0; c < 2; ++c)
-            mbarrier_init(o_full0 + 8 * c, 1);
         *abort_flag = 0;
         fence_barrier_init();
         prefetch_map(&map_q);
@@ -304,10 +305,9 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint64_t q_desc = smem_descriptor(smem_q, 16, 1024), k_desc0 = smem_descriptor(smem_kv, 16, 1024),
                            v_desc0 = smem_descriptor(smem_kv + KeyBytes, 8192, 1024);
             bool ok = mbarrier_wait(q_full, 0, abort_flag, p.counters, 202);
-            int issued = 0;
-            auto issue_scores = [&]() { // S = Q K_j^T into a buffer of chain j % 2
-                const int ring = issued % Ring, buffer = issued % (2 * Buffers);
-                ok = mbarrier_wait(kv_full0 + 8 * ring, (issued / Ring) & 1, abort_flag, p.counters, 203);
+            auto issue_scores = [&](int j) { // S = Q K_j^T into a buffer of chain j % 2
+                const int ring = j % Ring, buffer = j % (2 * Buffers);
+                ok = mbarrier_wait(kv_full0 + 8 * ring, (j / Ring) & 1, abort_flag, p.counters, 203);
                 if (!ok)
                     return;
                 tcgen05_fence_after();
@@ -317,10 +317,9 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     tcgen05_mma_bf16(tmem_s0 + 64 * buffer, descriptor_at(q_desc, ks * 32), descriptor_at(k_desc, ks * 32),
                                      idesc_s, ks > 0);
                 tcgen05_commit(s_full0 + 8 * buffer);
-                ++issued;
             };
-            while (ok && issued < min(steps, 2 * Buffers))
-                issue_scores();
+            for (int j = 0; ok && j < min(steps, 2 * Buffers); ++j)
+                issue_scores(j);
             for (int j = 0; j < steps && ok; ++j) {
                 const int chain = j & 1, ring = j % Ring;
                 ok = mbarrier_wait(p_full0 + 8 * (j % (2 * Buffers)), (j / (2 * Buffers)) & 1, abort_flag, p.counters, 204);
@@ -332,10 +331,11 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 for (int ks = 0; ks < KeyStep / 16; ++ks) // O_chain += P V_j: four 16-key steps
                     tcgen05_mma_bf16_ts(tmem_o0 + 64 * chain, tmem_s0 + 64 * (j % (2 * Buffers)) + ks * 8,
                                         descriptor_at(v_desc, ks * 2048), idesc_o, (j > 1 || ks > 0) ? 1u : 0u);
-                tcgen05_commit(o_full0 + 8 * chain);
                 tcgen05_commit(kv_empty0 + 8 * ring); // K_j and V_j are no longer read
-                if (issued < steps)
-                    issue_scores(); // step j + 2 Buffers takes this step's buffer: issued after the products that read it
+                if (j + 2 * Buffers < steps)
+                    issue_scores(j + 2 * Buffers); // takes this step's buffer: issued after the products that read it
+                else
+                    tcgen05_commit(s_full0 + 8 * (j % (2 * Buffers))); // the phase that tells of this step's product
             }
         }
     } else {
@@ -351,12 +351,12 @@ flash_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         RowSums sums;
         bool ok = true;
         const int mine = softmax_chain<2, Buffers>(chain, steps, tile * BlockM, row, tmem_s, tmem_o, s_full0 + 8 * chain, p_full0 + 8 * chain,
-                                                   o_full0 + 8 * chain, p, abort_flag, reference_max, sums, ok);
+                                                   p, abort_flag, reference_max, sums, ok);
         const float running_sum = sums.sum;
-        if (Buffers == 2 && ok && mine > 1) // up to two products may be under way: a phase is awaited by its parity, so each in turn
-            ok = mbarrier_wait(o_full0 + 8 * chain, mine & 1, abort_flag, p.counters, 208);
-        if (ok && mine > 0)
-            ok = mbarrier_wait(o_full0 + 8 * chain, (mine - 1) & 1, abort_flag, p.counters, 208);
+        if (ok && mine > 0) { // the last product, and with it all
+            const int buffer = Buffers == 2 ? (mine - 1) & 1 : 0;
+            ok = mbarrier_wait(s_full0 + 8 * chain + 16 * buffer, (Buffers == 2 ? (mine + 1) >> 1 : mine) & 1, abort_flag, p.counters, 208);
+        }
         // merge the two chains: each publishes its reference maximum and sum, then takes half of the
         // output columns of both accumulators
         exchange[chain * 2 * BlockM + row] = reference_max;
@@ -549,7 +549,7 @@ flash_forward_single_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         float reference_max = -CUDART_INF_F;
         RowSums sums;
         bool ok = true;
-        softmax_chain<1, 1>(0, steps, tile * BlockM, row, tmem_s + lanes, tmem_o + lanes, s_full, p_full, o_full, p, abort_flag,
+        softmax_chain<1, 1>(0, steps, tile * BlockM, row, tmem_s + lanes, tmem_o + lanes, s_full, p_full, p, abort_flag,
                          reference_max, sums, ok);
         if (ok)
             ok = mbarrier_wait(o_full, 0, abort_flag, p.counters, 208);
