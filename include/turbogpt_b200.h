@@ -185,7 +185,9 @@ int64_t tg_ex_read_activation(Engine *engine, int layer, const char *name, float
  * copy or tensor-core operation in flight.  Returns 1 when the wait gave up as designed and left code
  * 901 in the engine's device error word (0 if it reported completion, < 0 on a host error).  The
  * engine's next synchronising call (tg_batch, tg_get_training_losses, tg_predict, tg_optimizer_test)
- * then fails with "a device-side wait gave up (code 901)"; tg_set_weights clears the error word. */
+ * then fails with "a device-side wait gave up (code 901)"; tg_set_weights clears the error word.
+ * engine NULL: the code is left where the stand-alone attention calls on the current device leave theirs
+ * (tg_ex_last_device_error returns it). */
 int tg_ex_selftest_bounded_wait(Engine *engine, double limit_ms);
 
 /* Kernel microbenchmarks on device pointers (BF16 unless noted), enqueued on `stream`.
@@ -218,8 +220,9 @@ int tg_ex_gemm_schedule(int64_t a_row, int64_t a_col, int64_t b_row, int64_t b_c
  * cleared on `stream` first): calls that overlap on the GPU race.  Results equal tg_ex_gemm's. */
 int tg_ex_weight_gradient_static(const void *dy, const void *x, float *dw, int out, int in, int tokens,
                                  void *stream);
-/* tg_ex_gemm and tg_ex_weight_gradient_static return once their kernel is enqueued.  Every wait inside
- * the kernel is bounded (about two seconds); one that gives up leaves a code in a device error word
+/* The stand-alone tensor-core calls (tg_ex_gemm, tg_ex_head_cross_entropy, tg_ex_weight_gradient_static,
+ * tg_ex_attention_*) return once their kernels are enqueued.  Every wait inside
+ * a kernel is bounded (about two seconds); one that gives up leaves a code in a device error word
  * and the output partly unwritten.  This call synchronises `stream` and returns the first such code
  * recorded on the current device since the last query (0: none; < 0: host error), clearing it.
  * Allocates nothing. */

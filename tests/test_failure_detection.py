@@ -8,6 +8,9 @@ leaves an error code that the next synchronising call reports; the engine stays 
 import ctypes as C
 import os
 import socket
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -98,3 +101,33 @@ def test_a_wait_that_runs_out_is_reported_and_the_engine_survives():
         after, _, _ = engine.batch(x, x, backward=False)
         np.testing.assert_array_equal(before, after)
         assert engine.lib.tg_ex_selftest_bounded_wait(engine.handle, 0.0) < 0    # limit out of range
+
+
+@pytest.mark.gpu
+def test_stand_alone_attention_reports_a_wait_that_gave_up():
+    lib = bridge.load_library()
+    assert lib.tg_ex_last_device_error(None) == 0
+    assert lib.tg_ex_selftest_bounded_wait(None, 1.0) == 1
+    assert lib.tg_ex_last_device_error(None) == 901
+    assert lib.tg_ex_last_device_error(None) == 0
+
+
+@pytest.mark.gpu
+def test_the_first_stand_alone_attention_call_can_be_captured():
+    """The error word is found without an allocation, in a process that has made no other call."""
+    code = """
+import torch
+from turbogpt_b200 import load_library
+lib = load_library()
+qkv = torch.randn(256, 192, device="cuda").bfloat16()
+out, lse = torch.zeros(256, 64, dtype=torch.bfloat16, device="cuda"), torch.empty(2, 1, 128, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    assert lib.tg_ex_attention_forward(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), 2, 128, 1, 64, 1,
+                                       torch.cuda.current_stream().cuda_stream) == 0, lib.tg_error()
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(out[0], qkv[0, 128:]) and lib.tg_ex_last_device_error(None) == 0
+"""
+    root = Path(__file__).resolve().parents[1]
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=root)

@@ -677,7 +677,7 @@ void launch_flash_attention_backward_fused(const void *qkv, const void *out, con
     p.dq_count = reinterpret_cast<int *>(statistics + 2 * pairs * padded);
     p.scale = 1.f / sqrtf(float(HeadSize));
     p.scale_log2 = 1.4426950408889634f * p.scale;
-    p.counters = counters;
+    p.counters = counters ? counters : attention_error_word(true);
     const uint64_t rows = uint64_t(batch) * context;
     const int64_t vectors = int64_t(rows) * width / 8;
     if (padded != size_t(context)) // the padding is read (and masked): keep it finite

@@ -15,6 +15,7 @@
 // of shared memory each); in grids of up to one CTA per SM a chain has two score buffers and the ring eight slots.
 #include "device_utils.cuh"
 #include "sm100.cuh"
+#include <atomic>
 
 using namespace sm100;
 
@@ -1198,7 +1199,24 @@ flash_both_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_c
         dkv_block<true>(map_qkv128, map_qkv64, map_do64, p, blockIdx.x - half);
 }
 
+// Error word of the calls that have no engine: a symbol, so that they allocate nothing.
+__device__ StepCounters stand_alone_counters;
+std::atomic<StepCounters *> stand_alone_address[64]; // per device, looked up by its first such call
 } // namespace
+
+StepCounters *attention_error_word(bool look_up) {
+    int device = 0;
+    CHECK_CUDA(cudaGetDevice(&device));
+    if (device >= 64)
+        return nullptr;
+    StepCounters *word = stand_alone_address[device];
+    if (!word && look_up) {
+        void *address = nullptr;
+        CHECK_CUDA(cudaGetSymbolAddress(&address, stand_alone_counters));
+        stand_alone_address[device] = word = static_cast<StepCounters *>(address);
+    }
+    return word;
+}
 
 bool flash_attention_supported(int width, int heads) {
     return heads > 0 && width == heads * HeadSize;
@@ -1222,7 +1240,7 @@ void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int 
     p.batch = batch, p.context = context, p.heads = heads, p.width = width;
     p.tiles = (context + BlockM - 1) / BlockM;
     p.scale_log2 = 1.4426950408889634f / sqrtf(float(HeadSize));
-    p.counters = counters;
+    p.counters = counters ? counters : attention_error_word(true);
     const uint64_t rows = uint64_t(batch) * context;
     CUtensorMap map_q = make_map_bf16(qkv, uint64_t(3) * width, rows, 1, uint64_t(3) * width, 0, HeadSize, BlockM);
     CUtensorMap map_kv = make_map_bf16(qkv, uint64_t(3) * width, rows, 1, uint64_t(3) * width, 0, HeadSize, KeyStep);
@@ -1264,7 +1282,7 @@ int launch_flash_attention_backward(const void *qkv, const void *out, const void
     p.tiles = (context + BlockM - 1) / BlockM;
     p.scale = 1.f / sqrtf(float(HeadSize));
     p.scale_log2 = 1.4426950408889634f * p.scale;
-    p.counters = counters;
+    p.counters = counters ? counters : attention_error_word(true);
     const uint64_t rows = uint64_t(batch) * context;
     CUtensorMap qkv128 = make_map_bf16(qkv, uint64_t(3) * width, rows, 1, uint64_t(3) * width, 0, HeadSize, 128);
 

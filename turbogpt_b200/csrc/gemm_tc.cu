@@ -1173,14 +1173,14 @@ void launch_weight_gradient_static(const void *dy, const void *x, float *dw, int
                     reinterpret_cast<StepCounters *>(scratch + StaticErrorOffset), s);
 }
 
-// First device-side give-up code recorded by the stand-alone GEMM calls (tg_ex_gemm,
-// tg_ex_weight_gradient_static) on the current device since the last query; 0 when none.
+// First device-side give-up code recorded by the stand-alone calls (tg_ex_gemm, tg_ex_head_cross_entropy,
+// tg_ex_weight_gradient_static, attention) on the current device since the last query; 0 when none.
 // Synchronises `s`; allocates nothing.
 int gemm_tc_take_device_error(cudaStream_t s) {
     int device = 0;
     CHECK_CUDA(cudaGetDevice(&device));
     CHECK_CUDA(cudaStreamSynchronize(s));
-    StepCounters *words[2] = {nullptr, nullptr};
+    StepCounters *words[3] = {nullptr, nullptr, attention_error_word(false)};
     {
         std::lock_guard<std::mutex> lock(shared_workspace_mutex);
         auto found = shared_workspaces.find(device);

@@ -109,6 +109,9 @@ struct SoftmaxAttentionBackwardArgs {
 void launch_softmax_attention_backward(Dtype t, const SoftmaxAttentionBackwardArgs &a, cudaStream_t s);
 
 // ---- causal softmax attention on tcgen05 (BF16, head size 64) ----
+// `counters` nullptr: a wait that gives up is recorded in the current device's word for calls without an engine, below (nullptr: no such
+// call yet, unless `look_up`), which gemm_tc_take_device_error() reads too.
+StepCounters *attention_error_word(bool look_up);
 bool flash_attention_supported(int width, int heads);
 void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int batch, int context, int heads,
                                     StepCounters *counters, cudaStream_t s);

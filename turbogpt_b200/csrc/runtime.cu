@@ -266,6 +266,8 @@ int64_t tg_ex_read_activation(Engine *e, int layer, const char *name, float *out
 
 int tg_ex_selftest_bounded_wait(Engine *e, double limit_ms) {
     try {
+        if (!e)
+            return launch_starved_wait(attention_error_word(true), limit_ms, 901, nullptr);
         e->set_device();
         return launch_starved_wait(e->counters, limit_ms, 901, e->stream);
     } catch (const std::exception &error) {
