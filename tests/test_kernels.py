@@ -106,6 +106,30 @@ def test_products_of_every_tile_form_at_their_edges(m, n, k, b_mn):
     assert lib.tg_ex_last_device_error(None) == 0
 
 
+def test_batches_of_more_matrices_than_a_launch_takes():
+    """2^20 tiles to a launch: matrices on both sides of the border, the second tensor's too, against 64 bits.  Neighbouring matrices share
+    all but 16 bytes."""
+    lib, batch, n, k = load_library(), 2 ** 20 + 5, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, b = (torch.randn(8 * batch + size, generator=g, device="cuda").bfloat16() for size in (k, n * k))
+    r = torch.randn(batch, n, generator=g, device="cuda").bfloat16()
+    c, scaled = (torch.full((batch, n), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    for out, second in ((c, None), (scaled, r.data_ptr())):
+        assert lib.tg_ex_gemm_batched(a.data_ptr(), k, 1, 8, b.data_ptr(), k, 1, 8, out.data_ptr(), n, n, second, .5, 3.,
+                                      1, n, k, batch, 0, None) == 0, lib.tg_error()
+    torch.cuda.synchronize()
+    assert torch.isfinite(c).all() and torch.isfinite(scaled).all()
+    for first in (0, 2 ** 20 - 500):
+        some = slice(first, first + 505)
+        x, w = a.as_strided((505, 1, k), (8, k, 1), 8 * first).double(), b.as_strided((505, n, k), (8, k, 1), 8 * first).double()
+        exact, bound = ((x @ w.mT)[:, 0], k * 2.0 ** -24 * (x.abs() @ w.abs().mT)[:, 0])
+        assert ((c[some].double() - exact).abs() <= bound + 2.0 ** -8 * exact.abs()).all()
+        expected = .5 * exact + 3. * r[some].double()
+        assert ((scaled[some].double() - expected).abs() <=
+                .5 * bound + 2.0 ** -22 * (.5 * exact.abs() + 3. * r[some].double().abs()) + 2.0 ** -8 * expected.abs()).all()
+    assert lib.tg_ex_last_device_error(None) == 0
+
+
 @pytest.mark.parametrize("m,n,k,b_mn", [
     *((m, n, k, b_mn) for k in (64, 72, 192, 320, 1544)  # shorter than the ring of half an SM, as long, round after round
       for m, n, b_mn in ((320, 320, False), (320, 320, True), (129, 72, True), (64, 64, False),  # 64 columns, four stages

@@ -26,6 +26,8 @@
 // The head GEMM has an epilogue of its own: 256-way softmax cross-entropy on the FP32 accumulators.
 #include "device_utils.cuh"
 #include "sm100.cuh"
+#include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <atomic>
@@ -134,7 +136,7 @@ template <int Warps> __device__ __forceinline__ bool epilogue_all(bool ok) {
 }
 
 // Where a work item lies: the K splits of a tile follow one another, tiles run along n first, matrices of a batch last.  In 32 bits
-// (a tile has at least 8192 outputs: 2^31 of them do not fit any memory): 64-bit divisions cost every warp some 500 instructions an item.
+// (see MostItems): 64-bit divisions cost every warp some 500 instructions an item.
 struct Item {
     int split, tile, nt, mt, z;
 };
@@ -928,6 +930,10 @@ void grow(GemmWorkspace &w, const ScratchNeed &need, cudaStream_t s) {
     }
 }
 
+// The kernel counts work items in 32 bits.  Batches of more than this many go in several launches (one of 2^20 items takes milliseconds,
+// so another costs nothing; K is whole there); a single matrix of more would not fit any memory.
+constexpr long long MostItems = 1 << 20;
+
 // Builds the kernel parameters and tensor maps for `sc` and launches.  `partials` / `tickets` may be
 // null when the schedule does not split K.
 void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *partials, unsigned *tickets,
@@ -943,7 +949,21 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
     const int unit = sc.pair ? 2 : 1;
     const int m_tiles = (g.m + BM - 1) / BM, padded_m_tiles = (m_tiles + unit - 1) / unit * unit;
     const int n_tiles = (g.n + p.bn - 1) / p.bn;
-    const long long tiles = (long long)(padded_m_tiles / unit) * n_tiles * g.batch; // scheduling units
+    const long long matrix_tiles = (long long)(padded_m_tiles / unit) * n_tiles, tiles = matrix_tiles * g.batch; // scheduling units
+    if (tiles > MostItems && g.batch > 1) {
+        const int part = int(std::max(1ll, MostItems / matrix_tiles));
+        auto at = [](const void *base, int64_t elements, Dtype t) { return base ? static_cast<const char *>(base) + elements * int64_t(dtype_size(t)) : nullptr; };
+        for (int64_t z = 0; z < g.batch; z += part) {
+            GemmArgs some = g;
+            some.batch = int(std::min<int64_t>(part, g.batch - z));
+            some.a = at(g.a, z * g.a_batch, g.in), some.b = at(g.b, z * g.b_batch, g.in), some.r = at(g.r, z * g.r_batch, g.out);
+            some.c = const_cast<char *>(at(g.c, z * g.c_batch, g.out)), some.c2 = const_cast<char *>(at(g.c2, z * g.c_batch, g.out));
+            launch_schedule(some, sc, sms, partials, tickets, counters, s);
+        }
+        return;
+    }
+    if (tiles > INT_MAX / 2)
+        throw std::runtime_error("GEMM: too many tiles");
     const int bn_local = p.bn / unit;
     const int stage_bytes = StageABytes + bn_local * BK * 2;
     const int row_scratch = g.epilogue == Epilogue::CrossEntropy ? RowScratchBytes : 0;
