@@ -44,6 +44,18 @@ def test_outputs_of_whole_blocks_have_costs_of_their_own(library, m, n, k, b_mn,
     assert schedule(library, m, n, k, b_mn)[:3] == fastest
 
 
+# Measured us: single tiles of 256 columns, and pairs; the last two keep A in L2.
+@pytest.mark.parametrize("m,n,k,b_mn,fastest", [
+    (17871, 256, 3456, False, (256, 1, 1)),   # 36.6, 30.4
+    (13865, 256, 3520, False, (256, 1, 1)),   # 29.8, 26.1
+    (52096, 1024, 3072, True, (256, 1, 1)),   # 238.1, 221.7
+    (32768, 1024, 4096, False, (256, 1, 1)),  # 201.2, 180.7
+    (18719, 256, 960, False, (256, 1, 0)),    # 13.8, 14.6
+    (18078, 256, 1024, False, (256, 1, 0))])  # 13.2, 14.1
+def test_a_product_whose_input_streams_from_memory_takes_pairs(library, m, n, k, b_mn, fastest):
+    assert schedule(library, m, n, k, b_mn)[:3] == fastest
+
+
 def test_alignment_has_no_say_in_how_often_k_is_cut(library):
     cut = 0
     for m in (16, 100, 260, 445, 1140, 5000):

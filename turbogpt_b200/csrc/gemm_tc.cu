@@ -763,13 +763,20 @@ constexpr int SingleLaunch = 3240, PairLaunch = 4100;
 // per 128-byte line of an operand and 64-deep K block (the first is hidden where a pair stages half of B).  Rows of C off a sector
 // are written in parts: nanoseconds per tile column.
 constexpr int LineCost = 140, SectorCost = 500, RaggedStoreCost = 4;
-// Where N is whole 64-column blocks, as a model's are: costs fitted to 2698 products of 512 to 40000 tokens, N and K of widths 128 to 1024, in
-// every form.  A pair's tile costs half of what it did when its warps awaited their stores before they handed an accumulator over.  The choice
-// is 1.0 % slower than the best form (a third of the products kept out of the fit); by the costs above 3.0 %.  32768 x 768 x 768 41.0 -> 34.6 us, 8192 x 3072 x 768
-// 32.2 -> 27.6, 4096 x 3072 x 768 18.0 -> 15.9.  How often K is cut stays with the costs above: it decides the order of the sums.
+// Where N is whole 64-column blocks, as a model's are: costs fitted to 2698 products of 512 to 40000 tokens and models of widths 128 to 1024
+// (K and N up to 4096, one of them at most 1024), in every form.  A pair's tile costs half of what it did when its warps awaited their stores
+// before they handed an accumulator over.  The choice is 1.0 % slower than the best form (a third of the products kept out of the fit); by the costs above
+// 3.0 %.  Over 19853 others of 256 to 65536 tokens, N and K of 128 to 4096, it is 0.5 % slower than the best form (0.5 % over K up to 1024, 0.4 up to
+// 2048, 0.7 above; at worst 38 %), by the costs above 2.4 %, and over 6916 with K off whole blocks 0.4 and 1.8.
+// 32768 x 768 x 768 41.0 -> 34.6 us, 8192 x 3072 x 768 32.2 -> 27.6, 4096 x 3072 x 768 18.0 -> 15.9.  How often K is cut stays with the costs above: it
+// decides the order of the sums.
 constexpr TileCost WholeSingleCost[] = {{256, 312, 1090}, {192, 259, 999}, {128, 199, 633}, {64, 142, 391}};
 constexpr TileCost WholePairCost[] = {{256, 305, 725}, {192, 227, 781}, {128, 179, 494}};
 constexpr int WholeSingleLaunch = 2890, WholePairLaunch = 3719;
+// They know nothing of where A comes from.  Where it does not stay in L2, its 128 rows of a stage are what a CTA waits for, and the ring of
+// a 256-column single tile holds four of them to a pair's six: from 64 MB of A on, where the costs take that tile, the pair is 1.5 % faster up
+// to 80 MB and 6.6 % above (27 products; 17871 x 256 x 3456 36.6 and 30.4 us), up to 48 MB it is 3 % slower (1273).
+constexpr int64_t StreamedBytes = int64_t(64) << 20;
 // A K split of n: partial tiles, fence, ticket and read-back by one SM, or from four on a second launch, and the partial tiles'
 // passes through memory.
 constexpr long long split_cost(int splits, int bn, long long outputs) {
@@ -810,13 +817,14 @@ Schedule product_schedule(const GemmArgs &g, int sms) {
         }
     };
     auto consider_all = [&](int splits_allowed) {
-        const bool whole = splits_allowed == 1 && g.n % 64 == 0 && g.batch == 1;
+        const bool whole = splits_allowed == 1 && g.n % 64 == 0 && g.batch == 1, streamed = whole && int64_t(g.m) * g.k * 2 > StreamedBytes;
         best = {};
         if (m_tiles >= 2 && sms >= 2)
             for (const TileCost &cost : whole ? WholePairCost : PairCost)
                 consider(cost, 2, whole ? WholePairLaunch : PairLaunch, splits_allowed);
         for (const TileCost &cost : whole ? WholeSingleCost : SingleCost)
-            consider(cost, 1, whole ? WholeSingleLaunch : SingleLaunch, splits_allowed);
+            if (!(streamed && best.bn && cost.bn == 256))
+                consider(cost, 1, whole ? WholeSingleLaunch : SingleLaunch, splits_allowed);
     };
     consider_all(0); // how often K is cut decides the order of the sums: the alignment of the rows has no say in it
     consider_all(best.splits);
