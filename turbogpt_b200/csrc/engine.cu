@@ -379,10 +379,14 @@ void Engine::flush_profile() {
     }
     timed.clear();
 }
+bool Engine::on_tensor_cores(GemmArgs g) const {
+    g.in = act;
+    return tensor_cores && gemm_tc_supported(g);
+}
 void Engine::gemm(Family f, GemmArgs g) {
     g.in = act;
     run(f, [&](cudaStream_t s) {
-        if (tensor_cores && gemm_tc_supported(g))
+        if (on_tensor_cores(g))
             launches += launch_gemm_tc(g, gemm_sms, counters, s, &lanes[lane].workspace) - 1;
         else
             launch_gemm_simt(g, s, gemm_simt_scratch_bytes(g) <= SimtScratchBytes ? simt_scratch[lane] : nullptr);
@@ -516,7 +520,7 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
             run(FActivation, [&](cudaStream_t s) { launch_swiglu(act, a.wide, a.activated, M, Hd, s); });
         } else {
             up.n = Hd, up.ldc = Hd, up.epilogue = Epilogue::GeluDual, up.c2 = a.activated;
-            if (!want_gradient) // the derivative is for the backward pass
+            if (!want_gradient && on_tensor_cores(up)) // the derivative is for the backward pass
                 up.epilogue = Epilogue::Gelu, up.c = a.activated, up.c2 = nullptr;
             gemm(FGemmForward, up);
         }

@@ -183,6 +183,7 @@ struct Engine {
     void initialize();
     void release();
     template <class F> void run(Family f, F &&launch);
+    bool on_tensor_cores(GemmArgs g) const; // whether gemm() takes it there
     void gemm(Family f, GemmArgs g);
     void forward(bool want_gradient, bool dump_logits);
     void backward();

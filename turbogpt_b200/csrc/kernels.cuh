@@ -166,7 +166,7 @@ enum class Epilogue {
     // and the loss the same way; the logits never reach memory): n = 256; R = uint8 targets [m];
     // C2 = FP32 losses [m]; C = BF16 (softmax - onehot) * alpha, or nullptr for the loss alone.
     CrossEntropy = 5,
-    Gelu = 6, // C = gelu(round(acc)): calls that keep nothing for a backward pass
+    Gelu = 6, // C = gelu(round(acc)): calls that keep nothing for a backward pass; tensor cores only, like CrossEntropy
 };
 struct GemmArgs {
     Dtype in = Dtype::BF16, out = Dtype::BF16;
