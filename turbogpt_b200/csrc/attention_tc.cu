@@ -15,7 +15,6 @@
 // of shared memory each); in grids of up to one CTA per SM a chain has two score buffers and the ring eight slots.
 #include "device_utils.cuh"
 #include "sm100.cuh"
-#include <atomic>
 
 using namespace sm100;
 
@@ -1199,24 +1198,7 @@ flash_both_kernel(const __grid_constant__ CUtensorMap map_qkv128, const __grid_c
         dkv_block<true>(map_qkv128, map_qkv64, map_do64, p, blockIdx.x - half);
 }
 
-// Error word of the calls that have no engine: a symbol, so that they allocate nothing.
-__device__ StepCounters stand_alone_counters;
-std::atomic<StepCounters *> stand_alone_address[64]; // per device, looked up by its first such call
 } // namespace
-
-StepCounters *attention_error_word(bool look_up) {
-    int device = 0;
-    CHECK_CUDA(cudaGetDevice(&device));
-    if (device >= 64)
-        return nullptr;
-    StepCounters *word = stand_alone_address[device];
-    if (!word && look_up) {
-        void *address = nullptr;
-        CHECK_CUDA(cudaGetSymbolAddress(&address, stand_alone_counters));
-        stand_alone_address[device] = word = static_cast<StepCounters *>(address);
-    }
-    return word;
-}
 
 bool flash_attention_supported(int width, int heads) {
     return heads > 0 && width == heads * HeadSize;
