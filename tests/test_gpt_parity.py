@@ -270,6 +270,23 @@ def test_lanes_change_nothing_in_fp32(optimizer):
     lanes_against_one(3, 256, 5, 300, optimizer, bridge.PRECISION_FP32)
 
 
+@pytest.mark.parametrize("batch", [16, 64, 1024])  # 64 tokens: one lane of weight gradients; 256 and 4096: two
+def test_lanes_of_the_narrowest_fp32_products_change_nothing(batch):
+    """The reference architecture, operator by operator."""
+    data = np.random.default_rng(5).integers(0, 256, 1 << 15, dtype=np.uint8)
+    results = []
+    for flags in (0, bridge.FLAG_PROFILE):
+        ex = ConfigEx.reference(Config(depth=4, context=4, batch=batch))
+        ex.precision, ex.flags = bridge.PRECISION_FP32, flags
+        with Native(ex) as engine:
+            engine.set_weights(bridge.initialize_weights(ex))
+            engine.set_data(data)
+            engine.train(4)
+            results.append((engine.training_losses(4), engine.weights()))
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("depth,own", [(4, True), (5, False)])  # depth x 1024^2 at 2^22, and above: no lanes for the families
 def test_muon_scratch_is_shared_where_its_families_take_turns(depth, own):
     """What Muon adds to an engine's memory: X twice and two square matrices, for every family or for the largest one."""
@@ -445,6 +462,13 @@ def test_batch_results_leave_early_and_are_those_of_this_call(depth, width, batc
             results.append(outputs)
     for a, b in zip(*results):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("width,batch,context", [
+    (384, 32, 148), (384, 33, 148),   # 4736 rows: norms, and their gradients, start during the kernel before them; above: they do not
+    (512, 2, 4096), (512, 1, 8193)])  # tokens x width at 2^22: two lanes are joined before a finished piece leaves; above: one
+def test_batch_results_at_the_limits_of_early_norms_and_of_two_lanes(width, batch, context):
+    test_batch_results_leave_early_and_are_those_of_this_call(3, width, batch, context, 1)
 
 
 def test_predict_runs_one_sequence_and_matches_the_batched_forward():
