@@ -577,19 +577,19 @@ flash_forward_single_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 }
 
 // ------------------------------------------------------------------------------------------
-// Backward.  Two kernels, both deterministic (no atomics):
+// Backward.  Two kernels, or for small grids their blocks in one launch, all deterministic (no atomics):
 //   dq kernel    : one CTA per 128 query rows, stepping over keys 64 at a time.  S = Q K^T and
 //                  dP = dO V^T land in tensor memory; thread = query row computes
 //                  dS = P (dP - delta) with P = exp(S / sqrt(d) - lse), packs it to BF16 over S,
 //                  and dQ += dS K accumulates in tensor memory; 1 / sqrt(d) is applied once at the end.
-//                  It also computes delta = rowsum(dO * O) and leaves it for the second kernel.
-//   dk/dv kernel : one CTA per 128 keys, stepping over queries 32 at a time with everything
+//                  It also computes delta = rowsum(dO * O) and leaves it for the second kernel (in one launch the blocks of that
+//                  one compute it themselves).
+//   dk/dv kernel : one CTA per 128 keys, stepping over queries 64 at a time with everything
 //                  transposed (S^T = K Q^T, dP^T = V dO^T: thread = key row), so P^T and dS^T are
 //                  A operands in tensor memory for dV += P^T dO and dK += dS^T Q.
-// Both are software pipelines: score buffers are double-buffered in tensor memory and the MMA thread
-// issues the score products ahead of the accumulating products, so the tensor pipe works on the
-// neighbouring steps while the compute warps turn one step's scores into dS.  256 TMEM columns and
-// under 100 KB of shared memory per CTA: two CTAs share an SM.
+// Both are software pipelines: the MMA thread issues score products ahead of the accumulating products (how far, at each kernel), so
+// the tensor pipe works on the neighbouring steps while the compute warps turn one step's scores into dS.  256 TMEM columns and
+// 98 to 105 KB of shared memory per CTA: two CTAs share an SM.
 // ------------------------------------------------------------------------------------------
 constexpr int BackwardThreads = 320, BackwardTmemColumns = 256; // warp 0 TMA, warp 1 MMA, 8 compute warps
 
@@ -598,7 +598,8 @@ struct BackwardParams {
     bf16 *dqkv;
     const float *lse;
     // [2][batch * heads][tiles * 128]: every query's -lse in base 2, then its -delta, in rows padded to whole tiles
-    // (zeros in the padding; negated because the packed FP32 instructions only add); written by the dq kernel, fetched 64 at a time by the dk/dv kernel that follows it
+    // (zeros in the padding; negated because the packed FP32 instructions only add); written by the dq kernel, fetched 64 at a time by the
+    // dk/dv kernel that follows it, unused in one launch
     float *statistics;
     int batch, context, heads, width, tiles;
     float scale, scale_log2;

@@ -116,8 +116,8 @@ bool flash_attention_supported(int width, int heads);
 void launch_flash_attention_forward(const void *qkv, void *out, float *lse, int batch, int context, int heads,
                                     StepCounters *counters, cudaStream_t s);
 
-// `scratch`: flash_attention_backward_scratch_bytes() bytes; the dq kernel fills it with every query's lse
-// (base 2) and rowsum(dout * out) for the dk/dv kernel.
+// `scratch`: flash_attention_backward_scratch_bytes() bytes.  Where two kernels run, the dq kernel fills it with every query's lse
+// (base 2) and rowsum(dout * out) for the dk/dv kernel; in one launch for both (small grids) it stays as it is.
 size_t flash_attention_backward_scratch_bytes(int batch, int context, int heads);
 // Returns the number of kernels it launched.
 int launch_flash_attention_backward(const void *qkv, const void *out, const void *dout, const float *lse,

@@ -432,7 +432,7 @@ int tg_ex_attention_backward(const void *qkv, const void *out, const void *dout,
             launch_flash_attention_backward_fused(qkv, out, dout, lse, dqkv,
                                                   attention_scratch(flash_backward_scratch_bytes(batch, context, heads)), batch,
                                                   context, heads, nullptr, s);
-        } else if (tensor_cores) { // what the engine runs: dQ by query tile, then dK and dV by key tile
+        } else if (tensor_cores) { // what the engine runs: dQ by query tile, and dK and dV by key tile
             float *scratch = static_cast<float *>(attention_scratch(flash_attention_backward_scratch_bytes(batch, context, heads)));
             launch_flash_attention_backward(qkv, out, dout, lse, scratch, dqkv, batch, context, heads, nullptr, s);
         } else {
