@@ -999,7 +999,8 @@ static void map_pages(void *p, size_t bytes) {
 
 // With gradients, the results leave while the GPU is at work: the logits during the backward pass, the gradients in pieces of two
 // megabytes or more as their layers are finished.  15 MB into ordinary memory take 0.65 ms, longer than a small model's step: 4 layers
-// d 256, 2048 tokens 1.29 -> 1.21 ms, in FP32 3.2 -> 2.4 ms, into pinned arrays 0.73 -> 0.57 ms.
+// d 256, 2048 tokens 1.29 -> 1.21 ms, in FP32 3.2 -> 2.4 ms, into pinned arrays 0.73 -> 0.57 ms
+// (0.48 since the kernels became faster; ordinary memory as before within the host's 9 %).
 void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, float *gradient_out,
                    float *per_position) {
     set_device();
