@@ -629,15 +629,16 @@ __device__ __forceinline__ uint32_t score_gradient(uint32_t p0, uint32_t p1, uin
     return pack_bf16(d0, d1);
 }
 
-// delta = rowsum(dO * O) of a warp's 32 rows, lane = row.  Eight lanes take a row, so that a load covers four whole rows (a lane to a row
-// took 32 lines to a load).  A row's 32 sums of two neighbouring products are then brought together in one lane and added in the row's
-// order: dQ and dK keep the bits of one accumulator per row.  `gradient(r, chunk)`: 16 bytes of dO's row r.
+// delta = rowsum(dO * O) of 16 rows, in lane % 16 = row.  Eight lanes take a row, so that a load covers four whole rows (a lane to a row
+// takes 32 lines to a load).  The sums of two neighbouring products that a row's eight lanes hold are then brought together in two of
+// them, one for either half of the row, and added in the row's order: dQ and dK keep the bits of one accumulator per row.
+// `gradient(r, chunk)`: 16 bytes of dO's row r.
 template <class Gradient>
-__device__ __forceinline__ float output_dot_gradient(const uint4 (&o)[8], int lane, Gradient gradient) {
+__device__ __forceinline__ float output_dot_gradient(const uint4 (&o)[4], int lane, Gradient gradient) {
     const int group = lane / 8, chunk = lane % 8;
-    float sums[8][4]; // of row 4 i + group, this lane's chunk
+    float sums[4][4]; // of row 4 i + group, this lane's chunk
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 4; ++i) {
         const uint4 g = gradient(4 * i + group, chunk);
         const unsigned a4[4] = {o[i].x, o[i].y, o[i].z, o[i].w}, b4[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
@@ -645,12 +646,12 @@ __device__ __forceinline__ float output_dot_gradient(const uint4 (&o)[8], int la
             sums[i][k] = __uint_as_float(a4[k] << 16) * __uint_as_float(b4[k] << 16) +
                          __uint_as_float(a4[k] & 0xffff0000u) * __uint_as_float(b4[k] & 0xffff0000u);
     }
-    // The eight lanes of a group exchange rows for chunks: afterwards sums[c] is chunk c of row 4 (lane % 8) + group.
+    // Four neighbouring lanes exchange rows for chunks: afterwards sums[c] is chunk c + chunk / 4 * 4 of row 4 (chunk % 4) + group.
 #pragma unroll
-    for (int bit = 4; bit > 0; bit >>= 1) {
+    for (int bit = 2; bit > 0; bit >>= 1) {
         const bool upper = chunk & bit;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
             if (i & bit)
                 continue;
 #pragma unroll
@@ -663,17 +664,21 @@ __device__ __forceinline__ float output_dot_gradient(const uint4 (&o)[8], int la
     }
     float delta = 0.f;
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
+    for (int part = 0; part < 2; ++part) { // the row's first half, then, from its sum on, the second in the lane four further
+        delta = part ? __shfl_xor_sync(0xffffffffu, delta, 4) : 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            delta += sums[c][k];
-    return __shfl_sync(0xffffffffu, delta, (lane & 3) * 8 + lane / 4);
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                delta += sums[c][k];
+    }
+    return __shfl_sync(0xffffffffu, delta, (lane & 3) * 8 + 4 + (lane / 4 & 3));
 }
-// Row 4 i + lane / 8 of the 32 rows at `rows`, 16 bytes at lane % 8, for i = 0 .. 7; zeros from row `valid` on.
-__device__ __forceinline__ void load_four_rows_at_a_time(const bf16 *rows, int64_t row_elements, int valid, int lane, uint4 (&v)[8]) {
+// Row 4 i + lane / 8 of the 16 rows at `rows`, 16 bytes at lane % 8, for i = 0 .. 3; zeros from row `valid` on.
+__device__ __forceinline__ void load_four_rows_at_a_time(const bf16 *rows, int64_t row_elements, int valid, int lane, uint4 (&v)[4]) {
     const int group = lane / 8, chunk = lane % 8;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 4; ++i) {
         v[i] = make_uint4(0, 0, 0, 0);
         if (4 * i + group < valid)
             v[i] = *reinterpret_cast<const uint4 *>(rows + (4 * i + group) * row_elements + chunk * 8);
@@ -686,7 +691,7 @@ __device__ __forceinline__ void load_four_rows_at_a_time(const bf16 *rows, int64
 // needed for the final multiply.  Twelve MMAs per 64 keys (4 S, 4 dP, 4 dQ) keep the issuing thread,
 // which pays 40-80 clocks per small MMA, off the critical path.
 constexpr int DqStep = 64, DqStepBytes = DqStep * HeadSize * 2, DqRing = 4;
-constexpr int DqShared = 2 * TileBytes + DqRing * 2 * DqStepBytes + 1024 + 256; // Q, dO + ring of (K, V)
+constexpr int DqShared = 2 * TileBytes + DqRing * 2 * DqStepBytes + 1024 + 256 + BlockM * 4; // Q, dO + ring of (K, V), delta
 
 // `Statistics`: leaves -lse and -delta for the dk/dv kernel.
 template <bool Statistics>
@@ -701,6 +706,7 @@ __device__ __forceinline__ void dq_block(const CUtensorMap &map_qkv128, const CU
                    dq_done = dp_full + 8; // 1 + 2 DqRing + 2 + 2 + 1 + 1 = 15 barriers
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 7 + 2 * DqRing);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    float *delta_rows = reinterpret_cast<float *>(barriers + 32); // of the tile's queries
     const uint32_t smem_q = base, smem_do = base + TileBytes, smem_kv = base + 2 * TileBytes;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -818,16 +824,21 @@ __device__ __forceinline__ void dq_block(const CUtensorMap &map_qkv128, const CU
         const int64_t padded = int64_t(p.tiles) * BlockM, stat = bh * padded + position;
         const float lse2 = valid ? p.lse[(int64_t(b) * p.heads + h) * p.context + position] * 1.4426950408889634f : 0.f;
         // delta: O from global memory, dO from the tile the TMA warp loaded (row r of a 128-byte-swizzled tile keeps its 16-byte
-        // chunk c at position c ^ (r % 8)).
+        // chunk c at position c ^ (r % 8)).  Each of the quarter's two warps takes 16 of its rows.
         float delta = 0.f;
         bool ok = true;
         {
-            uint4 o[8];
-            load_four_rows_at_a_time(p.out + (int64_t(row0) + warp_first) * p.width + h * HeadSize, p.width, p.context - warp_first, lane, o);
+            const int mine = quarter * 32 + half * 16; // first of the warp's 16 rows in the tile
+            uint4 o[4];
+            load_four_rows_at_a_time(p.out + (int64_t(row0) + tile * BlockM + mine) * p.width + h * HeadSize, p.width,
+                                     p.context - tile * BlockM - mine, lane, o);
             ok = mbarrier_wait(qdo_full, 0, abort_flag, p.counters, 308);
-            const uint32_t tile_rows = smem_do + quarter * 32 * 128;
             if (__all_sync(0xffffffffu, ok))
-                delta = output_dot_gradient(o, lane, [&](int r, int chunk) { return load_shared16(tile_rows + r * 128 + ((chunk ^ (r & 7)) << 4)); });
+                delta = output_dot_gradient(o, lane, [&](int r, int chunk) { return load_shared16(smem_do + (mine + r) * 128 + ((chunk ^ (r & 7)) << 4)); });
+            if (lane < 16)
+                delta_rows[mine + lane] = delta;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); // the two warps meet
+            delta = delta_rows[row];
             if (!valid)
                 delta = 0.f;
             if (Statistics && ok && half == 0) { // rows past the end of the sequence hold zeros
@@ -1074,13 +1085,22 @@ __device__ __forceinline__ void dkv_block(const CUtensorMap &map_qkv128, const C
         bool ok = true;
         if (Own) { // the eight compute warps share out the queries from the tile's first key on
             for (int first = tile * BlockN + (warp - 2) * 32; first < p.tiles * BlockM; first += 256) {
-                uint4 o[8];
-                const int64_t rows = (int64_t(row0) + first) * p.width + h * HeadSize;
-                load_four_rows_at_a_time(p.out + rows, p.width, p.context - first, lane, o);
-                float delta = output_dot_gradient(o, lane, [&](int r, int chunk) {
-                    return first + r < p.context ? *reinterpret_cast<const uint4 *>(p.dout + rows + int64_t(r) * p.width + chunk * 8)
-                                                 : make_uint4(0, 0, 0, 0);
-                });
+                uint4 o[2][4];
+                float delta = 0.f;
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+                    load_four_rows_at_a_time(p.out + (int64_t(row0) + first + part * 16) * p.width + h * HeadSize, p.width,
+                                             p.context - first - part * 16, lane, o[part]);
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                    const int first_row = first + part * 16;
+                    const float sum = output_dot_gradient(o[part], lane, [&](int r, int chunk) {
+                        return first_row + r < p.context
+                                   ? *reinterpret_cast<const uint4 *>(p.dout + (int64_t(row0) + first_row + r) * p.width + h * HeadSize + chunk * 8)
+                                   : make_uint4(0, 0, 0, 0);
+                    });
+                    delta = lane / 16 == part ? sum : delta;
+                }
                 const int position = first + lane;
                 const float lse2 = position < p.context ? p.lse[(int64_t(b) * p.heads + h) * p.context + position] * 1.4426950408889634f : 0.f;
                 if (position >= p.context)
