@@ -10,8 +10,6 @@
 #include <cstring>
 #include <dlfcn.h>
 #include <iterator>
-#include <sys/mman.h>
-#include <unistd.h>
 #include <type_traits>
 
 constexpr int64_t TwoSideLanes = int64_t(1) << 22; // tokens x columns up to which weight gradients have two lanes
@@ -280,6 +278,7 @@ void Engine::initialize() {
         if (c.flags & TG_FLAG_BF16_GRADIENT_EXCHANGE)
             allocate(gradient_bf16, P, false);
     }
+    CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&mailbox), sizeof(Mailbox), cudaHostAllocDefault));
     copies.create(layout, depth, !comm); // under data parallelism the gradients are added up over the ranks after the pass
     CHECK_CUDA(cudaStreamSynchronize(stream));
 }
@@ -321,6 +320,9 @@ void Engine::release() {
     for (cudaEvent_t ev : fork_events)
         cudaEventDestroy(ev);
     copies.destroy();
+    results.destroy();
+    if (mailbox)
+        cudaFreeHost(mailbox);
     for (auto &t : timed) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
@@ -414,12 +416,19 @@ cudaEvent_t Engine::mark(int on) {
     return event;
 }
 void Engine::await(int on, cudaEvent_t event) { CHECK_CUDA(cudaStreamWaitEvent(lanes[on].stream, event, 0)); }
-void Engine::check_device_error() {
-    StepCounters host{};
-    CHECK_CUDA(cudaMemcpyAsync(&host, counters, sizeof(host), cudaMemcpyDeviceToHost, stream));
+// Waits for the stream, and reports what its kernels recorded.  `out` (may be null) first receives `count` values: through pinned memory,
+// so that they and the error word come with one wait (as copies of their own into ordinary memory each is a wait).
+void Engine::finish(float *out, const float *values, size_t count) {
+    const bool through = count <= std::size(mailbox->values);
+    if (out)
+        CHECK_CUDA(cudaMemcpyAsync(through ? mailbox->values : out, values, count * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    CHECK_CUDA(cudaMemcpyAsync(&mailbox->counters, counters, sizeof(StepCounters), cudaMemcpyDeviceToHost, stream));
     CHECK_CUDA(cudaStreamSynchronize(stream));
-    if (host.error)
-        throw std::runtime_error("a device-side wait gave up (code " + std::to_string(host.error) +
+    if (out && through)
+        memcpy(out, mailbox->values, count * sizeof(float));
+    flush_profile();
+    if (const int code = mailbox->counters.error)
+        throw std::runtime_error("a device-side wait gave up (code " + std::to_string(code) +
                                  "); results of this launch are invalid");
 }
 
@@ -961,10 +970,7 @@ void Engine::training_losses(float *out, int count) {
             v /= config.world;
         CHECK_CUDA(cudaMemcpyAsync(loss_history, all.data(), all.size() * 4, cudaMemcpyHostToDevice, stream));
     }
-    CHECK_CUDA(cudaMemcpyAsync(out, loss_history, size_t(count) * T * sizeof(float), cudaMemcpyDeviceToHost, stream));
-    CHECK_CUDA(cudaStreamSynchronize(stream));
-    flush_profile();
-    check_device_error();
+    finish(out, loss_history, size_t(count) * T);
 }
 
 float Engine::train_mean_loss(int steps) {
@@ -977,30 +983,24 @@ float Engine::train_mean_loss(int steps) {
     return float(sum / config.base.context);
 }
 
-// Has the kernel map the pages of a result before the copy into it needs them, on the host while the GPU computes.  Contents are
-// left alone; where the call is not known, the copy takes the faults itself.  For arrays of 32 MB and more: the C library maps such
-// an array afresh each time (76 MB of gradients 15.6 -> 11.9 ms a call, 340 MB 71 -> 51), smaller ones mostly lie in memory that it
-// has kept, and where they do not, the first call, which launches its kernels one by one, has nothing left to hide the walk behind
-// (2, 15 and 24 MB: calls 1.5 % slower, 1 % slower and 5 % faster with it, first calls 13, 10 and 16 % slower).  Memory that CUDA
-// knows has its pages: the walk over them cost pinned arrays 1.0 of 8.8 ms (12 layers d 768, 4096 tokens).  Both arrays are mapped before the first copy, which in ordinary memory holds the host until it is done: with the
-// gradients' pages after the logits' copy, fresh arrays take up to 5 % longer, mapped ones up to 7 % less.
-static void map_pages(void *p, size_t bytes) {
-#ifdef MADV_POPULATE_WRITE
-    if (!p || bytes < size_t(32) << 20)
-        return;
-    cudaPointerAttributes known{};
-    CHECK_CUDA(cudaPointerGetAttributes(&known, p));
-    const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE)), begin = (reinterpret_cast<uintptr_t>(p) + page - 1) / page * page,
-                    end = (reinterpret_cast<uintptr_t>(p) + bytes) / page * page;
-    if (known.type == cudaMemoryTypeUnregistered && begin < end)
-        (void)madvise(reinterpret_cast<void *>(begin), end - begin, MADV_POPULATE_WRITE);
-#endif
+// Whether a call's results go through the ring: arrays in ordinary memory only, a megabyte of them together.  Memory that CUDA knows
+// (pinned, managed) is the copy engine's to fill, and small results are there as soon by the driver's way.
+static bool through_ring(const std::vector<ResultCopies::Segment> &arrays) {
+    size_t bytes = 0;
+    for (const ResultCopies::Segment &s : arrays) {
+        for (const char *end : {static_cast<const char *>(s.to), static_cast<const char *>(s.to) + s.bytes - 1}) {
+            cudaPointerAttributes known{};
+            CHECK_CUDA(cudaPointerGetAttributes(&known, end));
+            if (known.type != cudaMemoryTypeUnregistered)
+                return false;
+        }
+        bytes += s.bytes;
+    }
+    return bytes >= size_t(1) << 20;
 }
 
 // With gradients, the results leave while the GPU is at work: the logits during the backward pass, the gradients in pieces of two
-// megabytes or more as their layers are finished.  15 MB into ordinary memory take 0.65 ms, longer than a small model's step: 4 layers
-// d 256, 2048 tokens 1.29 -> 1.21 ms, in FP32 3.2 -> 2.4 ms, into pinned arrays 0.73 -> 0.57 ms
-// (0.48 since the kernels became faster; ordinary memory as before within the host's 9 %).
+// megabytes or more as their layers are finished.
 void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, float *gradient_out,
                    float *per_position) {
     set_device();
@@ -1008,34 +1008,43 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
     std::vector<float> losses(tokens); // here, so that it cannot throw between the first copy into the caller's arrays and the wait for it
     if (!logits_fp32)
         allocate(logits_fp32, size_t(tokens) * Vocabulary, false);
+    const size_t logit_bytes = size_t(tokens) * Vocabulary * 4, gradient_bytes = size_t(layout.count) * 4;
+    // What leaves, in this order: the logits, the layers as they are finished, last first, then what is left.
+    std::vector<ResultCopies::Segment> segments, arrays;
+    if (logits_out) {
+        segments.push_back({logits_out, logits_fp32, logit_bytes, gradient_out ? copies.stream : stream, gradient_out ? copies.forward_done : nullptr});
+        arrays.push_back(segments.back());
+    }
+    if (gradient_out) {
+        int64_t left = layout.count;
+        for (const BatchCopies::Piece &piece : copies.pieces) {
+            segments.push_back({gradient_out + piece.begin, gradient + piece.begin, size_t(left - piece.begin) * 4, copies.stream, piece.ready});
+            left = piece.begin;
+        }
+        segments.push_back({gradient_out, gradient, size_t(left) * 4, stream, nullptr});
+        arrays.push_back({gradient_out, gradient, gradient_bytes, stream, nullptr});
+    }
+    const bool large = through_ring(arrays);
     CHECK_CUDA(cudaMemcpyAsync(x, bx, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemcpyAsync(y, by, tokens, cudaMemcpyHostToDevice, stream));
     replay(gradient_out ? GraphGradients : GraphEvaluate,
            [&] { one_step(gradient_out ? RunMode::Gradients : RunMode::Evaluate); });
-    const size_t logit_bytes = size_t(tokens) * Vocabulary * 4;
-    map_pages(logits_out, logit_bytes);
-    map_pages(gradient_out, size_t(layout.count) * 4);
-    if (logits_out) {
-        if (gradient_out) // beside the backward pass
-            CHECK_CUDA(cudaStreamWaitEvent(copies.stream, copies.forward_done, 0));
-        CHECK_CUDA(cudaMemcpyAsync(logits_out, logits_fp32, logit_bytes, cudaMemcpyDeviceToHost, gradient_out ? copies.stream : stream));
-    }
-    if (gradient_out) { // the layers as they are finished, last first, then what is left
-        int64_t left = layout.count;
-        for (const BatchCopies::Piece &piece : copies.pieces) {
-            CHECK_CUDA(cudaStreamWaitEvent(copies.stream, piece.ready, 0));
-            CHECK_CUDA(cudaMemcpyAsync(gradient_out + piece.begin, gradient + piece.begin, (left - piece.begin) * 4, cudaMemcpyDeviceToHost,
-                                       copies.stream));
-            left = piece.begin;
+    if (large && results.ready()) {
+        auto small = [](const ResultCopies::Segment &s) { return s.bytes < size_t(32) << 20; }; // smaller arrays mostly lie in memory that the C library has kept
+        arrays.erase(std::remove_if(arrays.begin(), arrays.end(), small), arrays.end());
+        results.run(segments.data(), segments.size(), arrays.data(), arrays.size());
+    } else {
+        for (const ResultCopies::Segment &s : segments) {
+            if (s.ready)
+                CHECK_CUDA(cudaStreamWaitEvent(s.stream, s.ready, 0));
+            CHECK_CUDA(cudaMemcpyAsync(s.to, s.from, s.bytes, cudaMemcpyDeviceToHost, s.stream));
         }
-        CHECK_CUDA(cudaMemcpyAsync(gradient_out, gradient, left * 4, cudaMemcpyDeviceToHost, stream));
+        if (gradient_out)
+            CHECK_CUDA(cudaStreamSynchronize(copies.stream)); // a pinned array's copy returns before it is done
     }
-    CHECK_CUDA(cudaMemcpyAsync(losses.data(), token_losses, size_t(tokens) * 4, cudaMemcpyDeviceToHost, stream));
-    if (gradient_out)
-        CHECK_CUDA(cudaStreamSynchronize(copies.stream)); // a pinned array's copy returns before it is done
-    CHECK_CUDA(cudaStreamSynchronize(stream));
-    flush_profile();
-    check_device_error();
+    finish(losses.data(), token_losses, size_t(tokens));
+    if (large) // for the next call
+        results.begin(ResultCopies::threads_for(std::thread::hardware_concurrency()), config.base.device);
     if (per_position)
         for (int p = 0; p < T; ++p) { // reference cuda/runtime.cu:279-290
             double sum = 0;
@@ -1065,10 +1074,7 @@ void Engine::predict(const uint8_t *context, float *logits256) {
         throw;
     }
     forward_batch = 0;
-    CHECK_CUDA(cudaMemcpyAsync(logits256, logits_fp32 + size_t(T - 1) * Vocabulary, Vocabulary * sizeof(float),
-                               cudaMemcpyDeviceToHost, stream));
-    CHECK_CUDA(cudaStreamSynchronize(stream));
-    check_device_error();
+    finish(logits256, logits_fp32 + size_t(T - 1) * Vocabulary, Vocabulary);
 }
 
 void Engine::optimizer_test(const float *g, int steps) {
@@ -1081,8 +1087,7 @@ void Engine::optimizer_test(const float *g, int steps) {
     for (int i = 0; i < steps; ++i)
         one_step(RunMode::OptimizerOnly);
     step += steps;
-    CHECK_CUDA(cudaStreamSynchronize(stream));
-    check_device_error();
+    finish();
 }
 
 void Engine::sample(uint64_t at_step, uint8_t *bx, uint8_t *by) {

@@ -3,6 +3,7 @@
 #pragma once
 #include "batch_copies.h"
 #include "kernels.cuh"
+#include "result_copies.h"
 #include <memory>
 #include <string>
 #include <vector>
@@ -143,6 +144,11 @@ struct Engine {
     size_t next_fork_event = 0;
     float *simt_scratch[3] = {nullptr, nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
     BatchCopies copies; // of tg_batch's results
+    ResultCopies results; // into ordinary memory, from the second call on that has use for them
+    struct Mailbox { // pinned: what a call brings back with its last wait
+        StepCounters counters;
+        float values[16384];
+    } *mailbox = nullptr;
     bool announce_gradients = false;
     StepGraph graphs[GraphKinds];
     int forward_batch = 0; // sequences the next forward pass covers (0: the configured batch)
@@ -203,5 +209,5 @@ struct Engine {
     void prepare_reference_step();
     void reference_train_step(bool sample, bool save);
     void one_step(RunMode mode, bool last = true);
-    void check_device_error();
+    void finish(float *out = nullptr, const float *values = nullptr, size_t count = 0);
 };

@@ -1,0 +1,254 @@
+// How large results reach ordinary (pageable) host memory: through a ring of pinned slices that the copy engine fills and a few
+// host threads empty into the caller's arrays, both while the GPU is still computing.  The driver's own copy into such memory does
+// the two in turn on the calling thread (15 MB in 0.65 to 0.75 ms, 21 GB/s, of a call whose kernels take 0.48).  tg_batch, the driver's
+// way and this: 2 MB of results 305 and 256 us, 6 MB 620 and 385, 15 MB 1290 and 600, 31 MB 2220 and 1080, 80 MB 13.3 and 4.2 ms, 345 MB 56 and
+// 18.5 ms (from 32 MB on the C library maps an array afresh for every call, and the threads take its page faults).  The first call that would have had
+// use for it starts the threads when it is done, and one of them makes the ring: as part of that call it took 0.5 to 1 ms of two.
+#pragma once
+#include "common.h"
+#include <atomic>
+#include <condition_variable>
+#include <cstdlib>
+#include <cstring>
+#include <memory>
+#include <mutex>
+#include <sys/mman.h>
+#include <thread>
+#include <unistd.h>
+
+class ResultCopies {
+  public:
+    // A slice crosses in 10 us and a thread empties it in 50.  15 and 345 MB with 8 slices 720 us and 21.5 ms, 12 658 us and 18.5, 16 594 us and 18.4;
+    // 24 and 32 of half the size 735 us and 20.1 ms, 680 us and 19.6.
+    static constexpr size_t SliceBytes = size_t(1) << 19, Slices = 16;
+    static constexpr int MostThreads = 4;
+
+    struct Segment { // to[0, bytes) = from, device memory that is complete on `stream` after `ready` (null: after what `stream` holds)
+        void *to;
+        const void *from;
+        size_t bytes;
+        cudaStream_t stream;
+        cudaEvent_t ready;
+    };
+
+    // A quarter of the processors this process may use, or none: results then take the driver's way.
+    static int threads_for(unsigned processors) { return int(processors / 4) < MostThreads ? int(processors / 4) : MostThreads; }
+
+    ResultCopies() = default;
+    ResultCopies(const ResultCopies &) = delete;
+    ~ResultCopies() { destroy(); }
+
+    // Starts the threads, the first of which makes the ring; the caller does not wait for it.  Nothing where they are there already.
+    void begin(int thread_count, int device) {
+        if (!threads.empty() || thread_count < 1)
+            return;
+        state = Making;
+        try {
+            threads.emplace_back([this, device] {
+                state.store(make(device) ? Ready : Failed, std::memory_order_release);
+                work();
+            });
+            while (int(threads.size()) < thread_count)
+                threads.emplace_back([this] { work(); });
+        } catch (const std::exception &) { // no thread, or no memory for one: those that run will do, if any
+        }
+    }
+    // Ring, events and threads are there.  (After a failure none of them is, and begin() may try again.)
+    bool ready() {
+        if (threads.empty())
+            return false;
+        const State now = state.load(std::memory_order_acquire);
+        if (now == Failed)
+            destroy();
+        return now == Ready;
+    }
+    bool making() const { return state.load(std::memory_order_acquire) == Making; }
+    void destroy() {
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            stopping = true;
+        }
+        wake.notify_all();
+        for (std::thread &t : threads)
+            t.join();
+        threads.clear();
+        stopping = false, state = None;
+        for (cudaEvent_t &e : landed) {
+            if (e)
+                cudaEventDestroy(e);
+            e = nullptr;
+        }
+        if (pinned)
+            cudaHostUnregister(ring);
+        free(ring);
+        ring = nullptr, pinned = false;
+    }
+
+    // Copies every segment, in order; returns when the last byte is in its place.  `map`: arrays whose pages the threads have the kernel map before
+    // the first results arrive.
+    void run(const Segment *segments, size_t count, const Segment *map, size_t map_count) {
+        try {
+            copy(segments, count, map, map_count);
+        } catch (...) { // nothing may be on its way into the ring when the next call uses it
+            for (size_t i = 0; i < count; ++i)
+                (void)cudaStreamSynchronize(segments[i].stream);
+            throw;
+        }
+    }
+
+  private:
+    bool make(int device) {
+        // Huge pages, where there are any, are mapped and pinned in 1 ms; cudaHostAlloc takes 3.5 to 4.5 for eight megabytes.
+        constexpr size_t HugePage = size_t(2) << 20;
+        ring = static_cast<uint8_t *>(aligned_alloc(HugePage, RingBytes));
+        if (ring)
+            (void)madvise(ring, RingBytes, MADV_HUGEPAGE);
+        bool made = ring && cudaSetDevice(device) == cudaSuccess;
+        made = pinned = made && cudaHostRegister(ring, RingBytes, cudaHostRegisterDefault) == cudaSuccess;
+        for (size_t i = 0; made && i < Slices; ++i)
+            if (cudaEventCreateWithFlags(&landed[i], cudaEventDisableTiming) != cudaSuccess)
+                landed[i] = nullptr, made = false;
+        if (!made)
+            (void)cudaGetLastError();
+        return made;
+    }
+    void copy(const Segment *segments, size_t count, const Segment *map, size_t map_count) {
+        size_t slices = 0;
+        for (size_t i = 0; i < count; ++i)
+            slices += (segments[i].bytes + SliceBytes - 1) / SliceBytes;
+        size_t total = slices;
+        for (size_t i = 0; i < map_count; ++i)
+            total += (map[i].bytes + MapBytes - 1) / MapBytes;
+        if (total > capacity)
+            jobs.reset(new Job[total]), capacity = total;
+        next.store(0, std::memory_order_relaxed);
+        published.store(0, std::memory_order_relaxed);
+        struct Active { // the threads take jobs while this lives; all have left the array when it is gone
+            ResultCopies &c;
+            explicit Active(ResultCopies &copies) : c(copies) {
+                {
+                    std::lock_guard<std::mutex> lock(c.mutex);
+                    c.active.store(true);
+                }
+                c.wake.notify_all();
+            }
+            ~Active() {
+                {
+                    std::lock_guard<std::mutex> lock(c.mutex);
+                    c.active.store(false);
+                }
+                while (c.inside.load(std::memory_order_acquire))
+                    std::this_thread::yield();
+            }
+        } active_now(*this);
+        size_t at = 0; // jobs made
+        auto publish = [&](void *to, const void *from, size_t bytes) {
+            jobs[at].to = to, jobs[at].from = from, jobs[at].bytes = bytes;
+            jobs[at].done.store(false, std::memory_order_relaxed);
+            published.store(++at, std::memory_order_release);
+        };
+        for (size_t i = 0; i < map_count; ++i) // the end first, as gradients arrive
+            for (size_t end = map[i].bytes; end;) {
+                const size_t begin = (end - 1) / MapBytes * MapBytes;
+                publish(static_cast<char *>(map[i].to) + begin, nullptr, end - begin);
+                end = begin;
+            }
+        // `issued` slices are on their way into the ring, the first `taken` of them have been handed to the threads.
+        const size_t first_job = at;
+        size_t issued = 0, taken = 0, segment = 0, offset = 0;
+        struct {
+            void *to;
+            size_t bytes;
+        } flying[Slices];
+        while (taken < slices) {
+            while (issued < slices && issued - taken < Slices &&
+                   (issued < Slices || jobs[first_job + issued - Slices].done.load(std::memory_order_acquire))) {
+                while (offset == segments[segment].bytes)
+                    ++segment, offset = 0;
+                const Segment &s = segments[segment];
+                if (!offset && s.ready)
+                    CHECK_CUDA(cudaStreamWaitEvent(s.stream, s.ready, 0));
+                const size_t bytes = s.bytes - offset < SliceBytes ? s.bytes - offset : SliceBytes, slot = issued % Slices;
+                CHECK_CUDA(cudaMemcpyAsync(ring + slot * SliceBytes, static_cast<const char *>(s.from) + offset, bytes, cudaMemcpyDeviceToHost, s.stream));
+                CHECK_CUDA(cudaEventRecord(landed[slot], s.stream));
+                flying[slot] = {static_cast<char *>(s.to) + offset, bytes};
+                offset += bytes, ++issued;
+            }
+            if (taken == issued) { // every slice of the ring is still being emptied
+                if (!take_one())
+                    std::this_thread::yield();
+                continue;
+            }
+            const size_t slot = taken % Slices;
+            CHECK_CUDA(cudaEventSynchronize(landed[slot]));
+            publish(flying[slot].to, ring + slot * SliceBytes, flying[slot].bytes);
+            ++taken;
+        }
+        while (take_one())
+            ;
+        for (size_t i = 0; i < at; ++i)
+            while (!jobs[i].done.load(std::memory_order_acquire))
+                std::this_thread::yield();
+    }
+
+    static constexpr size_t MapBytes = size_t(4) << 20, RingBytes = SliceBytes * Slices;
+    struct Job { // a copy, or (from null) pages to be mapped
+        void *to;
+        const void *from;
+        size_t bytes;
+        std::atomic<bool> done;
+    };
+    uint8_t *ring = nullptr;
+    bool pinned = false;
+    cudaEvent_t landed[Slices] = {};
+    std::vector<std::thread> threads;
+    std::unique_ptr<Job[]> jobs;
+    size_t capacity = 0;
+    std::atomic<size_t> next{0}, published{0};
+    std::atomic<int> inside{0};
+    std::atomic<bool> active{false};
+    std::mutex mutex;
+    std::condition_variable wake;
+    bool stopping = false;
+    enum State { None, Making, Ready, Failed };
+    std::atomic<State> state{None};
+
+    bool take_one() {
+        size_t i = next.load(std::memory_order_relaxed);
+        do
+            if (i >= published.load(std::memory_order_acquire))
+                return false;
+        while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+        Job &job = jobs[i];
+        if (job.from) {
+            memcpy(job.to, job.from, job.bytes);
+        } else {
+#ifdef MADV_POPULATE_WRITE
+            const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE)), begin = (reinterpret_cast<uintptr_t>(job.to) + page - 1) / page * page,
+                            end = (reinterpret_cast<uintptr_t>(job.to) + job.bytes) / page * page;
+            if (begin < end) // where the call is not known, the copies take the faults themselves
+                (void)madvise(reinterpret_cast<void *>(begin), end - begin, MADV_POPULATE_WRITE);
+#endif
+        }
+        job.done.store(true, std::memory_order_release);
+        return true;
+    }
+    void work() {
+        std::unique_lock<std::mutex> lock(mutex);
+        for (;;) {
+            wake.wait(lock, [&] { return stopping || active.load(); });
+            if (stopping)
+                return;
+            inside.fetch_add(1);
+            lock.unlock();
+            for (int idle = 0; active.load(std::memory_order_acquire);) {
+                if (take_one())
+                    idle = 0;
+                else if (++idle > 64)
+                    std::this_thread::yield();
+            }
+            inside.fetch_sub(1, std::memory_order_release);
+            lock.lock();
+        }
+    }
+};
