@@ -428,6 +428,13 @@ def test_norms_at_widths_off_the_register_tile(rows, width, kind):
     test_norms_match_torch(rows, width, kind)
 
 
+@pytest.mark.parametrize("rows,width", [(5000, 768), (4801, 776), (5000, 1016), (7103, 1024)])  # up to 768 columns a row's values stay in registers
+@pytest.mark.parametrize("kind", [0, 1])
+def test_norms_of_several_rows_a_warp(rows, width, kind):
+    """More rows than the backward kernel has warps, on both sides of its forms: same checks, same bounds."""
+    test_norms_match_torch(rows, width, kind)
+
+
 @pytest.mark.parametrize("d_head", [64, 32])  # tiles of 64 x 64 positions; a warp per row
 @pytest.mark.parametrize("at", [40, 90])      # in the first tile, in the last
 def test_cuda_core_attention_keeps_a_later_infinity_out(d_head, at):

@@ -247,17 +247,47 @@ __device__ __forceinline__ void fetch8(const bf16 *p, Packet<bf16> &r) { r.u = *
 __device__ __forceinline__ void fetch8(const float *p, Packet<float> &r) {
     r.a = *reinterpret_cast<const float4 *>(p), r.b = *reinterpret_cast<const float4 *>(p + 4);
 }
-__device__ __forceinline__ void unpack8(const Packet<bf16> &r, float (&v)[8]) {
-    const unsigned w[4] = {r.u.x, r.u.y, r.u.z, r.u.w};
+// Their FP32 values in pairs, for the packed instructions: these kernels issue for more than half of their time, one value at a time.
+__device__ __forceinline__ uint64_t pair_of(unsigned packed) { return sm100::float_pair(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u)); }
+__device__ __forceinline__ uint64_t both(float v) { return sm100::float_pair(v, v); }
+__device__ __forceinline__ unsigned packed_of(uint64_t pair) {
+    float lo, hi;
+    sm100::split_pair(pair, lo, hi);
+    return pack_bf16(lo, hi);
+}
+__device__ __forceinline__ void unpack8(const Packet<bf16> &r, uint64_t (&v)[4]) {
+    v[0] = pair_of(r.u.x), v[1] = pair_of(r.u.y), v[2] = pair_of(r.u.z), v[3] = pair_of(r.u.w);
+}
+__device__ __forceinline__ void unpack8(const Packet<float> &r, uint64_t (&v)[4]) {
+    v[0] = sm100::float_pair(r.a.x, r.a.y), v[1] = sm100::float_pair(r.a.z, r.a.w);
+    v[2] = sm100::float_pair(r.b.x, r.b.y), v[3] = sm100::float_pair(r.b.z, r.b.w);
+}
+__device__ __forceinline__ void store8(bf16 *p, const uint64_t (&v)[4]) {
+    *reinterpret_cast<uint4 *>(p) = make_uint4(packed_of(v[0]), packed_of(v[1]), packed_of(v[2]), packed_of(v[3]));
+}
+__device__ __forceinline__ void store8(float *p, const uint64_t (&v)[4]) {
+    float f[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        v[2 * i] = __uint_as_float(w[i] << 16);
-        v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
+    for (int j = 0; j < 4; ++j)
+        sm100::split_pair(v[j], f[2 * j], f[2 * j + 1]);
+    store8(p, f);
 }
-__device__ __forceinline__ void unpack8(const Packet<float> &r, float (&v)[8]) {
-    v[0] = r.a.x, v[1] = r.a.y, v[2] = r.a.z, v[3] = r.a.w, v[4] = r.b.x, v[5] = r.b.y, v[6] = r.b.z, v[7] = r.b.w;
+// A product that is rounded before anything is added to it: a packed one followed by a packed sum becomes one operation.
+__device__ __forceinline__ uint64_t product(uint64_t a, uint64_t b) {
+    float a0, a1, b0, b1;
+    sm100::split_pair(a, a0, a1);
+    sm100::split_pair(b, b0, b1);
+    return sm100::float_pair(__fmul_rn(a0, b0), __fmul_rn(a1, b1));
 }
+template <class T> __device__ __forceinline__ uint64_t rounded_pair(uint64_t v) {
+    if constexpr (sizeof(T) == 2)
+        return pair_of(packed_of(v));
+    else
+        return v;
+}
+// Makes the compiler take the packet for another: what is computed from it again is computed again, not kept in registers.
+__device__ __forceinline__ void renew(Packet<bf16> &r) { asm volatile("" : "+r"(r.u.x), "+r"(r.u.y), "+r"(r.u.z), "+r"(r.u.w)); }
+__device__ __forceinline__ void renew(Packet<float> &) {}
 
 // Widths up to 1024: the row lives in registers (one 128-bit load per 256 columns and lane), so x is read once; scale
 // and bias are read once per block into shared memory.  Ragged (a width that is no multiple of 256): some lanes have no
@@ -271,14 +301,14 @@ __device__ __forceinline__ int plane_of_column(int c) { // column -> index in th
     const int v = c / 256, lane = c % 256 / 8, half = c % 8 / 4, j = c % 4;
     return plane_index(v, half, lane) + j;
 }
-__device__ __forceinline__ void load_planes(const float *base, int v, int lane, float (&w)[8]) {
-    const float4 a = *reinterpret_cast<const float4 *>(base + plane_index(v, 0, lane));
-    const float4 b = *reinterpret_cast<const float4 *>(base + plane_index(v, 1, lane));
-    w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+__device__ __forceinline__ void load_planes(const float *base, int v, int lane, uint64_t (&w)[4]) {
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(base + plane_index(v, 0, lane));
+    const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(base + plane_index(v, 1, lane));
+    w[0] = a.x, w[1] = a.y, w[2] = b.x, w[3] = b.y;
 }
-__device__ __forceinline__ void store_planes(float *base, int v, int lane, const float (&w)[8]) {
-    *reinterpret_cast<float4 *>(base + plane_index(v, 0, lane)) = make_float4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<float4 *>(base + plane_index(v, 1, lane)) = make_float4(w[4], w[5], w[6], w[7]);
+__device__ __forceinline__ void store_planes(float *base, int v, int lane, const uint64_t (&w)[4]) {
+    *reinterpret_cast<ulonglong2 *>(base + plane_index(v, 0, lane)) = make_ulonglong2(w[0], w[1]);
+    *reinterpret_cast<ulonglong2 *>(base + plane_index(v, 1, lane)) = make_ulonglong2(w[2], w[3]);
 }
 // Two sums over the warp at once: the shuffles of the two values interleave, so the pair costs the
 // latency of one reduction.
@@ -295,43 +325,55 @@ __device__ __forceinline__ void warp_sum2(float &a, float &b) {
 // share one warp reduction: the row's dependent chain is one shuffle plus one reduction.
 // `tail`: the lane has columns in the last 256 (it holds zeros there otherwise).
 template <class T, int V, bool Ragged>
-__device__ __forceinline__ void row_moments(int kind, const float (&x)[V][8], int width, bool tail, float &mean, float &inv) {
-    float sums[4] = {0, 0, 0, 0}, squares[4] = {0, 0, 0, 0};
+__device__ __forceinline__ void row_moments(int kind, const uint64_t (&x)[V][4], int width, bool tail, float &mean, float &inv) {
+    uint64_t sums[2] = {0, 0}, squares[2] = {0, 0}; // of the columns 0 and 1, 2 and 3 of every four
+    auto total = [](const uint64_t (&v)[2]) {
+        float f[4];
+        sm100::split_pair(v[0], f[0], f[1]);
+        sm100::split_pair(v[1], f[2], f[3]);
+        return (f[0] + f[1]) + (f[2] + f[3]);
+    };
     if (kind == TG_NORM_RMS) {
 #pragma unroll
         for (int v = 0; v < V; ++v)
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                squares[j % 4] += x[v][j] * x[v][j];
+            for (int j = 0; j < 4; ++j)
+                squares[j % 2] = sm100::fma_pair(x[v][j], x[v][j], squares[j % 2]);
         mean = 0;
-        inv = rsqrtf(warp_sum((squares[0] + squares[1]) + (squares[2] + squares[3])) / width + 1e-6f);
+        inv = rsqrtf(warp_sum(total(squares)) / width + 1e-6f);
         return;
     }
     if constexpr (sizeof(T) == 4 || Ragged) {
 #pragma unroll
         for (int v = 0; v < V; ++v)
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                sums[j % 4] += x[v][j];
-        mean = warp_sum((sums[0] + sums[1]) + (sums[2] + sums[3])) / width;
+            for (int j = 0; j < 4; ++j)
+                sums[j % 2] = sm100::add_pair(sums[j % 2], x[v][j]);
+        mean = warp_sum(total(sums)) / width;
+        const uint64_t shift = both(-mean);
 #pragma unroll
         for (int v = 0; v < V; ++v)
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (!Ragged || v + 1 < V || tail)
-                    squares[j % 4] += (x[v][j] - mean) * (x[v][j] - mean);
-        inv = rsqrtf(warp_sum((squares[0] + squares[1]) + (squares[2] + squares[3])) / width + 1e-5f);
+            for (int j = 0; j < 4; ++j)
+                if (!Ragged || v + 1 < V || tail) {
+                    const uint64_t d = sm100::add_pair(x[v][j], shift);
+                    squares[j % 2] = sm100::fma_pair(d, d, squares[j % 2]);
+                }
+        inv = rsqrtf(warp_sum(total(squares)) / width + 1e-5f);
     } else {
-        const float shift = __shfl_sync(0xffffffffu, x[0][0], 0);
+        float first, second;
+        sm100::split_pair(x[0][0], first, second);
+        const float shift = __shfl_sync(0xffffffffu, first, 0);
+        const uint64_t back = both(-shift);
 #pragma unroll
         for (int v = 0; v < V; ++v)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float d = x[v][j] - shift;
-                sums[j % 4] += d;
-                squares[j % 4] += d * d;
+            for (int j = 0; j < 4; ++j) {
+                const uint64_t d = sm100::add_pair(x[v][j], back);
+                sums[j % 2] = sm100::add_pair(sums[j % 2], d);
+                squares[j % 2] = sm100::fma_pair(d, d, squares[j % 2]);
             }
-        float s1 = (sums[0] + sums[1]) + (sums[2] + sums[3]), s2 = (squares[0] + squares[1]) + (squares[2] + squares[3]);
+        float s1 = total(sums), s2 = total(squares);
         warp_sum2(s1, s2);
         const float offset = s1 / width;
         mean = shift + offset;
@@ -370,7 +412,7 @@ template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 4)
     __syncthreads();
     for (; row < a.rows; row += stride) {
         T *y = (T *)a.y + int64_t(row) * a.width;
-        float v[V][8];
+        uint64_t v[V][4];
 #pragma unroll
         for (int k = 0; k < V; ++k)
             unpack8(next[k], v[k]);
@@ -380,14 +422,21 @@ template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 4)
         row_moments<T, V, Ragged>(a.kind, v, a.width, tail, mean, inv);
         if (a.stats && lane == 0) // kept for the backward pass; a caller's array is aligned to its floats only
             a.stats[2 * int64_t(row)] = mean, a.stats[2 * int64_t(row) + 1] = inv;
+        const uint64_t shift = both(-mean), scaled = both(inv);
 #pragma unroll
         for (int k = 0; k < V; ++k) {
-            float out[8], w[8], b[8];
+            uint64_t out[4], w[4], b[4];
             load_planes(sw, k, lane, w);
-            load_planes(sb, k, lane, b);
+            if (a.kind == TG_NORM_RMS) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                out[j] = a.kind == TG_NORM_RMS ? v[k][j] * inv * w[j] : (v[k][j] - mean) * inv * w[j] + b[j];
+                for (int j = 0; j < 4; ++j)
+                    out[j] = sm100::mul_pair(sm100::mul_pair(v[k][j], scaled), w[j]);
+            } else {
+                load_planes(sb, k, lane, b);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    out[j] = sm100::fma_pair(sm100::mul_pair(sm100::add_pair(v[k][j], shift), scaled), w[j], b[j]);
+            }
             if (k + 1 < V || tail)
                 store8(y + (k * 32 + lane) * 8, out);
         }
@@ -513,7 +562,7 @@ __global__ void __launch_bounds__(256) norm_backward_reduce_kernel(const float *
     }
 }
 // Register-resident variant for widths up to 1024: x, dy and the residual gradient are read once, and
-// a warp fetches its next row while it works on the current one.  The row's mean and 1/sigma come
+// a warp fetches its next row while it works on the current one (the kernel issues for 57 % of its time at 768 columns: values go in pairs).  The row's mean and 1/sigma come
 // from the forward pass when it saved them (`stats`), so the only reduction a row waits for is the
 // pair sum(dz), sum(dz z).  Each warp keeps the scale/bias gradient sums of its rows in its own slice
 // of shared memory (plane layout: a lane owns its words, no conflicts, no atomics); warps are summed
@@ -526,9 +575,16 @@ template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 2)
     const bool residual = a.residual_in != nullptr, saved = a.stats != nullptr;
     const int stride = gridDim.x * warps;
     const bool tail = !Ragged || ((V - 1) * 32 + lane) * 8 < a.width;
-    Packet<T> nx[V], ng[V], nr[V];
+    // A row of more than 768 columns, its residual and the next row are more than 128 registers hold (they spilled 200 bytes, whose
+    // traffic the streamed rows pushed out of L1): the residual is fetched with its own row, and what the second half needs is computed again
+    // from the row as it came.  32768 x 1024 with the sums' kernel 100 -> 78 us, 8192 x 1024 55 -> 48, 32768 x 896 98 -> 78; narrower rows are
+    // level to 3 % slower that way (32768 x 640 62.8 and 64.7).
+    constexpr bool Lean = sizeof(T) == 2 && V > 3;
+    Packet<T> nx[V], ng[V], nr[Lean ? 1 : V];
     if (Ragged)
-        nx[V - 1] = ng[V - 1] = nr[V - 1] = Packet<T>{}; // stay zero in the lanes without a tail
+        nx[V - 1] = ng[V - 1] = Packet<T>{}; // stay zero in the lanes without a tail
+    if (Ragged && !Lean)
+        nr[V - 1] = Packet<T>{};
     float2 nstat = make_float2(0.f, 1.f);
     auto fetch = [&](int row) {
         const int64_t offset = int64_t(row) * a.width;
@@ -540,7 +596,7 @@ template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 2)
                 continue;
             fetch8((const T *)a.x + offset + (v * 32 + lane) * 8, nx[v]);
             fetch8((const T *)a.dy + offset + (v * 32 + lane) * 8, ng[v]);
-            if (residual)
+            if (!Lean && residual)
                 fetch8((const T *)a.residual_in + offset + (v * 32 + lane) * 8, nr[v]);
         }
     };
@@ -559,56 +615,85 @@ template <class T, int V, bool Ragged> __global__ void __launch_bounds__(256, 2)
     __syncthreads();
     for (; row < a.rows; row += stride) {
         const int64_t offset = int64_t(row) * a.width;
-        float x[V][8], g[V][8];
-        Packet<T> r[V];
+        Packet<T> px[V], pg[V], r[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            unpack8(nx[v], x[v]);
-            unpack8(ng[v], g[v]);
-            r[v] = nr[v];
+            px[v] = nx[v], pg[v] = ng[v];
+            if (!Lean)
+                r[v] = nr[v];
+            else if (residual && (v + 1 < V || tail))
+                fetch8((const T *)a.residual_in + offset + (v * 32 + lane) * 8, r[v]);
         }
         float mean = nstat.x, inv = nstat.y;
         if (row + stride < a.rows)
             fetch(row + stride); // in flight during this row's arithmetic
-        if (!saved)
+        if (!saved) {
+            uint64_t x[V][4];
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                unpack8(px[v], x[v]);
             row_moments<T, V, Ragged>(a.kind, x, a.width, tail, mean, inv);
-        float part_dz[4] = {0, 0, 0, 0}, part_dzz[4] = {0, 0, 0, 0};
+        }
+        const uint64_t shift = both(-mean), scaled = both(inv);
+        uint64_t zs[Lean ? 1 : V][4], dzs[Lean ? 1 : V][4]; // the normalised values and dy * scale
+        uint64_t part_dz[2] = {0, 0}, part_dzz[2] = {0, 0};
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            float w[8], dw[8], db[8];
+            uint64_t x[4], g[4], w[4], dw[4], db[4];
+            unpack8(px[v], x);
+            unpack8(pg[v], g);
             load_planes(scale, v, lane, w);
             load_planes(mine, v, lane, dw);
             load_planes(mine + V * 256, v, lane, db);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float z = (x[v][j] - mean) * inv, dz = g[v][j] * w[j];
-                x[v][j] = z; // keep the normalised value
-                part_dz[j % 4] += dz;
-                part_dzz[j % 4] += dz * z;
-                dw[j] += g[v][j] * z;
-                db[j] += g[v][j];
-                g[v][j] = dz; // keep dy * scale
+            for (int j = 0; j < 4; ++j) {
+                const uint64_t z = sm100::mul_pair(sm100::add_pair(x[j], shift), scaled), dz = product(g[j], w[j]);
+                part_dz[j % 2] = sm100::add_pair(part_dz[j % 2], dz);
+                part_dzz[j % 2] = sm100::fma_pair(dz, z, part_dzz[j % 2]);
+                dw[j] = sm100::fma_pair(g[j], z, dw[j]);
+                db[j] = sm100::add_pair(db[j], g[j]);
+                if (!Lean)
+                    zs[v][j] = z, dzs[v][j] = dz;
             }
             store_planes(mine, v, lane, dw);
             store_planes(mine + V * 256, v, lane, db);
         }
-        float sum_dzz = (part_dzz[0] + part_dzz[1]) + (part_dzz[2] + part_dzz[3]);
-        float sum_dz = (part_dz[0] + part_dz[1]) + (part_dz[2] + part_dz[3]);
+        float parts[4], sum_dzz, sum_dz;
+        sm100::split_pair(part_dzz[0], parts[0], parts[1]);
+        sm100::split_pair(part_dzz[1], parts[2], parts[3]);
+        sum_dzz = (parts[0] + parts[1]) + (parts[2] + parts[3]);
+        sm100::split_pair(part_dz[0], parts[0], parts[1]);
+        sm100::split_pair(part_dz[1], parts[2], parts[3]);
+        sum_dz = (parts[0] + parts[1]) + (parts[2] + parts[3]);
         warp_sum2(sum_dzz, sum_dz);
         sum_dzz /= a.width;
         sum_dz = a.kind == TG_NORM_LAYER ? sum_dz / a.width : 0.f;
+        const uint64_t less_dzz = both(-sum_dzz), less_dz = both(-sum_dz);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            float out[8];
+            uint64_t out[4];
+            if constexpr (Lean) {
+                uint64_t x[4], g[4], w[4];
+                renew(px[v]), renew(pg[v]);
+                unpack8(px[v], x);
+                unpack8(pg[v], g);
+                load_planes(scale, v, lane, w);
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                out[j] = (g[v][j] - sum_dz - x[v][j] * sum_dzz) * inv;
+                for (int j = 0; j < 4; ++j) {
+                    const uint64_t z = sm100::mul_pair(sm100::add_pair(x[j], shift), scaled), dz = product(g[j], w[j]);
+                    out[j] = sm100::mul_pair(sm100::fma_pair(z, less_dzz, sm100::add_pair(dz, less_dz)), scaled);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    out[j] = sm100::mul_pair(sm100::fma_pair(zs[v][j], less_dzz, sm100::add_pair(dzs[v][j], less_dz)), scaled);
+            }
             if (residual) {
-                float res[8];
+                uint64_t res[4];
                 unpack8(r[v], res);
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    out[j] = res[j] + rounded<T>(out[j]);
+                for (int j = 0; j < 4; ++j)
+                    out[j] = sm100::add_pair(res[j], rounded_pair<T>(out[j]));
             }
             if (v + 1 < V || tail)
                 store8((T *)a.dx + offset + (v * 32 + lane) * 8, out);
