@@ -379,6 +379,43 @@ def test_muon_on_the_tensor_core_path():
         assert relative(actual - w, opt.w - w) < .04  # verify.py:101's bound for the Muon part
 
 
+@pytest.mark.parametrize("depth,width,hidden,ns_steps", [
+    (2, 64, 72, 5),      # one tile a matrix, a last K block of eight
+    (3, 192, 200, 4),    # tiles of 64 columns, partly and wholly past the edge; the result in the first of the two buffers
+    (12, 128, 520, 5), (2, 448, 1000, 5), (3, 320, 264, 3),  # 64 and 128 columns; rows off 32 bytes; hidden < width
+    (6, 384, 1536, 2),   # 128 columns for A and B, 256 for X'
+    (2, 1032, 1544, 1)]) # 256 columns throughout, a last tile of eight rows
+def test_newton_schulz_of_all_families_in_one_launch(depth, width, hidden, ns_steps):
+    """Tiles, mirrored operands and waits at their edges: every hidden matrix against the CPU oracle (verify.py:101's bound; a wrong tile is an error
+    of order one), and the same bits family by family (one lane: other tile widths, other orders of tiles) and on a second run."""
+    heads = width // 8
+    arch = Arch.gpt(depth, width, heads, hidden)
+    w = Model(arch, seed=3).flat()
+    ex = ConfigEx.gpt(Config(depth=depth, context=16, batch=4, clip=1.0, ns_steps=ns_steps), width, heads, hidden, hidden_optimizer=bridge.HIDDEN_MUON)
+    rng = np.random.default_rng(depth)
+    results = []
+    for flags in (0, 0, bridge.FLAG_PROFILE):
+        ex.flags = flags
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            if not results:
+                gradients = (rng.standard_normal((2, engine.count)) * .01).astype(np.float32)
+            results.append([])
+            for gradient in gradients:
+                engine.optimizer_test(gradient, 1)
+                results[-1].append(engine.weights())
+    np.testing.assert_array_equal(results[0], results[1])
+    np.testing.assert_array_equal(results[0], results[2])
+    opt = Optimizer(arch, Hyper(clip=1.0, ns_steps=ns_steps), w, hidden="muon")
+    opt.step(gradients[0])
+    offset = 0
+    for name, shape in specification(arch):
+        part = slice(offset, offset + int(np.prod(shape)))
+        offset = part.stop
+        if len(shape) == 2 and name != "embedding":
+            assert relative(results[0][0][part] - w[part], opt.w[part] - w[part]) < .04, name
+
+
 def _structured_bytes(size, seed):
     """Learnable bytes: an order-1 Markov chain with sparse (Dirichlet 0.05) transition rows."""
     rng = np.random.default_rng(seed)

@@ -240,12 +240,17 @@ void Engine::initialize() {
         float *sumsq = nullptr;
         allocate(scratch, muon_lanes ? total : 2 * (matrix + square), false);
         allocate(sumsq, (muon_lanes ? muon.size() : 1) * depth * MuonBlocks);
+        unsigned *progress = nullptr;
+        allocate(progress, muon.size() * depth);
+        muon_persistent = tensor_cores && c.world == 1;
         for (MuonFamily &f : muon) {
             if (muon_lanes)
                 matrix = padded(size_t(f.rows) * f.cols), square = padded(side(f) * side(f));
             f.x[0] = scratch, f.x[1] = f.x[0] + matrix, f.a = f.x[1] + matrix, f.b = f.a + square, f.sumsq = sumsq;
             if (muon_lanes)
                 scratch = f.b + square, sumsq += depth * MuonBlocks;
+            f.progress = progress, progress += depth;
+            muon_persistent &= newton_schulz_supported(f.rows, f.cols, f.x[0]);
         }
     }
     if (tensor_cores && !profile && c.world == 1 && reference_step_supported(c))
@@ -732,7 +737,8 @@ void Engine::backward() {
 }
 
 // ------------------------------------------------------------------------------- optimizer ---
-void Engine::muon_family(const MuonFamily &family) {
+// Momentum, the normalised direction and, with `iterate`, its Newton-Schulz iterations; returns where every layer's result is.
+bf16 *Engine::muon_direction(const MuonFamily &family, bool iterate) {
     const TgConfigEx &c = config;
     const int depth = c.base.depth, rows = family.rows, cols = family.cols;
     const int64_t first_offset = family.first, stride = depth > 1 ? layout.layers[1].qkv - layout.layers[0].qkv : 0;
@@ -746,9 +752,11 @@ void Engine::muon_family(const MuonFamily &family) {
     const bool sharded = comm && depth % c.world == 0 && depth >= c.world;
     const int mine = sharded ? depth / c.world : depth, first = sharded ? c.rank * mine : 0;
     MuonPrepareArgs prep{gradient + first_offset, momentum + first_offset, family.x[0], family.sumsq, sumsq_partial,
-                         sumsq_blocks, schedule, counters, c.base.momentum, c.base.clip, rows, cols, depth, stride};
+                         sumsq_blocks, schedule, counters, c.base.momentum, c.base.clip, rows, cols, depth, stride, family.progress};
     run(FMuon, [&](cudaStream_t s) { launch_muon_prepare(prep, s); });
     run(FMuon, [&](cudaStream_t s) { launch_muon_normalize(family.x[0], family.sumsq, per, depth, sms, s); });
+    if (!iterate)
+        return family.x[c.base.ns_steps % 2];
     bf16 *cur = family.x[0] + first * per, *nxt = family.x[1] + first * per;
     bf16 *a_buffer = family.a + int64_t(first) * r * r, *b_buffer = family.b + int64_t(first) * r * r;
     const bool small = muon_newton_schulz_small_supported(r, n); // the reference architecture: one launch, in place
@@ -771,7 +779,7 @@ void Engine::muon_family(const MuonFamily &family) {
         x2.out = Dtype::BF16;
         for (GemmArgs *g : {&a, &b, &x2}) {
             run(FMuon, [&](cudaStream_t s) {
-                g->in = Dtype::BF16, g->beside_others = muon_lanes;
+                g->in = Dtype::BF16;
                 if (tensor_cores && gemm_tc_supported(*g))
                     launches += launch_gemm_tc(*g, sms, counters, s, &lanes[lane].workspace) - 1;
                 else
@@ -787,6 +795,20 @@ void Engine::muon_family(const MuonFamily &family) {
             nccl.check(nccl.AllGather(cur, all, size_t(mine) * per, Nccl::Bfloat16, comm, s), "ncclAllGather");
         });
     }
+    return all;
+}
+void Engine::muon_iterations(const MuonFamily *families, int count) {
+    NewtonSchulzArgs a;
+    for (int i = 0; i < count; ++i)
+        a.family[i] = {{families[i].x[0], families[i].x[1]}, families[i].a, families[i].b, families[i].rows, families[i].cols};
+    a.count = count, a.batch = config.base.depth, a.steps = config.base.ns_steps, a.progress = families[0].progress, a.counters = counters;
+    if (a.steps > 0)
+        run(FMuon, [&](cudaStream_t s) { launch_newton_schulz(a, sms, s); });
+}
+void Engine::muon_apply(const MuonFamily &family, bf16 *all) {
+    const TgConfigEx &c = config;
+    const int depth = c.base.depth, rows = family.rows, cols = family.cols;
+    const int64_t first_offset = family.first, stride = depth > 1 ? layout.layers[1].qkv - layout.layers[0].qkv : 0;
     MuonApplyArgs apply{all, weight_high + first_offset, weight_low + first_offset,
                         weight_fp32 ? weight_fp32 + first_offset : nullptr, schedule, counters, c.base.muon_lr,
                         c.base.weight_decay, rows, cols, depth, stride};
@@ -802,16 +824,36 @@ void Engine::optimize() {
     next_fork_event = 0; // backward has joined its lanes
     const cudaEvent_t norm_ready = muon_lanes && !muon.empty() ? mark(0) : nullptr;
     run(FOptimizer, [&](cudaStream_t s) { launch_adamw(a, sms, s); });
-    // The families are independent chains of small products: each on a lane of its own.
+    // The families are independent of one another: each on a lane of its own, but for the iterations in one launch.
     const int chains = muon_lanes ? std::min(int(muon.size()), LaneCount - 1) : 0;
+    const bool together = chains && muon_persistent;
+    auto join = [&] {
+        for (int l = 1; l <= chains; ++l)
+            fork(l, 0);
+    };
+    std::vector<bf16 *> directions(muon.size());
     for (int l = 1; l <= chains; ++l)
         await(l, norm_ready);
     for (size_t f = 0; f < muon.size(); ++f) {
         OnLane on(*this, chains ? 1 + int(f) % chains : 0);
-        muon_family(muon[f]);
+        directions[f] = muon_direction(muon[f], !muon_persistent);
+        if (together)
+            continue;
+        if (muon_persistent)
+            muon_iterations(&muon[f], 1);
+        muon_apply(muon[f], directions[f]);
     }
-    for (int l = 1; l <= chains; ++l)
-        fork(l, 0); // join
+    join();
+    if (together) {
+        muon_iterations(muon.data(), int(muon.size()));
+        for (int l = 1; l <= chains; ++l)
+            fork(0, l);
+        for (size_t f = 0; f < muon.size(); ++f) {
+            OnLane on(*this, 1 + int(f) % chains);
+            muon_apply(muon[f], directions[f]);
+        }
+        join();
+    }
     run(FMisc, [&](cudaStream_t s) { launch_advance(counters, s); });
 }
 

@@ -106,8 +106,10 @@ struct Engine {
         int rows = 0, cols = 0;
         bf16 *x[2] = {nullptr, nullptr}, *a = nullptr, *b = nullptr;
         float *sumsq = nullptr;
+        unsigned *progress = nullptr;
     };
     std::vector<MuonFamily> muon;
+    bool muon_persistent = false; // the iterations in one launch for all families, or, where they share scratch, for each
     // the reference architecture's step in three kernels (reference_step.cu, small_optimizer_kernel); unset: operator by operator
     bool reference_step = false;
     ReferenceStepPlan reference_plan;
@@ -196,7 +198,9 @@ struct Engine {
     void exchange_bucket(int64_t begin, int64_t end, int index);
     void finish_exchange();
     void optimize();
-    void muon_family(const MuonFamily &family);
+    bf16 *muon_direction(const MuonFamily &family, bool iterate);
+    void muon_iterations(const MuonFamily *families, int count);
+    void muon_apply(const MuonFamily &family, bf16 *direction);
     bool use_graphs() const { return !profile && !comm && !(config.flags & TG_FLAG_NO_GRAPH); }
     template <class F> void replay(GraphKind kind, F &&body);
     void announce(cudaEvent_t event, int on);

@@ -283,12 +283,26 @@ struct MuonPrepareArgs { // momentum, Nesterov direction, BF16 cast (+ transpose
     float momentum_rate, clip;
     int rows, cols, batch;
     int64_t stride;      // elements between consecutive matrices of the batch in the flat arrays
+    unsigned *progress = nullptr; // [batch], set to zero for launch_newton_schulz
 };
 void launch_muon_prepare(const MuonPrepareArgs &a, cudaStream_t s);
 void launch_muon_normalize(bf16 *x, const float *sumsq, int64_t per_matrix, int batch, int sms, cudaStream_t s);
 // `matrices` consecutive [r, n] BF16 matrices (r <= n), orthogonalised in place by `steps` Newton-Schulz iterations.
 bool muon_newton_schulz_small_supported(int r, int n);
 void launch_muon_newton_schulz_small(bf16 *x, int r, int n, int steps, int matrices, cudaStream_t s);
+// The iterations of up to five families of `batch` matrices each, between which nothing but X (in x[0], and after an odd number of steps in
+// x[1]) and the two squares is kept.
+struct NewtonSchulzArgs {
+    struct Family {
+        bf16 *x[2], *a, *b; // [batch][r][n] with r = min(rows, cols), n the other; [batch][r][r]
+        int rows, cols;
+    } family[5];
+    int count = 0, batch = 0, steps = 0;
+    unsigned *progress = nullptr; // [count][batch], zero
+    StepCounters *counters = nullptr;
+};
+bool newton_schulz_supported(int rows, int cols, const void *x);
+void launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s);
 struct MuonApplyArgs {
     const bf16 *x;
     bf16 *weight_high;

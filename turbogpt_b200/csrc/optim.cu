@@ -140,6 +140,12 @@ void launch_adamw(const AdamArgs &a, int sms, cudaStream_t s) {
 
 // ---- Muon (reference cuda/optim.cuh:16-65) ----
 
+__device__ __forceinline__ void finish_block(const MuonPrepareArgs &a, int matrix, float squares) { // one thread
+    a.sumsq[matrix * MuonBlocks + blockIdx.x] = squares;
+    if (a.progress && blockIdx.x == 0)
+        a.progress[matrix] = 0;
+}
+
 __global__ void __launch_bounds__(256) muon_prepare_kernel(MuonPrepareArgs a) {
     __shared__ float scratch[32];
     const float clip = clip_factor(a.norm_partial, a.norm_blocks, a.clip, scratch);
@@ -162,7 +168,7 @@ __global__ void __launch_bounds__(256) muon_prepare_kernel(MuonPrepareArgs a) {
     }
     squares = block_sum(squares, scratch);
     if (threadIdx.x == 0)
-        a.sumsq[matrix * MuonBlocks + blockIdx.x] = squares;
+        finish_block(a, matrix, squares);
 }
 // The same stage, 128-bit: eight consecutive elements per thread (matrices stored in the orientation the
 // iterations use, rows <= cols).
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(256) muon_prepare_vector_kernel(MuonPrepareArg
     }
     squares = block_sum(squares, scratch);
     if (threadIdx.x == 0)
-        a.sumsq[matrix * MuonBlocks + blockIdx.x] = squares;
+        finish_block(a, matrix, squares);
 }
 // Tall matrices (rows > cols) are orthogonalised transposed.  64 x 64 tiles go through shared memory so
 // that gradient and momentum are read, and the transposed BF16 matrix written, in whole 128-byte lines.
@@ -256,7 +262,7 @@ __global__ void __launch_bounds__(256) muon_prepare_transpose_kernel(MuonPrepare
     }
     squares = block_sum(squares, scratch);
     if (threadIdx.x == 0)
-        a.sumsq[matrix * MuonBlocks + blockIdx.x] = squares;
+        finish_block(a, matrix, squares);
 }
 void launch_muon_prepare(const MuonPrepareArgs &a, cudaStream_t s) {
     const dim3 grid(MuonBlocks, a.batch);
