@@ -416,6 +416,66 @@ def test_newton_schulz_of_all_families_in_one_launch(depth, width, hidden, ns_st
             assert relative(results[0][0][part] - w[part], opt.w[part] - w[part]) < .04, name
 
 
+@pytest.mark.parametrize("width,hidden,context,batch", [
+    (64, 72, 13, 5),      # 65 tokens: a last row, a last K block of one token, outputs of 72 columns
+    (128, 200, 37, 3), (192, 1000, 64, 2), (320, 264, 333, 1), (256, 1024, 130, 1),
+    (256, 1024, 1024, 3), # tiles of 128 columns; K cut for the weight gradients
+    (512, 64, 517, 4)])   # K cut in the chain, more tiles than SMs
+def test_fp32_products_on_tensor_cores(width, hidden, context, batch):
+    """FP32 engines with and without tensor cores: every activation, logit and gradient at the FP32 mode's own bound."""
+    rng = np.random.default_rng(width)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    arch = Arch.gpt(2, width, width // 64, hidden)
+    w = Model(arch, seed=5, scale=.05).flat()
+    results = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.gpt(Config(depth=2, context=context, batch=batch), width, width // 64, hidden, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            logits, gradients, losses = engine.batch(x, y)
+            again = engine.batch(x, y)
+            np.testing.assert_array_equal(gradients, again[1])  # replayed
+            activations = [engine.activation(l, name) for l in range(2) for name in ("qkv", "middle", "activated")]
+            results.append([logits, losses, *activations, gradients])
+    for got, expected in zip(*results):
+        assert relative(got, expected) <= 1e-5
+    offset = 0
+    for name, shape in specification(arch):
+        part = slice(offset, offset + int(np.prod(shape)))
+        offset = part.stop
+        assert relative(results[0][-1][part], results[1][-1][part]) <= 1e-5, name
+
+
+def test_fp32_products_of_infinities_and_of_values_that_round_to_them():
+    """Infinities and NaN stay what FP32 multiply-adds make of them, and nothing else is touched by them; so do finite weights beyond the largest BF16
+    value, and products that overflow."""
+    width, context, batch = 128, 40, 2
+    rng = np.random.default_rng(2)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    arch = Arch.gpt(1, width, 2)
+    w = Model(arch, seed=5, scale=.05).flat()
+    qkv = w[256 * width + 2 * width:][:3 * width * width].reshape(3 * width, width)  # behind the embedding and the norm's scale and bias
+    qkv[3, 5], qkv[10, 0], qkv[100, 7], qkv[200, 9], qkv[300, 11] = np.inf, np.nan, 3.4e38, -3.395e38, 1e38
+    qkv[300, 12] = -1e38
+    results = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.gpt(Config(depth=1, context=context, batch=batch), width, 2, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            engine.batch(x, y, backward=False)
+            results.append((engine.activation(0, "normed1"), engine.activation(0, "qkv")))
+    (normed, got), (same, expected) = results
+    np.testing.assert_array_equal(normed, same)
+    assert not np.isfinite(got[:, [3, 10]]).any() and np.isinf(got[:, 100]).any() and np.isfinite(got[:, 100]).any()
+    untouched = np.setdiff1d(np.arange(3 * width), [3, 10, 100, 200, 300])
+    assert np.isfinite(got[:, untouched]).all()
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(expected))
+    np.testing.assert_array_equal(np.isinf(got), np.isinf(expected))
+    finite = np.isfinite(expected)
+    magnitude = np.abs(normed).astype(np.float64) @ np.abs(np.where(np.isfinite(qkv), qkv, 0)).T.astype(np.float64)
+    assert (np.abs(got[finite] - expected[finite].astype(np.float64)) <= 2 * width * 2.0 ** -24 * magnitude[finite]).all()
+
+
 def _structured_bytes(size, seed):
     """Learnable bytes: an order-1 Markov chain with sparse (Dirichlet 0.05) transition rows."""
     rng = np.random.default_rng(seed)

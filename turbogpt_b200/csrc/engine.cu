@@ -13,7 +13,7 @@
 #include <type_traits>
 
 constexpr int64_t TwoSideLanes = int64_t(1) << 22; // tokens x columns up to which weight gradients have two lanes
-constexpr size_t SimtScratchBytes = size_t(6) << 20; // bounds gemm_simt_scratch_bytes for every shape it cuts
+constexpr size_t SimtScratchBytes = SplitScratchBytes; // bounds gemm_simt_scratch_bytes for every shape it cuts
 
 const char *const family_names[FamilyCount] = {
     "sample", "embedding", "norm", "gemm_forward", "gemm_input_grad", "gemm_weight_grad", "attention_forward",
@@ -399,6 +399,8 @@ void Engine::gemm(Family f, GemmArgs g) {
     run(f, [&](cudaStream_t s) {
         if (on_tensor_cores(g))
             launches += launch_gemm_tc(g, gemm_sms, counters, s, &lanes[lane].workspace) - 1;
+        else if (tensor_cores && gemm_split_supported(g))
+            launch_gemm_split(g, sms, counters, s, simt_scratch[lane]);
         else
             launch_gemm_simt(g, s, gemm_simt_scratch_bytes(g) <= SimtScratchBytes ? simt_scratch[lane] : nullptr);
     });

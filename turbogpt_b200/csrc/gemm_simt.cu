@@ -1,51 +1,15 @@
 // GEMM on CUDA cores: C[m,n] = sum_k A[m,k] * B[n,k] with arbitrary element strides, BF16 or
-// FP32 operands, FP32 accumulation.  It serves the shapes the tensor-core kernel does not take
-// (the reference architecture's 16/48-wide matrices), the FP32 check mode, and is the on-device
-// cross-check of the tcgen05 kernel.  Two kernels: gemm_simt_kernel takes any strides, sizes and
+// FP32 operands, FP32 accumulation.  It serves the shapes the tensor-core kernels do not take
+// (the reference architecture's 16/48-wide matrices) and engines without tensor cores, and is the on-device
+// cross-check of the tcgen05 kernels.  Two kernels: gemm_simt_kernel takes any strides, sizes and
 // alignments (64x64 output tile, 16-deep shared-memory slices, 4x4 outputs per thread, scalar loads);
 // gemm_simt_wide_kernel (BF16 operands) and gemm_fp32_kernel (FP32) take what 16-byte pieces can reach and every shape of
 // a real model (see there).
-#include "device_utils.cuh"
-#include "kernels.cuh"
+#include "epilogue_ops.cuh"
 #include <algorithm>
 #include <type_traits>
 
 constexpr int TileM = 64, TileN = 64, TileK = 16;
-
-// Every case is inlined for each output of a thread: a second GELU here made the code a fifth longer and small calls, which fetch it anew,
-// 5 to 12 % slower (the reference architecture's gradients of 64 tokens 555 -> 631 us), so that Epilogue::Gelu is the tensor cores' alone.
-template <class Out> struct EpilogueOps {
-    // `value` is the FP32 accumulator; returns what is stored to C (already in storage rounding).
-    __device__ static void apply(const GemmArgs &g, float value, int64_t c_index, int64_t r_index, int z) {
-        Out *c = (Out *)g.c + z * g.c_batch;
-        switch (g.epilogue) {
-        case Epilogue::Store:
-            c[c_index] = from_float<Out>(value);
-            break;
-        case Epilogue::Residual: {
-            const Out *r = (const Out *)g.r + z * g.r_batch;
-            c[c_index] = from_float<Out>(rounded<Out>(value) + to_float(r[r_index]));
-            break;
-        }
-        case Epilogue::GeluDual: {
-            float pre = rounded<Out>(value);
-            c[c_index] = from_float<Out>(gelu_derivative(pre));
-            ((Out *)g.c2 + z * g.c_batch)[c_index] = from_float<Out>(gelu(pre));
-            break;
-        }
-        case Epilogue::GeluGrad: {
-            const Out *r = (const Out *)g.r + z * g.r_batch;
-            c[c_index] = from_float<Out>(rounded<Out>(value) * to_float(r[r_index]));
-            break;
-        }
-        case Epilogue::Axpby: {
-            const Out *r = (const Out *)g.r + z * g.r_batch;
-            c[c_index] = from_float<Out>(g.alpha * value + g.beta * to_float(r[r_index]));
-            break;
-        }
-        }
-    }
-};
 
 // `partials` == nullptr: blockIdx.z is the batch index and the block walks all of K.  Otherwise (batch 1)
 // blockIdx.z is a slice of K, `slice_k` elements long, and the block writes its FP32 partial tile to
@@ -442,6 +406,9 @@ template <class In, class Out> static void launch_simt(const GemmArgs &g, const 
         gemm_simt_wide_kernel<Out, 4><<<grid, 128, 0, s>>>(g, partials, slice_k);
     if (partials)
         gemm_simt_reduce_kernel<Out><<<unsigned((int64_t(g.m) * g.n + 255) / 256), 256, 0, s>>>(g, partials, used);
+}
+void launch_gemm_slices(const GemmArgs &g, const float *partials, int slices, cudaStream_t s) {
+    gemm_simt_reduce_kernel<float><<<unsigned((int64_t(g.m) * g.n + 255) / 256), 256, 0, s>>>(g, partials, slices);
 }
 void launch_gemm_simt(const GemmArgs &g, cudaStream_t s, float *scratch) {
     if (g.epilogue == Epilogue::Gelu || g.epilogue == Epilogue::CrossEntropy)

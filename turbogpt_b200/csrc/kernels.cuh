@@ -190,6 +190,12 @@ struct GemmArgs {
 // partial tiles added in a fixed order); nullptr: never cut.
 size_t gemm_simt_scratch_bytes(const GemmArgs &g);
 void launch_gemm_simt(const GemmArgs &g, cudaStream_t s, float *scratch = nullptr);
+// FP32 operands, FP32 products: on tensor cores as products of BF16 parts (gemm_split.cu); `scratch`: SplitScratchBytes, or nullptr (K is not cut).
+bool gemm_split_supported(const GemmArgs &g);
+constexpr size_t SplitScratchBytes = size_t(6) << 20; // its plans need no more
+void launch_gemm_split(const GemmArgs &g, int sms, StepCounters *counters, cudaStream_t s, float *scratch = nullptr);
+// Adds `slices` partial products [m][n] in order, and applies the epilogue.
+void launch_gemm_slices(const GemmArgs &g, const float *partials, int slices, cudaStream_t s);
 // tcgen05 path; returns false when the shape/layout is outside what it supports.
 bool gemm_tc_supported(const GemmArgs &g);
 // Split-K scratch of the tcgen05 GEMM: FP32 partial tiles, one ticket per output tile (zero between
