@@ -2,9 +2,9 @@
 //
 // Every operand value is the sum of three BF16 parts, x = h + m + l, each the rounded rest of what the parts before it leave (24 bits of
 // significand in three times eight).  Of the nine products of parts the six above 2^-24 of x y are formed, exact in FP32: h h into one
-// accumulator, h m, m h, m m, h l and l h into another.  The tensor core's sums lose bits with their length (4.4e-6 after 256 steps),
-// so the first accumulator only ever holds one 64-deep block of K, four steps, and is added to FP32 registers; the second is 2^-8 of the
-// result and runs over all of K.  Against 64 bits (N(0,1) operands, K 16 to 4096) 0.4 to 1.3e-7,
+// accumulator, h m, m h, m m, h l and l h into another.  The tensor core cuts its sums off instead of rounding them (1.2e-8 of the
+// result for every step, 4.4e-6 after 256), so the first accumulator only ever holds 32 of K, two steps, and is added to FP32 registers; the second is
+// 2^-8 of the result and runs over all of K.  Against 64 bits (N(0,1) operands, K 16 to 4096) 0.4 to 1.3e-7,
 // where the CUDA cores' sums have 0.7 to 4.1e-7.
 //
 // What bounds it: 24 products of 128 x BN x 16 a block read their operands from shared memory, 6 (4 + BN / 32) KB each, at 128 B/clk, beside the
@@ -95,16 +95,17 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
     const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
     uint8_t *aligned = raw_shared + (base - smem_address(raw_shared));
     uint64_t *barriers = reinterpret_cast<uint64_t *>(aligned + 2 * stage_bytes(BN));
-    const uint32_t full0 = smem_address(barriers), done0 = full0 + 16;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 4);
+    const uint32_t full0 = smem_address(barriers), done0 = full0 + 16, added = done0 + 16;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 5);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    constexpr int Columns = BN == 128 ? 512 : 256; // of tensor memory: two accumulators of h h, one of the rest
+    constexpr int Columns = BN == 128 ? 512 : 256; // of tensor memory: an accumulator of h h for either half of a block, one of the rest
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
             mbarrier_init(full0 + 8 * s, Workers);
             mbarrier_init(done0 + 8 * s, 1);
         }
+        mbarrier_init(added, Workers);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
                            b_desc = smem_descriptor(base + 3 * part_bytes(BM), BK ? 16 : 64 * RowBytes, 1024);
             for (int b = 0; b < blocks && ok; ++b) {
                 const int s = b % 2;
-                ok = mbarrier_wait(full0 + 8 * s, b / 2 & 1, abort_flag, counters, 411); // the block is there, and the accumulator has been read
+                ok = mbarrier_wait(full0 + 8 * s, b / 2 & 1, abort_flag, counters, 411); // the block is there
                 if (!ok)
                     break;
                 tcgen05_fence_after();
@@ -145,13 +146,18 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
                 };
 #pragma unroll
                 for (int ks = 0; ks < Block / 16; ++ks) {
-                    multiply(tmem_base + s * BN, 0, 0, ks, ks > 0);
                     multiply(tmem_base + 2 * BN, 0, 1, ks, b > 0 || ks > 0);
                     multiply(tmem_base + 2 * BN, 1, 0, ks, true);
                     multiply(tmem_base + 2 * BN, 1, 1, ks, true);
                     multiply(tmem_base + 2 * BN, 0, 2, ks, true);
                     multiply(tmem_base + 2 * BN, 2, 0, ks, true);
                 }
+                if (b > 0 && !(ok = mbarrier_wait(added, (b - 1) & 1, abort_flag, counters, 413))) // the block before has been added to the registers
+                    break;
+                tcgen05_fence_after();
+#pragma unroll
+                for (int ks = 0; ks < Block / 16; ++ks)
+                    multiply(tmem_base + ks / 2 * BN, 0, 0, ks, ks % 2);
                 tcgen05_commit(done0 + 8 * s);
             }
         }
@@ -162,24 +168,26 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
 #pragma unroll
         for (int j = 0; j < Share; ++j)
             sums[j] = 0.f;
-        auto add = [&](int accumulator) { // columns of tensor memory, all blocks of which are complete
-            const uint32_t address = tmem_base + (uint32_t(quarter * 32) << 16) + accumulator * BN + first_column;
-#pragma unroll
-            for (int c = 0; c < Share; c += 16) {
-                uint32_t v[16];
-                tmem_load_32x16_async(address + c, v);
-                tmem_wait_load(v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    sums[c + j] += __uint_as_float(v[j]);
-            }
-        };
+        const uint32_t accumulators = tmem_base + (uint32_t(quarter * 32) << 16) + first_column;
         auto finish = [&](int block) {
             if (!mbarrier_wait(done0 + 8 * (block % 2), block / 2 & 1, abort_flag, counters, 412))
                 return false;
             tcgen05_fence_after();
-            add(block % 2);
+#pragma unroll
+            for (int c = 0; c < Share; c += 8) { // more columns at a time spill
+                uint32_t v[8], w[8];
+                tmem_load_32x8_async(accumulators + c, v);
+                tmem_load_32x8_async(accumulators + BN + c, w);
+                tmem_wait_load(v);
+                tmem_wait_load(w);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    sums[c + j] += __uint_as_float(v[j]) + __uint_as_float(w[j]);
+            }
             tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbarrier_arrive(added);
             return true;
         };
         a.load(k_end);
@@ -200,8 +208,17 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
                 break;
         }
         ok = ok && finish(blocks - 1);
-        if (ok)
-            add(2);
+#pragma unroll
+        for (int c = 0; c < Share; c += 16) {
+            if (!ok)
+                break;
+            uint32_t v[16];
+            tmem_load_32x16_async(accumulators + 2 * BN + c, v);
+            tmem_wait_load(v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                sums[c + j] += __uint_as_float(v[j]);
+        }
     }
     ok = __syncthreads_and(ok); // every product is done: the stages take the sums
     constexpr int Pitch = BN + 4;

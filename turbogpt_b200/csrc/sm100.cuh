@@ -285,6 +285,19 @@ __device__ __forceinline__ void tmem_wait_load(uint32_t (&r)[16]) {
                  :
                  : "memory");
 }
+// 8-column forms.
+__device__ __forceinline__ void tmem_load_32x8_async(uint32_t address, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(address)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_load(uint32_t (&r)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
+}
 // 32 lanes x 32 consecutive 32-bit columns from registers: thread i writes row (lane base + i).
 __device__ __forceinline__ void tmem_store_32x32(uint32_t address, const uint32_t (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
