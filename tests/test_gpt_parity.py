@@ -476,6 +476,35 @@ def test_fp32_products_of_infinities_and_of_values_that_round_to_them():
     assert (np.abs(got[finite] - expected[finite].astype(np.float64)) <= 2 * width * 2.0 ** -24 * magnitude[finite]).all()
 
 
+@pytest.mark.parametrize("context,batch,heads", [(2, 70, 1), (64, 2, 2), (65, 3, 1), (129, 2, 3), (200, 40, 2), (1000, 1, 1)])
+def test_fp32_attention_on_tensor_cores(context, batch, heads):
+    """Sequence ends on and off the 64-row tiles, two tokens a sequence, more tiles than SMs: what attention saves, and the gradients that it
+    passes on, against the CUDA cores' kernels at the FP32 mode's own bound."""
+    test_fp32_products_on_tensor_cores(64 * heads, 128 * heads, context, batch)
+
+
+def test_fp32_attention_keeps_a_later_infinity_out():
+    """An infinite embedding at one position: what precedes it stays finite and as it was, what follows is what the CUDA cores' kernels make of it."""
+    width, context, batch, at = 128, 150, 2, 70
+    rng = np.random.default_rng(3)
+    x, y = rng.integers(0, 255, (2, batch, context), dtype=np.uint8)
+    x[1, at] = 255  # read there only
+    arch = Arch.gpt(2, width, 2)
+    w = Model(arch, seed=5, scale=.05).flat()
+    results = []
+    for value, flags in ((.5, 0), (np.inf, 0), (np.inf, bridge.FLAG_NO_TENSOR_CORES)):
+        w[255 * width + 3] = value
+        ex = ConfigEx.gpt(Config(depth=2, context=context, batch=batch), width, 2, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            engine.batch(x, y, backward=False)
+            results.append(engine.activation(0, "attended").reshape(batch, context, width))
+    without, got, expected = results
+    assert relative(got[0], without[0]) <= 1e-5 and relative(got[1, :at], without[1, :at]) <= 1e-5
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(expected))
+    assert not np.isfinite(got[1, at:]).any()
+
+
 def _structured_bytes(size, seed):
     """Learnable bytes: an order-1 Markov chain with sparse (Dirichlet 0.05) transition rows."""
     rng = np.random.default_rng(seed)

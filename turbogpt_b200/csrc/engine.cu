@@ -521,6 +521,8 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
             run(FAttentionForward, [&](cudaStream_t s) {
                 if (tensor_cores && act == Dtype::BF16 && flash_attention_supported(W, H))
                     launch_flash_attention_forward(a.qkv, a.attended, a.lse, B, T, H, counters, s);
+                else if (tensor_cores && act == Dtype::FP32 && attention_split_supported(W, H))
+                    launch_attention_split_forward(at, s);
                 else
                     launch_softmax_attention(act, at, s);
             });
@@ -703,6 +705,8 @@ void Engine::backward() {
                 if (tensor_cores && act == Dtype::BF16 && flash_attention_supported(W, H)) {
                     launches += launch_flash_attention_backward(a.qkv, a.attended, dbranch, a.lse, attention_scratch, dqkv, B, T, H,
                                                                 counters, s) - 1;
+                } else if (tensor_cores && act == Dtype::FP32 && attention_split_supported(W, H)) {
+                    launch_attention_split_backward(at, s);
                 } else {
                     launch_softmax_attention_backward(act, at, s);
                 }

@@ -107,6 +107,10 @@ struct SoftmaxAttentionBackwardArgs {
     int batch, context, width, heads;
 };
 void launch_softmax_attention_backward(Dtype t, const SoftmaxAttentionBackwardArgs &a, cudaStream_t s);
+// FP32, head size 64, on tensor cores (attention_split.cu).
+bool attention_split_supported(int width, int heads);
+void launch_attention_split_forward(const SoftmaxAttentionArgs &a, cudaStream_t s);
+void launch_attention_split_backward(const SoftmaxAttentionBackwardArgs &a, cudaStream_t s);
 
 // ---- causal softmax attention on tcgen05 (BF16, head size 64) ----
 // `counters` nullptr: a wait that gives up is recorded in the current device's word for calls without an engine, below (nullptr: no such
