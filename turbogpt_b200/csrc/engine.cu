@@ -202,6 +202,7 @@ void Engine::initialize() {
         allocate(embedding_partial, size_t(EmbeddingSlices) * Vocabulary * W, false);
     sumsq_blocks = sms * 8;
     allocate(sumsq_partial, sumsq_blocks);
+    allocate(adam_ticket, 1);
 
     // Per 8 parameters: 0 = Muon, 1 = AdamW, 2 = AdamW with decay (reference cuda/optim.cuh:5-15:
     // decay on the head only; with AdamW on hidden matrices they decay too; a tied embedding is the head).
@@ -490,7 +491,8 @@ void Engine::set_onecycle(const TgOneCycle &s) {
 }
 
 // ------------------------------------------------------------------------------- forward -----
-void Engine::forward(bool want_gradient, bool dump_logits) {
+// `embedded`: the sampling kernel has left the embeddings.
+void Engine::forward(bool want_gradient, bool dump_logits, bool embedded) {
     const TgConfigEx &c = config;
     const int B = forward_batch ? forward_batch : c.base.batch, T = c.base.context, M = B * T;
     const int W = c.width, Hd = c.hidden, H = c.heads;
@@ -501,7 +503,8 @@ void Engine::forward(bool want_gradient, bool dump_logits) {
                    layer_norm ? weight_low + bias : nullptr, out, M, W, stats, true}; // the embedding, at least, lies between them and the optimizer
         run(FNorm, [&](cudaStream_t s) { launch_norm(act, a, s); });
     };
-    run(FEmbedding, [&](cudaStream_t s) { launch_embedding(act, weight(layout.embedding), x, layers[0].x, M, W, s); });
+    if (!embedded)
+        run(FEmbedding, [&](cudaStream_t s) { launch_embedding(act, weight(layout.embedding), x, layers[0].x, M, W, s); });
     for (int l = 0; l < depth; ++l) {
         LayerActivations &a = layers[l];
         const LayerOffsets &p = layout.layers[l];
@@ -597,6 +600,15 @@ void Engine::finish_exchange() {
         return;
     CHECK_CUDA(cudaEventRecord(exchange_done, exchange_stream));
     CHECK_CUDA(cudaStreamWaitEvent(stream, exchange_done, 0));
+}
+
+// Nothing of the step waits for its row of the losses but the count of steps: beside the backward pass, which joins its lanes.
+void Engine::record_losses() {
+    next_fork_event = 0;
+    if (side_lanes)
+        fork(0, 1);
+    OnLane on(*this, side_lanes ? 1 : 0);
+    run(FMisc, [&](cudaStream_t s) { launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context, s); });
 }
 
 void Engine::backward() {
@@ -827,6 +839,8 @@ void Engine::optimize() {
     AdamArgs a{gradient, momentum, variance, weight_high, weight_low, weight_fp32, adam_mode, sumsq_partial,
                sumsq_blocks, schedule, counters, c.base.learning_rate, c.base.beta1, c.base.beta2,
                c.base.weight_decay, c.base.epsilon, c.base.clip, layout.count};
+    if (muon.empty()) // the step's last kernel
+        a.advance = counters, a.ticket = adam_ticket;
     next_fork_event = 0; // backward has joined its lanes
     const cudaEvent_t norm_ready = muon_lanes && !muon.empty() ? mark(0) : nullptr;
     run(FOptimizer, [&](cudaStream_t s) { launch_adamw(a, sms, s); });
@@ -860,7 +874,8 @@ void Engine::optimize() {
         }
         join();
     }
-    run(FMisc, [&](cudaStream_t s) { launch_advance(counters, s); });
+    if (!muon.empty())
+        run(FMisc, [&](cudaStream_t s) { launch_advance(counters, s); });
 }
 
 // ------------------------------------------------------------------------------- modes -------
@@ -896,19 +911,21 @@ void Engine::one_step(RunMode mode, bool last) {
     if (mode == RunMode::Train) {
         SampleArgs sampling{data, data_size, config.base.seed, counters, -1, config.base.batch, config.base.context,
                      config.world, config.rank, x, y};
-        run(FSample, [&](cudaStream_t s) { launch_sample(sampling, s); });
+        run(FSample, [&](cudaStream_t s) {
+            if (profile) // every family has its own kernels there
+                launch_sample(sampling, s);
+            else
+                launch_sample_embedding(act, sampling, weight(layout.embedding), layers[0].x, config.width, s);
+        });
     }
     if (mode != RunMode::OptimizerOnly) {
-        forward(mode != RunMode::Evaluate, mode != RunMode::Train && logits_fp32 != nullptr);
+        forward(mode != RunMode::Evaluate, mode != RunMode::Train && logits_fp32 != nullptr, mode == RunMode::Train && !profile);
         if (mode == RunMode::Gradients)
             announce(copies.forward_done, 0);
         if (mode == RunMode::Evaluate)
             return;
         if (mode == RunMode::Train)
-            run(FMisc, [&](cudaStream_t s) {
-                launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context,
-                                    s);
-            });
+            record_losses();
         announce_gradients = mode == RunMode::Gradients;
         backward();
         announce_gradients = false;
@@ -1241,9 +1258,7 @@ void Engine::train_batch(const uint8_t *bx, const uint8_t *by, float *per_positi
             return;
         }
         forward(true, false);
-        run(FMisc, [&](cudaStream_t s) {
-            launch_loss_history(token_losses, loss_history, counters, config.base.batch, config.base.context, s);
-        });
+        record_losses();
         backward();
         optimize();
     });

@@ -117,7 +117,7 @@ struct Engine {
     float2 *reference_rope = nullptr;
     SmallMatrix *small_matrices = nullptr;
     int small_matrix_count = 0;
-    unsigned *small_ticket = nullptr;
+    unsigned *small_ticket = nullptr, *adam_ticket = nullptr;
     // host mirrors
     uint64_t step = 0;
     int last_train_steps = 0;
@@ -193,7 +193,8 @@ struct Engine {
     template <class F> void run(Family f, F &&launch);
     bool on_tensor_cores(GemmArgs g) const; // whether gemm() takes it there
     void gemm(Family f, GemmArgs g);
-    void forward(bool want_gradient, bool dump_logits);
+    void forward(bool want_gradient, bool dump_logits, bool embedded = false);
+    void record_losses();
     void backward();
     void exchange_bucket(int64_t begin, int64_t end, int index);
     void finish_exchange();

@@ -27,6 +27,8 @@ struct SampleArgs {
     uint8_t *x, *y; // [batch*context]
 };
 void launch_sample(const SampleArgs &a, cudaStream_t s);
+// The same, and the embeddings of x to `hidden`.
+void launch_sample_embedding(Dtype t, const SampleArgs &a, const void *table, void *hidden, int width, cudaStream_t s);
 void launch_embedding(Dtype t, const void *table, const uint8_t *x, void *hidden, int tokens, int width,
                       cudaStream_t s);
 // grad[x[t]*width + c] += dhidden[t, c] in FP32 (reference cuda/model.cuh:96-97), deterministic:
@@ -278,7 +280,10 @@ struct AdamArgs {
     const StepCounters *counters;
     float learning_rate, beta1, beta2, weight_decay, epsilon, clip;
     int64_t count;
+    StepCounters *advance = nullptr; // counted up by the last block, where this kernel is the step's last; `ticket` is zero between launches
+    unsigned *ticket = nullptr;
 };
+// Follows launch_sum_squares in the stream.
 void launch_adamw(const AdamArgs &a, int sms, cudaStream_t s);
 constexpr int MuonBlocks = 32; // blocks per matrix in the Muon prepare stage = partial sums per matrix
 struct MuonPrepareArgs { // momentum, Nesterov direction, BF16 cast (+ transpose when rows > cols), sum of squares
