@@ -10,6 +10,7 @@
 #include <cstring>
 #include <dlfcn.h>
 #include <iterator>
+#include <new>
 #include <type_traits>
 
 constexpr int64_t TwoSideLanes = int64_t(1) << 22; // tokens x columns up to which weight gradients have two lanes
@@ -284,7 +285,9 @@ void Engine::initialize() {
         if (c.flags & TG_FLAG_BF16_GRADIENT_EXCHANGE)
             allocate(gradient_bf16, P, false);
     }
-    CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&mailbox), sizeof(Mailbox), cudaHostAllocDefault));
+    mailbox = new (std::align_val_t(4096)) Mailbox;
+    CHECK_CUDA(cudaHostRegister(mailbox, sizeof(Mailbox), cudaHostRegisterDefault)); // cudaHostAlloc: 2.5 ms longer
+    mailbox_pinned = true;
     copies.create(layout, depth, !comm); // under data parallelism the gradients are added up over the ranks after the pass
     CHECK_CUDA(cudaStreamSynchronize(stream));
 }
@@ -327,8 +330,10 @@ void Engine::release() {
         cudaEventDestroy(ev);
     copies.destroy();
     results.destroy();
+    if (mailbox_pinned)
+        cudaHostUnregister(mailbox);
     if (mailbox)
-        cudaFreeHost(mailbox);
+        operator delete(mailbox, std::align_val_t(4096));
     for (auto &t : timed) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);

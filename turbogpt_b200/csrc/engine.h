@@ -151,6 +151,7 @@ struct Engine {
         StepCounters counters;
         float values[16384];
     } *mailbox = nullptr;
+    bool mailbox_pinned = false;
     bool announce_gradients = false;
     StepGraph graphs[GraphKinds];
     int forward_batch = 0; // sequences the next forward pass covers (0: the configured batch)
