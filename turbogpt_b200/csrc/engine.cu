@@ -298,7 +298,6 @@ void Engine::prepare_reference_step() {
     reference_plan = reference_step_plan(c, sms);
     allocate(reference_partial, size_t(reference_plan.blocks) * reference_plan.partial_stride, false);
     allocate(reference_norm, reference_plan.gradient_blocks);
-    allocate(small_ticket, 1);
     std::vector<float2> rope(c.base.context);
     for (int p = 0; p < c.base.context; ++p)
         rope[p] = make_float2(float(std::cos(double(p))), float(std::sin(double(p))));
@@ -903,7 +902,7 @@ void Engine::reference_train_step(bool sample, bool save) {
     SmallOptimizerArgs update{{gradient, momentum, variance, weight_high, weight_low, nullptr, adam_mode, reference_norm,
                                reference_plan.gradient_blocks, schedule, counters, b.learning_rate, b.beta1, b.beta2, b.weight_decay,
                                b.epsilon, b.clip, layout.count},
-                              b.muon_lr, b.momentum, b.ns_steps, small_matrices, small_matrix_count, counters, small_ticket};
+                              b.muon_lr, b.momentum, b.ns_steps, small_matrices, small_matrix_count, counters};
     run(FOptimizer, [&](cudaStream_t s) { launch_small_optimizer(update, s); });
 }
 

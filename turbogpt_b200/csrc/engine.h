@@ -117,7 +117,7 @@ struct Engine {
     float2 *reference_rope = nullptr;
     SmallMatrix *small_matrices = nullptr;
     int small_matrix_count = 0;
-    unsigned *small_ticket = nullptr, *adam_ticket = nullptr;
+    unsigned *adam_ticket = nullptr;
     // host mirrors
     uint64_t step = 0;
     int last_train_steps = 0;

@@ -250,7 +250,7 @@ struct ReferenceStepArgs {
     int64_t data_size;
     uint64_t seed;
     const uint8_t *x, *y;
-    const StepCounters *counters;
+    StepCounters *counters; // the step's number is counted up when its gradients are reduced
     const bf16 *weight_high;
     const uint16_t *weight_low;
     const float2 *rope;  // [context] cos, sin of the position in radians
@@ -331,7 +331,7 @@ struct MuonApplyArgs {
 };
 void launch_muon_apply(const MuonApplyArgs &a, int sms, cudaStream_t s);
 void launch_advance(StepCounters *counters, cudaStream_t s);
-// AdamW, Muon and the advance of the step counters in one kernel, for models whose hidden matrices are at most 16 x 48
+// AdamW and Muon in one kernel, for models whose hidden matrices are at most 16 x 48
 // (or 48 x 16): one warp orthogonalises one matrix in registers.
 struct SmallMatrix {
     int offset, rows, cols;
@@ -342,8 +342,7 @@ struct SmallOptimizerArgs {
     int ns_steps;
     const SmallMatrix *matrices; // device
     int matrix_count;
-    StepCounters *counters;      // advanced by the last block
-    unsigned *ticket;            // zero between launches
+    StepCounters *counters;      // the step has been counted up already (launch_reference_step), the iteration is by this
 };
 void launch_small_optimizer(const SmallOptimizerArgs &a, cudaStream_t s);
 

@@ -59,8 +59,7 @@ __device__ __forceinline__ float clip_factor(const float *norm_partial, int norm
 // correction with the current, possibly cycled, beta1 as torch.optim.AdamW does.
 struct AdamRates {
     float clip = 1.f, lr, beta1, step_size, inv_sqrt_bc2;
-    __device__ __forceinline__ explicit AdamRates(const AdamArgs &a) {
-        const unsigned long long step = a.counters->step;
+    __device__ __forceinline__ AdamRates(const AdamArgs &a, unsigned long long step) {
         float multiplier = 1;
         beta1 = a.beta1;
         if (a.schedule) {
@@ -131,7 +130,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a) {
     __shared__ float scratch[32];
     sm100::grid_launch_dependents();
     const int64_t groups = a.count / 8;
-    AdamRates rates(a);
+    AdamRates rates(a, a.counters->step);
     sm100::grid_dependency_wait();
     rates.clip = clip_factor(a.norm_partial, a.norm_blocks, a.clip, scratch);
     for (int64_t group = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; group < groups;
@@ -515,7 +514,7 @@ void launch_advance(StepCounters *counters, cudaStream_t s) {
 
 // ------------------------------------------------------------------------------------------
 // Whole update of a model of 16-wide matrices.  As separate kernels it was 5 x (prepare, normalise, Newton-Schulz in
-// shared memory, apply), AdamW and the counter: 22 launches and 0.2 ms, all latency (now ~9 us).  One warp takes one matrix: X
+// shared memory, apply), AdamW and the counter: 22 launches and 0.2 ms, all latency (now 5 us).  One warp takes one matrix: X
 // (16 x n, n = 16 or 48, the wide orientation) lives in registers as m16n8k16 operand fragments, and an iteration is
 // n/8 + 2 + n/8 products per 16-deep step with the roundings of muon_newton_schulz_small_kernel:
 //   A = X X^T     X's fragments are both operands
@@ -562,7 +561,7 @@ template <int Steps> struct SmallMuon { // Steps: columns of X / 16
             high[k][i][j] = a.adam.weight_high[at], low[k][i][j] = a.adam.weight_low[at];
         });
         if (a.adam.schedule) {
-            const TgStepRates rates = a.adam.schedule[a.adam.counters->step];
+            const TgStepRates rates = a.adam.schedule[a.counters->step - 1];
             mu = rates.momentum, multiplier = rates.multiplier;
         }
     }
@@ -640,18 +639,18 @@ __device__ __forceinline__ float clip_of_warp(const AdamArgs &a) {
     return fminf(1.f, a.clip / (sqrtf(warp_sum(local)) + 1e-6f));
 }
 __global__ void __launch_bounds__(SmallWarps * 32) small_optimizer_kernel(const __grid_constant__ SmallOptimizerArgs a, int matrix_blocks) {
-    sm100::grid_launch_dependents();
     const int index = blockIdx.x * SmallWarps + threadIdx.x / 32;
     SmallMatrix matrix{0, 16, 16};
     if (index < a.matrix_count)
         matrix = a.matrices[index];
     sm100::grid_dependency_wait();
+    sm100::grid_launch_dependents(); // the next step's kernel reads the step's number, which is this one's and has been counted up by now
     if (int(blockIdx.x) >= matrix_blocks) {
         const int64_t group = int64_t(blockIdx.x - matrix_blocks) * blockDim.x + threadIdx.x;
         AdamGroup parameters;
         if (group < a.adam.count / 8)
             parameters = AdamGroup(a.adam, group);
-        AdamRates rates(a.adam);
+        AdamRates rates(a.adam, a.counters->step - 1);
         rates.clip = clip_of_warp(a.adam);
         parameters.update<false>(a.adam, rates, group);
     } else {
@@ -663,11 +662,8 @@ __global__ void __launch_bounds__(SmallWarps * 32) small_optimizer_kernel(const 
             muon.update(a, clip_of_warp(a.adam));
         }
     }
-    __syncthreads(); // every thread has read the step before the block's arrival is counted
-    if (threadIdx.x == 0 && atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1) {
-        a.counters->step += 1;
-        a.counters->iteration += 1;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        a.counters->iteration += 1; // its readers have ended
 }
 void launch_small_optimizer(const SmallOptimizerArgs &a, cudaStream_t s) {
     const int matrix_blocks = (a.matrix_count + SmallWarps - 1) / SmallWarps, per_block = SmallWarps * 32;

@@ -3,7 +3,7 @@
 //
 // What bounds it: a token's whole step is 52 k multiply-adds over matrices of 16 columns, so as separate
 // kernels (one per operator, ~150 launches) a step is launch latency and half-empty tiles: 1.43 ms at depth 4,
-// context 4, batch 2880, and 0.86 ms at batch 16 (now 49 and 31 us with reduction and update: the latency of the chain of
+// context 4, batch 2880, and 0.86 ms at batch 16 (now 49 and 30 us with reduction and update: the latency of the chain of
 // dependent products).  Here a block takes whole sequences (up to 128 tokens) through
 // every layer and back: each warp keeps its 16 tokens' residual stream in registers, the weights sit in shared
 // memory once, and only k and v (forward) and the attention gradients (backward) pass between warps.
@@ -404,30 +404,36 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
     grid_launch_dependents();
     for (int i = threadIdx.x; i < p.context; i += StepThreads)
         reinterpret_cast<float2 *>(shared + at.rope)[i] = p.rope[i];
-    grid_dependency_wait(); // the weights and the step count of the update before this step
 
-    // ---- a tile's bytes and the embeddings of its tokens (into the attention gradients' memory), one thread per row ----
-    auto fetch_tokens = [&](int tile) {
+    // ---- a tile's bytes, one thread per row; then the embeddings of its tokens, into the attention gradients' memory ----
+    auto fetch_bytes = [&](int tile) {
         const int r = threadIdx.x, first_sequence = tile * p.sequences, valid = min(p.sequences, p.batch - first_sequence) * p.context;
-        if (r >= p.rows)
-            return;
-        int x = 0, y = 0;
-        if (r < valid) {
+        int x = -1, y = 0;
+        if (r < valid && r < p.rows) {
             if (p.data) { // endpoint = lo + hash(seed + step * batch + sequence) % (size - lo), see sample_kernel
                 const int64_t lo = p.context > 8 ? p.context : 8;
-                const uint64_t seed = p.seed + uint64_t(p.counters->step) * uint64_t(p.batch) + uint64_t(first_sequence + r / p.context);
+                const uint64_t seed = p.seed + __ldcg(&p.counters->step) * uint64_t(p.batch) + uint64_t(first_sequence + r / p.context);
                 const uint8_t *source = p.data + lo + (long long)(hash_u64(seed) % uint64_t(p.data_size - lo)) - p.context + r % p.context;
                 x = source[0], y = source[1];
             } else {
                 x = p.x[int64_t(first_sequence) * p.context + r], y = p.y[int64_t(first_sequence) * p.context + r];
             }
+        }
+        if (r < p.rows)
+            xs[r] = uint8_t(max(x, 0)), ys[r] = uint8_t(y);
+        return x;
+    };
+    auto fetch_embeddings = [&](int x) {
+        if (x >= 0)
 #pragma unroll
             for (int half = 0; half < 2; ++half)
-                copy_async<16>(base + at.dy + r * 32 + half * 16, p.weight_high + x * Width + half * 8);
-        }
-        xs[r] = uint8_t(x), ys[r] = uint8_t(y);
+                copy_async<16>(base + at.dy + threadIdx.x * 32 + half * 16, p.weight_high + x * Width + half * 8);
     };
-    fetch_tokens(blockIdx.x);
+    // The bytes are found while the update before this step runs: the step's number is counted up by the reduction before that update, which has ended
+    // when the update lets this kernel start.
+    const int first_byte = fetch_bytes(blockIdx.x);
+    grid_dependency_wait(); // the weights of the update before this step
+    fetch_embeddings(first_byte);
 
     // ---- weights to shared memory; they are awaited before the first product ----
     const int final_norm = Layer0 + p.depth * LayerParameters, head = final_norm + Width, head_rows = p.depth * LayerRows;
@@ -520,7 +526,7 @@ __global__ void __launch_bounds__(StepThreads, 1) reference_step_kernel(const __
         const int64_t token0 = int64_t(first_sequence) * p.context;
         if (accumulate) {
             __syncthreads(); // the previous tile has been read
-            fetch_tokens(tile);
+            fetch_embeddings(fetch_bytes(tile));
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
@@ -1021,7 +1027,7 @@ struct ReduceParams {
     float *gradient, *norm_partial;
     const float *token_losses;
     float *history;
-    const StepCounters *counters;
+    StepCounters *counters;
     int batch, context;
 };
 __global__ void __launch_bounds__(256) reduce_gradients_kernel(const __grid_constant__ ReduceParams p) {
@@ -1029,6 +1035,12 @@ __global__ void __launch_bounds__(256) reduce_gradients_kernel(const __grid_cons
     __shared__ double loss_sums[8];
     grid_launch_dependents();
     grid_dependency_wait();
+    // The step's number is read by the step kernel, which has ended, and by the update, which knows that it has been counted up; the update in turn
+    // counts the rows of losses, which only this kernel reads.  (The update's last block counted both by a ticket, a microsecond at its end, and the bytes'
+    // chain of loads began after it: 64 tokens 31.5 -> 30.2 us a step, 11520 tokens 50.6 -> 49.5.  More of the rows below at a time: 1.4 us slower, the code
+    // being fetched anew for every step.)
+    if (blockIdx.x == 0 && threadIdx.x == 255)
+        p.counters->step += 1;
     if (int(blockIdx.x) >= p.gradient_blocks) {
         const int position = blockIdx.x - p.gradient_blocks;
         double total = 0;
