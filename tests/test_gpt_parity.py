@@ -613,6 +613,32 @@ def test_predict_runs_one_sequence_and_matches_the_batched_forward():
     assert relative(logits, expected) <= 1e-2
 
 
+@pytest.mark.parametrize("depth,width,context,batch,swiglu", [
+    (2, 64, 72, 1, False),    # one K block of 64, fewer than the ring holds
+    (3, 448, 200, 3, True),   # seven
+    (2, 768, 129, 2, False),  # more than the ring holds
+    (2, 1024, 1300, 8, True)])  # pairs of thread blocks, several tiles to each
+def test_weights_fetched_ahead_in_evaluation(depth, width, context, batch, swiglu):
+    """Calls without gradients fetch a product's weights while the kernel before it ends, calls with gradients do not: the logits are
+    the same bits, and those of the weights set last."""
+    rng = np.random.default_rng(width)
+    ex = ConfigEx.gpt(Config(depth=depth, context=context, batch=batch), width, width // 64)
+    if swiglu:
+        ex.mlp = bridge.MLP_SWIGLU
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    with Native(ex) as engine:
+        w = rng.standard_normal(engine.count).astype(np.float32) * .05
+        for i in range(3):
+            engine.set_weights(w * (1 + i))
+            evaluated, again = engine.batch(x, y, backward=False)[0], engine.batch(x, y, backward=False)[0]
+            expected = engine.batch(x, y)[0]
+            np.testing.assert_array_equal(evaluated, again)
+            np.testing.assert_array_equal(evaluated, expected)
+            # One sequence alone may take other splits of K: the residual stream is stored 2 depth + 1 times, and each time a value
+            # may round to the next of BF16 (2^-8).
+            assert relative(engine.predict(x[0]), expected[0, -1]) <= (2 * depth + 1) ** .5 * 2 ** -8
+
+
 @pytest.mark.parametrize("context,batch", [(200, 3), (72, 5)])
 def test_ragged_context_on_the_tensor_core_path(context, batch):
     """Contexts off the 128-row attention tile and the 64-key step, odd batch, head size 64 (the tcgen05

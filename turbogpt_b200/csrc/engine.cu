@@ -517,6 +517,7 @@ void Engine::forward(bool want_gradient, bool dump_logits, bool embedded) {
         GemmArgs qkv;
         qkv.a = a.normed1, qkv.a_row = W, qkv.b = weight(p.qkv), qkv.b_row = W, qkv.c = a.qkv, qkv.ldc = 3 * W;
         qkv.m = M, qkv.n = 3 * W, qkv.k = W, qkv.out = act;
+        qkv.b_settled = !want_gradient; // the embedding, at least, lies between the weights and what wrote them
         gemm(FGemmForward, qkv);
         if (c.rope == TG_ROPE_PARTIAL)
             run(FMisc, [&](cudaStream_t s) { launch_rope(act, a.qkv, M, T, W, H, false, s); });
@@ -538,11 +539,13 @@ void Engine::forward(bool want_gradient, bool dump_logits, bool embedded) {
         proj.a = a.attended, proj.a_row = W, proj.b = weight(p.attention), proj.b_row = W, proj.c = a.middle;
         proj.ldc = W, proj.m = M, proj.n = W, proj.k = W, proj.out = act;
         proj.epilogue = Epilogue::Residual, proj.r = a.x, proj.ldr = W;
+        proj.b_settled = !want_gradient;
         gemm(FGemmForward, proj);
         norm(a.middle, p.mlp_norm, p.mlp_norm_bias, a.normed2, a.stats2);
         GemmArgs up;
         up.a = a.normed2, up.a_row = W, up.b = weight(p.gate), up.b_row = W, up.c = a.wide, up.m = M, up.k = W;
         up.out = act;
+        up.b_settled = !want_gradient;
         if (c.mlp == TG_MLP_SWIGLU) { // gate and up are adjacent: one projection computes both
             up.n = 2 * Hd, up.ldc = 2 * Hd;
             gemm(FGemmForward, up);
@@ -557,12 +560,14 @@ void Engine::forward(bool want_gradient, bool dump_logits, bool embedded) {
         down.a = a.activated, down.a_row = Hd, down.b = weight(p.down), down.b_row = Hd, down.c = next;
         down.ldc = W, down.m = M, down.n = W, down.k = Hd, down.out = act;
         down.epilogue = Epilogue::Residual, down.r = a.middle, down.ldr = W;
+        down.b_settled = !want_gradient;
         gemm(FGemmForward, down);
     }
     norm(final_x, layout.final_norm, layout.final_norm_bias, final_normed, final_stats);
     GemmArgs head;
     head.a = final_normed, head.a_row = W, head.b = weight(layout.head), head.b_row = W, head.c = logits;
     head.ldc = Vocabulary, head.m = M, head.n = Vocabulary, head.k = W, head.out = act;
+    head.b_settled = !want_gradient;
     const float divisor = float(int64_t(B) * c.world * T);
     // Training steps take the loss and its gradient from the head product's FP32 accumulators (the reference
     // fuses them the same way, cuda/model.cuh:31-58); calls that return logits run the two kernels.

@@ -162,7 +162,7 @@ __device__ __forceinline__ Item locate(const TcParams &p, int work, int n_tiles,
 // cta_group::2 MMAs issued by the pair's first CTA.  Each CTA stages its own 128 rows of A and half
 // of the B tile (the tensor core reads the other half from the partner's shared memory), so a
 // K block costs each SM 16 KB + BN/2 x 128 B instead of 16 KB + BN x 128 B and the ring is deeper.
-template <int Kind, bool OutFp32, bool Pair, int EpilogueWarps>
+template <int Kind, bool OutFp32, bool Pair, int EpilogueWarps, bool EarlyB = false>
 __global__ void __launch_bounds__(threads_of(EpilogueWarps), EpilogueWarps == 8 ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcParams p) {
     extern __shared__ uint8_t raw_shared[];
@@ -213,7 +213,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // Barriers, tensor memory and descriptors are set up; only now wait for the kernel before this one
     // (its tail overlaps the set-up above when this kernel was launched programmatically).
     grid_launch_dependents();
-    grid_dependency_wait();
+    if (!EarlyB || warp != 0)
+        grid_dependency_wait();
 
     // Tiles along M are scheduled per CTA pair; m_tiles counts 128-row tiles including padding.
     const int m_tiles = ((p.m + BM * Unit - 1) / (BM * Unit)) * Unit, n_tiles = (p.n + p.bn - 1) / p.bn;
@@ -233,6 +234,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int b_boxes = p.b_mn ? bn_local / 64 : 1;
             int stage = 0;
             uint32_t phase = 0;
+            auto load = [&](uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+                if constexpr (Pair)
+                    tma_load_3d_pair(dst, map, x, y, z, bar);
+                else
+                    tma_load_3d(dst, map, x, y, z, bar);
+            };
+            // A weight is there before the activations that it multiplies: the ring's first round of it is fetched while the kernel before this one ends.
+            int early = 0; // K blocks whose B is on its way
+            if constexpr (EarlyB) {
+                if (first_item < work_items) {
+                    const Item item = locate(p, first_item, n_tiles, m_units, Unit, int(rank));
+                    const int n_first = item.nt * p.bn + int(rank) * bn_local;
+                    int bx = p.b_mn ? n_first : 0, by = p.b_mn ? 0 : n_first;
+                    for (const int most = min(p.stages, k_blocks); early < most; ++early) {
+                        const uint32_t sb = base + early * stage_bytes + StageABytes, bar = landed0 + 8 * early;
+                        if (rank == 0)
+                            mbarrier_expect_tx(full0 + 8 * early, stage_tx);
+                        for (int j = 0; j < b_boxes; ++j)
+                            load(sb + j * 64 * BK * 2, &map_b, bx + j * 64, by, item.z, bar);
+                        bx += b_dx, by += b_dy;
+                    }
+                }
+                grid_dependency_wait();
+            }
             for (int w = first_item; w < work_items; w += item_stride) {
                 const Item item = locate(p, w, n_tiles, m_units, Unit, int(rank));
                 const int kb0 = item.split * p.k_blocks_per_split;
@@ -241,25 +266,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 int ax = p.a_mn ? m_first : kb0 * BK, ay = p.a_mn ? kb0 * BK : m_first;
                 int bx = p.b_mn ? n_first : kb0 * BK, by = p.b_mn ? kb0 * BK : n_first;
                 bool ok = true;
-                for (int kb = kb0; kb < kb1; ++kb) {
+                int kb = kb0;
+                if constexpr (EarlyB) {
+                    for (; early; --early, ++kb) { // nothing has used these stages yet
+                        const uint32_t sa = base + stage * stage_bytes, bar = landed0 + 8 * stage;
+                        load(sa, &map_a, ax, ay, z, bar);
+                        if (p.a_mn)
+                            load(sa + 64 * BK * 2, &map_a, ax + 64, ay, z, bar);
+                        ax += a_dx, ay += a_dy, bx += b_dx, by += b_dy;
+                        if (++stage == p.stages) {
+                            stage = 0;
+                            phase ^= 1;
+                        }
+                    }
+                }
+                for (; kb < kb1; ++kb) {
                     ok = mbarrier_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, p.counters, 101);
                     if (!ok)
                         break;
                     const uint32_t sa = base + stage * stage_bytes, sb = sa + StageABytes, bar = landed0 + 8 * stage;
                     if (rank == 0)
                         mbarrier_expect_tx(full0 + 8 * stage, stage_tx);
-                    auto load = [&](uint32_t dst, const CUtensorMap *map, int x, int y) {
-                        if constexpr (Pair)
-                            tma_load_3d_pair(dst, map, x, y, z, bar);
-                        else
-                            tma_load_3d(dst, map, x, y, z, bar);
-                    };
-                    load(sa, &map_a, ax, ay);
+                    load(sa, &map_a, ax, ay, z, bar);
                     if (p.a_mn)
-                        load(sa + 64 * BK * 2, &map_a, ax + 64, ay);
-                    load(sb, &map_b, bx, by);
+                        load(sa + 64 * BK * 2, &map_a, ax + 64, ay, z, bar);
+                    load(sb, &map_b, bx, by, z, bar);
                     for (int j = 1; j < b_boxes; ++j)
-                        load(sb + j * 64 * BK * 2, &map_b, bx + j * 64, by);
+                        load(sb + j * 64 * BK * 2, &map_b, bx + j * 64, by, z, bar);
                     ax += a_dx, ay += a_dy, bx += b_dx, by += b_dy;
                     if (++stage == p.stages) {
                         stage = 0;
@@ -995,11 +1028,21 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
         if (p.out_fp32) {
             launch(gemm_tc_kernel<int(Epilogue::Store), true, P, 16>);
         } else {
+            // Few rows: a product is hardly longer than the fetch of its weights, and most of that is hidden (tg_predict 12 layers d 768
+            // 636 -> 624 us, 16 layers d 640, 74 tokens 572 -> 547, 2 layers d 896, 1381 tokens 187 -> 181).  In the training step, where
+            // products are long, the same costs more than it gives (4 layers d 256, 2048 tokens: 343 -> 346 us a step): the engine does not ask for it there.
+            const bool early = g.b_settled && p.splits == 1;
             switch (g.epilogue) {
-            case Epilogue::Store: launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16>); break;
-            case Epilogue::Residual: launch(gemm_tc_kernel<int(Epilogue::Residual), false, P, 16>); break;
+            case Epilogue::Store:
+                early ? launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16, true>) : launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16>);
+                break;
+            case Epilogue::Residual:
+                early ? launch(gemm_tc_kernel<int(Epilogue::Residual), false, P, 16, true>) : launch(gemm_tc_kernel<int(Epilogue::Residual), false, P, 16>);
+                break;
             case Epilogue::GeluDual: launch(gemm_tc_kernel<int(Epilogue::GeluDual), false, P, 16>); break;
-            case Epilogue::Gelu: launch(gemm_tc_kernel<int(Epilogue::Gelu), false, P, 16>); break;
+            case Epilogue::Gelu:
+                early ? launch(gemm_tc_kernel<int(Epilogue::Gelu), false, P, 16, true>) : launch(gemm_tc_kernel<int(Epilogue::Gelu), false, P, 16>);
+                break;
             case Epilogue::GeluGrad: launch(gemm_tc_kernel<int(Epilogue::GeluGrad), false, P, 16>); break;
             case Epilogue::Axpby: launch(gemm_tc_kernel<int(Epilogue::Axpby), false, P, 16>); break;
             case Epilogue::CrossEntropy: launch(gemm_tc_kernel<int(Epilogue::CrossEntropy), false, P, 16>); break;

@@ -190,6 +190,8 @@ struct GemmArgs {
     float alpha = 1.f, beta = 0.f;
     int batch = 1;           // batched over z with element strides below
     int64_t a_batch = 0, b_batch = 0, c_batch = 0, r_batch = 0;
+    bool b_settled = false;  // B was written before the kernel that precedes this one in the stream began: it may be read while that one runs
+                             // (plain, residual and GELU products of BF16 results do so)
     bool beside_others = false; // other lanes' products run at the same time: leave them half of an SM where that is enough
 };
 // `scratch`: gemm_simt_scratch_bytes(g) bytes for shapes that are cut along K (small outputs over a long K,
