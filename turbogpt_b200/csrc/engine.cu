@@ -121,9 +121,9 @@ void Engine::initialize() {
     // 12 layers d 768, 4096 tokens 1 %, 8192 tokens level; 8 layers d 640, 8192 tokens and 14 layers d 960, 8192 tokens 0.2 and 0.7 % slower.  Three: slower
     // than two everywhere (361 -> 369 us).
     const int64_t work = int64_t(tokens) * c.width;
-    // FP32 products fill the GPU from width 64 on, and a second lane of them is in the chain's way: training steps, one lane -> two, 4 layers d 256,
-    // 2048 tokens 2065 -> 2142 us, 2 layers d 768, 1024 tokens 3150 -> 3357, 4 layers d 64, 4096 tokens 1101 -> 1133; the widths of the reference
-    // architecture leave it idle over many tokens: 4 layers d 16, 64 tokens 560 -> 567, 256 tokens 1127 -> 725, 11520 tokens 1096 -> 973.
+    // FP32 products fill the GPU from width 64 on, and a second lane of them is in the chain's way (training steps, one lane -> two, level to 4 %
+    // longer; no lane at all 5 to 15 %); the widths of the reference architecture, on CUDA cores, leave it idle over many tokens: 4 layers d 16, 64 tokens
+    // 560 -> 567 us, 256 tokens 1127 -> 725, 11520 tokens 1096 -> 973.
     const bool second = work <= TwoSideLanes && (act == Dtype::BF16 || (c.width < 64 && tokens >= 256));
     side_lanes = !concurrent || work > int64_t(1) << 24 ? 0 : second ? 2 : 1;
     muon_lanes = concurrent && c.hidden_optimizer == TG_HIDDEN_MUON && int64_t(c.base.depth) * c.width * c.width <= int64_t(1) << 22;

@@ -47,10 +47,10 @@ constexpr int RowScratchBytes = 2 * 4 * BM * 4; // CrossEntropy: row maxima and 
 constexpr int MaxShared = 232448 - 1024; // 227 KB less the runtime's own reservation
 // Where the caller says that others run beside it (GemmArgs::beside_others), a batched product of at most one tile per SM, up to 128
 // columns wide, runs in half an SM: eight epilogue warps, one accumulator of its own width, and a ring of half the shared memory.
-// Those are Muon's Newton-Schulz products when the families' chains run beside each other on four lanes: of 60 in a step of 6 layers
-// d 384 the 45 of 128 columns, 108 blocks each, which as whole SMs are kept waiting for one another (4 steps 5400 -> 5150 us, eight
-// optimizer steps alone 4.56 -> 3.82 ms, 6 layers d 320 3.92 -> 3.10, the same bits; two blocks to an SM above one tile per SM measured level).  Products in a chain of their own, a sharded or profiled
-// optimizer's among them, keep the deep ring: tg_predict of 12 layers d 768 takes 838 us with halves, 735 without.  Every kernel that takes tensor memory lets its
+// Measured with Newton-Schulz products as launches of their own, four chains of them beside each other: of 60 in a step of 6 layers
+// d 384 the 45 of 128 columns, 108 blocks each, as whole SMs were kept waiting for one another (eight optimizer steps
+// 4.56 -> 3.82 ms, 6 layers d 320 3.92 -> 3.10, the same bits; two blocks to an SM above one tile per SM measured level).  Products in a chain of their own,
+// a sharded optimizer's among them, keep the deep ring: tg_predict of 12 layers d 768 takes 838 us with halves, 735 without.  Every kernel that takes tensor memory lets its
 // dependents launch only once it holds it, so none can wait for columns that a kernel waiting for it holds.
 constexpr int HalfShared = 113 * 1024;
 
