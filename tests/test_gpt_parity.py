@@ -617,9 +617,10 @@ def test_predict_runs_one_sequence_and_matches_the_batched_forward():
     (2, 64, 72, 1, False),    # one K block of 64, fewer than the ring holds
     (3, 448, 200, 3, True),   # seven
     (2, 768, 129, 2, False),  # more than the ring holds
+    (1, 1024, 512, 4, False),   # one tile to a thread block or pair in some products, several in others
     (2, 1024, 1300, 8, True)])  # pairs of thread blocks, several tiles to each
 def test_weights_fetched_ahead_in_evaluation(depth, width, context, batch, swiglu):
-    """Calls without gradients fetch a product's weights while the kernel before it ends, calls with gradients do not: the logits are
+    """Calls without gradients fetch a product's weights while the kernel before it ends where a block has one tile, calls with gradients do not: the logits are
     the same bits, and those of the weights set last."""
     rng = np.random.default_rng(width)
     ex = ConfigEx.gpt(Config(depth=depth, context=context, batch=batch), width, width // 64)

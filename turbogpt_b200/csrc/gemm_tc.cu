@@ -1028,10 +1028,11 @@ void launch_schedule(const GemmArgs &g, const Schedule &sc, int sms, float *part
         if (p.out_fp32) {
             launch(gemm_tc_kernel<int(Epilogue::Store), true, P, 16>);
         } else {
-            // Few rows: a product is hardly longer than the fetch of its weights, and most of that is hidden (tg_predict 12 layers d 768
-            // 636 -> 624 us, 16 layers d 640, 74 tokens 572 -> 547, 2 layers d 896, 1381 tokens 187 -> 181).  In the training step, where
-            // products are long, the same costs more than it gives (4 layers d 256, 2048 tokens: 343 -> 346 us a step): the engine does not ask for it there.
-            const bool early = g.b_settled && p.splits == 1;
+            // A CTA's only tile: the product is hardly longer than the fetch of its weights, and most of that is hidden (tg_predict 12 layers d 768
+            // 636 -> 624 us, 16 layers d 640, 74 tokens 572 -> 547, 2 layers d 896, 1381 tokens 187 -> 181).  With further tiles to come it is level or costs
+            // more than it gives (evaluation of 6 layers d 512, 4096 tokens 366 -> 377), as it does in the training step, where the engine does not ask for
+            // it (4 layers d 256, 2048 tokens: 343 -> 346 us a step).
+            const bool early = g.b_settled && p.splits == 1 && work <= slots;
             switch (g.epilogue) {
             case Epilogue::Store:
                 early ? launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16, true>) : launch(gemm_tc_kernel<int(Epilogue::Store), false, P, 16>);
