@@ -152,6 +152,7 @@ struct Engine {
         float values[16384];
     } *mailbox = nullptr;
     bool mailbox_pinned = false;
+    int finishes = 0; // up to two
     bool announce_gradients = false;
     StepGraph graphs[GraphKinds];
     int forward_batch = 0; // sequences the next forward pass covers (0: the configured batch)
