@@ -13,7 +13,9 @@ struct Copy {
 static std::deque<Copy> queue;
 static size_t made = 0, queued = 0;
 static std::map<void *, size_t> recorded;
-static int calls = 0, failing = 0, waits = 0, handles = 0;
+static int calls = 0, failing = 0, waits = 0, handles = 0, calls_in_own_mode = 0;
+static std::atomic<int> wrong_at_once{0};
+static thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
 static std::atomic<int> alive{0};
 static bool fails() { return ++calls == failing; }
 static void make(size_t until) {
@@ -21,8 +23,11 @@ static void make(size_t until) {
         memcpy(queue.front().to, queue.front().from, queue.front().bytes);
 }
 extern "C" {
-cudaError_t cudaSetDevice(int) { return fails() ? cudaErrorInvalidDevice : cudaSuccess; }
-cudaError_t cudaHostRegister(void *, size_t, unsigned) { return fails() ? cudaErrorMemoryAllocation : (++alive, cudaSuccess); }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) { return std::swap(*m, mode), cudaSuccess; }
+cudaError_t cudaHostRegister(void *, size_t, unsigned) {
+    calls_in_own_mode += mode != cudaStreamCaptureModeRelaxed; // would end another thread's capture
+    return fails() ? cudaErrorMemoryAllocation : (++alive, cudaSuccess);
+}
 cudaError_t cudaHostUnregister(void *) { return --alive, cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
     if (fails())
@@ -45,12 +50,6 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "refused"; }
 }
 
-static bool ready(ResultCopies &c) { // once the ring has been made, or not
-    while (c.making())
-        std::this_thread::yield();
-    return c.ready();
-}
-
 int main() {
     int wrong = 0;
     constexpr size_t Slice = ResultCopies::SliceBytes;
@@ -65,18 +64,18 @@ int main() {
         }
         for (size_t i = 0; i < sizes.size(); ++i)
             segments.push_back({to[i].data(), from[i].data(), sizes[i], nullptr, i % 2 ? event : nullptr});
-        c.run(segments.data(), segments.size(), segments.data(), map ? segments.size() : 0);
-        wrong += from != to;
+        const bool done = c.run(segments.data(), segments.size(), segments.data(), map ? segments.size() : 0);
+        wrong += done && from != to;
+        return done;
     };
     const std::vector<std::vector<size_t>> calls_of = {{1}, {Slice}, {Slice - 1, Slice + 1}, {0, 5, 0, 3 * Slice + 7},
                                                        {ResultCopies::Slices * Slice, 1}, {2 * ResultCopies::Slices * Slice + 13, Slice / 2, 40 * Slice + 1}};
     for (int threads = 1; threads <= ResultCopies::MostThreads; ++threads) {
         ResultCopies c;
-        c.begin(threads, 0), c.begin(threads, 0);
-        wrong += !ready(c) || !ready(c);
+        wrong += !c.create(threads);
         for (int round = 0; round < 3; ++round)
             for (const auto &sizes : calls_of)
-                run(c, sizes, unsigned(round * 7 + threads), round == 1);
+                wrong += !run(c, sizes, unsigned(round * 7 + threads), round == 1);
         wrong += !queue.empty();
         for (int n : {1, 3, int(ResultCopies::Slices) + 5}) { // the n-th copy is refused: reported, and the next call is as ever
             calls = 0, failing = n;
@@ -92,21 +91,47 @@ int main() {
             run(c, {30 * Slice + 1, 17}, 2, false);
         }
     }
-    for (int n = 1; n <= 2 + int(ResultCopies::Slices); ++n) { // the n-th creation is refused: nothing is left, and the next one serves
+    for (int n = 1; n <= 1 + int(ResultCopies::Slices); ++n) { // the n-th creation is refused: nothing is left, and the next one serves
         ResultCopies c;
         calls = 0, failing = n;
-        c.begin(2, 0);
-        wrong += ready(c) || alive;
+        wrong += c.create(2) || alive;
         failing = 0;
-        c.begin(2, 0);
-        wrong += !ready(c);
+        wrong += !c.create(2);
         run(c, {Slice + 3}, 5, false);
         c.destroy(), c.destroy();
         wrong += alive;
     }
-    ResultCopies none;
-    none.begin(0, 0);
-    wrong += none.ready() || ResultCopies::threads_for(3) || ResultCopies::threads_for(4) != 1 || ResultCopies::threads_for(200) != ResultCopies::MostThreads;
+    { // made when it is worth it, shared, given back with its last owner; a call that finds it in use does without
+        const auto of = [](int device, size_t bytes) { return ResultCopies::of(device, bytes, 2); };
+        wrong += of(3, ResultCopies::Worth - 1) || of(4, 1);
+        auto a = of(3, 1), b = of(3, 0), other = of(4, ResultCopies::Worth - 1);
+        wrong += !a || a != b || !other || other == a;
+        std::atomic<int> refused{0}, done{0};
+        std::vector<std::thread> engines;
+        for (int i = 0; i < 4; ++i)
+            engines.emplace_back([&, i, ring = of(3, 0)] {
+                std::vector<uint8_t> from(3 * Slice + i, uint8_t(i + 1)), to(from.size());
+                const ResultCopies::Segment segment{to.data(), from.data(), from.size(), nullptr, nullptr};
+                for (int call = 0; call < 50; ++call) {
+                    std::fill(to.begin(), to.end(), uint8_t(0));
+                    const bool ran = ring->run(&segment, 1, nullptr, 0);
+                    ++(ran ? done : refused);
+                    wrong_at_once += ran ? from != to : to != std::vector<uint8_t>(to.size());
+                }
+            });
+        for (std::thread &t : engines)
+            t.join();
+        wrong += wrong_at_once || done + refused != 200 || !done;
+        a.reset();
+        wrong += of(3, 0) != b;
+        b.reset(), other.reset();
+        wrong += alive || of(3, 1);
+        calls = 0, failing = 1; // refused for good
+        wrong += of(3, ResultCopies::Worth) || of(3, ResultCopies::Worth) || calls != 1;
+        failing = 0;
+    }
+    wrong += ResultCopies::of(5, ResultCopies::Worth, 0) || ResultCopies::of(-1, ResultCopies::Worth, 1) || alive;
+    wrong += calls_in_own_mode || ResultCopies::threads_for(3) || ResultCopies::threads_for(4) != 1 || ResultCopies::threads_for(200) != ResultCopies::MostThreads;
     printf("wrong %d alive %d waits %d\n", wrong, alive.load(), waits > 0);
     return 0;
 }

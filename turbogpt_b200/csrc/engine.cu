@@ -326,7 +326,7 @@ void Engine::release() {
     for (cudaEvent_t ev : fork_events)
         cudaEventDestroy(ev);
     copies.destroy();
-    results.destroy();
+    results.reset();
     if (mailbox_pinned)
         cudaHostUnregister(mailbox);
     if (mailbox)
@@ -1071,16 +1071,16 @@ static bool ordinary(const ResultCopies::Segment &s) {
     }
     return true;
 }
-// Whether a call's results go through the ring: arrays in ordinary memory only, a megabyte of them together.  Small results are there as
+// Bytes of a call's results where they may go through the ring: arrays in ordinary memory only, a megabyte of them together.  Small results are there as
 // soon by the driver's way.
-static bool through_ring(const std::vector<ResultCopies::Segment> &arrays) {
+static size_t for_the_ring(const std::vector<ResultCopies::Segment> &arrays) {
     size_t bytes = 0;
     for (const ResultCopies::Segment &s : arrays) {
         if (!ordinary(s))
-            return false;
+            return 0;
         bytes += s.bytes;
     }
-    return bytes >= size_t(1) << 20;
+    return bytes >= size_t(1) << 20 ? bytes : 0;
 }
 
 // With gradients, the results leave while the GPU is at work: the logits during the backward pass, the gradients in pieces of two
@@ -1108,7 +1108,7 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
         segments.push_back({gradient_out, gradient, size_t(left) * 4, stream, nullptr});
         arrays.push_back({gradient_out, gradient, gradient_bytes, stream, nullptr});
     }
-    const bool large = through_ring(arrays);
+    const size_t large = for_the_ring(arrays);
     CHECK_CUDA(cudaMemcpyAsync(x, bx, tokens, cudaMemcpyHostToDevice, stream));
     CHECK_CUDA(cudaMemcpyAsync(y, by, tokens, cudaMemcpyHostToDevice, stream));
     replay(gradient_out ? GraphGradients : GraphEvaluate,
@@ -1116,9 +1116,9 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
     // Of 32 MB and more the C library maps an array afresh each time; smaller ones mostly lie in memory that it has kept.
     auto kept = [](const ResultCopies::Segment &s) { return s.bytes < size_t(32) << 20 || !ordinary(s); };
     arrays.erase(std::remove_if(arrays.begin(), arrays.end(), kept), arrays.end());
-    if (large && results.ready()) {
-        results.run(segments.data(), segments.size(), arrays.data(), arrays.size());
-    } else {
+    if (large && !results)
+        results = ResultCopies::of(config.base.device, large, ResultCopies::threads_for(std::thread::hardware_concurrency()));
+    if (!large || !results || !results->run(segments.data(), segments.size(), arrays.data(), arrays.size())) {
         for (const ResultCopies::Segment &s : arrays) // while the GPU computes (first calls: 76 MB 19.2 -> 16.1 ms, 340 MB 78 -> 59)
             ResultCopies::map_pages(s.to, s.bytes);
         for (const ResultCopies::Segment &s : segments) {
@@ -1130,8 +1130,6 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
             CHECK_CUDA(cudaStreamSynchronize(copies.stream)); // a pinned array's copy returns before it is done
     }
     finish(losses.data(), token_losses, size_t(tokens));
-    if (large) // for the next call
-        results.begin(ResultCopies::threads_for(std::thread::hardware_concurrency()), config.base.device);
     if (per_position)
         for (int p = 0; p < T; ++p) { // reference cuda/runtime.cu:279-290
             double sum = 0;

@@ -146,7 +146,7 @@ struct Engine {
     size_t next_fork_event = 0;
     float *simt_scratch[3] = {nullptr, nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
     BatchCopies copies; // of tg_batch's results
-    ResultCopies results; // into ordinary memory, from the second call on that has use for them
+    std::shared_ptr<ResultCopies> results; // the device's, once a call has had use for it
     struct Mailbox { // pinned: what a call brings back with its last wait
         StepCounters counters;
         float values[16384];

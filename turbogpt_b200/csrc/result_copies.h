@@ -2,13 +2,15 @@
 // host threads empty into the caller's arrays, both while the GPU is still computing.  The driver's own copy into such memory does
 // the two in turn on the calling thread (15 MB in 0.65 to 0.75 ms, 21 GB/s, of a call whose kernels take 0.48).  tg_batch, the driver's
 // way and this: 2 MB of results 305 and 256 us, 6 MB 620 and 385, 15 MB 1290 and 600, 31 MB 2220 and 1080, 80 MB 13.3 and 4.2 ms, 345 MB 56 and
-// 18.5 ms (from 32 MB on the C library maps an array afresh for every call, and the threads take its page faults).  The first call that would have had
-// use for it starts the threads when it is done, and one of them makes the ring: as part of that call it took 0.5 to 1 ms of two.
+// 18.5 ms (from 32 MB on the C library maps an array afresh for every call, and the threads take its page faults).
+//
+// Making the ring takes 1.5 ms, giving it back 0.5, so that it is shared by a device's engines, belongs to those that have used it, and is made by the call that
+// brings the results that left the driver's way to 32 MB, while that call's kernels run (made for every engine: second calls of 2 to 15 MB 1.0 -> 3.1 and
+// 2.6 -> 4.2 ms).
 #pragma once
 #include "common.h"
 #include <atomic>
 #include <condition_variable>
-#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -22,6 +24,7 @@ class ResultCopies {
     // 24 and 32 of half the size 735 us and 20.1 ms, 680 us and 19.6.
     static constexpr size_t SliceBytes = size_t(1) << 19, Slices = 16;
     static constexpr int MostThreads = 4;
+    static constexpr size_t Worth = size_t(32) << 20; // 40 us are saved for every megabyte
 
     struct Segment { // to[0, bytes) = from, device memory that is complete on `stream` after `ready` (null: after what `stream` holds)
         void *to;
@@ -38,49 +41,57 @@ class ResultCopies {
     ResultCopies(const ResultCopies &) = delete;
     ~ResultCopies() { destroy(); }
 
-    // Starts a thread that makes the ring and starts the others; the caller does not wait for it.  Nothing where it is there already.  (The caller
-    // starting all four while the first maps the ring: 50 to 180 us of a call of 0.6 to 2.2 ms.)
-    void begin(int thread_count, int device) {
-        if (maker.joinable() || thread_count < 1)
-            return;
-        state = Making;
+    // The ring of a device, made now where that is worth its time; null: `bytes` of results take the driver's way.  The current device is the one meant.
+    static std::shared_ptr<ResultCopies> of(int device, size_t bytes, int thread_count) {
+        struct Entry {
+            std::mutex mutex;
+            std::weak_ptr<ResultCopies> ring;
+            size_t passed = 0; // bytes since there was no ring
+            bool refused = false;
+        };
+        constexpr int Devices = 64;
+        static Entry *const entries = new Entry[Devices]; // outlives every engine
+        if (device < 0 || device >= Devices || thread_count < 1)
+            return nullptr;
+        Entry &entry = entries[device];
+        std::unique_lock<std::mutex> lock(entry.mutex, std::try_to_lock);
+        if (!lock) // another engine is making it
+            return nullptr;
+        if (std::shared_ptr<ResultCopies> ring = entry.ring.lock())
+            return ring;
+        if (entry.refused || (entry.passed += bytes) < Worth)
+            return nullptr;
+        entry.passed = 0;
+        auto ring = std::make_shared<ResultCopies>();
+        entry.refused = !ring->create(thread_count); // is not tried again
+        if (entry.refused)
+            return nullptr;
+        entry.ring = ring;
+        return ring;
+    }
+    // Ring, events and threads, or nothing.
+    bool create(int thread_count) {
+        bool made = make();
         try {
-            maker = std::thread([this, device, thread_count] {
-                const bool made = make(device);
-                try {
-                    while (made && int(others.size()) + 1 < thread_count)
-                        others.emplace_back([this] { work(); });
-                } catch (const std::exception &) { // no thread, or no memory for one: those that run will do
-                }
-                state.store(made ? Ready : Failed, std::memory_order_release);
-                work();
-            });
-        } catch (const std::exception &) {
-            state = None;
+            while (made && int(threads.size()) < thread_count)
+                threads.emplace_back([this] { work(); });
+        } catch (const std::exception &) { // no thread, or no memory for one: those that run will do
         }
-    }
-    // Ring, events and threads are there.  (After a failure none of them is, and begin() may try again.)
-    bool ready() {
-        if (!maker.joinable())
-            return false;
-        const State now = state.load(std::memory_order_acquire);
-        if (now == Failed)
+        made = !threads.empty();
+        if (!made)
             destroy();
-        return now == Ready;
+        return made;
     }
-    bool making() const { return state.load(std::memory_order_acquire) == Making; }
     void destroy() {
         {
             std::lock_guard<std::mutex> lock(mutex);
             stopping = true;
         }
         wake.notify_all();
-        if (maker.joinable())
-            maker.join(); // first: until then the others are its to start
-        for (std::thread &t : others)
+        for (std::thread &t : threads)
             t.join();
-        others.clear();
-        stopping = false, state = None;
+        threads.clear();
+        stopping = false;
         for (cudaEvent_t &e : landed) {
             if (e)
                 cudaEventDestroy(e);
@@ -88,8 +99,9 @@ class ResultCopies {
         }
         if (pinned)
             cudaHostUnregister(ring);
-        free(ring);
-        ring = nullptr, pinned = false;
+        if (mapped)
+            munmap(mapped, RingBytes + HugePage);
+        ring = nullptr, mapped = nullptr, pinned = false;
     }
 
     // Has the kernel map pages before the copies into them need them.  Contents are left alone; where the call is not known, the copies take
@@ -104,8 +116,11 @@ class ResultCopies {
     }
 
     // Copies every segment, in order; returns when the last byte is in its place.  `map`: arrays whose pages the threads have the kernel map before
-    // the first results arrive.
-    void run(const Segment *segments, size_t count, const Segment *map, size_t map_count) {
+    // the first results arrive.  False: another engine's call has the ring, and nothing was done.
+    bool run(const Segment *segments, size_t count, const Segment *map, size_t map_count) {
+        std::unique_lock<std::mutex> lease(busy, std::try_to_lock);
+        if (!lease)
+            return false;
         try {
             copy(segments, count, map, map_count);
         } catch (...) { // nothing may be on its way into the ring when the next call uses it
@@ -113,17 +128,21 @@ class ResultCopies {
                 (void)cudaStreamSynchronize(segments[i].stream);
             throw;
         }
+        return true;
     }
 
   private:
-    bool make(int device) {
-        // Huge pages, where there are any, are mapped and pinned in 1 ms; cudaHostAlloc takes 3.5 to 4.5 for eight megabytes.
-        constexpr size_t HugePage = size_t(2) << 20;
-        ring = static_cast<uint8_t *>(aligned_alloc(HugePage, RingBytes));
-        if (ring)
-            (void)madvise(ring, RingBytes, MADV_HUGEPAGE);
-        bool made = ring && cudaSetDevice(device) == cudaSuccess;
-        made = pinned = made && cudaHostRegister(ring, RingBytes, cudaHostRegisterDefault) == cudaSuccess;
+    // Huge pages, where there are any, are mapped and pinned in 1 ms; cudaHostAlloc takes 3.5 to 4.5 for eight megabytes.  Mapped here and not by the C library,
+    // which when it got such a block back might give away the memory that it keeps for the caller's arrays.
+    bool make() {
+        void *memory = mmap(nullptr, RingBytes + HugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        if (memory == MAP_FAILED)
+            return false;
+        mapped = memory;
+        ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(mapped) + HugePage - 1) / HugePage * HugePage);
+        (void)madvise(ring, RingBytes, MADV_HUGEPAGE);
+        RelaxedCapture relaxed;
+        bool made = pinned = cudaHostRegister(ring, RingBytes, cudaHostRegisterDefault) == cudaSuccess;
         for (size_t i = 0; made && i < Slices; ++i)
             if (cudaEventCreateWithFlags(&landed[i], cudaEventDisableTiming) != cudaSuccess)
                 landed[i] = nullptr, made = false;
@@ -210,28 +229,26 @@ class ResultCopies {
                 std::this_thread::yield();
     }
 
-    static constexpr size_t MapBytes = size_t(4) << 20, RingBytes = SliceBytes * Slices;
+    static constexpr size_t MapBytes = size_t(4) << 20, RingBytes = SliceBytes * Slices, HugePage = size_t(2) << 20;
     struct Job { // a copy, or (from null) pages to be mapped
         void *to;
         const void *from;
         size_t bytes;
         std::atomic<bool> done;
     };
+    void *mapped = nullptr;
     uint8_t *ring = nullptr;
     bool pinned = false;
     cudaEvent_t landed[Slices] = {};
-    std::thread maker;
-    std::vector<std::thread> others;
+    std::vector<std::thread> threads;
     std::unique_ptr<Job[]> jobs;
     size_t capacity = 0;
     std::atomic<size_t> next{0}, published{0};
     std::atomic<int> inside{0};
     std::atomic<bool> active{false};
-    std::mutex mutex;
+    std::mutex mutex, busy; // of the threads' state; for the length of a call
     std::condition_variable wake;
     bool stopping = false;
-    enum State { None, Making, Ready, Failed };
-    std::atomic<State> state{None};
 
     bool take_one() {
         size_t i = next.load(std::memory_order_relaxed);
