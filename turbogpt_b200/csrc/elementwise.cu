@@ -936,6 +936,16 @@ void launch_loss_history(const float *token_losses, float *history, const StepCo
                          int context, cudaStream_t s) {
     loss_history_kernel<<<blocks_for(context, 64), 64, 0, s>>>(token_losses, history, counters, batch, context);
 }
+__global__ void __launch_bounds__(256) collect_kernel(const StepCounters *counters, const float *values, int count, Outbox *out) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i == 0)
+        out->counters = *counters;
+    if (i < count)
+        out->values[i] = values[i];
+}
+void launch_collect(const StepCounters *counters, const float *values, int count, Outbox *out, cudaStream_t s) {
+    collect_kernel<<<blocks_for(std::max(count, 1), 256), 256, 0, s>>>(counters, values, count, out);
+}
 
 // ------------------------------------------------------------------------------------------
 // Conversions.

@@ -147,12 +147,8 @@ struct Engine {
     float *simt_scratch[3] = {nullptr, nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
     BatchCopies copies; // of tg_batch's results
     std::shared_ptr<ResultCopies> results; // the device's, once a call has had use for it
-    struct Mailbox { // pinned: what a call brings back with its last wait
-        StepCounters counters;
-        float values[16384];
-    } *mailbox = nullptr;
-    bool mailbox_pinned = false;
-    int finishes = 0; // up to two
+    Outbox *outbox = nullptr;          // what a call brings back with its last wait,
+    std::unique_ptr<Outbox> mailbox;   // and where it arrives
     bool announce_gradients = false;
     StepGraph graphs[GraphKinds];
     int forward_batch = 0; // sequences the next forward pass covers (0: the configured batch)

@@ -159,6 +159,12 @@ void launch_cross_entropy(Dtype t, const CrossEntropyArgs &a, cudaStream_t s);
 // ---- per-position loss history (reference cuda/trainer.cuh:79-100) ----
 void launch_loss_history(const float *token_losses, float *history, const StepCounters *counters, int batch,
                          int context, cudaStream_t s);
+struct Outbox {
+    StepCounters counters;
+    float values[16384];
+};
+// The counters and `count` values into one place, for one copy to the host.
+void launch_collect(const StepCounters *counters, const float *values, int count, Outbox *out, cudaStream_t s);
 
 // ---- GEMM dispatcher: C[m,n] = sum_k A[m,k] * B[n,k] (reference cuda/mma.cuh:77-108,
 //      cuda/ops.cuh:30-55,83-117) ----
