@@ -13,9 +13,8 @@ struct Copy {
 static std::deque<Copy> queue;
 static size_t made = 0, queued = 0;
 static std::map<void *, size_t> recorded;
-static int calls = 0, failing = 0, waits = 0, handles = 0, calls_in_own_mode = 0;
+static int calls = 0, failing = 0, waits = 0, handles = 0;
 static std::atomic<int> wrong_at_once{0};
-static thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
 static std::atomic<int> alive{0};
 static bool fails() { return ++calls == failing; }
 static void make(size_t until) {
@@ -23,11 +22,7 @@ static void make(size_t until) {
         memcpy(queue.front().to, queue.front().from, queue.front().bytes);
 }
 extern "C" {
-cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) { return std::swap(*m, mode), cudaSuccess; }
-cudaError_t cudaHostRegister(void *, size_t, unsigned) {
-    calls_in_own_mode += mode != cudaStreamCaptureModeRelaxed; // would end another thread's capture
-    return fails() ? cudaErrorMemoryAllocation : (++alive, cudaSuccess);
-}
+cudaError_t cudaHostRegister(void *, size_t, unsigned) { return fails() ? cudaErrorMemoryAllocation : (++alive, cudaSuccess); }
 cudaError_t cudaHostUnregister(void *) { return --alive, cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
     if (fails())
@@ -131,7 +126,7 @@ int main() {
         failing = 0;
     }
     wrong += ResultCopies::of(5, ResultCopies::Worth, 0) || ResultCopies::of(-1, ResultCopies::Worth, 1) || alive;
-    wrong += calls_in_own_mode || ResultCopies::threads_for(3) || ResultCopies::threads_for(4) != 1 || ResultCopies::threads_for(200) != ResultCopies::MostThreads;
+    wrong += ResultCopies::threads_for(3) || ResultCopies::threads_for(4) != 1 || ResultCopies::threads_for(200) != ResultCopies::MostThreads;
     printf("wrong %d alive %d waits %d\n", wrong, alive.load(), waits > 0);
     return 0;
 }

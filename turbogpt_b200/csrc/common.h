@@ -16,15 +16,6 @@ inline void check_cuda(cudaError_t error, const char *what = nullptr) {
 }
 #define CHECK_CUDA(expr) check_cuda((expr), #expr)
 
-// While it lives, this thread's calls leave every stream capture in the process alone: registering host memory would otherwise end a global-mode capture,
-// on whatever thread, with an error.  Only for calls that no capture depends on.
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
-    RelaxedCapture(const RelaxedCapture &) = delete;
-    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 // splitmix64 finaliser; defines the data indexing (reference utils.h:13-18) and must be bit-exact.
 __host__ __device__ inline uint64_t hash_u64(uint64_t x) {
     x += 0x9e3779b97f4a7c15ULL;

@@ -141,7 +141,6 @@ class ResultCopies {
         mapped = memory;
         ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(mapped) + HugePage - 1) / HugePage * HugePage);
         (void)madvise(ring, RingBytes, MADV_HUGEPAGE);
-        RelaxedCapture relaxed;
         bool made = pinned = cudaHostRegister(ring, RingBytes, cudaHostRegisterDefault) == cudaSuccess;
         for (size_t i = 0; made && i < Slices; ++i)
             if (cudaEventCreateWithFlags(&landed[i], cudaEventDisableTiming) != cudaSuccess)
