@@ -45,7 +45,9 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "refused"; }
 }
 
-int main() {
+int main(int count, char **) {
+    if (count > 1)
+        return printf("%u\n", ResultCopies::processors()), 0;
     int wrong = 0;
     constexpr size_t Slice = ResultCopies::SliceBytes;
     const auto event = reinterpret_cast<cudaEvent_t>(uintptr_t(1));

@@ -14,6 +14,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <sched.h>
 #include <sys/mman.h>
 #include <thread>
 #include <unistd.h>
@@ -34,7 +35,12 @@ class ResultCopies {
         cudaEvent_t ready;
     };
 
-    // A quarter of the processors this process may use, or none: results then take the driver's way.
+    // Processors that the calling thread may run on (hardware_concurrency counts those it may not, too).
+    static unsigned processors() {
+        cpu_set_t set;
+        return sched_getaffinity(0, sizeof(set), &set) == 0 ? unsigned(CPU_COUNT(&set)) : std::thread::hardware_concurrency(); // more than a set holds
+    }
+    // A quarter of them, or none: results then take the driver's way.
     static int threads_for(unsigned processors) { return int(processors / 4) < MostThreads ? int(processors / 4) : MostThreads; }
 
     ResultCopies() = default;
