@@ -2,8 +2,10 @@
 // waited for, never earlier, so a slice that is emptied too soon, or filled again too soon, shows in the result.  The fake's n-th call fails on request.
 #include "../turbogpt_b200/csrc/result_copies.h"
 #include <cstdio>
+#include <ctime>
 #include <deque>
 #include <map>
+#include <utility>
 
 struct Copy {
     void *to;
@@ -13,7 +15,7 @@ struct Copy {
 static std::deque<Copy> queue;
 static size_t made = 0, queued = 0;
 static std::map<void *, size_t> recorded;
-static int calls = 0, failing = 0, waits = 0, handles = 0;
+static int calls = 0, failing = 0, stall = 0, waits = 0, handles = 0;
 static std::atomic<int> wrong_at_once{0};
 static std::atomic<int> alive{0};
 static bool fails() { return ++calls == failing; }
@@ -38,7 +40,10 @@ cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t bytes, cudaMemcpy
     return cudaSuccess;
 }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return recorded[e] = queued, cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t e) { return make(recorded[e]), cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    std::this_thread::sleep_for(std::chrono::milliseconds(std::exchange(stall, 0)));
+    return make(recorded[e]), cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return make(queued), cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return ++waits, cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
@@ -126,6 +131,15 @@ int main(int count, char **) {
         calls = 0, failing = 1; // refused for good
         wrong += of(3, ResultCopies::Worth) || of(3, ResultCopies::Worth) || calls != 1;
         failing = 0;
+    }
+    { // the threads sleep while the GPU computes: processor time, of this process
+        ResultCopies c;
+        wrong += !c.create(4);
+        run(c, {Slice}, 6, false);
+        const std::clock_t begin = std::clock();
+        stall = 400;
+        wrong += !run(c, {4 * Slice}, 7, true);
+        wrong += double(std::clock() - begin) / CLOCKS_PER_SEC > .2;
     }
     wrong += ResultCopies::of(5, ResultCopies::Worth, 0) || ResultCopies::of(-1, ResultCopies::Worth, 1) || alive;
     wrong += ResultCopies::threads_for(3) || ResultCopies::threads_for(4) != 1 || ResultCopies::threads_for(200) != ResultCopies::MostThreads;
