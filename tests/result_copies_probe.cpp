@@ -5,6 +5,7 @@
 #include <ctime>
 #include <deque>
 #include <map>
+#include <sys/wait.h>
 #include <utility>
 
 struct Copy {
@@ -126,6 +127,14 @@ int main(int count, char **) {
         wrong += wrong_at_once || done + refused != 200 || !done;
         a.reset();
         wrong += of(3, 0) != b;
+        const pid_t child = fork();
+        if (!child) { // has no threads to wait for
+            alarm(20);
+            b.reset(), other.reset();
+            _exit(0);
+        }
+        int status = -1;
+        wrong += waitpid(child, &status, 0) != child || status;
         b.reset(), other.reset();
         wrong += alive || of(3, 1);
         calls = 0, failing = 1; // refused for good

@@ -70,7 +70,11 @@ class ResultCopies {
         if (entry.refused || (entry.passed += bytes) < Worth)
             return nullptr;
         entry.passed = 0;
-        auto ring = std::make_shared<ResultCopies>();
+        // A forked child has the memory but not the threads: it leaves both alone, since nothing there would end a wait for them.
+        std::shared_ptr<ResultCopies> ring(new ResultCopies, [owner = getpid()](ResultCopies *r) {
+            if (getpid() == owner)
+                delete r;
+        });
         entry.refused = !ring->create(thread_count); // is not tried again
         if (entry.refused)
             return nullptr;
