@@ -476,6 +476,57 @@ def test_fp32_products_of_infinities_and_of_values_that_round_to_them():
     assert (np.abs(got[finite] - expected[finite].astype(np.float64)) <= 2 * width * 2.0 ** -24 * magnitude[finite]).all()
 
 
+@pytest.mark.parametrize("context,batch", [(150, 2), (1024, 3)])  # K of the weight gradients uncut, and cut
+def test_fp32_gradients_beside_values_that_round_to_infinities(context, batch):
+    """Operands beyond the largest BF16 value in every layout of a product (x w, dy w, dy x) and in attention, where zeros meet them: what they touch is computed
+    once more, and every gradient is finite and what the CUDA cores make of it."""
+    width, hidden, huge, column, unit, query = 128, 256, 3.395e38, 7, 100, 40
+    rng = np.random.default_rng(context)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    arch = Arch.gpt(1, width, 2, hidden)
+    w = Model(arch, seed=5, scale=.05).flat()
+    offset, sizes, parts = 0, {}, {}
+    for name, shape in specification(arch):
+        parts[name] = slice(offset, offset + int(np.prod(shape)))
+        sizes[name], offset = shape, parts[name].stop
+    names = list(parts)  # embedding, norm scale and bias, q k v (one matrix or three), proj, norm scale and bias, up, down, ...
+    matrices = [name for name in names if len(sizes[name]) == 2 and name != "embedding"]
+    view = {name: w[parts[name]].reshape(sizes[name]) for name in names}
+    qkv = w[parts[matrices[0]].start:][:3 * width * width].reshape(3 * width, width)
+    up, down = view[matrices[-2]], view[matrices[-1]]
+    assert up.shape == (hidden, width) and down.shape == (width, hidden)
+    view[names[1]][column], view[names[2]][column] = 0, huge  # every token's normalised value there
+    qkv[:, column] = 0
+    qkv[query, column] = 1  # and one of q's, which meets
+    qkv[width + query] = 0  # zeros in k
+    up[unit] = 0
+    down[:9, unit] = huge
+    both = parts[matrices[0]].start + (width + query) * width + column  # the one gradient that sums products of two such values
+    results = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.gpt(Config(depth=1, context=context, batch=batch), width, 2, hidden, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            logits, gradients, losses = engine.batch(x, y)
+            assert not np.isfinite(gradients[both])
+            gradients[both] = 0
+            np.testing.assert_array_equal(engine.activation(0, "normed1").reshape(-1, width)[:, column], np.float32(huge))
+            results.append([logits, losses, gradients])
+    (logits, losses, got), (expected_logits, expected_losses, expected) = results
+    assert np.isfinite(logits).all() and relative(logits, expected_logits) <= 1e-5 and relative(losses, expected_losses) <= 1e-5
+    assert np.isfinite(expected).all() and np.isfinite(got).all()
+    for name in names:
+        a, b = got[parts[name]].reshape(sizes[name]).astype(np.float64), expected[parts[name]].reshape(sizes[name]).astype(np.float64)
+        large = np.zeros(b.shape, bool)  # sums of products with the large values
+        if name == matrices[-2]:
+            large[unit] = True
+        elif name == matrices[0]:
+            large[:, column] = large[width + query] = True
+        assert not large.any() or np.linalg.norm(b[large]) > 1e30
+        for some in (large, ~large):
+            assert relative(a[some], b[some]) <= 1e-5, name
+
+
 @pytest.mark.parametrize("context,batch,heads", [(2, 70, 1), (64, 2, 2), (65, 3, 1), (129, 2, 3), (200, 40, 2), (1000, 1, 1)])
 def test_fp32_attention_on_tensor_cores(context, batch, heads):
     """Sequence ends on and off the 64-row tiles, two tokens a sequence, more tiles than SMs: what attention saves, and the gradients that it

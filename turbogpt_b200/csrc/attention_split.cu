@@ -369,13 +369,14 @@ template <bool Queries> __device__ __forceinline__ void split_backward(const Sof
     }
     if (__syncthreads_and(finite))
         return;
-    // delta as the CUDA cores' code wants it: of every query it will read
-    for (int i = threadIdx.x / 4; i < a.context; i += SideThreads / 4) {
+    // delta as the CUDA cores' code wants it: of every query it will read.  Whole warps go round: a query's four lanes add up through a shuffle of all 32.
+    for (int first = 0; first < a.context; first += SideThreads / 4) {
+        const int i = first + threadIdx.x / 4;
         float total = 0.f;
-        for (int c = threadIdx.x % 4; c < Side; c += 4)
+        for (int c = threadIdx.x % 4; i < a.context && c < Side; c += 4)
             total += dout[int64_t(i) * a.width + c] * out[int64_t(i) * a.width + c];
         total = quad_sum(total);
-        if (threadIdx.x % 4 == 0)
+        if (i < a.context && threadIdx.x % 4 == 0)
             a.delta[block.statistics + i] = total; // the same value from every block that comes here
     }
     __syncthreads();
