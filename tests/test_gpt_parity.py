@@ -2,6 +2,8 @@
 head) against the CPU oracle: BF16 mode within 1e-2, FP32 check mode within 1e-5, on the
 BASELINE configuration "CPU reference step": 4 layers, d_model 256, 4 heads, ctx 256, batch 8,
 bytes uniform from seed 0, weights N(0, 0.02) from seed 1, one AdamW step."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -525,6 +527,26 @@ def test_fp32_gradients_beside_values_that_round_to_infinities(context, batch):
         assert not large.any() or np.linalg.norm(b[large]) > 1e30
         for some in (large, ~large):
             assert relative(a[some], b[some]) <= 1e-5, name
+
+
+def test_fp32_run_that_diverged_is_no_slower_than_on_cuda_cores():
+    """A NaN in every product: recomputed a tile at a time (one output at a time took 19 times as long as the CUDA cores' kernels)."""
+    context, batch = 256, 8
+    rng = np.random.default_rng(0)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    seconds = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.gpt(Config(depth=2, context=context, batch=batch), 256, 4, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(np.full(engine.count, np.nan, np.float32))
+            times = []
+            for _ in range(6):
+                begin = time.perf_counter()
+                logits, gradients, _ = engine.batch(x, y)
+                times.append(time.perf_counter() - begin)
+            assert np.isnan(logits).all()
+            seconds.append(min(times))
+    assert seconds[0] < 4 * seconds[1], seconds
 
 
 @pytest.mark.parametrize("context,batch,heads", [(2, 70, 1), (64, 2, 2), (65, 3, 1), (129, 2, 3), (200, 40, 2), (1000, 1, 1)])
