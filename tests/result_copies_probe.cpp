@@ -106,8 +106,8 @@ int main(int count, char **) {
     }
     { // made when it is worth it, shared, given back with its last owner; a call that finds it in use does without
         const auto of = [](int device, size_t bytes) { return ResultCopies::of(device, bytes, 2); };
-        wrong += of(3, ResultCopies::Worth - 1) || of(4, 1);
-        auto a = of(3, 1), b = of(3, 0), other = of(4, ResultCopies::Worth - 1);
+        wrong += of(3, ResultCopies::Worth - 1) || of(4, 1) || of(3, 1);
+        auto a = of(3, ResultCopies::Worth), b = of(3, 0), other = of(4, ResultCopies::Worth + 1);
         wrong += !a || a != b || !other || other == a;
         std::atomic<int> refused{0}, done{0};
         std::vector<std::thread> engines;
@@ -136,7 +136,7 @@ int main(int count, char **) {
         int status = -1;
         wrong += waitpid(child, &status, 0) != child || status;
         b.reset(), other.reset();
-        wrong += alive || of(3, 1);
+        wrong += alive || of(3, ResultCopies::Worth - 1);
         calls = 0, failing = 1; // refused for good
         wrong += of(3, ResultCopies::Worth) || of(3, ResultCopies::Worth) || calls != 1;
         failing = 0;

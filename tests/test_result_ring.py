@@ -38,7 +38,7 @@ def captured(before, during):
     return begun == ended == 0
 
 
-WORTH = 32 << 20  # bytes of results that take the driver's way before there is a ring
+WORTH = 32 << 20  # bytes of an engine's results from which on a ring is made
 
 
 @pytest.mark.parametrize("context,batch", [(128, 4), (512, 24)])  # 2 and 14 MB of results, less and more than the ring holds
@@ -67,7 +67,8 @@ def test_results_through_the_ring_are_those_of_pinned_memory(library, context, b
         while threads() == before:
             check(native.batch(x, y))
             calls += 1
-            assert calls <= WORTH // (logits.nbytes + gradients.nbytes) + 1
+            assert calls <= -(-WORTH // (logits.nbytes + gradients.nbytes))
+        assert calls == -(-WORTH // (logits.nbytes + gradients.nbytes))
         assert threads() == before + helpers
         for _ in range(3):
             check(other.batch(x, y))  # the first one too

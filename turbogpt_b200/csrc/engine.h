@@ -146,7 +146,8 @@ struct Engine {
     size_t next_fork_event = 0;
     float *simt_scratch[3] = {nullptr, nullptr, nullptr}; // per lane: partial tiles of CUDA-core GEMMs that are cut along K (6 MB bounds every shape)
     BatchCopies copies; // of tg_batch's results
-    std::shared_ptr<ResultCopies> results; // the device's, once a call has had use for it
+    std::shared_ptr<ResultCopies> results; // the device's, once it is worth its making
+    size_t result_bytes = 0;               // that calls without it have returned
     Outbox *outbox = nullptr;          // what a call brings back with its last wait,
     std::unique_ptr<Outbox> mailbox;   // and where it arrives
     bool announce_gradients = false;

@@ -5,7 +5,7 @@
 // 18.5 ms (from 32 MB on the C library maps an array afresh for every call, and the threads take its page faults).
 //
 // Making the ring takes 1.5 ms, giving it back 0.5, so that it is shared by a device's engines, belongs to those that have used it, and is made by the call that
-// brings the results that left the driver's way to 32 MB, while that call's kernels run (made for every engine: second calls of 2 to 15 MB 1.0 -> 3.1 and
+// brings an engine's results to 32 MB, while that call's kernels run (made for every engine: second calls of 2 to 15 MB 1.0 -> 3.1 and
 // 2.6 -> 4.2 ms).
 #pragma once
 #include "common.h"
@@ -49,12 +49,12 @@ class ResultCopies {
     ResultCopies(const ResultCopies &) = delete;
     ~ResultCopies() { destroy(); }
 
-    // The ring of a device, made now where that is worth its time; null: `bytes` of results take the driver's way.  The current device is the one meant.
+    // The ring of a device, which is the current one, for an engine whose results so far are `bytes`: made now where that is worth its time; null: results take
+    // the driver's way.
     static std::shared_ptr<ResultCopies> of(int device, size_t bytes, int thread_count) {
         struct Entry {
             std::mutex mutex;
             std::weak_ptr<ResultCopies> ring;
-            size_t passed = 0; // bytes since there was no ring
             bool refused = false;
         };
         constexpr int Devices = 64;
@@ -67,9 +67,8 @@ class ResultCopies {
             return nullptr;
         if (std::shared_ptr<ResultCopies> ring = entry.ring.lock())
             return ring;
-        if (entry.refused || (entry.passed += bytes) < Worth)
+        if (entry.refused || bytes < Worth)
             return nullptr;
-        entry.passed = 0;
         // A forked child has the memory but not the threads: it leaves both alone, since nothing there would end a wait for them.
         std::shared_ptr<ResultCopies> ring(new ResultCopies, [owner = getpid()](ResultCopies *r) {
             if (getpid() == owner)
