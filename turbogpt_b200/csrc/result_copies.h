@@ -26,7 +26,7 @@ class ResultCopies {
     // 24 and 32 of half the size 735 us and 20.1 ms, 680 us and 19.6.
     static constexpr size_t SliceBytes = size_t(1) << 19, Slices = 16;
     static constexpr int MostThreads = 4;
-    static constexpr std::chrono::microseconds Patience{50}; // 20, 100 and 300 give the same calls
+    static constexpr std::chrono::microseconds Patience{1000}; // without work; 300 is too short for evaluations of FP32 engines (500 -> 830 us after a pause), 3000 level
     static constexpr size_t Worth = size_t(32) << 20; // 40 us are saved for every megabyte
 
     struct Segment { // to[0, bytes) = from, device memory that is complete on `stream` after `ready` (null: after what `stream` holds)
@@ -174,8 +174,12 @@ class ResultCopies {
         struct Active { // the threads take jobs while this lives; all have left the array when it is gone
             ResultCopies &c;
             explicit Active(ResultCopies &copies) : c(copies) {
-                std::lock_guard<std::mutex> lock(c.mutex);
-                c.active.store(true);
+                {
+                    std::lock_guard<std::mutex> lock(c.mutex);
+                    c.active.store(true);
+                    ++c.call;
+                }
+                c.wake.notify_all();
             }
             ~Active() {
                 {
@@ -260,6 +264,7 @@ class ResultCopies {
     std::mutex mutex, busy; // of the threads' state; for the length of a call
     std::condition_variable wake;
     bool stopping = false;
+    unsigned call = 0;
 
     bool take_one() {
         size_t i = next.load(std::memory_order_relaxed);
@@ -276,16 +281,17 @@ class ResultCopies {
         job.done.store(true, std::memory_order_release);
         return true;
     }
-    // A thread that finds nothing to do for a while sleeps: polling through a call's kernels took four processors for all of it (15 MB after 0.48 and 1.0 ms of
-    // kernels: 2.75 -> 2.0 and 5.7 -> 3.0 ms of processor time).
+    // Awake from a call's beginning on, since waking takes 0.1 to 0.2 ms (woken for the first slice: 2 MB 270 -> 450 us a call), but a thread that finds nothing
+    // to do for a while sleeps: polling through the kernels of a long call took four processors for all of it.
     void work() {
         std::unique_lock<std::mutex> lock(mutex);
-        for (;;) {
+        for (unsigned seen = 0;;) {
             ++asleep;
-            wake.wait(lock, [&] { return stopping || (active.load() && next.load() < published.load()); });
+            wake.wait(lock, [&] { return stopping || (active.load() && (seen != call || next.load() < published.load())); });
             --asleep;
             if (stopping)
                 return;
+            seen = call;
             inside.fetch_add(1);
             lock.unlock();
             auto last = std::chrono::steady_clock::now();
