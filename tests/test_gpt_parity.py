@@ -12,7 +12,7 @@ from oracle.model import Arch, Model, specification
 from oracle.optim import Hyper, Optimizer
 from turbogpt_b200 import Config, ConfigEx, Native
 from turbogpt_b200 import bridge
-from helpers import max_relative, relative
+from helpers import evaluation_in_64_bits, max_relative, relative
 
 pytestmark = pytest.mark.gpu
 
@@ -547,6 +547,44 @@ def test_fp32_run_that_diverged_is_no_slower_than_on_cuda_cores():
             assert np.isnan(logits).all()
             seconds.append(min(times))
     assert seconds[0] < 4 * seconds[1], seconds
+
+
+def fp32_errors(depth, width, hidden, context, batch):
+    """Errors against 64 bits of an FP32 evaluation's logits, gradients and each parameter's gradient, with tensor cores and without."""
+    rng = np.random.default_rng(width)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    arch = Arch.gpt(depth, width, width // 64, hidden)
+    w = Model(arch, seed=5).flat()
+    logits, gradients = evaluation_in_64_bits(arch, w, x, y)
+    errors = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.gpt(Config(depth=depth, context=context, batch=batch), width, width // 64, hidden, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            got = engine.batch(x, y)
+        errors.append({"logits": relative(got[0], logits), "gradients": relative(got[1], gradients)})
+        offset = 0
+        for name, shape in specification(arch):
+            part = slice(offset, offset + int(np.prod(shape)))
+            offset = part.stop
+            errors[-1][name] = relative(got[1][part], gradients[part])
+    return errors
+
+
+@pytest.mark.parametrize("depth,width,hidden,context,batch", [
+    (4, 256, 1024, 256, 8), (2, 128, 512, 32, 8), (6, 128, 512, 260, 12), (3, 192, 768, 77, 3), (5, 512, 2048, 98, 11), (1, 64, 256, 1024, 64)])
+def test_fp32_engines_are_no_further_from_64_bits_than_on_cuda_cores(depth, width, hidden, context, batch):
+    ours, cuda_cores = fp32_errors(depth, width, hidden, context, batch)
+    for name in ("logits", "gradients"):
+        assert ours[name] <= cuda_cores[name], (name, ours[name], cuda_cores[name])
+
+
+def test_fp32_errors_do_not_grow_with_the_tokens_of_a_weight_gradient():
+    """Uncut sums over 262144 tokens, which the tensor core cuts off at every step: none of its accumulators may hold all of them.  In FP32 registers one in 64 additions
+    of the CUDA cores' is left, which is an eighth of their rounding; held whole, the smaller parts' sums made it as large as all of it."""
+    ours, cuda_cores = fp32_errors(1, 1024, 1024, 64, 4096)
+    for name in ("0.qkv", "0.attention", "0.gate", "0.projection"):
+        assert ours[name] <= cuda_cores[name] / 2, (name, ours[name], cuda_cores[name])
 
 
 @pytest.mark.parametrize("context,batch,heads", [(2, 70, 1), (64, 2, 2), (65, 3, 1), (129, 2, 3), (200, 40, 2), (1000, 1, 1)])

@@ -4,8 +4,8 @@
 // significand in three times eight).  Of the nine products of parts the six above 2^-24 of x y are formed, exact in FP32: h h into one
 // accumulator, h m, m h, m m, h l and l h into another.  The tensor core cuts its sums off instead of rounding them (1.2e-8 of the
 // result for every step, 4.4e-6 after 256), so the first accumulator only ever holds 32 of K, two steps, and is added to FP32 registers; the second is
-// 2^-8 of the result and runs over all of K.  Against 64 bits (N(0,1) operands, K 16 to 4096) 0.4 to 1.3e-7,
-// where the CUDA cores' sums have 0.7 to 4.1e-7.
+// 2^-8 of the result and holds 2048 (all of K: a weight gradient's error grew with its tokens, 262144 of them 2.7e-6, now 1.0e-6; CUDA cores 2.9e-6).
+// Against 64 bits (N(0,1) operands, K 16 to 4096) 0.4 to 1.3e-7, where the CUDA cores' sums have 0.7 to 4.1e-7.
 //
 // What bounds it: 24 products of 128 x BN x 16 a block read their operands from shared memory, 6 (4 + BN / 32) KB each, at 128 B/clk, beside the
 // 48 + 3/8 BN KB that the split operands are written with: 1560 clocks a 128 x 128 x 64 block where the CUDA cores take 8192 for the
@@ -26,6 +26,7 @@ using namespace sm100;
 
 namespace {
 constexpr int BM = 128, Block = 64; // rows of a tile, K elements of a block
+constexpr int RestBlocks = 32;      // that the second accumulator holds
 constexpr int Workers = 16, Threads = 32 * (Workers + 1), WorkerThreads = 32 * Workers;
 constexpr int RowBytes = Block * 2; // of a K-major part; an MN-major one has 128 bytes (64 rows) per k
 constexpr int ControlBytes = 64;
@@ -227,21 +228,25 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
                 ok = mbarrier_wait(full0 + 8 * s, b / 2 & 1, abort_flag, counters, 411); // the block is there
                 if (!ok)
                     break;
-                tcgen05_fence_after();
                 const uint64_t da = descriptor_at(a_desc, s * stage_bytes(BN)), db = descriptor_at(b_desc, s * stage_bytes(BN));
+                const bool emptied = b % RestBlocks == 0; // the second accumulator, with the block before
+                auto block_before_added = [&] { return b == 0 || (ok = mbarrier_wait(added, (b - 1) & 1, abort_flag, counters, 413)); };
+                if (emptied && !block_before_added())
+                    break;
+                tcgen05_fence_after();
                 auto multiply = [&](uint32_t accumulator, int a_part, int b_part, int ks, bool add) {
                     tcgen05_mma_bf16(accumulator, descriptor_at(da, a_part * part_bytes(BM) + ks * a_step),
                                      descriptor_at(db, b_part * part_bytes(BN) + ks * b_step), instruction, add);
                 };
 #pragma unroll
                 for (int ks = 0; ks < Block / 16; ++ks) {
-                    multiply(tmem_base + 2 * BN, 0, 1, ks, b > 0 || ks > 0);
+                    multiply(tmem_base + 2 * BN, 0, 1, ks, !emptied || ks > 0);
                     multiply(tmem_base + 2 * BN, 1, 0, ks, true);
                     multiply(tmem_base + 2 * BN, 1, 1, ks, true);
                     multiply(tmem_base + 2 * BN, 0, 2, ks, true);
                     multiply(tmem_base + 2 * BN, 2, 0, ks, true);
                 }
-                if (b > 0 && !(ok = mbarrier_wait(added, (b - 1) & 1, abort_flag, counters, 413))) // the block before has been added to the registers
+                if (!emptied && !block_before_added())
                     break;
                 tcgen05_fence_after();
 #pragma unroll
@@ -273,6 +278,17 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
                 for (int j = 0; j < 8; ++j)
                     sums[c + j] += __uint_as_float(v[j]) + __uint_as_float(w[j]);
             }
+            if (block == blocks - 1 || block % RestBlocks == RestBlocks - 1) {
+#pragma unroll
+                for (int c = 0; c < Share; c += 16) {
+                    uint32_t v[16];
+                    tmem_load_32x16_async(accumulators + 2 * BN + c, v);
+                    tmem_wait_load(v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        sums[c + j] += __uint_as_float(v[j]);
+                }
+            }
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0)
@@ -297,17 +313,6 @@ __global__ void __launch_bounds__(Threads, 1) gemm_split_kernel(const __grid_con
                 break;
         }
         ok = ok && finish(blocks - 1);
-#pragma unroll
-        for (int c = 0; c < Share; c += 16) {
-            if (!ok)
-                break;
-            uint32_t v[16];
-            tmem_load_32x16_async(accumulators + 2 * BN + c, v);
-            tmem_wait_load(v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                sums[c + j] += __uint_as_float(v[j]);
-        }
     }
     ok = __syncthreads_and(ok); // every product is done: the stages take the sums
     constexpr int Pitch = BN + 4;
