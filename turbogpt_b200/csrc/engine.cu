@@ -760,11 +760,20 @@ void Engine::backward() {
 }
 
 // ------------------------------------------------------------------------------- optimizer ---
-// Momentum, the normalised direction and, with `iterate`, its Newton-Schulz iterations; returns where every layer's result is.
-bf16 *Engine::muon_direction(const MuonFamily &family, bool iterate) {
+// Momentum and the normalised direction, in x[0].
+void Engine::muon_direction(const MuonFamily &family) {
     const TgConfigEx &c = config;
     const int depth = c.base.depth, rows = family.rows, cols = family.cols;
     const int64_t first_offset = family.first, stride = depth > 1 ? layout.layers[1].qkv - layout.layers[0].qkv : 0;
+    MuonPrepareArgs prep{gradient + first_offset, momentum + first_offset, family.x[0], family.sumsq, sumsq_partial,
+                         sumsq_blocks, schedule, counters, c.base.momentum, c.base.clip, rows, cols, depth, stride, family.progress};
+    run(FMuon, [&](cudaStream_t s) { launch_muon_prepare(prep, s); });
+    run(FMuon, [&](cudaStream_t s) { launch_muon_normalize(family.x[0], family.sumsq, int64_t(rows) * cols, depth, sms, s); });
+}
+// The Newton-Schulz iterations as products of their own; returns where every layer's result is.
+bf16 *Engine::muon_products(const MuonFamily &family) {
+    const TgConfigEx &c = config;
+    const int depth = c.base.depth, rows = family.rows, cols = family.cols;
     const int r = std::min(rows, cols), n = std::max(rows, cols); // orthogonalise the wide orientation
     const int64_t per = int64_t(rows) * cols;
     // Under data parallelism the gradients are identical on every rank after the exchange, so the
@@ -774,12 +783,6 @@ bf16 *Engine::muon_direction(const MuonFamily &family, bool iterate) {
     // stay bit-identical and any rank can write a checkpoint.
     const bool sharded = comm && depth % c.world == 0 && depth >= c.world;
     const int mine = sharded ? depth / c.world : depth, first = sharded ? c.rank * mine : 0;
-    MuonPrepareArgs prep{gradient + first_offset, momentum + first_offset, family.x[0], family.sumsq, sumsq_partial,
-                         sumsq_blocks, schedule, counters, c.base.momentum, c.base.clip, rows, cols, depth, stride, family.progress};
-    run(FMuon, [&](cudaStream_t s) { launch_muon_prepare(prep, s); });
-    run(FMuon, [&](cudaStream_t s) { launch_muon_normalize(family.x[0], family.sumsq, per, depth, sms, s); });
-    if (!iterate)
-        return family.x[c.base.ns_steps % 2];
     bf16 *cur = family.x[0] + first * per, *nxt = family.x[1] + first * per;
     bf16 *a_buffer = family.a + int64_t(first) * r * r, *b_buffer = family.b + int64_t(first) * r * r;
     const bool small = muon_newton_schulz_small_supported(r, n); // the reference architecture: one launch, in place
@@ -820,13 +823,15 @@ bf16 *Engine::muon_direction(const MuonFamily &family, bool iterate) {
     }
     return all;
 }
-void Engine::muon_iterations(const MuonFamily *families, int count) {
+// The same in one launch; false: it was refused, and the products are to be launched instead, from now on.
+bool Engine::muon_iterations(const MuonFamily *families, int count) {
     NewtonSchulzArgs a;
     for (int i = 0; i < count; ++i)
         a.family[i] = {{families[i].x[0], families[i].x[1]}, families[i].a, families[i].b, families[i].rows, families[i].cols};
     a.count = count, a.batch = config.base.depth, a.steps = config.base.ns_steps, a.progress = families[0].progress, a.counters = counters;
     if (a.steps > 0)
-        run(FMuon, [&](cudaStream_t s) { launch_newton_schulz(a, sms, s); });
+        run(FMuon, [&](cudaStream_t s) { muon_persistent = launch_newton_schulz(a, sms, s); });
+    return muon_persistent;
 }
 void Engine::muon_apply(const MuonFamily &family, bf16 *all) {
     const TgConfigEx &c = config;
@@ -856,26 +861,25 @@ void Engine::optimize() {
         for (int l = 1; l <= chains; ++l)
             fork(l, 0);
     };
-    std::vector<bf16 *> directions(muon.size());
+    auto finish_family = [&](const MuonFamily &family, bool iterated) {
+        muon_apply(family, iterated ? family.x[c.base.ns_steps % 2] : muon_products(family));
+    };
     for (int l = 1; l <= chains; ++l)
         await(l, norm_ready);
     for (size_t f = 0; f < muon.size(); ++f) {
         OnLane on(*this, chains ? 1 + int(f) % chains : 0);
-        directions[f] = muon_direction(muon[f], !muon_persistent);
-        if (together)
-            continue;
-        if (muon_persistent)
-            muon_iterations(&muon[f], 1);
-        muon_apply(muon[f], directions[f]);
+        muon_direction(muon[f]);
+        if (!together)
+            finish_family(muon[f], muon_persistent && muon_iterations(&muon[f], 1));
     }
     join();
     if (together) {
-        muon_iterations(muon.data(), int(muon.size()));
+        const bool iterated = muon_iterations(muon.data(), int(muon.size()));
         for (int l = 1; l <= chains; ++l)
             fork(0, l);
         for (size_t f = 0; f < muon.size(); ++f) {
             OnLane on(*this, 1 + int(f) % chains);
-            muon_apply(muon[f], directions[f]);
+            finish_family(muon[f], iterated);
         }
         join();
     }

@@ -198,8 +198,9 @@ struct Engine {
     void exchange_bucket(int64_t begin, int64_t end, int index);
     void finish_exchange();
     void optimize();
-    bf16 *muon_direction(const MuonFamily &family, bool iterate);
-    void muon_iterations(const MuonFamily *families, int count);
+    void muon_direction(const MuonFamily &family);
+    bf16 *muon_products(const MuonFamily &family);
+    bool muon_iterations(const MuonFamily *families, int count);
     void muon_apply(const MuonFamily &family, bf16 *direction);
     bool use_graphs() const { return !profile && !comm && !(config.flags & TG_FLAG_NO_GRAPH); }
     template <class F> void replay(GraphKind kind, F &&body);

@@ -325,7 +325,8 @@ struct NewtonSchulzArgs {
     StepCounters *counters = nullptr;
 };
 bool newton_schulz_supported(int rows, int cols, const void *x);
-void launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s);
+// False: the GPU, or the part of it that this process may use, does not hold all its blocks at once, or there are more tiles than it counts; nothing was launched.
+bool launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s);
 struct MuonApplyArgs {
     const bf16 *x;
     bf16 *weight_high;

@@ -393,7 +393,7 @@ bool newton_schulz_supported(int rows, int cols, const void *x) {
     return r >= 64 && r % 8 == 0 && n % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
 }
 
-void launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s) {
+bool launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s) {
     if (a.count < 1 || a.count > MaxFamilies || a.steps < 1)
         throw std::runtime_error("Newton-Schulz: one to five families, at least one step");
     static thread_local Params p; // 5 KB
@@ -459,7 +459,7 @@ void launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s) {
     }
     p.per_step = p.items[Gram] + p.items[Square] + p.items[Update];
     if ((long long)p.per_step * a.steps > (1 << 30))
-        throw std::runtime_error("Newton-Schulz: too many tiles");
+        return false;
     const int shared = p.stages * p.stage_bytes + ControlBytes + 1024;
     CHECK_CUDA(cudaFuncSetAttribute(newton_schulz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MaxShared));
     cudaLaunchConfig_t config{};
@@ -468,5 +468,11 @@ void launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s) {
     attribute.id = cudaLaunchAttributeCooperative; // every CTA is resident: they wait for one another
     attribute.val.cooperative = 1;
     config.attrs = &attribute, config.numAttrs = 1;
-    CHECK_CUDA(cudaLaunchKernelEx(&config, newton_schulz_kernel, p));
+    const cudaError_t status = cudaLaunchKernelEx(&config, newton_schulz_kernel, p);
+    if (status == cudaErrorCooperativeLaunchTooLarge) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    CHECK_CUDA(status);
+    return true;
 }
