@@ -5,6 +5,7 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -28,8 +29,6 @@ with Native(ex) as engine:
 
 @pytest.mark.parametrize("depth,width", [(3, 192), (5, 960)])  # the families in one launch, and one by one
 def test_refused_newton_schulz_launch(library, tmp_path, depth, width):
-    import numpy as np
-
     shim = tmp_path / "refused.so"
     subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-I/usr/local/cuda/include", str(SHIM), "-o", str(shim), "-ldl"], check=True)
     results, refusals = [], []

@@ -396,7 +396,8 @@ bool newton_schulz_supported(int rows, int cols, const void *x) {
 bool launch_newton_schulz(const NewtonSchulzArgs &a, int sms, cudaStream_t s) {
     if (a.count < 1 || a.count > MaxFamilies || a.steps < 1)
         throw std::runtime_error("Newton-Schulz: one to five families, at least one step");
-    static thread_local Params p; // 5 KB
+    static_assert(sizeof(Params) <= 32764, "the most a kernel's parameters may take");
+    static thread_local Params p;
     p = Params{};
     int order[MaxFamilies]; // the longest products first: what follows them fills the gaps
     for (int i = 0; i < a.count; ++i)
