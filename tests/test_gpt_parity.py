@@ -594,6 +594,25 @@ def test_fp32_attention_on_tensor_cores(context, batch, heads):
     test_fp32_products_on_tensor_cores(64 * heads, 128 * heads, context, batch)
 
 
+@pytest.mark.parametrize("head_size,heads", [(2, 4), (4, 4), (12, 2), (20, 4), (6, 12)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_softmax_attention_of_head_sizes_off_eight(head_size, heads, fp32):
+    """Even head sizes that are no multiple of eight: rows of q, k and v are aligned to two values only, and end where another head's begin."""
+    width, context, batch = head_size * heads, 45, 3
+    rng = np.random.default_rng(head_size)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    model = Model(Arch.gpt(2, width, heads), seed=1, scale=.1, fp32=fp32)
+    logits, gradients, losses = model.batch(x, y)
+    precision = bridge.PRECISION_FP32 if fp32 else bridge.PRECISION_BF16
+    tolerance = 1e-5 if fp32 else 1e-2
+    with Native(ConfigEx.gpt(Config(depth=2, context=context, batch=batch, clip=0), width, heads, precision=precision)) as engine:
+        engine.set_weights(model.flat())
+        got = engine.batch(x, y)
+    assert relative(got[0], logits) <= tolerance
+    assert relative(got[1], gradients) <= tolerance
+    np.testing.assert_allclose(got[2], losses, rtol=tolerance, atol=tolerance)
+
+
 def test_fp32_attention_keeps_a_later_infinity_out():
     """An infinite embedding at one position: what precedes it stays finite and as it was, what follows is what the CUDA cores' kernels make of it."""
     width, context, batch, at = 128, 150, 2, 70

@@ -111,9 +111,15 @@ void launch_argmax_attention_backward(Dtype t, const ArgmaxAttentionBackwardArgs
 constexpr int MaxHeadChunks = 8; // head size up to 256 = 8 chunks of 32 lanes
 constexpr int AttentionWarps = 4;
 
-// Dot product of a row held in shared memory (FP32) with a row in global memory.
+// Dot product of a row held in shared memory (FP32) with a row in global memory.  Where the head size is no multiple of eight, rows are not aligned to eight
+// values, and what follows them is not theirs.
 template <class T> __device__ __forceinline__ float dot_row(const float *shared_row, const T *row, int d) {
     float sum = 0;
+    if (d % 8) {
+        for (int c = 0; c < d; ++c)
+            sum += shared_row[c] * to_float(row[c]);
+        return sum;
+    }
     for (int c = 0; c < d; c += 8) {
         float v[8];
         load8(row + c, v);
