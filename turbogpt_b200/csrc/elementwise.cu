@@ -908,6 +908,16 @@ template <class T> __global__ void __launch_bounds__(256) cross_entropy_kernel(C
         a.losses[row] = high + logf(sum) - picked;
     if (a.logits_fp32)
         store8(a.logits_fp32 + int64_t(row) * Vocabulary + lane * 8, v);
+    if (a.outbox) {
+        if (row == 0 && lane == 0)
+            a.outbox->counters = *a.counters;
+        if (a.last_logits ? row + 1 == a.rows : lane == 0) {
+            if (a.last_logits)
+                store8(a.outbox->values + lane * 8, v);
+            else
+                a.outbox->values[row] = high + logf(sum) - picked;
+        }
+    }
     if (a.dlogits) {
         float g[8];
 #pragma unroll

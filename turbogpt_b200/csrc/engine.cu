@@ -424,13 +424,9 @@ cudaEvent_t Engine::mark(int on) {
     return event;
 }
 void Engine::await(int on, cudaEvent_t event) { CHECK_CUDA(cudaStreamWaitEvent(lanes[on].stream, event, 0)); }
-// What finish() brings back in one copy with the error word: copied behind it, with the call's last kernels.  Each copy into ordinary memory is a wait.
-void Engine::collect(const float *values, size_t count) {
-    if (count <= std::size(outbox->values))
-        run(FMisc, [&](cudaStream_t s) { launch_collect(counters, values, int(count), outbox, s); });
-}
-// Waits for the stream, and reports what its kernels recorded.  `out` (may be null) first receives `count` values, collected or the losses, which lie behind
-// the counters.  Losses of a finished step: 14.7 us; counters and losses in copies of their own 27, in one through pinned memory 15.7 (and 0.65 ms to pin it).
+// Waits for the stream, and reports what its kernels recorded.  `out` (may be null) first receives `count` values: the losses of training steps, which lie
+// behind the counters, or what the call's last kernel has left in the outbox.  One copy, since each into ordinary memory is a wait: losses of a finished step
+// 14.7 us, counters and losses in copies of their own 27, both through pinned memory 15.7 (and 0.65 ms to pin it).
 void Engine::finish(float *out, const float *values, size_t count) {
     const bool together = count <= std::size(outbox->values), collected = values != loss_history;
     const size_t behind = out && together ? count : 0;
@@ -583,6 +579,8 @@ void Engine::forward(bool want_gradient, bool dump_logits, bool embedded) {
     gemm(FGemmForward, head);
     CrossEntropyArgs ce{logits, y, token_losses, want_gradient ? logits : nullptr,
                         dump_logits ? logits_fp32 : nullptr, divisor, M};
+    if (!want_gradient && (forward_batch || size_t(M) <= std::size(outbox->values))) // an evaluation's last kernel
+        ce.outbox = outbox, ce.counters = counters, ce.last_logits = forward_batch;
     run(FCrossEntropy, [&](cudaStream_t s) { launch_cross_entropy(act, ce, s); });
 }
 
@@ -1116,7 +1114,8 @@ void Engine::batch(const uint8_t *bx, const uint8_t *by, float *logits_out, floa
     replay(gradient_out ? GraphGradients : GraphEvaluate,
            [&] {
                one_step(gradient_out ? RunMode::Gradients : RunMode::Evaluate);
-               collect(token_losses, size_t(tokens));
+               if (gradient_out && size_t(tokens) <= std::size(outbox->values))
+                   run(FMisc, [&](cudaStream_t s) { launch_collect(counters, token_losses, tokens, outbox, s); });
            });
     // Of 32 MB and more the C library maps an array afresh each time; smaller ones mostly lie in memory that it has kept.
     auto kept = [](const ResultCopies::Segment &s) { return s.bytes < size_t(32) << 20 || !ordinary(s); };
@@ -1158,10 +1157,7 @@ void Engine::predict(const uint8_t *context, float *logits256) {
     CHECK_CUDA(cudaMemsetAsync(y, 0, T, stream));
     forward_batch = 1;
     try {
-        replay(GraphPredict, [&] {
-            one_step(RunMode::Evaluate);
-            collect(logits_fp32 + size_t(T - 1) * Vocabulary, Vocabulary);
-        });
+        replay(GraphPredict, [&] { one_step(RunMode::Evaluate); });
     } catch (...) {
         forward_batch = 0;
         throw;

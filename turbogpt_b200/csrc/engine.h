@@ -214,6 +214,5 @@ struct Engine {
     void prepare_reference_step();
     void reference_train_step(bool sample, bool save);
     void one_step(RunMode mode, bool last = true);
-    void collect(const float *values, size_t count);
     void finish(float *out = nullptr, const float *values = nullptr, size_t count = 0);
 };

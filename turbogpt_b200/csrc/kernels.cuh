@@ -144,6 +144,12 @@ void launch_swiglu(Dtype t, const void *wide, void *out, int tokens, int hidden,
 void launch_swiglu_backward(Dtype t, const void *wide, const void *dout, void *dwide, int tokens, int hidden,
                             cudaStream_t s);
 
+// What a call brings back with its last wait.
+struct Outbox {
+    StepCounters counters;
+    float values[16384];
+};
+
 // ---- 256-way softmax cross-entropy (reference cuda/model.cuh:33-57) ----
 struct CrossEntropyArgs {
     const void *logits;  // [rows, 256]
@@ -153,16 +159,15 @@ struct CrossEntropyArgs {
     float *logits_fp32;  // optional FP32 copy of the logits (diagnostic calls)
     float divisor;       // global batch * context
     int rows;
+    Outbox *outbox = nullptr;  // optional, where this is a call's last kernel: receives the counters and
+    const StepCounters *counters = nullptr;
+    bool last_logits = false;  // the last row's logits, else the losses
 };
 void launch_cross_entropy(Dtype t, const CrossEntropyArgs &a, cudaStream_t s);
 
 // ---- per-position loss history (reference cuda/trainer.cuh:79-100) ----
 void launch_loss_history(const float *token_losses, float *history, const StepCounters *counters, int batch,
                          int context, cudaStream_t s);
-struct Outbox {
-    StepCounters counters;
-    float values[16384];
-};
 // The counters and `count` values into one place, for one copy to the host.
 void launch_collect(const StepCounters *counters, const float *values, int count, Outbox *out, cudaStream_t s);
 
