@@ -529,6 +529,36 @@ def test_fp32_gradients_beside_values_that_round_to_infinities(context, batch):
             assert relative(a[some], b[some]) <= 1e-5, name
 
 
+@pytest.mark.parametrize("size", [1e3, 1e5])
+@pytest.mark.parametrize("context,batch,heads", [(40, 3, 2), (200, 2, 2), (333, 1, 3)])
+def test_fp32_attention_of_large_scores(size, context, batch, heads):
+    """q and k so large that a score's last place is worth more than any exponential: the backward pass has to find the forward pass's scores to the bit, or
+    probabilities of one become zero or infinite.  Gradients that such probabilities scale, and everything before them, are what the CUDA cores' kernels make of it."""
+    width = 64 * heads
+    rng = np.random.default_rng(context)
+    x, y = rng.integers(0, 256, (2, batch, context), dtype=np.uint8)
+    arch = Arch.gpt(1, width, heads)
+    w = Model(arch, seed=5, scale=.05).flat()
+    offset, parts = 0, {}
+    for name, shape in specification(arch):
+        parts[name] = slice(offset, offset + int(np.prod(shape)))
+        offset = parts[name].stop
+    w[parts["0.qkv"]][:2 * width * width] *= size
+    results = []
+    for flags in (0, bridge.FLAG_NO_TENSOR_CORES):
+        ex = ConfigEx.gpt(Config(depth=1, context=context, batch=batch), width, heads, precision=bridge.PRECISION_FP32, flags=flags)
+        with Native(ex) as engine:
+            engine.set_weights(w)
+            logits, gradients, losses = engine.batch(x, y)
+            results.append([logits, losses, gradients])
+    (logits, losses, got), (expected_logits, expected_losses, expected) = results
+    assert relative(logits, expected_logits) <= 1e-5 and relative(losses, expected_losses) <= 1e-5
+    assert np.isfinite(expected).all() and np.isfinite(got).all()
+    values = slice(parts["0.qkv"].start + 2 * width * width, parts["0.qkv"].stop)  # v's; q's and k's are differences of equal numbers
+    for part in (values, *(parts[name] for name in list(parts)[4:])):
+        assert relative(got[part], expected[part]) <= 1e-5
+
+
 def test_fp32_run_that_diverged_is_no_slower_than_on_cuda_cores():
     """A NaN in every product: recomputed a tile at a time (one output at a time took 19 times as long as the CUDA cores' kernels)."""
     context, batch = 256, 8

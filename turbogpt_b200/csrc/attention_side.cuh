@@ -122,8 +122,9 @@ template <class T> __device__ void side_forward(const SoftmaxAttentionArgs &a, S
     }
 }
 // Queries == true: dq of a tile of queries, over the keys at or before it; false: dk and dv of a tile of keys, over the
-// queries at or after it.  P = exp(S - lse), dS = P (dO V^T - delta) / sqrt(d).
-template <class T, bool Queries>
+// queries at or after it.  P = exp(S - lse), dS = P (dO V^T - delta) / sqrt(d).  Bounded: lse may come from scores of other bits than these, and an
+// exponential above one from their difference is one.
+template <class T, bool Queries, bool Bounded = false>
 __device__ void side_backward(const SoftmaxAttentionBackwardArgs &a, SideTile *side_tiles, const SideBlock &block) { // five tiles for queries, else six
     SideTile &q = side_tiles[0], &k = side_tiles[1], &v = side_tiles[2], &dy = side_tiles[3], &ds = side_tiles[4], &p = side_tiles[5];
     const int tx = block.tx, ty = block.ty, fixed = block.tile * Side;
@@ -160,7 +161,7 @@ __device__ void side_backward(const SoftmaxAttentionBackwardArgs &a, SideTile *s
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const bool seen = k0 + tx + 16 * j <= query && query < a.context;
-                const float e = seen ? expf(s[i][j] * .125f - lse) : 0.f;
+                const float x = s[i][j] * .125f - lse, e = seen ? expf(Bounded && x > 0.f ? 0.f : x) : 0.f;
                 ds[ty + 16 * i][tx + 16 * j] = seen ? e * (dp[i][j] - delta) * .125f : 0.f;
                 if (!Queries)
                     p[ty + 16 * i][tx + 16 * j] = e;

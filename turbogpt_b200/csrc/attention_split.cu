@@ -69,9 +69,15 @@ __device__ __forceinline__ void load_matrices_transposed(uint32_t address, uint3
 }
 __device__ __forceinline__ uint32_t piece(uint32_t tile, int row, int column16) { return tile + row * 128 + ((column16 ^ (row & 7)) << 4); }
 
-// Six products of parts into the leading parts' sums and the others'.
+// Six products of parts into the leading parts' sums and the others'.  Mirrored: in the order that gives the bits of the transposed product.
+template <bool Mirrored = false>
 __device__ __forceinline__ void multiply_parts(Fragment &lead, Fragment &rest, const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int n) {
-    auto multiply = [&](Fragment &d, int i, int j) { mma_bf16(d[0], d[1], d[2], d[3], a[i], b[j][2 * n], b[j][2 * n + 1]); };
+    auto multiply = [&](Fragment &d, int i, int j) {
+        if (Mirrored)
+            mma_bf16(d[0], d[1], d[2], d[3], a[j], b[i][2 * n], b[i][2 * n + 1]);
+        else
+            mma_bf16(d[0], d[1], d[2], d[3], a[i], b[j][2 * n], b[j][2 * n + 1]);
+    };
     multiply(lead, 0, 0);
     multiply(rest, 0, 1);
     multiply(rest, 1, 0);
@@ -80,7 +86,7 @@ __device__ __forceinline__ void multiply_parts(Fragment &lead, Fragment &rest, c
     multiply(rest, 2, 0);
 }
 // out[16 rows x 32] = A's rows from `row` on times B's rows from `column` on, transposed, over the 64 columns of both.
-__device__ __forceinline__ void multiply_rows(Fragment (&out)[Frags], uint32_t a_tile, int row, uint32_t b_tile, int column, int lane) {
+template <bool Mirrored = false> __device__ __forceinline__ void multiply_rows(Fragment (&out)[Frags], uint32_t a_tile, int row, uint32_t b_tile, int column, int lane) {
 #pragma unroll
     for (int n = 0; n < Frags / 2; ++n) {
         Fragment lead[2][2] = {}, rest[2] = {}; // of either half of K; of both
@@ -92,8 +98,8 @@ __device__ __forceinline__ void multiply_rows(Fragment (&out)[Frags], uint32_t a
                 load_matrices(piece(a_tile + part * PartBytes, row + ((lane >> 3) & 1) * 8 + (lane & 7), k * 2 + (lane >> 4)), a[part]);
                 load_matrices(piece(b_tile + part * PartBytes, column + n * 16 + (lane >> 4) * 8 + (lane & 7), k * 2 + ((lane >> 3) & 1)), b[part]);
             }
-            multiply_parts(lead[k / 2][0], rest[0], a, b, 0);
-            multiply_parts(lead[k / 2][1], rest[1], a, b, 1);
+            multiply_parts<Mirrored>(lead[k / 2][0], rest[0], a, b, 0);
+            multiply_parts<Mirrored>(lead[k / 2][1], rest[1], a, b, 1);
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
@@ -321,7 +327,8 @@ template <bool Queries> __device__ __forceinline__ void split_backward(const Sof
         __syncthreads();
         const int q0 = Queries ? fixed : moving, k0 = Queries ? moving : fixed;
         Fragment s[Frags], dp[Frags]; // rows: the tile's own; columns: the other side's
-        multiply_rows(s, Queries ? q_tile : k_tile, own * Rows, Queries ? k_tile : q_tile, half * Half, lane);
+        // The scores to the bit of the forward pass: where their last place is large, exp(s - lse) is one for the same bits only.
+        multiply_rows<!Queries>(s, Queries ? q_tile : k_tile, own * Rows, Queries ? k_tile : q_tile, half * Half, lane);
         multiply_rows(dp, Queries ? dy_tile : v_tile, own * Rows, Queries ? v_tile : dy_tile, half * Half, lane);
 #pragma unroll
         for (int f = 0; f < Frags; ++f)
@@ -380,7 +387,7 @@ template <bool Queries> __device__ __forceinline__ void split_backward(const Sof
             a.delta[block.statistics + i] = total; // the same value from every block that comes here
     }
     __syncthreads();
-    side_backward<float, Queries>(a, reinterpret_cast<SideTile *>(shared), block);
+    side_backward<float, Queries, true>(a, reinterpret_cast<SideTile *>(shared), block);
 }
 // Blocks of either kind in turn, the longest first.
 __global__ void __launch_bounds__(SideThreads, 1) attention_split_backward_kernel(SoftmaxAttentionBackwardArgs a) {
