@@ -5,7 +5,8 @@
 // accumulator, h m, m h, m m, h l and l h into another.  The tensor core cuts its sums off instead of rounding them (1.2e-8 of the
 // result for every step, 4.4e-6 after 256), so the first accumulator only ever holds 32 of K, two steps, and is added to FP32 registers; the second is
 // 2^-8 of the result and holds 2048 (all of K: a weight gradient's error grew with its tokens, 262144 of them 2.7e-6, now 1.0e-6; CUDA cores 2.9e-6).
-// Against 64 bits (N(0,1) operands, K 16 to 4096) 0.4 to 1.3e-7, where the CUDA cores' sums have 0.7 to 4.1e-7.
+// Against 64 bits (N(0,1) operands, K 64 to 8192) 0.5 to 2.2e-7, where the CUDA cores' sums have 0.8 to 8.1e-7; what is cut off has the result's sign, 1 to 5e-8 of it.
+// BF16 ends at 2^-133: a result all of whose terms have an operand below 2^-112 has fewer bits (2^-116 2e-6, 2^-120 4e-5).
 //
 // What bounds it: 24 products of 128 x BN x 16 a block read their operands from shared memory, 6 (4 + BN / 32) KB each, at 128 B/clk, beside the
 // 48 + 3/8 BN KB that the split operands are written with: 1560 clocks a 128 x 128 x 64 block where the CUDA cores take 8192 for the
